@@ -725,14 +725,17 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
         dsk[2 * c4] = pack2<kInterBF16<BF16>>(u0.x, u0.y);
         dsk[2 * c4 + 1] = pack2<kInterBF16<BF16>>(u1.x, u1.y);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(C::kBarStatsFree + b));  // the row statistics are consumed
       {
         uint4* dst = ds_scratch + out_off;
 #pragma unroll
         for (int pc = 0; pc < 8; ++pc)
           dst[pc * 128] = make_uint4(dsk[4 * pc], dsk[4 * pc + 1], dsk[4 * pc + 2], dsk[4 * pc + 3]);
       }
+      // The row statistics are given back only after the stores of the values computed from them:
+      // an arrive that merely follows the loads in program order can overtake the last of them, and
+      // the copy engine then refills the buffer under it (seen as four wrong q columns of a tile).
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(C::kBarStatsFree + b));
     }
   }
 

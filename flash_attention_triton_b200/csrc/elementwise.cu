@@ -281,20 +281,28 @@ __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
         b[i] = make_uint4(0, 0, 0, 0);
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty(s));  // the pieces are in registers
+    // Products and maxima first: the stage is given back once every piece has been used, not when
+    // its load has been issued (an arrive can overtake a load that is still in flight).
+    float dot[kPasses];
     unsigned amax2 = 0;
-    const int cb = it & 1;
 #pragma unroll
     for (int i = 0; i < kPasses; ++i) {
-      float acc = dot8<BF16>(a[i], b[i]);
-#pragma unroll
-      for (int off = kLanesPerRow / 2; off > 0; off >>= 1)
-        acc += __shfl_xor_sync(0xffffffffu, acc, off);
+      dot[i] = dot8<BF16>(a[i], b[i]);
       amax2 = __vmaxu2(amax2, b[i].x & 0x7fff7fffu);
       amax2 = __vmaxu2(amax2, b[i].y & 0x7fff7fffu);
       amax2 = __vmaxu2(amax2, b[i].z & 0x7fff7fffu);
       amax2 = __vmaxu2(amax2, b[i].w & 0x7fff7fffu);
+      dot[i] += __shfl_xor_sync(0xffffffffu, dot[i], kLanesPerRow / 2);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty(s));
+    const int cb = it & 1;
+#pragma unroll
+    for (int i = 0; i < kPasses; ++i) {
+      float acc = dot[i];
+#pragma unroll
+      for (int off = kLanesPerRow / 4; off > 0; off >>= 1)
+        acc += __shfl_xor_sync(0xffffffffu, acc, off);
       const int r = i * kRowsPerPass + row_in_pass;
       if (sub == 0) {
         const bool valid = r < rows;
