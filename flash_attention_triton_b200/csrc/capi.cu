@@ -249,9 +249,10 @@ int fa2_fwd_strided(const void* q, const void* k, const void* v, void* o, float*
   DeviceState* d = nullptr;
   if (int e = device_state(&d)) return e;
   CUtensorMap tq, tk, tv, to;
+  const int kv_rows = fwd_kv_rows(padded_head_dim(D));
   if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, 128)) return e;
-  if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, 128)) return e;
-  if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, 128)) return e;
+  if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, kv_rows)) return e;
+  if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, kv_rows)) return e;
   if (int e = make_map_of(&to, o, strides, 3, dtype, B, H, N, D, 32)) return e;
   const AttnShape s = make_shape(B, H, N, Nk, D, dtype, scale);
   cudaStream_t st = static_cast<cudaStream_t>(stream);

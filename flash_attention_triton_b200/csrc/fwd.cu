@@ -2,7 +2,7 @@
 //
 // Replaces _forward_kernel (src/flash_attention_triton/_triton_kernels_v2.py:11-189 of the
 // reference).  One CTA owns two adjacent 128-row Q tiles of one (batch, head) and walks the KV
-// tiles 0..diagonal.  Warp roles:
+// tiles 0..diagonal.  (What follows describes head dims above 64; the last paragraph the others.)  Warp roles:
 //   warps 0-3   softmax for Q tile 0   (thread = one score row = one tensor-memory lane)
 //   warps 4-7   softmax for Q tile 1
 //   warp  8     issues S = Q_i K_j^T          } one elected lane each; two warps so that neither
@@ -20,34 +20,58 @@
 // back to back.
 //
 // The online softmax works in the exp2 domain with the scale folded in, and rescales O only
-// when the running maximum has moved by more than 2^8 ("lazy rescale"); masking code runs on
+// when the running maximum has moved by more than kRescaleThreshold ("lazy rescale"); masking code runs on
 // the diagonal tile only.  A fixed fraction of the exponentials is evaluated with a
 // polynomial on the FMA pipe because the MUFU rate (16 / clk / SM) would otherwise bound the
 // kernel: 2 x 128 x 128 exponentials per KV step cost as many cycles as the four MMAs.
+//
+// Head dims up to 64: the MMAs of a tile are short (512 cycles or less per 128 x 128 scores) and the
+// softmax instruction stream is what takes the time; with two softmax warps per scheduler it issues
+// in half of the cycles only, the rest is latency of dependent instructions.  So the KV tiles are
+// 64 rows there: a thread holds 64 instead of 128 scores, 96 registers do instead of 208, 256
+// columns of tensor memory instead of 512, and TWO CTAs run on an SM, four softmax warps per
+// scheduler.  The exponentials then all go to the MUFU, which has time (the polynomial costs five
+// times the issue slots).  Measured against 128-row tiles and one CTA, microseconds:
+// [4,16,2048,64] 70.5 -> 61.6, [8,12,4095,32] 296 -> 269, [2,16,8192,64] 388 -> 382.
 #include "common.cuh"
 #include "mma_issue.cuh"
 #include "ptx.cuh"
 
 #ifndef FA2_FWD_POLY_PAIRS_PER_8
-#define FA2_FWD_POLY_PAIRS_PER_8 3  // of every 8 column pairs, this many use ex2_poly2
+#define FA2_FWD_POLY_PAIRS_PER_8 3  // of every 8 column pairs, this many use ex2_poly2 (D > 64)
 #endif
 
 namespace fa2 {
 namespace {
 
 constexpr int kFwdThreads = 384;
-constexpr float kRescaleThreshold = 8.0f;  // log2 units
 constexpr float kLn2 = 0.6931471805599453f;
 
 template <int D>
 struct FwdCfg {
   using T = Tile<D>;
+  static constexpr int kW = fwd_kv_rows(D);  // rows of a KV tile = columns of a score tile
+  static constexpr int kPolyShare = kW == 64 ? 0 : FA2_FWD_POLY_PAIRS_PER_8;
+  static constexpr int kCtasPerSm = kW == 64 ? 2 : 1;
+  // O is rescaled when the running maximum has moved by more than this (log2 units).  A row's
+  // largest P is exactly 1, without rounding error, when its maximum is fresh: 64-row tiles, whose
+  // maxima settle later, use a lower threshold and none after their first tile, which keeps the
+  // error of O below that of 128-row tiles (peaked softmax, fp16: 1.78e-4 against 1.84e-4).
+  static constexpr float kRescaleThreshold = kW == 64 ? 4.0f : 8.0f;
+  static constexpr int kKvBytes = T::kTileBytes / 128 * kW;
+  // registers of a producer / softmax thread; the launch gives every thread
+  // kLaunchRegs (the launch bounds' limit, rounded down to a multiple of 8)
+  static constexpr int kLaunchRegs = 65536 / (kFwdThreads * kCtasPerSm) / 8 * 8;
+  static constexpr int kProducerRegs = kW == 64 ? 48 : 72;
+  static constexpr int kSoftmaxRegs = kW == 64 ? 96 : 208;
+  static_assert(128 * kProducerRegs + 256 * kSoftmaxRegs <= kFwdThreads * kLaunchRegs,
+                "setmaxnreg.inc waits for registers that setmaxnreg.dec has released");
   static constexpr int kKStages = D == 128 ? 3 : 4;
   static constexpr int kVStages = D == 128 ? 2 : 4;
   static constexpr int kOffQ = 0;
   static constexpr int kOffK = kOffQ + 2 * T::kTileBytes;
-  static constexpr int kOffV = kOffK + kKStages * T::kTileBytes;
-  static constexpr int kOffBar = kOffV + kVStages * T::kTileBytes;
+  static constexpr int kOffV = kOffK + kKStages * kKvBytes;
+  static constexpr int kOffBar = kOffV + kVStages * kKvBytes;
   // barrier slots
   static constexpr int kBarQFull = 0;
   static constexpr int kBarKFull = 1;
@@ -62,9 +86,11 @@ struct FwdCfg {
   static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;  // + tmem slot, abort, work slot
   // tensor-memory columns
   static constexpr int kColS = 0;
-  static constexpr int kColP = 128;  // P0 at 128, P1 at 192 (64 columns of 16-bit pairs each)
-  static constexpr int kColO = 256;  // O0 at 256, O1 at 256 + D
-  static constexpr int kTmemCols = 512;
+  static constexpr int kColP = kW;      // P0, then P1 (kW / 2 columns of 16-bit pairs each)
+  static constexpr int kColO = 2 * kW;  // O0, then O1 (D columns each)
+  static constexpr int kTmemCols = 512 / kCtasPerSm;
+  static_assert(kColO + 2 * D <= kTmemCols, "tensor memory of one CTA");
+  static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "shared memory of one SM");
 };
 
 enum FwdSite {
@@ -82,7 +108,7 @@ enum FwdSite {
 };
 
 template <int D, bool BF16>
-__global__ void __launch_bounds__(kFwdThreads, 1)
+__global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtasPerSm)
     fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap to,
                float* __restrict__ lse, int N, int Nk, int num_bh, int num_heads, int group,
@@ -96,6 +122,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   constexpr int HALVES = WIDE ? 2 : 1;  // staged tiles per 128 rows
   using C = FwdCfg<DT>;
   using T = Tile<DT>;
+  constexpr int W = C::kW;  // rows of a KV tile
   extern __shared__ __align__(1024) uint8_t smem[];
 
   // Role index: hardware warps 0-3 take roles 8-11 (MMA, TMA, idle, idle) and hardware warps
@@ -116,7 +143,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   auto bar = [&](int i) { return smem_base + C::kOffBar + 8u * i; };
 
   const int ntiles = (N + 127) >> 7;
-  const int nktiles = (Nk + 127) >> 7;
+  const int nktiles = (Nk + W - 1) / W;  // KV tiles of W rows
   const int npairs = WIDE ? ntiles : (ntiles + 1) >> 1;  // work items per (batch, head)
   const int total_items = npairs * num_bh;
 
@@ -131,7 +158,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
 
-  // One CTA per SM; work items (one Q-tile pair of one (batch, head)) are fetched from a
+  // One or two CTAs per SM; work items (one Q-tile pair of one (batch, head)) are fetched from a
   // global counter in head-major, heavy-pair-first order, like a hardware block scheduler
   // would hand them out, but without the launch gap and with tensor memory kept allocated.
   // Between items all roles meet at a barrier and the mbarriers are re-initialised, so each
@@ -173,13 +200,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     const int pair = npairs - 1 - ht.rank;  // the last pair of Q tiles meets the most KV tiles
     const int qt0 = WIDE ? pair : 2 * pair, qt1 = qt0 + 1;
     const bool has1 = !WIDE && qt1 < ntiles;
-    // KV tiles of Q tile i: 0 .. min(i, last KV tile)  (N = query rows, Nk <= N = key rows)
-    const int n0 = qt0 + 1 < nktiles ? qt0 + 1 : nktiles;
-    const int n1 = has1 ? (qt1 + 1 < nktiles ? qt1 + 1 : nktiles) : 0;
+    // KV tiles of Q tile i: those up to its diagonal, or to the last key  (N = query rows,
+    // Nk <= N = key rows)
+    constexpr int kPerQ = 128 / W;
+    const int n0 = min((qt0 + 1) * kPerQ, nktiles);
+    const int n1 = has1 ? min((qt1 + 1) * kPerQ, nktiles) : 0;
     const int nkv = n1 > n0 ? n1 : n0;
 
   if (warp >= 8) {
-    reg_dec<72>();  // whole warpgroup (warps 8-11) gives registers to the softmax groups
+    reg_dec<C::kProducerRegs>();  // whole warpgroup (warps 8-11) gives registers to the softmax groups
     if (warp == 9) {
       // ---------------------------------------------------------------- TMA producer
       // (whole warp, converged; only the elected lane arms barriers and issues copies)
@@ -204,11 +233,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
           const int ks = t % C::kKStages, kph = (t / C::kKStages) & 1;
           if (!mbar_wait_warp(bar(C::kBarKEmpty + ks), kph ^ 1, w, kSiteLoadK)) break;
           if (elected) {
-            mbar_arrive_expect_tx(bar(C::kBarKFull + ks), T::kTileBytes);
+            mbar_arrive_expect_tx(bar(C::kBarKFull + ks), C::kKvBytes);
 #pragma unroll
             for (int ch = 0; ch < T::kChunks; ++ch)
-              tma_load_4d(smem_base + C::kOffK + ks * T::kTileBytes + ch * T::kChunkTileBytes, &tk,
-                          (t % HALVES) * 128 + ch * T::kChunkElems, (t / HALVES) * 128, hc,
+              tma_load_4d(smem_base + C::kOffK + ks * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tk,
+                          (t % HALVES) * 128 + ch * T::kChunkElems, (t / HALVES) * W, hc,
                           bar(C::kBarKFull + ks));
           }
         }
@@ -217,11 +246,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
           const int vs = tv_ % C::kVStages, vph = (tv_ / C::kVStages) & 1;
           if (!mbar_wait_warp(bar(C::kBarVEmpty + vs), vph ^ 1, w, kSiteLoadV)) break;
           if (elected) {
-            mbar_arrive_expect_tx(bar(C::kBarVFull + vs), T::kTileBytes);
+            mbar_arrive_expect_tx(bar(C::kBarVFull + vs), C::kKvBytes);
 #pragma unroll
             for (int ch = 0; ch < T::kChunks; ++ch)
-              tma_load_4d(smem_base + C::kOffV + vs * T::kTileBytes + ch * T::kChunkTileBytes, &tv,
-                          (tv_ % HALVES) * 128 + ch * T::kChunkElems, (tv_ / HALVES) * 128, hc,
+              tma_load_4d(smem_base + C::kOffV + vs * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tv,
+                          (tv_ % HALVES) * 128 + ch * T::kChunkElems, (tv_ / HALVES) * W, hc,
                           bar(C::kBarVFull + vs));
           }
         }
@@ -259,17 +288,17 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             // S = Q_lo K_lo^T + Q_hi K_hi^T: the Q slots hold the halves, K arrives half by half
             for (int half = 0; ok && half < 2; ++half) {
               if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
-              issue_rows_x_rows<DT, BF16>(elected, tmem_base + C::kColS,
+              issue_rows_x_rows<DT, BF16, W>(elected, tmem_base + C::kColS,
                                           smem_base + C::kOffQ + half * T::kTileBytes,
-                                          smem_base + C::kOffK + ks * T::kTileBytes, half);
+                                          smem_base + C::kOffK + ks * C::kKvBytes, half);
               if (elected) mma_commit(bar(C::kBarKEmpty + ks));
               next_k();
             }
             if (!ok) break;
           } else {
-            issue_rows_x_rows<DT, BF16>(elected, tmem_base + C::kColS,
+            issue_rows_x_rows<DT, BF16, W>(elected, tmem_base + C::kColS,
                                         smem_base + C::kOffQ + i * T::kTileBytes,
-                                        smem_base + C::kOffK + ks * T::kTileBytes);
+                                        smem_base + C::kOffK + ks * C::kKvBytes);
           }
           if (elected) mma_commit(bar(C::kBarSFull + i));
           prev_i = i;
@@ -305,17 +334,17 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             // O_lo += P V_lo, O_hi += P V_hi: the O0 / O1 columns hold the two halves of O
             for (int half = 0; ok && half < 2; ++half) {
               if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
-              issue_tmem_x_tile<DT, BF16>(elected, tmem_base + C::kColO + half * DT,
-                                          tmem_base + C::kColP, 32,
-                                          smem_base + C::kOffV + vs * T::kTileBytes, j > 0);
+              issue_tmem_x_tile<DT, BF16, W>(elected, tmem_base + C::kColO + half * DT,
+                                          tmem_base + C::kColP, W / 4,
+                                          smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
               if (elected) mma_commit(bar(C::kBarVEmpty + vs));
               next_v();
             }
             if (!ok) break;
           } else {
-            issue_tmem_x_tile<DT, BF16>(elected, tmem_base + C::kColO + i * DT,
-                                        tmem_base + C::kColP + i * 64, 32,
-                                        smem_base + C::kOffV + vs * T::kTileBytes, j > 0);
+            issue_tmem_x_tile<DT, BF16, W>(elected, tmem_base + C::kColO + i * DT,
+                                        tmem_base + C::kColP + i * (W / 2), W / 4,
+                                        smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
           }
           if (elected) mma_commit(bar(C::kBarPvDone + i));
         }
@@ -329,47 +358,46 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ softmax groups
-    reg_inc<208>();
+    reg_inc<C::kSoftmaxRegs>();
     const int wg = warp >> 2;
     const int qt = wg == 0 ? qt0 : qt1;
     const int nj = wg == 0 ? n0 : n1;
     const int r = (warp & 3) * 32 + lane;  // row inside the Q tile = tensor-memory lane
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tS = tmem_base + lane_base + C::kColS;
-    const uint32_t tP = tmem_base + lane_base + C::kColP + wg * 64;
+    const uint32_t tP = tmem_base + lane_base + C::kColP + wg * (W / 2);
     const uint32_t tO = tmem_base + lane_base + C::kColO + wg * DT;  // wide: 256 columns, wg 0 only
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < nj; ++j) {
       if (!(ok = mbar_wait_warp(bar(C::kBarSFull + wg), j & 1, w, kSiteSoftS))) break;
       tc_fence_after();
-      uint32_t sr[128];
-      tmem_ld_x32(tS + 0, sr + 0);
-      tmem_ld_x32(tS + 32, sr + 32);
-      tmem_ld_x32(tS + 64, sr + 64);
-      tmem_ld_x32(tS + 96, sr + 96);
+      uint32_t sr[W];
+#pragma unroll
+      for (int c = 0; c < W; c += 32) tmem_ld_x32(tS + c, sr + c);
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(C::kBarSFree + wg));  // S may be overwritten now
       float* s = reinterpret_cast<float*>(sr);
-      if (j == qt || j * 128 + 128 > Nk) {
-        // diagonal tile: keep col <= row; last KV tile: drop the columns beyond the last key
-        int last = j == qt ? r : 127;
-        last = last < Nk - 1 - j * 128 ? last : Nk - 1 - j * 128;
+      if (j * W + W > qt * 128 || j * W + W > Nk) {
+        // diagonal tiles: keep col <= row; last KV tile: drop the columns beyond the last key
+        const int last = min(qt * 128 + r, Nk - 1) - j * W;
 #pragma unroll
-        for (int c = 0; c < 128; ++c) s[c] = (c <= last) ? s[c] : -INFINITY;
+        for (int c = 0; c < W; ++c) s[c] = (c <= last) ? s[c] : -INFINITY;
       }
-      float mx[4];
+      float mx[W / 32];
 #pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) {
+      for (int q4 = 0; q4 < W / 32; ++q4) {
         mx[q4] = max3(s[32 * q4], s[32 * q4 + 1], s[32 * q4 + 2]);
 #pragma unroll
         for (int c = 3; c < 31; c += 2) mx[q4] = max3(mx[q4], s[32 * q4 + c], s[32 * q4 + c + 1]);
         mx[q4] = fmaxf(mx[q4], s[32 * q4 + 31]);
       }
-      const float m_new = fmaxf(max3(m_run, mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      const bool need = (m_new - m_run) * scale_log2 > kRescaleThreshold;
+      float m_new = max3(m_run, mx[0], mx[1]);
+      if constexpr (W == 128) m_new = fmaxf(m_new, fmaxf(mx[2], mx[3]));
+      const float threshold = W == 128 ? C::kRescaleThreshold : (j == 1 ? 0.f : C::kRescaleThreshold);
+      const bool need = (m_new - m_run) * scale_log2 > threshold;
       bool pv_waited = false;
       if (__any_sync(0xffffffffu, need)) {
         const float alpha = ex2((m_run - m_new) * scale_log2);
@@ -380,14 +408,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
           if (!(ok = mbar_wait_warp(bar(C::kBarPvDone + wg), (j - 1) & 1, w, kSiteSoftPv))) break;
           tc_fence_after();
           pv_waited = true;
+          constexpr int kStep = W == 64 ? 16 : 32;  // the score row stays in registers meanwhile
 #pragma unroll
-          for (int c0 = 0; c0 < D; c0 += 32) {
-            uint32_t orr[32];
-            tmem_ld_x32(tO + c0, orr);
+          for (int c0 = 0; c0 < D; c0 += kStep) {
+            uint32_t orr[kStep];
+            if constexpr (kStep == 16) tmem_ld_x16(tO + c0, orr); else tmem_ld_x32(tO + c0, orr);
             tmem_wait_ld();
 #pragma unroll
-            for (int c = 0; c < 32; ++c) orr[c] = __float_as_uint(__uint_as_float(orr[c]) * alpha);
-            tmem_st_x32(tO + c0, orr);
+            for (int c = 0; c < kStep; ++c) orr[c] = __float_as_uint(__uint_as_float(orr[c]) * alpha);
+            if constexpr (kStep == 16) tmem_st_x16(tO + c0, orr); else tmem_st_x32(tO + c0, orr);
           }
         }
       }
@@ -395,11 +424,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
       const float2 sc2 = make_float2(scale_log2, scale_log2);
       const float2 nm2 = make_float2(-m_run * scale_log2, -m_run * scale_log2);
       float2 acc[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-      uint32_t pk[64];
+      uint32_t pk[W / 2];
 #pragma unroll
-      for (int c = 0; c < 64; ++c) {
+      for (int c = 0; c < W / 2; ++c) {
         float2 t = __ffma2_rn(make_float2(s[2 * c], s[2 * c + 1]), sc2, nm2);
-        if ((c & 7) < FA2_FWD_POLY_PAIRS_PER_8) {
+        if ((c & 7) < C::kPolyShare) {
           t = ex2_poly2(t);
         } else {
           t.x = ex2(t.x);
@@ -412,8 +441,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         // P_i still feeds O_i += P_i(j-1) V_(j-1) until that product has completed
         if (!(ok = mbar_wait_warp(bar(C::kBarPvDone + wg), (j - 1) & 1, w, kSiteSoftPv))) break;
       }
-      tmem_st_x32(tP, pk);
-      tmem_st_x32(tP + 32, pk + 32);
+#pragma unroll
+      for (int c = 0; c < W / 2; c += 32) tmem_st_x32(tP + c, pk + c);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -492,7 +521,8 @@ cudaError_t launch_fwd_t(const AttnShape& s, const CUtensorMap& tq, const CUtens
   const int ntiles = (s.N + 127) / 128;
   const int npairs = D == 256 ? ntiles : (ntiles + 1) / 2;
   const long long items = static_cast<long long>(npairs) * s.B * s.H;
-  const unsigned grid = static_cast<unsigned>(items < ctx.num_sms ? items : ctx.num_sms);
+  const long long slots = static_cast<long long>(ctx.num_sms) * C::kCtasPerSm;
+  const unsigned grid = static_cast<unsigned>(items < slots ? items : slots);
   const float scale_log2 = s.scale * 1.4426950408889634f;
   kern<<<grid, kFwdThreads, C::kSmemBytes, stream>>>(tq, tk, tv, to, lse, s.N, s.Nk, s.B * s.H, s.H,
                                                      heads_per_group(s), scale_log2, ctx.status,

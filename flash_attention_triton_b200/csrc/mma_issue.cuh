@@ -29,40 +29,41 @@ __device__ __forceinline__ uint32_t desc_lo_word(uint32_t saddr, uint32_t lbo_by
   return ((saddr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
 }
 
-// acc[128, 128] (+)= A[128 rows, D] * B[128 rows, D]^T.  Both tiles are K-major (row = M / N
-// index, the contiguous dimension is the reduction index d), as TMA stages a [128, D] tile.
-template <int D, bool BF16>
+// acc[128, W] (+)= A[128 rows, D] * B[W rows, D]^T.  Both tiles are K-major (row = M / N
+// index, the contiguous dimension is the reduction index d), as TMA stages a [rows, D] tile.
+template <int D, bool BF16, int W = 128>
 __device__ __forceinline__ void issue_rows_x_rows(uint32_t elected, uint32_t d_tmem,
                                                   uint32_t a_addr, uint32_t b_addr,
                                                   uint32_t accumulate = 0u) {
   using T = Tile<D>;
-  constexpr uint32_t idesc = make_idesc(128, 128, BF16, false, false);
+  constexpr uint32_t idesc = make_idesc(128, W, BF16, false, false);
   constexpr uint32_t hi = desc_hi_word(T::kAtomBytes, T::kSwizzleMode);
   const uint32_t a_lo = desc_lo_word(a_addr, 16), b_lo = desc_lo_word(b_addr, 16);
 #pragma unroll
   for (int k = 0; k < D / 16; ++k) {
     constexpr int kpc = T::kKStepsPerChunk;
-    const uint32_t off16 = ((k / kpc) * T::kChunkTileBytes + (k % kpc) * 32) >> 4;
+    const uint32_t a16 = ((k / kpc) * T::kChunkTileBytes + (k % kpc) * 32) >> 4;
+    const uint32_t b16 = ((k / kpc) * (T::kChunkTileBytes / 128 * W) + (k % kpc) * 32) >> 4;
     if (elected)
-      mma_ss(d_tmem, desc_from_words(a_lo + off16, hi), desc_from_words(b_lo + off16, hi), idesc,
+      mma_ss(d_tmem, desc_from_words(a_lo + a16, hi), desc_from_words(b_lo + b16, hi), idesc,
              k > 0 ? 1u : accumulate);
   }
 }
 
-// acc[128, D] (+)= A[128, 128] * B[128 rows, D].  A is 16-bit in tensor memory, two values per
-// column: reduction indices 0..63 at columns a_tmem .. +31 and 64..127 at a_tmem + a_col_half ..
-// (+31).  B is a staged [128, D] tile used MN-major (row = reduction index, d contiguous).
-template <int D, bool BF16>
+// acc[128, D] (+)= A[128, W] * B[W rows, D].  A is 16-bit in tensor memory, two values per
+// column: the first W/2 reduction indices at columns a_tmem .., the others at a_tmem + a_col_half ..
+// (W/4 columns each).  B is a staged [W, D] tile used MN-major (row = reduction index, d contiguous).
+template <int D, bool BF16, int W = 128>
 __device__ __forceinline__ void issue_tmem_x_tile(uint32_t elected, uint32_t d_tmem,
                                                   uint32_t a_tmem, uint32_t a_col_half,
                                                   uint32_t b_addr, uint32_t accumulate) {
   using T = Tile<D>;
   constexpr uint32_t idesc = make_idesc_ab(128, D, kInterBF16<BF16>, BF16, false, true);
   constexpr uint32_t hi = desc_hi_word(T::kAtomBytes, T::kSwizzleMode);
-  const uint32_t b_lo = desc_lo_word(b_addr, T::kChunkTileBytes);
+  const uint32_t b_lo = desc_lo_word(b_addr, T::kChunkTileBytes / 128 * W);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const uint32_t a = a_tmem + (k < 4 ? k * 8 : a_col_half + (k - 4) * 8);
+  for (int k = 0; k < W / 16; ++k) {
+    const uint32_t a = a_tmem + (k < W / 32 ? k * 8 : a_col_half + (k - W / 32) * 8);
     if (elected)
       mma_ts(d_tmem, a, desc_from_words(b_lo + ((k * 2 * T::kAtomBytes) >> 4), hi), idesc,
              k > 0 ? 1u : accumulate);

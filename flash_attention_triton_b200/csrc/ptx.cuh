@@ -77,11 +77,33 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const W
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, w, site);
 }
-// Warp-uniform variant for warps that go on to execute .sync.aligned instructions.
+// Warp-uniform variant for converged warps: the vote makes the outcome, and with it every branch
+// around the wait, uniform, so no lane has to be brought back together afterwards.  (A lane that has
+// already seen the phase complete sees it again when the others retry: the barrier cannot
+// complete its next phase before this warp has gone on.)
+__device__ __forceinline__ bool mbar_wait_warp_slow(uint32_t bar, uint32_t parity, const WaitCtx& w,
+                                                 int site) {
+  const long long t0 = clock64();
+  uint32_t it = 0;
+  for (;;) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((++it & 63u) == 0) {
+      const bool late = clock64() - t0 > kWaitLimitCycles;
+      if (__any_sync(0xffffffffu, late)) {
+        if ((threadIdx.x & 31u) == 0) {
+          *w.abort_flag = 1;
+          atomicCAS(w.status, 0, 0x10000 | site);
+        }
+        return false;
+      }
+      if (__any_sync(0xffffffffu, *w.abort_flag != 0)) return false;
+    }
+  }
+}
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const WaitCtx& w,
                                                int site) {
-  const bool ok = mbar_wait(bar, parity, w, site);
-  return __all_sync(0xffffffffu, ok);
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return mbar_wait_warp_slow(bar, parity, w, site);
 }
 
 // ----------------------------------------------------------------------------------------
