@@ -30,7 +30,7 @@ namespace {
 // dK / dV (+ fused dQ) kernel: one CTA per KV tile of one (batch, head); see dkdv_roles.
 // =========================================================================================
 template <int D, bool BF16, int MODE>
-__global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, 1)
+__global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::kCtasPerSm)
     bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                     const __grid_constant__ CUtensorMap tdk,
@@ -101,19 +101,32 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, 1)
 // buffer they just read, and the MMA warp then issues dQ += dS(j) K_j followed by S(j+2) into
 // the same buffer.  S(j+1) is already in the other buffer, so the tensor pipe and the compute
 // warps overlap instead of alternating.
+// Head dims up to 64 walk the KV tiles in steps of 64 rows with two CTAs per SM, for the reasons given
+// at DkdvCfg; the polynomial's share of the exponentials is that of the dK/dV kernel.
 template <int D>
 struct DqCfg {
   using T = Tile<D>;
-  static constexpr int kKStages = 3;  // K_j is needed by S(j) and, later, by dQ(j)
-  static constexpr int kVStages = 2;
-  static constexpr int kThreads = 384;
-  static constexpr int kMmaWarp = 8;
-  static constexpr int kLoadWarp = 9;
+  static constexpr int kW = bwd_step_rows(D);  // rows of a KV tile = score columns of a step
+  static constexpr int kCtasPerSm = kW == 64 ? 2 : 1;
+  static constexpr int kGroups = 2;           // compute groups of four warps
+  static constexpr int kCols = kW / kGroups;  // score columns of a compute thread
+  static constexpr int kKvBytes = T::kTileBytes / 128 * kW;
+  static constexpr int kKStages = kW == 64 ? 4 : 3;  // K_j is needed by S(j) and, later, by dQ(j)
+  static constexpr int kVStages = kW == 64 ? 3 : 2;
+  static constexpr int kMmaWarp = 4 * kGroups;
+  static constexpr int kThreads = 32 * (kMmaWarp + 4);
+  static constexpr int kLoadWarp = kMmaWarp + 1;
+  // registers per thread of the producer / compute warps; the launch gives every thread kLaunchRegs
+  static constexpr int kLaunchRegs = 65536 / (kThreads * kCtasPerSm) / 8 * 8;
+  static constexpr int kProducerRegs = kW == 64 ? 48 : 72;
+  static constexpr int kComputeRegs = kW == 64 ? 96 : 208;
+  static_assert(128 * kProducerRegs + 128 * kGroups * kComputeRegs <= kThreads * kLaunchRegs,
+                "setmaxnreg.inc waits for registers that setmaxnreg.dec has released");
   static constexpr int kOffQ = 0;
   static constexpr int kOffDO = kOffQ + T::kTileBytes;
   static constexpr int kOffK = kOffDO + T::kTileBytes;
-  static constexpr int kOffV = kOffK + kKStages * T::kTileBytes;
-  static constexpr int kOffStats = kOffV + kVStages * T::kTileBytes;  // [256] fp32
+  static constexpr int kOffV = kOffK + kKStages * kKvBytes;
+  static constexpr int kOffStats = kOffV + kVStages * kKvBytes;  // [256] fp32
   static constexpr int kOffBar = kOffStats + 1024;
   static constexpr int kBarQ = 0;  // Q, dO and rowstats
   static constexpr int kBarKFull = 1;
@@ -122,20 +135,22 @@ struct DqCfg {
   static constexpr int kBarVEmpty = kBarVFull + kVStages;
   static constexpr int kBarSFull = kBarVEmpty + kVStages;  // 2 (one per score buffer)
   static constexpr int kBarDpFull = kBarSFull + 2;
-  static constexpr int kBarDpConsumed = kBarDpFull + 1;  // 8 arrivals (one per compute warp)
-  static constexpr int kBarDsReady = kBarDpConsumed + 1;  // 8 arrivals
+  static constexpr int kBarDpConsumed = kBarDpFull + 1;  // one arrival per compute warp
+  static constexpr int kBarDsReady = kBarDpConsumed + 1;  // one arrival per compute warp
   static constexpr int kBarDqDone = kBarDsReady + 1;      // 2: dQ += dS(j) K_j completed, by j%2
   static constexpr int kBarDone = kBarDqDone + 2;
   static constexpr int kNumBars = kBarDone + 1;
   static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;
-  static constexpr int kColS = 0;     // score buffers at 0 and 128; dS (16-bit) overwrites them
-  static constexpr int kColDp = 256;
-  static constexpr int kColDQ = 384;
-  static constexpr int kTmemCols = 512;
+  static constexpr int kColS = 0;     // score buffers at 0 and kW; dS (16-bit) overwrites them
+  static constexpr int kColDp = 2 * kW;
+  static constexpr int kColDQ = 3 * kW;
+  static constexpr int kTmemCols = 512 / kCtasPerSm;
+  static_assert(kColDQ + D <= kTmemCols, "tensor memory of one CTA");
+  static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "shared memory of one SM");
 };
 
 template <int D, bool BF16>
-__global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
+__global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
     bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                   const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                   const __grid_constant__ CUtensorMap tdq, const float* __restrict__ rowstats,
@@ -143,6 +158,9 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
                   int group, float scale, float scale_log2, int* status) {
   using C = DqCfg<D>;
   using T = Tile<D>;
+  constexpr int W = C::kW;  // rows of a KV tile
+  constexpr int kCols = C::kCols, kPairs = kCols / 2;
+  constexpr uint32_t kHalf = kCols;  // columns between the two groups' halves of dS
   extern __shared__ __align__(1024) uint8_t smem[];
   // Role index: producer / MMA group on hardware warps 0-3, compute groups on 4-11.
   const int warp = ((threadIdx.x >> 5) + C::kMmaWarp) % (C::kThreads / 32), lane = threadIdx.x & 31;
@@ -161,8 +179,8 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
   const int qt = ntiles - 1 - ht.rank;  // the last Q tile meets the most KV tiles
   const int bh = ht.bh;
   const HeadCoord hc{bh % num_heads, bh / num_heads};
-  const int nktiles = (Nk + 127) >> 7;               // N = query rows, Nk <= N = key rows
-  const int nkv = qt + 1 < nktiles ? qt + 1 : nktiles;  // KV tiles 0 .. min(qt, last)
+  // KV tiles up to the diagonal, or to the last key (N = query rows, Nk <= N = key rows)
+  const int nkv = min((qt + 1) * (128 / W), (Nk + W - 1) / W);
 
   if (threadIdx.x == 0) {
     mbar_init(bar(C::kBarQ), 1);
@@ -177,8 +195,8 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
     mbar_init(bar(C::kBarSFull + 0), 1);
     mbar_init(bar(C::kBarSFull + 1), 1);
     mbar_init(bar(C::kBarDpFull), 1);
-    mbar_init(bar(C::kBarDpConsumed), 8);
-    mbar_init(bar(C::kBarDsReady), 8);
+    mbar_init(bar(C::kBarDpConsumed), 4 * C::kGroups);
+    mbar_init(bar(C::kBarDsReady), 4 * C::kGroups);
     mbar_init(bar(C::kBarDqDone + 0), 1);
     mbar_init(bar(C::kBarDqDone + 1), 1);
     mbar_init(bar(C::kBarDone), 1);
@@ -197,7 +215,7 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
   const WaitCtx w{abort_flag, status};
 
   if (warp >= C::kMmaWarp) {
-    reg_dec<72>();
+    reg_dec<C::kProducerRegs>();
     if (warp == C::kLoadWarp) {
       // TMA producer: whole warp, converged; the elected lane arms barriers and issues copies.
       const uint32_t elected = elect_one();
@@ -220,20 +238,20 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
         const int ks = j % C::kKStages, kph = (j / C::kKStages) & 1;
         if (!mbar_wait_warp(bar(C::kBarKEmpty + ks), kph ^ 1, w, kBSiteLoadQ)) break;
         if (elected) {
-          mbar_arrive_expect_tx(bar(C::kBarKFull + ks), T::kTileBytes);
+          mbar_arrive_expect_tx(bar(C::kBarKFull + ks), C::kKvBytes);
 #pragma unroll
           for (int ch = 0; ch < T::kChunks; ++ch)
-            tma_load_4d(smem_base + C::kOffK + ks * T::kTileBytes + ch * T::kChunkTileBytes, &tk,
-                        ch * T::kChunkElems, j * 128, hc, bar(C::kBarKFull + ks));
+            tma_load_4d(smem_base + C::kOffK + ks * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tk,
+                        ch * T::kChunkElems, j * W, hc, bar(C::kBarKFull + ks));
         }
         const int vs = j % C::kVStages, vph = (j / C::kVStages) & 1;
         if (!mbar_wait_warp(bar(C::kBarVEmpty + vs), vph ^ 1, w, kBSiteLoadDO)) break;
         if (elected) {
-          mbar_arrive_expect_tx(bar(C::kBarVFull + vs), T::kTileBytes);
+          mbar_arrive_expect_tx(bar(C::kBarVFull + vs), C::kKvBytes);
 #pragma unroll
           for (int ch = 0; ch < T::kChunks; ++ch)
-            tma_load_4d(smem_base + C::kOffV + vs * T::kTileBytes + ch * T::kChunkTileBytes, &tv,
-                        ch * T::kChunkElems, j * 128, hc, bar(C::kBarVFull + vs));
+            tma_load_4d(smem_base + C::kOffV + vs * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tv,
+                        ch * T::kChunkElems, j * W, hc, bar(C::kBarVFull + vs));
         }
       }
     } else if (warp == C::kMmaWarp) {
@@ -257,8 +275,8 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
           tc_fence_after();
         }
         if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kBSiteMmaDO))) break;
-        issue_rows_x_rows<D, BF16>(elected, tmem_base + C::kColDp, doa,
-                                   smem_base + C::kOffV + vs * T::kTileBytes);
+        issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColDp, doa,
+                                   smem_base + C::kOffV + vs * C::kKvBytes);
         commit(C::kBarDpFull);
         commit(C::kBarVEmpty + vs);  // V is free once dP has read it
         if (++vs == C::kVStages) {
@@ -283,8 +301,8 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
           tc_fence_after();
         }
         if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kBSiteMmaKV))) break;
-        issue_rows_x_rows<D, BF16>(elected, tmem_base + C::kColS + (j & 1) * 128, qa,
-                                   smem_base + C::kOffK + ks * T::kTileBytes);
+        issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColS + (j & 1) * W, qa,
+                                   smem_base + C::kOffK + ks * C::kKvBytes);
         commit(C::kBarSFull + (j & 1));
         commit(C::kBarKEmpty + ks);
         if (++ks == C::kKStages) {
@@ -305,8 +323,8 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
         if (!(ok = mbar_wait(bar(C::kBarDsReady), j & 1, w, kBSiteMmaDs))) break;
         tc_fence_after();
         // A = 16-bit dS over score buffer j%2, B = K_j as MN-major tile
-        issue_tmem_x_tile<D, BF16>(elected, tmem_base + C::kColDQ, tmem_base + C::kColS + (j & 1) * 128,
-                                   64, smem_base + C::kOffK + ks * T::kTileBytes, j > 0);
+        issue_tmem_x_tile<D, BF16, W>(elected, tmem_base + C::kColDQ, tmem_base + C::kColS + (j & 1) * W,
+                                   kHalf, smem_base + C::kOffK + ks * C::kKvBytes, j > 0);
         commit(C::kBarDqDone + (j & 1));
         commit(C::kBarKEmpty + ks);
         if (++ks == C::kKStages) {
@@ -318,12 +336,12 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
     }
     __syncwarp();
   } else {
-    reg_inc<208>();
+    reg_inc<C::kComputeRegs>();
     const int wg = warp >> 2;
     const int w4 = warp & 3;
     const int r = w4 * 32 + lane;  // q row in the tile = tensor-memory lane
     const uint32_t lane_base = static_cast<uint32_t>(w4 * 32) << 16;
-    const uint32_t tDp = tmem_base + lane_base + C::kColDp + wg * 64;
+    const uint32_t tDp = tmem_base + lane_base + C::kColDp + wg * kCols;
     const float2 sc2 = make_float2(scale_log2, scale_log2);
     // dS is formed as dS * 2^k in fp16 and dQ multiplied by 2^-k at the end (head_dscale)
     float inv_dscale;
@@ -338,50 +356,50 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, 1)
       ndlt2 = make_float2(stats[128 + r], stats[128 + r]);  // -delta of this row
     }
     for (int j = 0; ok && j < nkv; ++j) {
-      const uint32_t tS = tmem_base + lane_base + C::kColS + (j & 1) * 128 + wg * 64;
+      const uint32_t tS = tmem_base + lane_base + C::kColS + (j & 1) * W + wg * kCols;
       if (!(ok = mbar_wait_warp(bar(C::kBarSFull + (j & 1)), (j >> 1) & 1, w, kBSiteCmpSt))) break;
       tc_fence_after();
-      float2 p[32];
+      float2 p[kPairs];
       {
-        uint32_t sr[64];
-        tmem_ld_x32(tS, sr);
-        tmem_ld_x32(tS + 32, sr + 32);
+        uint32_t sr[kCols];
+#pragma unroll
+        for (int c = 0; c < kCols; c += 32) tmem_ld_x32(tS + c, sr + c);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
+        for (int c = 0; c < kPairs; ++c) {
           const float2 t = __ffma2_rn(
               make_float2(__uint_as_float(sr[2 * c]), __uint_as_float(sr[2 * c + 1])), sc2, nlse2);
-          p[c] = exp2_pair(t, c);
+          p[c] = exp2_pair<kPolyShareT<D>>(t, c);
         }
       }
-      if (j == qt || j * 128 + 128 > Nk) {
-        // diagonal tile: keep kv <= q; last KV tile: drop the columns beyond the last key
-        int last = j == qt ? r : 127;
-        last = last < Nk - 1 - j * 128 ? last : Nk - 1 - j * 128;
+      if (j * W + W > qt * 128 || j * W + W > Nk) {
+        // diagonal tiles: keep kv <= q; last KV tile: drop the columns beyond the last key
+        const int last = min(qt * 128 + r, Nk - 1) - j * W - wg * kCols;
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          p[c].x = (wg * 64 + 2 * c <= last) ? p[c].x : 0.f;
-          p[c].y = (wg * 64 + 2 * c + 1 <= last) ? p[c].y : 0.f;
+        for (int c = 0; c < kPairs; ++c) {
+          p[c].x = (2 * c <= last) ? p[c].x : 0.f;
+          p[c].y = (2 * c + 1 <= last) ? p[c].y : 0.f;
         }
       }
       if (!(ok = mbar_wait_warp(bar(C::kBarDpFull), j & 1, w, kBSiteCmpDpt))) break;
       tc_fence_after();
-      uint32_t dp[64];
-      tmem_ld_x32(tDp, dp);
-      tmem_ld_x32(tDp + 32, dp + 32);
+      uint32_t dp[kCols];
+#pragma unroll
+      for (int c = 0; c < kCols; c += 32) tmem_ld_x32(tDp + c, dp + c);
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(C::kBarDpConsumed));
-      uint32_t dsk[32];
+      uint32_t dsk[kPairs];
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
+      for (int c = 0; c < kPairs; ++c) {
         float2 u = __fadd2_rn(
             make_float2(__uint_as_float(dp[2 * c]), __uint_as_float(dp[2 * c + 1])), ndlt2);
         u = __fmul2_rn(__fmul2_rn(p[c], u), scale2);
         dsk[c] = pack2<kInterBF16<BF16>>(u.x, u.y);
       }
-      tmem_st_x32(tS, dsk);  // over the score columns this thread has already read
+      // over the score columns this thread has already read
+      if constexpr (kPairs == 16) tmem_st_x16(tS, dsk); else tmem_st_x32(tS, dsk);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();

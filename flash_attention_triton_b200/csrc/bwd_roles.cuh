@@ -42,11 +42,11 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
 // row and 64 q columns of a tile.  probabilities_of_row: p = 2^(s * c - lse2[q]) from the raw
 // scores `sr` and the negated, log2-scaled row statistics of the 64 columns (`nlse`, read with
 // warp-wide broadcasts).  mask_row: keep only the q columns >= `first` (128 keeps nothing).
-template <int SHARE = FA2_BWD_POLY_PAIRS_PER_8>
-__device__ __forceinline__ void probabilities_of_row(const uint32_t (&sr)[64], const float4* nlse,
-                                                     float2 sc2, float2 (&p)[32]) {
+template <int SHARE = FA2_BWD_POLY_PAIRS_PER_8, int PAIRS>
+__device__ __forceinline__ void probabilities_of_row(const uint32_t (&sr)[2 * PAIRS], const float4* nlse,
+                                                     float2 sc2, float2 (&p)[PAIRS]) {
 #pragma unroll
-  for (int c4 = 0; c4 < 16; ++c4) {
+  for (int c4 = 0; c4 < PAIRS / 2; ++c4) {
     const float4 l = nlse[c4];
     const float2 t0 = __ffma2_rn(
         make_float2(__uint_as_float(sr[4 * c4]), __uint_as_float(sr[4 * c4 + 1])), sc2,
@@ -58,9 +58,10 @@ __device__ __forceinline__ void probabilities_of_row(const uint32_t (&sr)[64], c
     p[2 * c4 + 1] = exp2_pair<SHARE>(t1, 2 * c4 + 1);
   }
 }
-__device__ __forceinline__ void mask_row(float2 (&p)[32], int first_column, int column0) {
+template <int PAIRS>
+__device__ __forceinline__ void mask_row(float2 (&p)[PAIRS], int first_column, int column0) {
 #pragma unroll
-  for (int c = 0; c < 32; ++c) {
+  for (int c = 0; c < PAIRS; ++c) {
     p[c].x = (column0 + 2 * c >= first_column) ? p[c].x : 0.f;
     p[c].y = (column0 + 2 * c + 1 >= first_column) ? p[c].y : 0.f;
   }
@@ -145,22 +146,49 @@ __host__ __device__ __forceinline__ int dstile_count(int ntiles, int jt) {
 // an fp32 buffer with atomic adds by a fourth warp group.  MODE 2 (spill): also stores every
 // 16-bit dS^T tile to a scratch tensor, from which a consumer forms dQ with one product per tile
 // pair instead of recomputing S, P, dP.
+//
+// Modes 0 and 1 take head dims up to 64 in steps of 64 Q rows (kW).  The products of a 128 x 128 tile
+// pair are short there and a step is a chain of latencies: score product, copy-out, exponentials,
+// copy-in, dP product, ...; all eight compute warps of a CTA stand at the same link of it.  With 64
+// score columns a CTA needs half of the tensor memory and registers, so two CTAs run on an SM and
+// fill each other's waits, at the price of score products that read their A operand twice as often
+// (shared-memory bound: 384 instead of 256 cycles per tile pair at head dim 64).  Measured, whole
+// backward call, microseconds, 128- against 64-row steps: [4,16,2048,64] mode 0 207 -> 171, mode 1
+// 178 -> 169; [8,12,4095,32] mode 0 850 -> 743, mode 1 638 -> 576; [8,16,1000,64] mode 0 147 -> 120,
+// mode 1 124 -> 115; [2,16,8192,64] mode 0 1258 -> 1149, mode 1 986 -> 997 (bound by the fp32
+// reductions in L2, 2.2 TB/s: without them it takes 791).  One compute group of 64 columns per thread
+// instead of two of 32 was 2-6 % slower.
 template <int D, int MODE>
 struct DkdvCfg {
   using T = Tile<D>;
   static constexpr bool FUSE = MODE == 1;
   static constexpr bool SPILL = MODE == 2;
-  static constexpr int kStages = 2;  // Q (+rowstats) ring and dO ring (the code relies on 2)
-  static constexpr int kThreads = FUSE ? 512 : 384;
-  static constexpr int kMmaWarp = FUSE ? 12 : 8;
+  static constexpr int kW = SPILL ? 128 : bwd_step_rows(D);  // Q rows of a step = score columns
+  static constexpr int kCtasPerSm = kW == 64 ? 2 : 1;
+  static constexpr int kGroups = 2;  // compute groups of four warps
+  static constexpr int kCols = kW / kGroups;     // score columns of a compute thread
+  static constexpr int kStepBytes = T::kTileBytes / 128 * kW;
+  static constexpr int kStages = kW == 64 && !FUSE ? 4 : 2;  // Q (+rowstats) ring and dO ring
+  static constexpr int kRedWarp = 4 * kGroups;   // first reduction warp (FUSE)
+  static constexpr int kMmaWarp = kRedWarp + (FUSE ? 4 : 0);
+  static constexpr int kThreads = 32 * (kMmaWarp + 4);
+  // registers per thread of the producer / reduction / compute warps; the launch gives every
+  // thread kLaunchRegs
+  static constexpr int kLaunchRegs = 65536 / (kThreads * kCtasPerSm) / 8 * 8;
+  static constexpr int kProducerRegs = kW == 64 ? (FUSE ? 40 : 48) : 72;
+  static constexpr int kReduceRegs = kW == 64 ? 56 : 136;
+  static constexpr int kComputeRegs = kW == 64 ? (FUSE ? 80 : 96) : (FUSE ? 152 : 208);
+  static_assert(128 * kProducerRegs + (FUSE ? 128 * kReduceRegs : 0) + 128 * kGroups * kComputeRegs <=
+                    kThreads * kLaunchRegs,
+                "setmaxnreg.inc waits for registers that setmaxnreg.dec has released");
   static constexpr int kLoadWarp = kMmaWarp + 1;
   static constexpr int kOffK = 0;
   static constexpr int kOffV = kOffK + T::kTileBytes;
   static constexpr int kOffQ = kOffV + T::kTileBytes;
-  static constexpr int kOffDO = kOffQ + kStages * T::kTileBytes;
-  static constexpr int kOffDS = kOffDO + kStages * T::kTileBytes;  // [2][128 kv][64 q] 16-bit
-  static constexpr int kOffStats = kOffDS + (FUSE ? 32768 : 0);    // [kStages][256] fp32
-  static constexpr int kOffBar = kOffStats + kStages * 1024;
+  static constexpr int kOffDO = kOffQ + kStages * kStepBytes;
+  static constexpr int kOffDS = kOffDO + kStages * kStepBytes;  // [2][128 kv][64 q] 16-bit
+  static constexpr int kOffStats = kOffDS + (FUSE ? 32768 : 0);    // [kStages][2][kW] fp32
+  static constexpr int kOffBar = kOffStats + kStages * kW * 8;
   static constexpr int kBarKV = 0;
   static constexpr int kBarQFull = 1;                      // kStages
   static constexpr int kBarQEmpty = kBarQFull + kStages;   // kStages
@@ -168,19 +196,21 @@ struct DkdvCfg {
   static constexpr int kBarDOEmpty = kBarDOFull + kStages;
   static constexpr int kBarStFull = kBarDOEmpty + kStages;
   static constexpr int kBarDptFull = kBarStFull + 1;
-  static constexpr int kBarPtReady = kBarDptFull + 1;   // 8 arrivals (one per compute warp)
-  static constexpr int kBarDsReady = kBarPtReady + 1;   // 8 arrivals
+  static constexpr int kBarPtReady = kBarDptFull + 1;   // one arrival per compute warp
+  static constexpr int kBarDsReady = kBarPtReady + 1;   // one arrival per compute warp
   static constexpr int kBarDqFull = kBarDsReady + 1;
   static constexpr int kBarDqDrained = kBarDqFull + 1;  // 4 arrivals
   static constexpr int kBarDone = kBarDqDrained + 1;
   static constexpr int kNumBars = kBarDone + 1;
   static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;
-  static_assert(kSmemBytes <= 232448, "shared memory budget of one CTA");
+  static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "shared memory of one SM");
+  static_assert(kStages * kStepBytes >= T::kTileBytes, "the rings stage dK and dV at the end");
   static constexpr int kColSt = 0;
-  static constexpr int kColDpt = 128;  // dQ (fused) reuses these columns
-  static constexpr int kColDV = 256;
-  static constexpr int kColDK = 256 + D;
-  static constexpr int kTmemCols = 512;
+  static constexpr int kColDpt = kW;  // dQ (fused) reuses these columns
+  static constexpr int kColDV = 2 * kW;
+  static constexpr int kColDK = 2 * kW + D;
+  static constexpr int kTmemCols = 512 / kCtasPerSm;
+  static_assert(kColDK + D <= kTmemCols && (!FUSE || D <= kW), "tensor memory of one CTA");
 };
 
 enum BwdSite {
@@ -222,8 +252,8 @@ __device__ __forceinline__ void dkdv_init_barriers(uint32_t bar0) {
   }
   mbar_init(bar(C::kBarStFull), 1);
   mbar_init(bar(C::kBarDptFull), 1);
-  mbar_init(bar(C::kBarPtReady), 8);
-  mbar_init(bar(C::kBarDsReady), 8);
+  mbar_init(bar(C::kBarPtReady), 4 * C::kGroups);
+  mbar_init(bar(C::kBarDsReady), 4 * C::kGroups);
   mbar_init(bar(C::kBarDqFull), 1);
   mbar_init(bar(C::kBarDqDrained), 4);
   mbar_init(bar(C::kBarDone), 2);  // last dV (warp X) and last dK (warp Y)
@@ -265,10 +295,16 @@ __device__ __forceinline__ void dkdv_roles(
   const int bh = item.bh;
   const int nq = ntiles - jt;  // Q tiles ntiles-1 down to jt (N = query rows, Nk <= N = key rows)
   const bool kv_ragged = jt * 128 + 128 > Nk;  // this KV tile has rows beyond the last key
+  // A Q tile is worked through in kSub steps of W rows, first rows first, so that dK and dV add the
+  // same products in the same order whatever W is.
+  constexpr int W = C::kW;
+  constexpr int kSub = 128 / W;
+  const int nsteps = nq * kSub;
+  auto q_row = [&](int t) { return (ntiles - 1 - t / kSub) * 128 + (t % kSub) * W; };
 
   if (warp >= C::kMmaWarp) {
     // ---------------------------------------------------------------- producer / MMA group
-    reg_dec<72>();
+    reg_dec<C::kProducerRegs>();
     if (warp == C::kLoadWarp) {
       // TMA producer: whole warp, converged; the elected lane arms barriers and issues copies.
       const uint32_t elected = elect_one();
@@ -285,27 +321,33 @@ __device__ __forceinline__ void dkdv_roles(
                       jt * 128, hc, bar(C::kBarKV));
         }
       }
-      for (int ii = 0; ii < nq; ++ii) {
-        const int s = ii % C::kStages, ph = (ii / C::kStages) & 1;
-        const int qt = ntiles - 1 - ii;
+      for (int t = 0; t < nsteps; ++t) {
+        const int s = t % C::kStages, ph = (t / C::kStages) & 1;
+        const int row = q_row(t);
         if (!mbar_wait_warp(bar(C::kBarQEmpty + s), ph ^ 1, w, kBSiteLoadQ)) break;
         if (elected) {
-          mbar_arrive_expect_tx(bar(C::kBarQFull + s), T::kTileBytes + 1024);
+          mbar_arrive_expect_tx(bar(C::kBarQFull + s), C::kStepBytes + W * 8);
 #pragma unroll
           for (int ch = 0; ch < T::kChunks; ++ch)
-            tma_load_4d(smem_base + C::kOffQ + s * T::kTileBytes + ch * T::kChunkTileBytes, tq,
-                        ch * T::kChunkElems, qt * 128, hc, bar(C::kBarQFull + s));
-          bulk_load_1d(smem_base + C::kOffStats + s * 1024,
-                       rowstats + (static_cast<size_t>(bh) * ntiles + qt) * 256, 1024,
-                       bar(C::kBarQFull + s));
+            tma_load_4d(smem_base + C::kOffQ + s * C::kStepBytes + ch * (C::kStepBytes / T::kChunks), tq,
+                        ch * T::kChunkElems, row, hc, bar(C::kBarQFull + s));
+          const float* stats = rowstats + (static_cast<size_t>(bh) * ntiles + (row >> 7)) * 256;
+          if constexpr (W == 128) {
+            bulk_load_1d(smem_base + C::kOffStats + s * 1024, stats, 1024, bar(C::kBarQFull + s));
+          } else {
+            const int half = row & 64;
+            bulk_load_1d(smem_base + C::kOffStats + s * 512, stats + half, 256, bar(C::kBarQFull + s));
+            bulk_load_1d(smem_base + C::kOffStats + s * 512 + 256, stats + 128 + half, 256,
+                         bar(C::kBarQFull + s));
+          }
         }
         if (!mbar_wait_warp(bar(C::kBarDOEmpty + s), ph ^ 1, w, kBSiteLoadDO)) break;
         if (elected) {
-          mbar_arrive_expect_tx(bar(C::kBarDOFull + s), T::kTileBytes);
+          mbar_arrive_expect_tx(bar(C::kBarDOFull + s), C::kStepBytes);
 #pragma unroll
           for (int ch = 0; ch < T::kChunks; ++ch)
-            tma_load_4d(smem_base + C::kOffDO + s * T::kTileBytes + ch * T::kChunkTileBytes, tdo,
-                        ch * T::kChunkElems, qt * 128, hc, bar(C::kBarDOFull + s));
+            tma_load_4d(smem_base + C::kOffDO + s * C::kStepBytes + ch * (C::kStepBytes / T::kChunks),
+                        tdo, ch * T::kChunkElems, row, hc, bar(C::kBarDOFull + s));
         }
       }
     } else if (warp == C::kMmaWarp || warp == C::kMmaWarp + 2) {
@@ -324,84 +366,90 @@ __device__ __forceinline__ void dkdv_roles(
         if (elected) mma_commit(bar(b));
       };
       bool ok = mbar_wait(bar(C::kBarKV), 0, w, kBSiteMmaKV);
-      int s = 0, ph = 0;  // ring stage / phase of step ii (both rings advance together)
+      int s = 0, ph = 0;  // ring stage / phase of step t (both rings advance together)
+      constexpr uint32_t kHalf = C::kCols;  // columns between the two groups' halves of Pt and dSt
       if (warp == C::kMmaWarp) {
         // ------------------------------------------------------------ warp X
         if (ok && (ok = mbar_wait(bar(C::kBarQFull + 0), 0, w, kBSiteMmaQ))) {
-          issue_rows_x_rows<D, BF16>(elected, tmem_base + C::kColSt, ka, smem_base + C::kOffQ);
+          issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColSt, ka, smem_base + C::kOffQ);
           commit(C::kBarStFull);
           commit(C::kBarQEmpty + 0);
         }
-        for (int ii = 0; ok && ii < nq; ++ii) {
-          const int s1 = s ^ 1, ph1 = ph ^ s;  // stage / phase of step ii+1 (two stages)
-          const uint32_t doa = smem_base + C::kOffDO + s * T::kTileBytes;
+        for (int t = 0; ok && t < nsteps; ++t) {
+          const int s1 = s + 1 == C::kStages ? 0 : s + 1, ph1 = s1 ? ph : ph ^ 1;  // of step t+1
+          const uint32_t doa = smem_base + C::kOffDO + s * C::kStepBytes;
           if (!(ok = mbar_wait(bar(C::kBarDOFull + s), ph, w, kBSiteMmaDO))) break;
-          if (!(ok = mbar_wait(bar(C::kBarPtReady), ii & 1, w, kBSiteMmaPt))) break;
+          if (!(ok = mbar_wait(bar(C::kBarPtReady), t & 1, w, kBSiteMmaPt))) break;
           tc_fence_after();
-          issue_tmem_x_tile<D, BF16>(elected, tmem_base + C::kColDV, tmem_base + C::kColSt, 64, doa,
-                                     ii > 0);  // dV += Pt dO_i
+          issue_tmem_x_tile<D, BF16, W>(elected, tmem_base + C::kColDV, tmem_base + C::kColSt, kHalf,
+                                        doa, t > 0);  // dV += Pt dO_t
           commit(C::kBarDOEmpty + s);
-          if (ii + 1 < nq) {
+          if (t + 1 < nsteps) {
             if (!(ok = mbar_wait(bar(C::kBarQFull + s1), ph1, w, kBSiteMmaQ))) break;
-            issue_rows_x_rows<D, BF16>(elected, tmem_base + C::kColSt, ka,
-                                       smem_base + C::kOffQ + s1 * T::kTileBytes);  // St(i+1)
+            issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColSt, ka,
+                                          smem_base + C::kOffQ + s1 * C::kStepBytes);  // St(t+1)
             commit(C::kBarStFull);
             commit(C::kBarQEmpty + s1);
           }
-          ph ^= s;
-          s ^= 1;
+          s = s1;
+          ph = ph1;
         }
         if (ok) commit(C::kBarDone);
       } else {
         // ------------------------------------------------------------ warp Y
         if (ok && (ok = mbar_wait(bar(C::kBarDOFull + 0), 0, w, kBSiteMmaDO))) {
-          issue_rows_x_rows<D, BF16>(elected, tmem_base + C::kColDpt, va, smem_base + C::kOffDO);
+          issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColDpt, va, smem_base + C::kOffDO);
           commit(C::kBarDptFull);
           commit(C::kBarDOEmpty + 0);
         }
-        for (int ii = 0; ok && ii < nq; ++ii) {
-          const int s1 = s ^ 1, ph1 = ph ^ s;
-          const uint32_t qa = smem_base + C::kOffQ + s * T::kTileBytes;
+        for (int t = 0; ok && t < nsteps; ++t) {
+          const int s1 = s + 1 == C::kStages ? 0 : s + 1, ph1 = s1 ? ph : ph ^ 1;
+          const uint32_t qa = smem_base + C::kOffQ + s * C::kStepBytes;
+          const bool tile_end = (t + 1) % kSub == 0;  // last step of a Q tile
           if (!(ok = mbar_wait(bar(C::kBarQFull + s), ph, w, kBSiteMmaQ))) break;
-          if (!(ok = mbar_wait(bar(C::kBarDsReady), ii & 1, w, kBSiteMmaDs))) break;
+          if (!(ok = mbar_wait(bar(C::kBarDsReady), t & 1, w, kBSiteMmaDs))) break;
           if constexpr (!FUSE) {
-            // St(i+1) sits on the critical chain St -> Pt -> dV -> St; let warp X get it into
-            // the in-order pipe first, dK and dPt(i+1) then run under the next exponentials.
-            if (ii + 1 < nq) {
-              if (!(ok = mbar_wait(bar(C::kBarStFull), (ii + 1) & 1, w, kBSiteMmaQ))) break;
+            // St(t+1) sits on the critical chain St -> Pt -> dV -> St; let warp X get it into
+            // the in-order pipe first, dK and dPt(t+1) then run under the next exponentials.
+            if (t + 1 < nsteps) {
+              if (!(ok = mbar_wait(bar(C::kBarStFull), (t + 1) & 1, w, kBSiteMmaQ))) break;
             }
           }
           tc_fence_after();
-          issue_tmem_x_tile<D, BF16>(elected, tmem_base + C::kColDK, tmem_base + C::kColDpt, 64, qa,
-                                     ii > 0);  // dK += dSt Q_i
+          issue_tmem_x_tile<D, BF16, W>(elected, tmem_base + C::kColDK, tmem_base + C::kColDpt, kHalf,
+                                        qa, t > 0);  // dK += dSt Q_t
           commit(C::kBarQEmpty + s);
           if constexpr (FUSE) {
-            // dQ_i[128 q, D] = dS[q, kv] * K[kv, d]: A = dS^T tile in smem (q contiguous ->
-            // MN-major), B = K tile (d contiguous -> MN-major); lands over the dPt columns.
-            issue_tileT_x_tile<D, BF16>(elected, tmem_base + C::kColDpt, smem_base + C::kOffDS, ka);
-            commit(C::kBarDqFull);
+            // dQ[128 q, D] of a whole Q tile = dS[q, kv] * K[kv, d]: A = dS^T tile in smem (q
+            // contiguous -> MN-major), B = K tile (d contiguous -> MN-major); lands over the dPt columns.
+            if (tile_end) {
+              issue_tileT_x_tile<D, BF16>(elected, tmem_base + C::kColDpt, smem_base + C::kOffDS, ka);
+              commit(C::kBarDqFull);
+            }
           }
-          if (ii + 1 < nq) {
+          if (t + 1 < nsteps) {
             if constexpr (FUSE) {
-              if (!(ok = mbar_wait(bar(C::kBarDqDrained), ii & 1, w, kBSiteMmaDrain))) break;
-              tc_fence_after();
+              if (tile_end) {
+                if (!(ok = mbar_wait(bar(C::kBarDqDrained), (t / kSub) & 1, w, kBSiteMmaDrain))) break;
+                tc_fence_after();
+              }
             }
             if (!(ok = mbar_wait(bar(C::kBarDOFull + s1), ph1, w, kBSiteMmaDO))) break;
-            issue_rows_x_rows<D, BF16>(elected, tmem_base + C::kColDpt, va,
-                                       smem_base + C::kOffDO + s1 * T::kTileBytes);  // dPt(i+1)
+            issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColDpt, va,
+                                          smem_base + C::kOffDO + s1 * C::kStepBytes);  // dPt(t+1)
             commit(C::kBarDptFull);
             commit(C::kBarDOEmpty + s1);
           }
-          ph ^= s;
-          s ^= 1;
+          s = s1;
+          ph = ph1;
         }
         if (ok) commit(C::kBarDone);
       }
     }
     __syncwarp();
-  } else if (FUSE && warp >= 8) {
+  } else if (FUSE && warp >= C::kRedWarp) {
     // ---------------------------------------------------------------- dQ reduction group
-    reg_inc<136>();  // 512-thread kernel starts at 128 registers per thread
+    if constexpr (C::kReduceRegs > C::kLaunchRegs) reg_inc<C::kReduceRegs>(); else reg_dec<C::kReduceRegs>();
     const int w4 = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(w4 * 32) << 16;
     float inv_dscale;
@@ -414,71 +462,79 @@ __device__ __forceinline__ void dkdv_roles(
                    lane * 4;
       // Whole dQ tile into registers first, so the MMA warp can reuse the columns at once;
       // the atomics follow at leisure.
-      uint32_t v[D];
+      constexpr int kPart = C::kReduceRegs < 72 ? 32 : D;  // what the registers hold at a time
 #pragma unroll
-      for (int c0 = 0; c0 < D; c0 += 32) tmem_ld_x32(tmem_base + lane_base + C::kColDpt + c0, v + c0);
-      tmem_wait_ld();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(C::kBarDqDrained));
+      for (int d0 = 0; d0 < D; d0 += kPart) {
+        uint32_t v[kPart];
 #pragma unroll
-      for (int k = 0; k < D / 4; ++k)
-        red_add_v4(dst + k * 128, __uint_as_float(v[4 * k]) * inv_dscale,
-                   __uint_as_float(v[4 * k + 1]) * inv_dscale, __uint_as_float(v[4 * k + 2]) * inv_dscale,
-                   __uint_as_float(v[4 * k + 3]) * inv_dscale);
+        for (int c0 = 0; c0 < kPart; c0 += 32)
+          tmem_ld_x32(tmem_base + lane_base + C::kColDpt + d0 + c0, v + c0);
+        tmem_wait_ld();
+        if (d0 + kPart == D) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(C::kBarDqDrained));
+        }
+#pragma unroll
+        for (int k = 0; k < kPart / 4; ++k)
+          red_add_v4(dst + (d0 / 4 + k) * 128, __uint_as_float(v[4 * k]) * inv_dscale,
+                     __uint_as_float(v[4 * k + 1]) * inv_dscale, __uint_as_float(v[4 * k + 2]) * inv_dscale,
+                     __uint_as_float(v[4 * k + 3]) * inv_dscale);
+      }
     }
   } else {
     // ---------------------------------------------------------------- compute groups
-    if constexpr (FUSE) reg_inc<152>(); else reg_inc<208>();
-    const int wg = warp >> 2;  // 0: score columns (q) 0..63, 1: 64..127
+    reg_inc<C::kComputeRegs>();
+    constexpr int kCols = C::kCols, kPairs = kCols / 2;
+    const int wg = warp >> 2;  // score columns (q) wg * kCols ..
     const int w4 = warp & 3;
     const int r = w4 * 32 + lane;  // kv row in the tile = tensor-memory lane
     const uint32_t lane_base = static_cast<uint32_t>(w4 * 32) << 16;
-    const uint32_t tSt = tmem_base + lane_base + C::kColSt + wg * 64;
-    const uint32_t tDpt = tmem_base + lane_base + C::kColDpt + wg * 64;
+    const uint32_t tSt = tmem_base + lane_base + C::kColSt + wg * kCols;
+    const uint32_t tDpt = tmem_base + lane_base + C::kColDpt + wg * kCols;
     const float2 sc2 = make_float2(scale_log2, scale_log2);
     float inv_dscale;
     const float dscale = head_dscale<BF16>(item.tile_amax, ntiles, lane, &inv_dscale);
     const float2 scale2 = make_float2(scale * dscale, scale * dscale);  // dS = P (dP - delta) scale 2^k
     bool ok = true;
-    for (int ii = 0; ii < nq; ++ii) {
-      const int s = ii % C::kStages, ph = (ii / C::kStages) & 1;
-      const int qt = ntiles - 1 - ii;
-      const float* stats = reinterpret_cast<const float*>(smem + C::kOffStats + s * 1024);
-      const float4* nlse = reinterpret_cast<const float4*>(stats + wg * 64);        // -lse*log2e
-      const float4* ndlt = reinterpret_cast<const float4*>(stats + 128 + wg * 64);  // -delta
+    for (int t = 0; t < nsteps; ++t) {
+      const int s = t % C::kStages, ph = (t / C::kStages) & 1;
+      const int row = q_row(t), qt = row >> 7;
+      const float* stats = reinterpret_cast<const float*>(smem + C::kOffStats + s * (W * 8));
+      const float4* nlse = reinterpret_cast<const float4*>(stats + wg * kCols);      // -lse*log2e
+      const float4* ndlt = reinterpret_cast<const float4*>(stats + W + wg * kCols);  // -delta
       if (!(ok = mbar_wait_warp(bar(C::kBarQFull + s), ph, w, kBSiteCmpQ))) break;
-      if (!(ok = mbar_wait_warp(bar(C::kBarStFull), ii & 1, w, kBSiteCmpSt))) break;
+      if (!(ok = mbar_wait_warp(bar(C::kBarStFull), t & 1, w, kBSiteCmpSt))) break;
       tc_fence_after();
-      float2 p[32];  // P^T for this thread's kv row, q columns wg*64 .. wg*64+63
+      float2 p[kPairs];  // P^T for this thread's kv row, q columns wg*kCols ..
       {
-        uint32_t sr[64];
-        tmem_ld_x32(tSt, sr);
-        tmem_ld_x32(tSt + 32, sr + 32);
+        uint32_t sr[kCols];
+#pragma unroll
+        for (int c = 0; c < kCols; c += 32) tmem_ld_x32(tSt + c, sr + c);
         tmem_wait_ld();
         probabilities_of_row<kPolyShareT<D>>(sr, nlse, sc2, p);
       }
       if (qt == jt || kv_ragged) {
         // diagonal tile: keep q >= kv; rows beyond the last key (zero-filled K, V) keep nothing,
         // so that a huge 2^(-lse) never meets their zeros
-        mask_row(p, (jt * 128 + r >= Nk) ? 128 : (qt == jt ? r : 0), wg * 64);
+        mask_row(p, (jt * 128 + r >= Nk) ? 128 : (qt == jt ? r : 0), (row & 127) + wg * kCols);
       }
       {
-        uint32_t pk[32];
+        uint32_t pk[kPairs];
 #pragma unroll
-        for (int c = 0; c < 32; ++c) pk[c] = pack2<kInterBF16<BF16>>(p[c].x, p[c].y);
-        tmem_st_x32(tSt, pk);  // columns wg*64 .. wg*64+31 of the St region
+        for (int c = 0; c < kPairs; ++c) pk[c] = pack2<kInterBF16<BF16>>(p[c].x, p[c].y);
+        if constexpr (kPairs == 16) tmem_st_x16(tSt, pk); else tmem_st_x32(tSt, pk);
         tmem_wait_st();
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(C::kBarPtReady));
 
-      if (!(ok = mbar_wait_warp(bar(C::kBarDptFull), ii & 1, w, kBSiteCmpDpt))) break;
+      if (!(ok = mbar_wait_warp(bar(C::kBarDptFull), t & 1, w, kBSiteCmpDpt))) break;
       tc_fence_after();
-      uint32_t dsk[32];
+      uint32_t dsk[kPairs];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      for (int h = 0; h < kCols / 32; ++h) {
         uint32_t dp[32];
         tmem_ld_x32(tDpt + 32 * h, dp);
         tmem_wait_ld();
@@ -496,7 +552,7 @@ __device__ __forceinline__ void dkdv_roles(
           dsk[16 * h + 2 * c4 + 1] = pack2<kInterBF16<BF16>>(u1.x, u1.y);
         }
       }
-      tmem_st_x32(tDpt, dsk);  // columns 128 + wg*64 .. +31
+      if constexpr (kPairs == 16) tmem_st_x16(tDpt, dsk); else tmem_st_x32(tDpt, dsk);
       if constexpr (SPILL) {
         // This thread's 64 values of dS^T(jt, qt) (kv row r, q columns wg*64 ..) straight to pair
         // `tile0 + (qt - jt)` of the scratch tensor.  A tile is stored piece-major: the 16-byte
@@ -511,10 +567,11 @@ __device__ __forceinline__ void dkdv_roles(
           dst[pc * 128] = make_uint4(dsk[4 * pc], dsk[4 * pc + 1], dsk[4 * pc + 2], dsk[4 * pc + 3]);
       }
       if constexpr (FUSE) {
-        uint8_t* ds_tile = smem + C::kOffDS + wg * 16384;
+        const int col = (row & 127) + wg * kCols;  // first q column inside the Q tile
+        uint8_t* ds_tile = smem + C::kOffDS + (col >> 6) * 16384;
 #pragma unroll
-        for (int pc = 0; pc < 8; ++pc)
-          *reinterpret_cast<uint4*>(ds_tile + swizzled_offset_128B(r, pc)) =
+        for (int pc = 0; pc < kCols / 8; ++pc)
+          *reinterpret_cast<uint4*>(ds_tile + swizzled_offset_128B(r, ((col & 63) >> 3) + pc)) =
               make_uint4(dsk[4 * pc], dsk[4 * pc + 1], dsk[4 * pc + 2], dsk[4 * pc + 3]);
         fence_proxy_async_smem();
       }

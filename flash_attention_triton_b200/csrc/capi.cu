@@ -383,10 +383,12 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
   }
 
   CUtensorMap tq, tk, tv, tdo, tdq, tdk, tdv;
-  if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, 128)) return e;
+  // boxes of the resident tiles are 128 rows high, those of the tiles a kernel walks step_rows
+  const int step_rows = deterministic == 2 ? 128 : bwd_step_rows(padded_head_dim(D));
+  if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, step_rows)) return e;
   if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, 128)) return e;
   if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, 128)) return e;
-  if (int e = make_map_of(&tdo, dout, strides, 3, dtype, B, H, N, D, 128)) return e;
+  if (int e = make_map_of(&tdo, dout, strides, 3, dtype, B, H, N, D, step_rows)) return e;
   if (int e = make_map_of(&tdk, dk, strides, 5, dtype, B, H, Nk, D, 32)) return e;
   if (int e = make_map_of(&tdv, dv, strides, 6, dtype, B, H, Nk, D, 32)) return e;
   const Strides sdq{st_all[12], st_all[13], st_all[14]};
@@ -400,6 +402,12 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
         launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, rs, nullptr, 0, d->status, st);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     record_mark_between(st);
+    if (step_rows != 128) {  // here Q and dO are resident, K and V are walked
+      if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, 128)) return e;
+      if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, step_rows)) return e;
+      if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, step_rows)) return e;
+      if (int e = make_map_of(&tdo, dout, strides, 3, dtype, B, H, N, D, 128)) return e;
+    }
     return static_cast<int>(launch_bwd_dq(s, tq, tk, tv, tdo, tdq, rs, d->status, st));
   }
   if (deterministic == 2) {

@@ -76,6 +76,10 @@ inline int padded_head_dim(int d) { return d <= 32 ? 32 : (d <= 64 ? 64 : (d <= 
 // Rows of the KV tiles the forward kernel walks (its K and V tensor maps use boxes of this height).
 __host__ __device__ constexpr int fwd_kv_rows(int padded_d) { return padded_d <= 64 ? 64 : 128; }
 
+// Rows of the tiles the backward kernels walk past their resident tile: Q and dO tiles of the dK/dV
+// kernel (its spill mode always takes 128), K and V tiles of the dQ kernel.
+__host__ __device__ constexpr int bwd_step_rows(int padded_d) { return padded_d <= 64 ? 64 : 128; }
+
 // Order in which the causal kernels take their (head, tile) work items.  A tile's work shrinks
 // with its rank (rank 0 is the tile that meets the most tiles of the other kind), so for an even
 // finish the long items must start first; but the items of one head share its tensors through

@@ -136,6 +136,21 @@ def test_forward_backward_match_oracle(shape, dtype, scale, qk_mul, mode, monkey
         check_against(ref, got, dtype)
 
 
+@pytest.mark.parametrize("mode", ["recompute", "atomic"])
+@pytest.mark.parametrize("d,dtype", [(64, torch.float16), (40, torch.bfloat16), (32, torch.float16)])
+@pytest.mark.parametrize("nq,nk", [(1, 1), (63, 63), (64, 64), (65, 65), (128, 64), (129, 65), (191, 191),
+                                   (192, 192), (193, 129), (257, 257), (320, 191), (449, 449)])
+def test_narrow_heads_at_the_edges_of_64_row_steps(nq, nk, d, dtype, mode, monkeypatch):
+    """Head dims up to 64 walk keys (forward, dQ) and queries (dK, dV) in steps of 64 rows inside
+    tiles of 128: one row below, at and above every boundary, odd and even step counts, fewer keys
+    than queries.  Bounds: those of every parity test here (conftest)."""
+    monkeypatch.setenv("FA2_B200_BWD_MODE", mode)
+    g = torch.Generator().manual_seed(nq * 1000 + nk + d)
+    q, do = (torch.randn(2, 2, nq, d, generator=g).to(dtype) for _ in range(2))
+    k, v = (torch.randn(2, 2, nk, d, generator=g).to(dtype) for _ in range(2))
+    check_against(naive_attention(q, k, v, do), run_api(q, k, v, do, None, mode != "atomic"), dtype)
+
+
 def test_spill_mode_chunks_change_no_bit(monkeypatch):
     """With a scratch bound of 3 MiB the spill mode works through [3, 5, 700, 64] (0.7 MiB per
     head) in chunks of 3 + 2 heads per batch entry; with 8 MiB in chunks of 2 + 1 batch
