@@ -7,10 +7,12 @@ cannot be loaded, :func:`lib` raises; nothing falls back to PyTorch or to the CP
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 from ctypes import c_char_p, c_float, c_int, c_size_t, c_void_p
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libfa2_b200.so"
+HOST_PATH = LIB_PATH.parent / "_host.so"
 
 FA2_DTYPE_FP16 = 0
 FA2_DTYPE_BF16 = 1
@@ -43,6 +45,7 @@ def stride_array(*tensors):
     return (ctypes.c_longlong * len(flat))(*flat)
 
 _lib = None
+_host = None
 
 
 class Fa2Error(RuntimeError):
@@ -70,6 +73,25 @@ def lib() -> ctypes.CDLL:
         fn.argtypes = argtypes
     _lib = handle
     return _lib
+
+
+def host():
+    """Load (once) and return the native host path (``csrc/host.cpp``)."""
+    global _host
+    if _host is None:
+        lib()
+        if not HOST_PATH.exists():
+            raise RuntimeError(
+                f"{HOST_PATH} is missing. Build it with `python -m flash_attention_triton_b200.build`. "
+                "There is no fallback path."
+            )
+        import torch  # noqa: F401  (its libraries resolve the module's symbols)
+
+        spec = importlib.util.spec_from_file_location("flash_attention_triton_b200._host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    return _host
 
 
 def check(fn: str, code: int) -> None:

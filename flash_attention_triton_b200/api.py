@@ -22,6 +22,7 @@ Everything runs through the C library on the tensors' CUDA device; there is no f
 
 from __future__ import annotations
 
+import functools
 import math
 import os
 from collections.abc import Callable
@@ -36,12 +37,7 @@ _MAX_HEAD_DIM = 256  # the reference's max_headdim on B200 (line 533)
 
 
 # ------------------------------------------------------------------ host launch wrappers
-def _dtype_code(dtype: torch.dtype) -> int:
-    if dtype == torch.float16:
-        return _lib.FA2_DTYPE_FP16
-    if dtype == torch.bfloat16:
-        return _lib.FA2_DTYPE_BF16
-    raise AssertionError("Supports only fp16 and bf16 compute dtypes")
+_COMPUTE_DTYPES = (torch.float16, torch.bfloat16)
 
 
 def _check_status_if_asked(fn: str) -> None:
@@ -55,26 +51,12 @@ def _check_status_if_asked(fn: str) -> None:
             raise _lib.Fa2Error(fn, -7, f"{_lib.lib().fa2_strerror(-7).decode()} (status {word:#x})")
 
 
-def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
-
-
-def _readable_in_place(t: torch.Tensor) -> bool:
-    """Whether the kernels can read a ``[B, H, N, D]`` tensor through its own strides: unit
-    last stride, 16-byte aligned base, batch / head / row strides that are positive multiples
-    of 8 elements (strides of size-1 dimensions do not matter)."""
-    if t.stride(-1) != 1 or t.data_ptr() % 16:
-        return False
-    for size, stride in zip(t.shape[:3], t.stride()[:3]):
-        if size > 1 and (stride <= 0 or stride % 8):
-            return False
-    return t.shape[2] == 1 or t.stride(2) >= t.shape[3]
-
-
 def _as_kernel_input(t: torch.Tensor) -> torch.Tensor:
-    """The tensor itself when it can be read in place (e.g. a transposed ``[B, N, H, D]``
-    buffer), else a contiguous copy (what the reference always makes, line 316)."""
-    return t if _readable_in_place(t) else t.contiguous()
+    """The tensor itself when the kernels can read it through its own strides (unit last stride,
+    16-byte aligned base, batch / head / row strides that are positive multiples of 8 elements;
+    e.g. a transposed ``[B, N, H, D]`` buffer), else a contiguous copy (what the reference always
+    makes, line 316)."""
+    return t if _lib.host().readable_in_place(t) else t.contiguous()
 
 
 def _flash_attention_forward(
@@ -97,19 +79,11 @@ def _flash_attention_forward(
     if seqlen_k > seqlen_q:  # no query sees the keys beyond seqlen_q - 1 (top-left aligned mask)
         k, v, seqlen_k = k[:, :, :seqlen_q], v[:, :, :seqlen_q], seqlen_q
     softmax_scale = softmax_scale or 1.0 / math.sqrt(headdim)
-    q, k, v = [_as_kernel_input(t) for t in (q, k, v)]
-    output = torch.empty(q.shape, device=q.device, dtype=q.dtype)  # dense, like the reference's O
-    lse = torch.empty((batch, nheads, seqlen_q), device=q.device, dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        _lib.check(
-            "fa2_fwd_strided",
-            _lib.lib().fa2_fwd_strided(
-                q.data_ptr(), k.data_ptr(), v.data_ptr(), output.data_ptr(), lse.data_ptr(),
-                batch, nheads, seqlen_q, seqlen_k, headdim, _dtype_code(q.dtype),
-                float(softmax_scale), _lib.stride_array(q, k, v, output), _stream(q),
-            ),
-        )
-        _check_status_if_asked("fa2_fwd_strided")
+    assert q.dtype in _COMPUTE_DTYPES, "Supports only fp16 and bf16 compute dtypes"
+    # output and LSE are dense, like the reference's
+    code, output, lse = _lib.host().forward(q, k, v, float(softmax_scale))
+    _lib.check("fa2_fwd_strided", code)
+    _check_status_if_asked("fa2_fwd_strided")
     return output, lse, softmax_scale
 
 
@@ -207,44 +181,26 @@ def _flash_attention_backward(
         seqlen_k = seqlen_q
     # The reference requires everything contiguous here (lines 183-192) and copies dO when it
     # is not (170-171); the inputs may keep their strides, only our own buffers are dense.
-    q, k, v, d_output = [_as_kernel_input(t) for t in (q, k, v, d_output)]
     assert lse.shape == (batch, nheads, seqlen_q)
     assert output.is_contiguous() and dq.is_contiguous()
-    assert _readable_in_place(dk) and _readable_in_place(dv)
-    lib = _lib.lib()
-    code = _dtype_code(q.dtype)
-    with torch.cuda.device(q.device):
-        stats_bytes = lib.fa2_rowstats_bytes(batch, nheads, seqlen_q)
-        rowstats = torch.empty(stats_bytes // 4, device=q.device, dtype=torch.float32)
-        _lib.check(
-            "fa2_bwd_preprocess_strided",
-            lib.fa2_bwd_preprocess_strided(
-                output.data_ptr(), d_output.data_ptr(), lse.data_ptr(), rowstats.data_ptr(),
-                batch, nheads, seqlen_q, headdim, code, _lib.stride_array(output, d_output),
-                _stream(q),
-            ),
-        )
-        mode = _backward_mode(bool(deterministic), headdim, seqlen_q)
-        workspace, ws_bytes, mode = _allocate_workspace(
-            lib, q.device, batch, nheads, seqlen_q, headdim, mode)
-        _lib.check(
-            "fa2_bwd_strided",
-            lib.fa2_bwd_strided(
-                q.data_ptr(), k.data_ptr(), v.data_ptr(), d_output.data_ptr(), rowstats.data_ptr(),
-                dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                workspace.data_ptr() if workspace is not None else None, ws_bytes,
-                batch, nheads, seqlen_q, seqlen_k, headdim, code, float(softmax_scale),
-                mode, _lib.stride_array(q, k, v, d_output, dq, dk, dv), _stream(q),
-            ),
-        )
-        _check_status_if_asked("fa2_bwd_strided")
+    assert q.dtype in _COMPUTE_DTYPES, "Supports only fp16 and bf16 compute dtypes"
+    host = _lib.host()
+    assert host.readable_in_place(dk) and host.readable_in_place(dv)
+    code, rowstats, d_output = host.preprocess(output, d_output, lse)
+    _lib.check("fa2_bwd_preprocess_strided", code)
+    mode = _backward_mode(bool(deterministic), headdim, seqlen_q)
+    workspace, _, mode = _allocate_workspace(
+        _lib.lib(), q.device, batch, nheads, seqlen_q, headdim, mode)
+    _lib.check("fa2_bwd_strided", host.backward(
+        q, k, v, d_output, dq, dk, dv, rowstats, workspace, float(softmax_scale), mode))
+    _check_status_if_asked("fa2_bwd_strided")
 
 
 # ------------------------------------------------------------------ autograd integration
 def _compute_dtype(dtype: torch.dtype) -> torch.dtype:
     # fp16 / bf16 run natively; everything else takes the reference's route (cast to fp16,
     # reference line 316).
-    return dtype if dtype in (torch.float16, torch.bfloat16) else torch.float16
+    return dtype if dtype in _COMPUTE_DTYPES else torch.float16
 
 
 class FlashAttentionV2Function(torch.autograd.Function):
@@ -258,7 +214,7 @@ class FlashAttentionV2Function(torch.autograd.Function):
         if headdim > _MAX_HEAD_DIM:
             raise ValueError(f"head dimension {headdim} is not supported (at most {_MAX_HEAD_DIM})")
         softmax_scale = softmax_scale or 1.0 / math.sqrt(headdim)  # reference line 94: 0.0 -> default
-        q, k, v = [_as_kernel_input(t.to(cdtype)) for t in (q, k, v)]
+        q, k, v = [_as_kernel_input(t if t.dtype == cdtype else t.to(cdtype)) for t in (q, k, v)]
         pad = -headdim % 8  # zero columns change neither the scores nor the real output columns
         if pad:
             q, k, v = [torch.nn.functional.pad(t, (0, pad)) for t in (q, k, v)]
@@ -266,13 +222,18 @@ class FlashAttentionV2Function(torch.autograd.Function):
         ctx.save_for_backward(q, k, v, output, lse)
         ctx.deterministic = bool(deterministic)
         ctx.headdim = headdim
-        return output[..., :headdim].contiguous().to(initial_dtype)
+        if pad:
+            output = output[..., :headdim].contiguous()
+        else:
+            output = output.view(output.shape)  # the tensor that is saved is not the one handed out
+        return output if initial_dtype == cdtype else output.to(initial_dtype)
 
     @staticmethod
     def backward(ctx: Any, d_output):  # noqa: ANN001
         q, k, v, output, lse = ctx.saved_tensors
-        dq, dk, dv = (torch.empty(t.shape, device=t.device, dtype=t.dtype) for t in (q, k, v))
-        d_output = d_output.to(q.dtype)
+        dq, dk, dv = _lib.host().gradients(q, k, v)
+        if d_output.dtype != q.dtype:
+            d_output = d_output.to(q.dtype)
         pad = q.shape[-1] - ctx.headdim
         if pad:
             d_output = torch.nn.functional.pad(d_output, (0, pad))
@@ -319,9 +280,14 @@ def init_to_zero_v2(name: str) -> Callable[[dict[str, torch.Tensor]], torch.Tens
 
 
 # ------------------------------------------------------------------ public API
+@functools.lru_cache(maxsize=None)
+def _capability(index: int) -> tuple[int, int]:
+    return torch.cuda.get_device_capability(index)
+
+
 def _check_device(q: torch.Tensor) -> None:
     assert q.is_cuda, "All tensors must reside on CUDA device"
-    cc = torch.cuda.get_device_capability(q.device)
+    cc = _capability(q.device.index)
     if cc[0] != 10:
         raise RuntimeError(
             f"compute capability {cc} is not supported: this library targets B200 (sm_100a) only"

@@ -1,7 +1,8 @@
 """In-tree nvcc build of the sm_100a shared library.
 
 ``python -m flash_attention_triton_b200.build`` compiles every ``csrc/*.cu`` for
-``compute_100a/sm_100a`` and links ``libfa2_b200.so`` next to this file.  nvcc
+``compute_100a/sm_100a``, links ``libfa2_b200.so`` next to this file, and compiles the Python module
+``_host.so`` that calls it.  nvcc
 cross-compiles without a GPU, so the build can run on a CPU-only machine and the
 resulting ``.so`` be carried to the B200 host.  Objects are rebuilt only when a source or
 header is newer than the object.
@@ -13,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -21,6 +23,7 @@ CSRC = PKG_DIR / "csrc"
 INCLUDE = PKG_DIR.parent / "include"
 BUILD_DIR = PKG_DIR / "build"
 LIB_PATH = PKG_DIR / "libfa2_b200.so"
+HOST_PATH = PKG_DIR / "_host.so"
 
 NVCC_FLAGS = [
     "-std=c++17",
@@ -63,13 +66,39 @@ def _compile(src: Path, verbose: bool) -> Path:
     return obj
 
 
+def _build_host(verbose: bool) -> None:
+    """The Python module with the host path (``csrc/host.cpp``), against torch's C++ headers and the
+    library next to it."""
+    src = CSRC / "host.cpp"
+    newest = max(src.stat().st_mtime, (INCLUDE / "fa2_b200.h").stat().st_mtime)
+    if HOST_PATH.exists() and HOST_PATH.stat().st_mtime >= newest:
+        return
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    includes = [INCLUDE, root / "include", root / "include/torch/csrc/api/include",
+                sysconfig.get_paths()["include"], cuda / "include"]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{p}" for p in includes), str(src), "-o", str(HOST_PATH),
+           f"-L{PKG_DIR}", f"-l:{LIB_PATH.name}", "-Wl,-rpath,$ORIGIN", f"-L{root / 'lib'}",
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]  # already loaded by `import torch`
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {src.name}:\n{res.stderr[-4000:]}")
+    if verbose:
+        print(f"[build] compiled {src.name}")
+
+
 def build(verbose: bool = True, force: bool = False) -> Path:
-    """Compile and link the library; returns the path of the ``.so``."""
+    """Compile and link the library and the host module; returns the path of the library."""
     BUILD_DIR.mkdir(exist_ok=True)
     sources = sorted(CSRC.glob("*.cu"))
     if force:
         for o in BUILD_DIR.glob("*.o"):
             o.unlink()
+        HOST_PATH.unlink(missing_ok=True)
     with ThreadPoolExecutor(max_workers=min(8, len(sources))) as pool:
         objs = list(pool.map(lambda s: _compile(s, verbose), sources))
     newest_obj = max(o.stat().st_mtime for o in objs)
@@ -81,6 +110,7 @@ def build(verbose: bool = True, force: bool = False) -> Path:
             raise RuntimeError(f"link failed:\n{res.stderr[-4000:]}")
         if verbose:
             print(f"[build] linked {LIB_PATH.name}")
+    _build_host(verbose)
     return LIB_PATH
 
 

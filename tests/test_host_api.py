@@ -118,3 +118,42 @@ def test_two_ranks_cover_the_problem_without_a_collective_on_the_data_path(tmp_p
         env=env, capture_output=True, text=True, timeout=240,
     )
     assert res.returncode == 0, res.stderr[-2000:]
+
+
+def _readable_by_definition(t):
+    """Unit last stride, 16-byte aligned base, positive batch / head / row strides in multiples of 8
+    elements where the dimension has more than one entry, rows that do not overlap."""
+    if t.stride(-1) != 1 or t.data_ptr() % 16:
+        return False
+    if any(n > 1 and (s <= 0 or s % 8) for n, s in zip(t.shape[:3], t.stride()[:3])):
+        return False
+    return t.shape[2] == 1 or t.stride(2) >= t.shape[3]
+
+
+@pytest.mark.parametrize("base", [torch.zeros(4096, dtype=torch.float16), torch.zeros(4096, dtype=torch.bfloat16)])
+def test_native_host_path_takes_the_same_tensors_in_place(base):
+    from flash_attention_triton_b200 import _lib
+
+    shapes = [(2, 3, 4, 16), (1, 3, 4, 16), (2, 1, 4, 16), (2, 3, 1, 16), (1, 1, 1, 8)]
+    strides = [(192, 64, 16, 1), (192, 16, 48, 1), (0, 64, 16, 1), (64, 0, 16, 1), (192, 60, 16, 1),
+               (196, 64, 16, 1), (192, 64, 8, 1), (192, 64, 20, 1), (192, 64, 16, 2), (192, 1, 16, 4), (5, 3, 7, 1)]
+    seen = set()
+    for shape in shapes:
+        for stride in strides:
+            for offset in (0, 1, 8):
+                t = base.as_strided(shape, stride, offset)
+                want = _readable_by_definition(t)
+                seen.add(want)
+                assert _lib.host().readable_in_place(t) is want, (shape, stride, offset)
+    assert seen == {True, False}
+
+
+def test_native_host_path_refuses_what_is_not_a_tensor():
+    from flash_attention_triton_b200 import _lib
+
+    t = torch.zeros(1, 1, 8, 8, dtype=torch.float16)
+    for call in (lambda h: h.forward(t, t, None, 0.1), lambda h: h.forward(t, t, t), lambda h: h.forward(t, t, t, "x"),
+                 lambda h: h.gradients(t, 1, t), lambda h: h.preprocess(t, t[0, 0], t), lambda h: h.readable_in_place(2),
+                 lambda h: h.backward(*([t] * 7), None, None, 0.1, 0), lambda h: h.backward(t)):
+        with pytest.raises(TypeError):
+            call(_lib.host())
