@@ -36,6 +36,9 @@ SYMBOLS = [
     ("fa2_bwd_preprocess_strided", c_int, [c_void_p] * 4 + [c_int] * 5 + [c_void_p, c_void_p]),
     ("fa2_bwd_strided", c_int,
      [c_void_p] * 9 + [c_size_t] + [c_int] * 6 + [c_float, c_int, c_void_p, c_void_p]),
+    ("fa2_fwd_strided_f32", c_int, [c_void_p] * 6 + [c_int] * 6 + [c_float, c_void_p, c_void_p]),
+    ("fa2_bwd_strided_f32", c_int,
+     [c_void_p] * 9 + [c_size_t] + [c_int] * 6 + [c_float, c_int, c_void_p, c_void_p]),
 ]
 
 

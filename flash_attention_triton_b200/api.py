@@ -60,9 +60,9 @@ def _as_kernel_input(t: torch.Tensor) -> torch.Tensor:
 
 
 def _flash_attention_forward(
-    q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, softmax_scale: float | None
-) -> tuple[torch.Tensor, torch.Tensor, float]:
-    """Validate, allocate O and LSE, launch ``fa2_fwd``.
+    q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, softmax_scale: float | None, f32: bool = False
+) -> tuple[torch.Tensor, torch.Tensor, float] | tuple[torch.Tensor, torch.Tensor, float, torch.Tensor]:
+    """Validate, allocate O and LSE, launch ``fa2_fwd``; with ``f32`` also return O as fp32.
 
     Counterpart of ``_flash_attention_forward`` (reference lines 61-144): the same asserts on
     shapes / device / dtype, ``softmax_scale or 1/sqrt(d)`` (so 0.0 means "default"), but
@@ -81,10 +81,10 @@ def _flash_attention_forward(
     softmax_scale = softmax_scale or 1.0 / math.sqrt(headdim)
     assert q.dtype in _COMPUTE_DTYPES, "Supports only fp16 and bf16 compute dtypes"
     # output and LSE are dense, like the reference's
-    code, output, lse = _lib.host().forward(q, k, v, float(softmax_scale))
+    code, output, lse, output32 = _lib.host().forward(q, k, v, float(softmax_scale), f32)
     _lib.check("fa2_fwd_strided", code)
     _check_status_if_asked("fa2_fwd_strided")
-    return output, lse, softmax_scale
+    return (output, lse, softmax_scale, output32) if f32 else (output, lse, softmax_scale)
 
 
 #: dQ strategies of the C library (the ``deterministic`` argument of ``fa2_bwd``)
@@ -170,7 +170,8 @@ def _flash_attention_backward(
     Counterpart of ``_flash_attention_backward`` (reference lines 147-277).  The workspace
     depends on the dQ strategy (:func:`_backward_mode`): an fp32 accumulator for the atomic
     kernel, the dS scratch for the spill mode, nothing for the recompute mode; the
-    deterministic modes write dQ once, already rounded.
+    deterministic modes write dQ once.  dq, dk and dv have the dtype of q, rounded once, or are
+    fp32, unrounded.
     """
     batch, nheads, seqlen_q, headdim = q.shape
     seqlen_k = k.shape[2]
@@ -210,6 +211,7 @@ class FlashAttentionV2Function(torch.autograd.Function):
     def forward(ctx: Any, q, k, v, softmax_scale, deterministic):  # noqa: ANN001
         initial_dtype = q.dtype
         cdtype = _compute_dtype(q.dtype)
+        f32 = q.dtype == k.dtype == v.dtype == torch.float32
         headdim = q.shape[-1]
         if headdim > _MAX_HEAD_DIM:
             raise ValueError(f"head dimension {headdim} is not supported (at most {_MAX_HEAD_DIM})")
@@ -218,10 +220,16 @@ class FlashAttentionV2Function(torch.autograd.Function):
         pad = -headdim % 8  # zero columns change neither the scores nor the real output columns
         if pad:
             q, k, v = [torch.nn.functional.pad(t, (0, pad)) for t in (q, k, v)]
-        output, lse, ctx.softmax_scale = _flash_attention_forward(q, k, v, softmax_scale)
-        ctx.save_for_backward(q, k, v, output, lse)
         ctx.deterministic = bool(deterministic)
         ctx.headdim = headdim
+        # fp32 callers get fp32 results from the kernels' accumulators, without a cast pass
+        ctx.f32 = f32 and not pad
+        if ctx.f32:
+            output, lse, ctx.softmax_scale, output32 = _flash_attention_forward(q, k, v, softmax_scale, True)
+            ctx.save_for_backward(q, k, v, output, lse)
+            return output32
+        output, lse, ctx.softmax_scale = _flash_attention_forward(q, k, v, softmax_scale)
+        ctx.save_for_backward(q, k, v, output, lse)
         if pad:
             output = output[..., :headdim].contiguous()
         else:
@@ -231,7 +239,7 @@ class FlashAttentionV2Function(torch.autograd.Function):
     @staticmethod
     def backward(ctx: Any, d_output):  # noqa: ANN001
         q, k, v, output, lse = ctx.saved_tensors
-        dq, dk, dv = _lib.host().gradients(q, k, v)
+        dq, dk, dv = _lib.host().gradients(q, k, v, ctx.f32)
         if d_output.dtype != q.dtype:
             d_output = d_output.to(q.dtype)
         pad = q.shape[-1] - ctx.headdim

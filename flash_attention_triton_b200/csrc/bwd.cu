@@ -34,7 +34,8 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::
     bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                     const __grid_constant__ CUtensorMap tdk,
-                    const __grid_constant__ CUtensorMap tdv, const float* __restrict__ rowstats,
+                    const __grid_constant__ CUtensorMap tdv, const __grid_constant__ F32Out dk32,
+                    const __grid_constant__ F32Out dv32, int cols, const float* __restrict__ rowstats,
                     const unsigned* __restrict__ tile_amax, float* __restrict__ dq_accum, int N,
                     int Nk, int num_bh, int num_heads, int group, float scale, float scale_log2,
                     int* status) {
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::
   const WaitCtx w{abort_flag, status};
 
   dkdv_roles<D, BF16, MODE>(smem, smem_base, tmem_base, warp, lane, &tq, &tk, &tv, &tdo, &tdk, &tdv,
-                            rowstats, dq_accum, N, Nk, scale, scale_log2, w, item);
+                            dk32, dv32, cols, rowstats, dq_accum, N, Nk, scale, scale_log2, w, item);
 
   tc_fence_before();
   __syncthreads();
@@ -153,7 +154,8 @@ template <int D, bool BF16>
 __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
     bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                   const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
-                  const __grid_constant__ CUtensorMap tdq, const float* __restrict__ rowstats,
+                  const __grid_constant__ CUtensorMap tdq, const __grid_constant__ F32Out dq32, int cols,
+                  const float* __restrict__ rowstats,
                   const unsigned* __restrict__ tile_amax, int N, int Nk, int num_bh, int num_heads,
                   int group, float scale, float scale_log2, int* status) {
   using C = DqCfg<D>;
@@ -407,7 +409,10 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
     }
     if (ok && wg == 0 && mbar_wait_warp(bar(C::kBarDone), 0, w, kBSiteCmpDone)) {
       tc_fence_after();
-      store_rows_16bit<D, BF16>(tmem_base + lane_base + C::kColDQ, smem + C::kOffDO, w4, lane, &tdq,
+      if (dq32.p != nullptr)
+        store_rows_f32<D>(tmem_base + lane_base + C::kColDQ, dq32, cols, qt * 128 + r, hc, N, inv_dscale);
+      else
+        store_rows_16bit<D, BF16>(tmem_base + lane_base + C::kColDQ, smem + C::kOffDO, w4, lane, &tdq,
                                 qt * 128, hc, N, inv_dscale);
     }
   }
@@ -442,7 +447,7 @@ struct ConsumeCfg {
 template <int D, bool BF16, int FORM>
 __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, 1)
     bwd_consume_kernel(const uint4* __restrict__ scratch, const __grid_constant__ CUtensorMap tb,
-                       const __grid_constant__ CUtensorMap tout,
+                       const __grid_constant__ CUtensorMap tout, const __grid_constant__ F32Out out32, int cols,
                        const unsigned* __restrict__ tile_amax, int N, int Nk, int num_bh,
                        int num_heads, int group, int* status) {
   using C = ConsumeCfg<D>;
@@ -487,7 +492,7 @@ __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, 1)
 
   consume_roles<D, BF16, FORM, C::kStages>(smem, smem_base, smem_base + C::kOffBar, tmem_base,
                                            warp == C::kLoadWarp, warp == C::kMmaWarp,
-                                           warp < 4 ? warp : -1, lane, scratch, &tb, &tout, N, Nk, w,
+                                           warp < 4 ? warp : -1, lane, scratch, &tb, &tout, out32, cols, N, Nk, w,
                                            item);
 
   tc_fence_before();
@@ -786,7 +791,8 @@ cudaError_t launch_scores_wide_t(const AttnShape& s, const CUtensorMap& tq, cons
 template <int D, bool BF16, int MODE>
 cudaError_t launch_dkdv_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                           const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdk,
-                          const CUtensorMap& tdv, const RowStats& rowstats, float* dq_accum,
+                          const CUtensorMap& tdv, const F32Out& dk32, const F32Out& dv32,
+                          const RowStats& rowstats, float* dq_accum,
                           int* status, cudaStream_t stream) {
   using C = DkdvCfg<D, MODE>;
   auto kern = bwd_dkdv_kernel<D, BF16, MODE>;
@@ -795,14 +801,14 @@ cudaError_t launch_dkdv_t(const AttnShape& s, const CUtensorMap& tq, const CUten
   if (e != cudaSuccess) return e;
   const unsigned grid = static_cast<unsigned>((s.Nk + 127) / 128) * s.B * s.H;  // one CTA per KV tile
   kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(
-      tq, tk, tv, tdo, tdk, tdv, rowstats.stats, rowstats.tile_amax, dq_accum, s.N, s.Nk, s.B * s.H,
+      tq, tk, tv, tdo, tdk, tdv, dk32, dv32, s.Dg, rowstats.stats, rowstats.tile_amax, dq_accum, s.N, s.Nk, s.B * s.H,
       s.H, heads_per_group(s), s.scale, s.scale * 1.4426950408889634f, status);
   return cudaGetLastError();
 }
 
 template <int D, bool BF16, int FORM>
 cudaError_t launch_consume_t(const AttnShape& s, const void* scratch, const CUtensorMap& tb,
-                             const CUtensorMap& tout, const RowStats& rowstats, int* status,
+                             const CUtensorMap& tout, const F32Out& out32, const RowStats& rowstats, int* status,
                              cudaStream_t stream) {
   using C = ConsumeCfg<D>;
   auto kern = bwd_consume_kernel<D, BF16, FORM>;
@@ -811,7 +817,7 @@ cudaError_t launch_consume_t(const AttnShape& s, const void* scratch, const CUte
   if (e != cudaSuccess) return e;
   const unsigned grid =
       static_cast<unsigned>(((FORM == 2 ? s.N : s.Nk) + 127) / 128) * s.B * s.H;  // one CTA per output tile
-  kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(static_cast<const uint4*>(scratch), tb, tout,
+  kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(static_cast<const uint4*>(scratch), tb, tout, out32, s.Dg,
                                                      rowstats.tile_amax, s.N, s.Nk, s.B * s.H, s.H,
                                                      heads_per_group(s), status);
   return cudaGetLastError();
@@ -820,7 +826,7 @@ cudaError_t launch_consume_t(const AttnShape& s, const void* scratch, const CUte
 template <int D, bool BF16>
 cudaError_t launch_dq_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                         const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
-                        const RowStats& rowstats, int* status, cudaStream_t stream) {
+                        const F32Out& dq32, const RowStats& rowstats, int* status, cudaStream_t stream) {
   using C = DqCfg<D>;
   auto kern = bwd_dq_kernel<D, BF16>;
   cudaError_t e =
@@ -828,7 +834,7 @@ cudaError_t launch_dq_t(const AttnShape& s, const CUtensorMap& tq, const CUtenso
   if (e != cudaSuccess) return e;
   const unsigned grid = static_cast<unsigned>((s.N + 127) / 128) * s.B * s.H;  // one CTA per Q tile
   kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(
-      tq, tk, tv, tdo, tdq, rowstats.stats, rowstats.tile_amax, s.N, s.Nk, s.B * s.H, s.H,
+      tq, tk, tv, tdo, tdq, dq32, s.Dg, rowstats.stats, rowstats.tile_amax, s.N, s.Nk, s.B * s.H, s.H,
       heads_per_group(s), s.scale, s.scale * 1.4426950408889634f, status);
   return cudaGetLastError();
 }
@@ -837,12 +843,12 @@ cudaError_t launch_dq_t(const AttnShape& s, const CUtensorMap& tq, const CUtenso
 
 cudaError_t launch_bwd_dkdv(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                             const CUtensorMap& tv, const CUtensorMap& tdo,
-                            const CUtensorMap& tdk, const CUtensorMap& tdv,
-                            const RowStats& rowstats, float* dq_accum, int mode, int* status,
+                            const CUtensorMap& tdk, const CUtensorMap& tdv, const F32Out& dk32,
+                            const F32Out& dv32, const RowStats& rowstats, float* dq_accum, int mode, int* status,
                             cudaStream_t stream) {
   // modes: 0 dK/dV only, 1 fused atomic dQ (dq_accum = fp32 accumulator), 2 spill dS tiles
   // (dq_accum = the 16-bit scratch tensor)
-#define FA2_ARGS s, tq, tk, tv, tdo, tdk, tdv, rowstats, dq_accum, status, stream
+#define FA2_ARGS s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rowstats, dq_accum, status, stream
 #define FA2_CASE(DD)                                                                        \
   case DD:                                                                                  \
     if (mode == 1)                                                                          \
@@ -865,8 +871,8 @@ cudaError_t launch_bwd_dkdv(const AttnShape& s, const CUtensorMap& tq, const CUt
 
 cudaError_t launch_bwd_dq(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                           const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
-                          const RowStats& rowstats, int* status, cudaStream_t stream) {
-#define FA2_ARGS s, tq, tk, tv, tdo, tdq, rowstats, status, stream
+                          const F32Out& dq32, const RowStats& rowstats, int* status, cudaStream_t stream) {
+#define FA2_ARGS s, tq, tk, tv, tdo, tdq, dq32, rowstats, status, stream
 #define FA2_CASE(DD)                                                   \
   case DD:                                                             \
     return s.dtype ? launch_dq_t<DD, true>(FA2_ARGS)                   \
@@ -892,9 +898,9 @@ cudaError_t launch_bwd_scores_wide(const AttnShape& s, const CUtensorMap& tq, co
 }
 
 cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch,
-                               const CUtensorMap& tb, const CUtensorMap& tout, const RowStats& rowstats,
-                               int* status, cudaStream_t stream) {
-#define FA2_ARGS s, scratch, tb, tout, rowstats, status, stream
+                               const CUtensorMap& tb, const CUtensorMap& tout, const F32Out& out32,
+                               const RowStats& rowstats, int* status, cudaStream_t stream) {
+#define FA2_ARGS s, scratch, tb, tout, out32, rowstats, status, stream
 #define FA2_CASE(DD)                                                      \
   case DD:                                                                \
     return s.dtype ? launch_consume_t<DD, true, 2>(FA2_ARGS)              \

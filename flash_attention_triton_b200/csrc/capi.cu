@@ -139,6 +139,9 @@ int make_map(CUtensorMap* m, const void* base, int dtype, int B, int H, int N, i
   return r == CUDA_SUCCESS ? FA2_OK : FA2_ERR_DRIVER;
 }
 
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
+
 // Map of tensor `idx` of a call (strides as get_strides resolves them).
 int make_map_of(CUtensorMap* m, const void* base, const long long* user, int idx, int dtype,
                 int B, int H, int N, int D, int box_rows) {
@@ -155,8 +158,6 @@ void make_ctx(DeviceState* d, LaunchCtx* ctx) {
   ctx->work_counter = d->counters + (d->next_counter.fetch_add(1) % kWorkCounterSlots);
   ctx->num_sms = d->num_sms;
 }
-
-bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 int check_shape(int B, int H, int N, int D, int dtype) {
   if (D < 8 || D > 256 || D % 8 != 0) return FA2_ERR_HEAD_DIM;
@@ -234,14 +235,18 @@ const char* fa2_strerror(int code) {
   return "unknown fa2 error code";
 }
 
-int fa2_fwd_strided(const void* q, const void* k, const void* v, void* o, float* lse, int B, int H,
-                    int N, int Nk, int D, int dtype, float scale, const long long* strides,
-                    fa2_stream_t stream) {
+static int fwd_strided(const void* q, const void* k, const void* v, void* o, float* o32, float* lse, int B,
+                       int H, int N, int Nk, int D, int dtype, float scale, const long long* strides,
+                       fa2_stream_t stream) {
   if (!q || !k || !v || !o || !lse) return FA2_ERR_NULL_POINTER;
   if (int e = check_shape(B, H, N, D, dtype)) return e;
   if (Nk < 1 || Nk > N) return FA2_ERR_SHAPE;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return FA2_ERR_MISALIGNED;
+  if (!aligned32(o32)) return FA2_ERR_MISALIGNED;
   if (!std::isfinite(scale) || !(scale > 0.f)) return FA2_ERR_SCALE;
+  F32Out out32{o32, {}};
+  if (o32)
+    if (int e = get_strides(strides, 4, B, H, N, D, &out32.st)) return e;
   for (int idx = 0; idx < 4; ++idx) {
     Strides unused;
     if (int e = get_strides(strides, idx, B, H, idx == 1 || idx == 2 ? Nk : N, D, &unused)) return e;
@@ -258,7 +263,20 @@ int fa2_fwd_strided(const void* q, const void* k, const void* v, void* o, float*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LaunchCtx ctx;
   make_ctx(d, &ctx);
-  return static_cast<int>(launch_fwd(s, tq, tk, tv, to, lse, ctx, st));
+  return static_cast<int>(launch_fwd(s, tq, tk, tv, to, out32, lse, ctx, st));
+}
+
+int fa2_fwd_strided(const void* q, const void* k, const void* v, void* o, float* lse, int B, int H,
+                    int N, int Nk, int D, int dtype, float scale, const long long* strides,
+                    fa2_stream_t stream) {
+  return fwd_strided(q, k, v, o, nullptr, lse, B, H, N, Nk, D, dtype, scale, strides, stream);
+}
+
+int fa2_fwd_strided_f32(const void* q, const void* k, const void* v, void* o, float* o32, float* lse, int B,
+                        int H, int N, int Nk, int D, int dtype, float scale, const long long* strides,
+                        fa2_stream_t stream) {
+  if (!o32) return FA2_ERR_NULL_POINTER;
+  return fwd_strided(q, k, v, o, o32, lse, B, H, N, Nk, D, dtype, scale, strides, stream);
 }
 
 int fa2_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int H, int N,
@@ -315,11 +333,12 @@ size_t fa2_bwd_workspace_bytes(int B, int H, int N, int D, int deterministic) {
 
 // fa2_bwd_strided with the two parts of the preprocess output given separately, so that a chunk of
 // a larger problem (see the chunk loop below) can point into the arrays of the whole problem.
+// grads_f32: dq, dk and dv are fp32 tensors (strides in their own elements).
 static int bwd_strided(const void* q, const void* k, const void* v, const void* dout,
                        const float* rowstats_ptr, const unsigned* tile_amax, void* dq, void* dk,
                        void* dv, void* workspace, size_t workspace_bytes, int B, int H, int N, int Nk,
                        int D, int dtype, float scale, int deterministic, const long long* strides,
-                       fa2_stream_t stream) {
+                       bool grads_f32, fa2_stream_t stream) {
   const float* rowstats = rowstats_ptr;
   if (!q || !k || !v || !dout || !rowstats || !dq || !dk || !dv) return FA2_ERR_NULL_POINTER;
   if (int e = check_shape(B, H, N, D, dtype)) return e;
@@ -331,6 +350,7 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(dout) || !aligned16(dq) ||
       !aligned16(dk) || !aligned16(dv) || !aligned16(rowstats))
     return FA2_ERR_MISALIGNED;
+  if (grads_f32 && (!aligned32(dq) || !aligned32(dk) || !aligned32(dv))) return FA2_ERR_MISALIGNED;
   if (!std::isfinite(scale) || !(scale > 0.f)) return FA2_ERR_SCALE;
   if (static_cast<long long>(B) * H * ((N + 127) / 128) > 0x7fffffffll) return FA2_ERR_SHAPE;  // one CTA per tile
   if (deterministic != 1 && !workspace) return FA2_ERR_WORKSPACE;
@@ -366,7 +386,8 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
         for (int h0 = 0; h0 < H; h0 += plan.nh) {
           const int nb = std::min(plan.nb, B - b0), nh = std::min(plan.nh, H - h0);
           auto at = [&](const void* p, int idx) {
-            return static_cast<const char*>(p) + 2 * (b0 * st_all[3 * idx] + h0 * st_all[3 * idx + 1]);
+            const long long element = idx >= 4 && grads_f32 ? 4 : 2;
+            return static_cast<const char*>(p) + element * (b0 * st_all[3 * idx] + h0 * st_all[3 * idx + 1]);
           };
           const int e = bwd_strided(
               at(in[0], 0), at(in[1], 1), at(in[2], 2), at(in[3], 3),
@@ -374,7 +395,7 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
               tile_amax + (static_cast<size_t>(b0) * H + h0) * ((N + 127) / 128),
               const_cast<char*>(at(out[0], 4)), const_cast<char*>(at(out[1], 5)),
               const_cast<char*>(at(out[2], 6)), workspace, workspace_bytes, nb, nh, N, Nk, D, dtype,
-              scale, 2, st_all, stream);
+              scale, 2, st_all, grads_f32, stream);
           if (e) return e;
         }
       return FA2_OK;
@@ -382,24 +403,32 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
     if (BH * dstile_pairs(N, Nk) >= (1ll << 31)) return FA2_ERR_SHAPE;
   }
 
-  CUtensorMap tq, tk, tv, tdo, tdq, tdk, tdv;
+  CUtensorMap tq, tk, tv, tdo;
+  CUtensorMap tdq{}, tdk{}, tdv{};  // of 16-bit gradients
+  F32Out dq32{nullptr, {}}, dk32{nullptr, {}}, dv32{nullptr, {}};
   // boxes of the resident tiles are 128 rows high, those of the tiles a kernel walks step_rows
   const int step_rows = deterministic == 2 ? 128 : bwd_step_rows(padded_head_dim(D));
   if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, step_rows)) return e;
   if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, 128)) return e;
   if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, 128)) return e;
   if (int e = make_map_of(&tdo, dout, strides, 3, dtype, B, H, N, D, step_rows)) return e;
-  if (int e = make_map_of(&tdk, dk, strides, 5, dtype, B, H, Nk, D, 32)) return e;
-  if (int e = make_map_of(&tdv, dv, strides, 6, dtype, B, H, Nk, D, 32)) return e;
   const Strides sdq{st_all[12], st_all[13], st_all[14]};
+  if (grads_f32) {
+    dq32 = {static_cast<float*>(dq), sdq};
+    dk32 = {static_cast<float*>(dk), {st_all[15], st_all[16], st_all[17]}};
+    dv32 = {static_cast<float*>(dv), {st_all[18], st_all[19], st_all[20]}};
+  } else {
+    if (int e = make_map_of(&tdk, dk, strides, 5, dtype, B, H, Nk, D, 32)) return e;
+    if (int e = make_map_of(&tdv, dv, strides, 6, dtype, B, H, Nk, D, 32)) return e;
+    if (deterministic != 0)
+      if (int e = make_map(&tdq, dq, dtype, B, H, N, D, sdq, 32)) return e;
+  }
   const AttnShape s = make_shape(B, H, N, Nk, D, dtype, scale);
   const RowStats rs{rowstats, tile_amax};
-  if (deterministic != 0)
-    if (int e = make_map(&tdq, dq, dtype, B, H, N, D, sdq, 32)) return e;
 
   if (deterministic == 1) {
     cudaError_t ce =
-        launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, rs, nullptr, 0, d->status, st);
+        launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, nullptr, 0, d->status, st);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     record_mark_between(st);
     if (step_rows != 128) {  // here Q and dO are resident, K and V are walked
@@ -408,7 +437,7 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
       if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, step_rows)) return e;
       if (int e = make_map_of(&tdo, dout, strides, 3, dtype, B, H, N, D, 128)) return e;
     }
-    return static_cast<int>(launch_bwd_dq(s, tq, tk, tv, tdo, tdq, rs, d->status, st));
+    return static_cast<int>(launch_bwd_dq(s, tq, tk, tv, tdo, tdq, dq32, rs, d->status, st));
   }
   if (deterministic == 2) {
     float* scratch = static_cast<float*>(workspace);
@@ -420,24 +449,38 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
       cudaError_t ce = launch_bwd_scores_wide(s, tq, tk, tv, tdo, rs, p_scratch, ds_scratch,
                                               d->status, st);
       if (ce != cudaSuccess) return static_cast<int>(ce);
-      if ((ce = launch_bwd_consume(s, 0, p_scratch, tdo, tdv, rs, d->status, st)) != cudaSuccess)
+      if ((ce = launch_bwd_consume(s, 0, p_scratch, tdo, tdv, dv32, rs, d->status, st)) != cudaSuccess)
         return static_cast<int>(ce);
-      if ((ce = launch_bwd_consume(s, 1, ds_scratch, tq, tdk, rs, d->status, st)) != cudaSuccess)
+      if ((ce = launch_bwd_consume(s, 1, ds_scratch, tq, tdk, dk32, rs, d->status, st)) != cudaSuccess)
         return static_cast<int>(ce);
-      return static_cast<int>(launch_bwd_consume(s, 2, ds_scratch, tk, tdq, rs, d->status, st));
+      return static_cast<int>(launch_bwd_consume(s, 2, ds_scratch, tk, tdq, dq32, rs, d->status, st));
     }
     cudaError_t ce =
-        launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, rs, scratch, 2, d->status, st);
+        launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, scratch, 2, d->status, st);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     record_mark_between(st);
-    return static_cast<int>(launch_bwd_consume(s, 2, scratch, tk, tdq, rs, d->status, st));
+    return static_cast<int>(launch_bwd_consume(s, 2, scratch, tk, tdq, dq32, rs, d->status, st));
   }
   float* dq_accum = static_cast<float*>(workspace);
   cudaError_t ce = cudaMemsetAsync(dq_accum, 0, fa2_bwd_workspace_bytes(B, H, N, D, 0), st);
   if (ce != cudaSuccess) return static_cast<int>(ce);
-  ce = launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, rs, dq_accum, 1, d->status, st);
+  ce = launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, dq_accum, 1, d->status, st);
   if (ce != cudaSuccess) return static_cast<int>(ce);
-  return static_cast<int>(launch_dq_convert(s, dq_accum, dq, sdq, st));
+  return static_cast<int>(launch_dq_convert(s, dq_accum, dq, sdq, dq32, st));
+}
+
+static int bwd_of_rowstats(const void* q, const void* k, const void* v, const void* dout,
+                           const float* rowstats, void* dq, void* dk, void* dv, void* workspace,
+                           size_t workspace_bytes, int B, int H, int N, int Nk, int D, int dtype,
+                           float scale, int deterministic, const long long* strides, bool grads_f32,
+                           fa2_stream_t stream) {
+  if (!rowstats) return FA2_ERR_NULL_POINTER;
+  if (int e = check_shape(B, H, N, D, dtype)) return e;
+  // the per-tile maxima of |dout| follow the last tile of the row statistics (fa2_bwd_preprocess)
+  const unsigned* tile_amax = reinterpret_cast<const unsigned*>(
+      rowstats + static_cast<size_t>(B) * H * ((N + 127) / 128) * 256);
+  return bwd_strided(q, k, v, dout, rowstats, tile_amax, dq, dk, dv, workspace, workspace_bytes, B,
+                     H, N, Nk, D, dtype, scale, deterministic, strides, grads_f32, stream);
 }
 
 int fa2_bwd_strided(const void* q, const void* k, const void* v, const void* dout,
@@ -445,13 +488,17 @@ int fa2_bwd_strided(const void* q, const void* k, const void* v, const void* dou
                     size_t workspace_bytes, int B, int H, int N, int Nk, int D, int dtype,
                     float scale, int deterministic, const long long* strides,
                     fa2_stream_t stream) {
-  if (!rowstats) return FA2_ERR_NULL_POINTER;
-  if (int e = check_shape(B, H, N, D, dtype)) return e;
-  // the per-tile maxima of |dout| follow the last tile of the row statistics (fa2_bwd_preprocess)
-  const unsigned* tile_amax = reinterpret_cast<const unsigned*>(
-      rowstats + static_cast<size_t>(B) * H * ((N + 127) / 128) * 256);
-  return bwd_strided(q, k, v, dout, rowstats, tile_amax, dq, dk, dv, workspace, workspace_bytes, B,
-                     H, N, Nk, D, dtype, scale, deterministic, strides, stream);
+  return bwd_of_rowstats(q, k, v, dout, rowstats, dq, dk, dv, workspace, workspace_bytes, B, H, N, Nk, D,
+                         dtype, scale, deterministic, strides, false, stream);
+}
+
+int fa2_bwd_strided_f32(const void* q, const void* k, const void* v, const void* dout,
+                        const float* rowstats, float* dq, float* dk, float* dv, void* workspace,
+                        size_t workspace_bytes, int B, int H, int N, int Nk, int D, int dtype,
+                        float scale, int deterministic, const long long* strides,
+                        fa2_stream_t stream) {
+  return bwd_of_rowstats(q, k, v, dout, rowstats, dq, dk, dv, workspace, workspace_bytes, B, H, N, Nk, D,
+                         dtype, scale, deterministic, strides, true, stream);
 }
 
 int fa2_bwd(const void* q, const void* k, const void* v, const void* dout, const float* rowstats,

@@ -62,6 +62,13 @@ struct Strides {
   long long b, h, n;
 };
 
+// An output written as fp32 straight from a kernel's accumulators (p == nullptr: the output is 16-bit
+// and goes through its tensor map).  Strides in elements, base 32-byte aligned.
+struct F32Out {
+  float* p;
+  Strides st;
+};
+
 // What the backward preprocess leaves for the backward kernels: the tile-blocked row statistics
 // and, one word per 128-row tile, the largest |dout| of the tile (16-bit pattern, sign cleared),
 // both indexed from the first (batch, head) problem of the launch.
@@ -131,7 +138,7 @@ __device__ __forceinline__ int fetch_work_item(unsigned int* work_counter, int t
 }
 
 cudaError_t launch_fwd(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
-                       const CUtensorMap& tv, const CUtensorMap& to, float* lse,
+                       const CUtensorMap& tv, const CUtensorMap& to, const F32Out& o32, float* lse,
                        const LaunchCtx& ctx, cudaStream_t stream);
 
 // rowstats[bh][t][0][r] = -lse * log2(e) (-inf for padded rows), rowstats[bh][t][1][r] = -delta;
@@ -149,8 +156,8 @@ cudaError_t launch_bwd_preprocess(const AttnShape& s, const void* o, const Strid
 // per head KV tile by KV tile, see dstile_pairs), from which launch_bwd_consume (form 2) forms dQ.
 cudaError_t launch_bwd_dkdv(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                             const CUtensorMap& tv, const CUtensorMap& tdo,
-                            const CUtensorMap& tdk, const CUtensorMap& tdv,
-                            const RowStats& rowstats, float* dq_accum, int mode, int* status,
+                            const CUtensorMap& tdk, const CUtensorMap& tdv, const F32Out& dk32,
+                            const F32Out& dv32, const RowStats& rowstats, float* dq_accum, int mode, int* status,
                             cudaStream_t stream);
 
 // Head dim 256: P^T and dS^T of every (KV tile, Q tile) pair as 16-bit piece-major tiles into two
@@ -167,8 +174,8 @@ cudaError_t launch_bwd_scores_wide(const AttnShape& s, const CUtensorMap& tq, co
 //   form 0: dV(jt) = sum_i P(jt, i)^T dO_i   (scratch = P tiles,  tb = dO, tout = dV)  head dim 256
 //   form 1: dK(jt) = sum_i dS(jt, i)^T Q_i   (scratch = dS tiles, tb = Q,  tout = dK)  head dim 256
 cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch,
-                               const CUtensorMap& tb, const CUtensorMap& tout, const RowStats& rowstats,
-                               int* status, cudaStream_t stream);
+                               const CUtensorMap& tb, const CUtensorMap& tout, const F32Out& out32,
+                               const RowStats& rowstats, int* status, cudaStream_t stream);
 
 // (KV tile, Q tile) pairs of one head: KV tile t < nktiles meets Q tiles t .. ntiles-1.
 inline long long dstile_pairs(int N, int Nk) {
@@ -179,11 +186,11 @@ inline long long dstile_pairs(int N, int Nk) {
 // dQ per Q tile, ascending KV order (deterministic path).
 cudaError_t launch_bwd_dq(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                           const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
-                          const RowStats& rowstats, int* status, cudaStream_t stream);
+                          const F32Out& dq32, const RowStats& rowstats, int* status, cudaStream_t stream);
 
-// dq = convert(dq_accum) (non-deterministic path).
+// dq = convert(dq_accum) (non-deterministic path); into dq32 when that is given.
 cudaError_t launch_dq_convert(const AttnShape& s, const float* dq_accum, void* dq,
-                              const Strides& sdq, cudaStream_t stream);
+                              const Strides& sdq, const F32Out& dq32, cudaStream_t stream);
 
 // One CTA whose waits run into the time limit on purpose (nothing ever arrives); it must end
 // by itself with the status word set.

@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
 // (the layout the fused backward kernel accumulates into).
 template <int D, bool BF16>
 __global__ void __launch_bounds__(256)
-    dq_convert_kernel(const float4* __restrict__ acc, uint4* __restrict__ dq, int N, int ntiles,
+    dq_convert_kernel(const float4* __restrict__ acc, uint4* __restrict__ dq, F32Out dq32, int N, int ntiles,
                       long long total, int d8, int H, Strides sdq) {
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= total) return;
@@ -353,12 +353,17 @@ __global__ void __launch_bounds__(256)
   const long long blk = (tile_global * 4 + w) * (D / 4);  // in units of [32 lanes][float4]
   const float4 x = acc[(blk + 2 * k8) * 32 + lane];
   const float4 y = acc[(blk + 2 * k8 + 1) * 32 + lane];
+  const long long bb = bh / H, hh = bh - bb * H;
+  if (dq32.p != nullptr) {
+    const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    st_global_8(dq32.p + bb * dq32.st.b + hh * dq32.st.h + row * dq32.st.n + k8 * 8, v);
+    return;
+  }
   uint4 r;
   r.x = pack2<BF16>(x.x, x.y);
   r.y = pack2<BF16>(x.z, x.w);
   r.z = pack2<BF16>(y.x, y.y);
   r.w = pack2<BF16>(y.z, y.w);
-  const long long bb = bh / H, hh = bh - bb * H;
   dq[bb * sdq.b + hh * sdq.h + row * sdq.n + k8] = r;  // strides in 16-byte units
 }
 
@@ -392,12 +397,12 @@ cudaError_t launch_pre_t(const AttnShape& s, const void* o, const Strides& so, c
 
 template <int D, bool BF16>
 cudaError_t launch_cvt_t(const AttnShape& s, const float* dq_accum, void* dq, const Strides& sdq,
-                         cudaStream_t stream) {
+                         const F32Out& dq32, cudaStream_t stream) {
   const int ntiles = (s.N + 127) / 128;
   const long long total = static_cast<long long>(s.B) * s.H * ntiles * 128 * (D / 8);
   const long long blocks = (total + 255) / 256;
   dq_convert_kernel<D, BF16><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
-      reinterpret_cast<const float4*>(dq_accum), static_cast<uint4*>(dq), s.N, ntiles, total,
+      reinterpret_cast<const float4*>(dq_accum), static_cast<uint4*>(dq), dq32, s.N, ntiles, total,
       s.Dg / 8, s.H, in_vec8(sdq));
   return cudaGetLastError();
 }
@@ -426,11 +431,11 @@ cudaError_t launch_bwd_preprocess(const AttnShape& s, const void* o, const Strid
 }
 
 cudaError_t launch_dq_convert(const AttnShape& s, const float* dq_accum, void* dq,
-                              const Strides& sdq, cudaStream_t stream) {
+                              const Strides& sdq, const F32Out& dq32, cudaStream_t stream) {
 #define FA2_CASE(DD)                                                        \
   case DD:                                                                  \
-    return s.dtype ? launch_cvt_t<DD, true>(s, dq_accum, dq, sdq, stream)   \
-                   : launch_cvt_t<DD, false>(s, dq_accum, dq, sdq, stream);
+    return s.dtype ? launch_cvt_t<DD, true>(s, dq_accum, dq, sdq, dq32, stream)   \
+                   : launch_cvt_t<DD, false>(s, dq_accum, dq, sdq, dq32, stream);
   switch (s.D) {
     FA2_CASE(32)
     FA2_CASE(64)

@@ -111,7 +111,7 @@ template <int D, bool BF16>
 __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtasPerSm)
     fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap to,
-               float* __restrict__ lse, int N, int Nk, int num_bh, int num_heads, int group,
+               const __grid_constant__ F32Out o32, int cols, float* __restrict__ lse, int N, int Nk, int num_bh, int num_heads, int group,
                float scale_log2, int* status, unsigned int* work_counter) {
   // Head dim 256 ("wide") runs on the staging and tensor-memory plan of head dim 128 with ONE
   // Q tile per work item: the two Q slots hold the two 128-column halves of that tile, K and V
@@ -456,6 +456,9 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
       // Stage the tile through the (now idle) Q buffer in the swizzled layout the output
       // tensor map expects; each warp stores its own 32 rows.
       uint8_t* sO = smem + C::kOffQ + wg * T::kTileBytes;
+      const int row = qt * 128 + r;
+      float* const dst32 =
+          o32.p != nullptr && row < N ? o32.p + hc.b * o32.st.b + hc.h * o32.st.h + row * o32.st.n : nullptr;
 #pragma unroll
       for (int c0 = 0; c0 < D; c0 += 32) {
         uint32_t orr[32];
@@ -476,6 +479,13 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
                               __uint_as_float(orr[8 * p + 7]) * inv_l);
           *reinterpret_cast<uint4*>(sO + chunk * T::kChunkTileBytes +
                                     swizzled_offset<DT>(r, piece0 + p)) = val;
+          // the unrounded row as well, for fp32 callers (see store_rows_f32 in bwd_roles.cuh)
+          if (dst32 != nullptr && c0 + 8 * p < cols) {
+            float x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = __uint_as_float(orr[8 * p + i]) * inv_l;
+            st_global_8(dst32 + c0 + 8 * p, x);
+          }
         }
       }
       fence_proxy_async_smem();
@@ -492,7 +502,6 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
           tma_store_wait_read();
         }
       }
-      const int row = qt * 128 + r;
       if (row < N)
         lse[static_cast<size_t>(bh) * N + row] = (m_run * scale_log2 + lg2(l_run)) * kLn2;
     }
@@ -511,7 +520,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
 
 template <int D, bool BF16>
 cudaError_t launch_fwd_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
-                         const CUtensorMap& tv, const CUtensorMap& to, float* lse,
+                         const CUtensorMap& tv, const CUtensorMap& to, const F32Out& o32, float* lse,
                          const LaunchCtx& ctx, cudaStream_t stream) {
   using C = FwdCfg<D == 256 ? 128 : D>;  // head dim 256 runs on the plan of head dim 128
   auto kern = fwd_kernel<D, BF16>;
@@ -524,7 +533,7 @@ cudaError_t launch_fwd_t(const AttnShape& s, const CUtensorMap& tq, const CUtens
   const long long slots = static_cast<long long>(ctx.num_sms) * C::kCtasPerSm;
   const unsigned grid = static_cast<unsigned>(items < slots ? items : slots);
   const float scale_log2 = s.scale * 1.4426950408889634f;
-  kern<<<grid, kFwdThreads, C::kSmemBytes, stream>>>(tq, tk, tv, to, lse, s.N, s.Nk, s.B * s.H, s.H,
+  kern<<<grid, kFwdThreads, C::kSmemBytes, stream>>>(tq, tk, tv, to, o32, s.Dg, lse, s.N, s.Nk, s.B * s.H, s.H,
                                                      heads_per_group(s), scale_log2, ctx.status,
                                                      ctx.work_counter);
   return cudaGetLastError();
@@ -533,12 +542,12 @@ cudaError_t launch_fwd_t(const AttnShape& s, const CUtensorMap& tq, const CUtens
 }  // namespace
 
 cudaError_t launch_fwd(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
-                       const CUtensorMap& tv, const CUtensorMap& to, float* lse,
+                       const CUtensorMap& tv, const CUtensorMap& to, const F32Out& o32, float* lse,
                        const LaunchCtx& ctx, cudaStream_t stream) {
 #define FA2_CASE(DD)                                                                 \
   case DD:                                                                           \
-    return s.dtype ? launch_fwd_t<DD, true>(s, tq, tk, tv, to, lse, ctx, stream)     \
-                   : launch_fwd_t<DD, false>(s, tq, tk, tv, to, lse, ctx, stream);
+    return s.dtype ? launch_fwd_t<DD, true>(s, tq, tk, tv, to, o32, lse, ctx, stream)     \
+                   : launch_fwd_t<DD, false>(s, tq, tk, tv, to, o32, lse, ctx, stream);
   switch (s.D) {
     FA2_CASE(32)
     FA2_CASE(64)

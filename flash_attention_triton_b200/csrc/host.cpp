@@ -50,16 +50,17 @@ bool tensors(PyObject* const* args, int n) {
   return true;
 }
 
-// forward(q, k, v, scale) -> (code, output, lse).  Shapes, devices and dtypes are the caller's
-// business; a non-zero code is that of fa2_fwd_strided.
+// forward(q, k, v, scale, f32) -> (code, output, lse, fp32 output or None).  Shapes, devices and
+// dtypes are the caller's business; a non-zero code is that of fa2_fwd_strided / fa2_fwd_strided_f32.
 PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 4) return PyErr_Format(PyExc_TypeError, "forward takes 4 arguments");
+  if (nargs != 5) return PyErr_Format(PyExc_TypeError, "forward takes 5 arguments");
   if (!tensors(args, 3)) return nullptr;
   const double scale = PyFloat_AsDouble(args[3]);
   if (scale == -1.0 && PyErr_Occurred()) return nullptr;
+  const bool f32 = args[4] == Py_True;
   at::Tensor q = THPVariable_Unpack(args[0]), k = THPVariable_Unpack(args[1]), v = THPVariable_Unpack(args[2]);
-  at::Tensor output, lse;
+  at::Tensor output, lse, output32;
   int code;
   {
     pybind11::gil_scoped_release no_gil;
@@ -67,13 +68,18 @@ PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     output = at::empty(q.sizes(), q.options().memory_format(at::MemoryFormat::Contiguous));
     lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
     const c10::cuda::CUDAGuard guard(q.device());
-    const StrideArray<4> strides({&q, &k, &v, &output});
-    code = fa2_fwd_strided(q.data_ptr(), k.data_ptr(), v.data_ptr(), output.data_ptr(), lse.data_ptr<float>(),
-                           q.size(0), q.size(1), q.size(2), k.size(2), q.size(3), dtype_code(q),
-                           static_cast<float>(scale), strides.v,
-                           c10::cuda::getCurrentCUDAStream(q.device().index()).stream());
+    if (f32) output32 = at::empty(q.sizes(), output.options().dtype(at::kFloat));
+    const StrideArray<5> strides({&q, &k, &v, &output, f32 ? &output32 : &output});
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+    const int b = q.size(0), h = q.size(1), n = q.size(2), nk = k.size(2), d = q.size(3);
+    code = f32 ? fa2_fwd_strided_f32(q.data_ptr(), k.data_ptr(), v.data_ptr(), output.data_ptr(),
+                                     output32.data_ptr<float>(), lse.data_ptr<float>(), b, h, n, nk, d,
+                                     dtype_code(q), static_cast<float>(scale), strides.v, stream)
+               : fa2_fwd_strided(q.data_ptr(), k.data_ptr(), v.data_ptr(), output.data_ptr(),
+                                 lse.data_ptr<float>(), b, h, n, nk, d, dtype_code(q),
+                                 static_cast<float>(scale), strides.v, stream);
   }
-  return Py_BuildValue("iNN", code, THPVariable_Wrap(output), THPVariable_Wrap(lse));
+  return Py_BuildValue("iNNN", code, THPVariable_Wrap(output), THPVariable_Wrap(lse), THPVariable_Wrap(output32));
   END_HANDLE_TH_ERRORS
 }
 
@@ -101,21 +107,23 @@ PyObject* preprocess(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// gradients(q, k, v) -> dense uninitialised (dq, dk, dv)
+// gradients(q, k, v, f32) -> dense uninitialised (dq, dk, dv), fp32 or in the dtype of q, k, v
 PyObject* gradients(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 3) return PyErr_Format(PyExc_TypeError, "gradients takes 3 arguments");
+  if (nargs != 4) return PyErr_Format(PyExc_TypeError, "gradients takes 4 arguments");
   if (!tensors(args, 3)) return nullptr;
   at::Tensor d[3];
   for (int i = 0; i < 3; ++i) {
     const at::Tensor& t = THPVariable_Unpack(args[i]);
-    d[i] = at::empty(t.sizes(), t.options().memory_format(at::MemoryFormat::Contiguous));
+    const auto options = t.options().memory_format(at::MemoryFormat::Contiguous);
+    d[i] = at::empty(t.sizes(), args[3] == Py_True ? options.dtype(at::kFloat) : options);
   }
   return Py_BuildValue("NNN", THPVariable_Wrap(d[0]), THPVariable_Wrap(d[1]), THPVariable_Wrap(d[2]));
   END_HANDLE_TH_ERRORS
 }
 
-// backward(q, k, v, d_output, dq, dk, dv, rowstats, workspace or None, scale, mode) -> code
+// backward(q, k, v, d_output, dq, dk, dv, rowstats, workspace or None, scale, mode) -> code; dq, dk
+// and dv all in the dtype of q, or all fp32
 PyObject* backward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   if (nargs != 11) return PyErr_Format(PyExc_TypeError, "backward takes 11 arguments");
@@ -129,6 +137,10 @@ PyObject* backward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   for (int i = 0; i < 7; ++i) t[i] = THPVariable_Unpack(args[i]);
   const at::Tensor rowstats = THPVariable_Unpack(args[7]);
   const at::Tensor workspace = args[8] == Py_None ? at::Tensor() : THPVariable_Unpack(args[8]);
+  const bool f32 = t[4].scalar_type() == at::kFloat;
+  for (int i = 4; i < 7; ++i)
+    if (t[i].scalar_type() != (f32 ? at::kFloat : t[0].scalar_type()))
+      return PyErr_Format(PyExc_TypeError, "dq, dk and dv must be all fp32 or all of the dtype of q");
   int code;
   {
     pybind11::gil_scoped_release no_gil;
@@ -136,13 +148,18 @@ PyObject* backward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const at::Tensor& q = t[0];
     const c10::cuda::CUDAGuard guard(q.device());
     const StrideArray<7> strides({&t[0], &t[1], &t[2], &t[3], &t[4], &t[5], &t[6]});
-    code = fa2_bwd_strided(q.data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(),
-                           rowstats.data_ptr<float>(), t[4].data_ptr(), t[5].data_ptr(), t[6].data_ptr(),
-                           workspace.defined() ? workspace.data_ptr() : nullptr,
-                           workspace.defined() ? workspace.nbytes() : 0, q.size(0), q.size(1), q.size(2),
-                           t[1].size(2), q.size(3), dtype_code(q), static_cast<float>(scale),
-                           static_cast<int>(mode), strides.v,
-                           c10::cuda::getCurrentCUDAStream(q.device().index()).stream());
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+    void* ws = workspace.defined() ? workspace.data_ptr() : nullptr;
+    const size_t ws_bytes = workspace.defined() ? workspace.nbytes() : 0;
+    const int b = q.size(0), h = q.size(1), n = q.size(2), nk = t[1].size(2), d = q.size(3);
+    code = f32 ? fa2_bwd_strided_f32(q.data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(),
+                                     rowstats.data_ptr<float>(), t[4].data_ptr<float>(), t[5].data_ptr<float>(),
+                                     t[6].data_ptr<float>(), ws, ws_bytes, b, h, n, nk, d, dtype_code(q),
+                                     static_cast<float>(scale), static_cast<int>(mode), strides.v, stream)
+               : fa2_bwd_strided(q.data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(),
+                                 rowstats.data_ptr<float>(), t[4].data_ptr(), t[5].data_ptr(), t[6].data_ptr(),
+                                 ws, ws_bytes, b, h, n, nk, d, dtype_code(q), static_cast<float>(scale),
+                                 static_cast<int>(mode), strides.v, stream);
   }
   return PyLong_FromLong(code);
   END_HANDLE_TH_ERRORS

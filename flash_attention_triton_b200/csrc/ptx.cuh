@@ -14,6 +14,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 }
 
 // ----------------------------------------------------------------------------------------
+// 32 bytes to global memory (32-byte aligned): a whole L2 sector from one thread.
+// ----------------------------------------------------------------------------------------
+__device__ __forceinline__ void st_global_8(float* p, const float (&v)[8]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]),
+               "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
+// ----------------------------------------------------------------------------------------
 // Bounded waits.  No wait in this library spins forever: after kWaitLimitCycles a waiter
 // raises the CTA-wide abort flag and records where it gave up in the device status word;
 // every other waiter of the CTA sees the flag and leaves too, the CTA drains and frees its

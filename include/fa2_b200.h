@@ -178,6 +178,23 @@ int fa2_bwd_strided(const void* q, const void* k, const void* v, const void* dou
                     int deterministic, const long long* strides, fa2_stream_t stream);
 
 /*
+ * For callers whose tensors are fp32 and who cast q, k, v and dout to 16 bits: the results written as
+ * fp32 from the kernels' accumulators, unrounded, instead of 16-bit results that the caller casts
+ * back.  fa2_fwd_strided_f32 writes the output twice, 16-bit to `o` (fa2_bwd_preprocess reads it) and
+ * fp32 to `o32` (strides: q, k, v, o, o32, 15 values); fa2_bwd_strided_f32 writes dq, dk and dv as
+ * fp32 only.  Strides of fp32 tensors count fp32 elements; their bases must be 32-byte aligned
+ * (FA2_ERR_MISALIGNED).  Everything else is as for the entry points above.
+ */
+int fa2_fwd_strided_f32(const void* q, const void* k, const void* v, void* o, float* o32, float* lse,
+                        int B, int H, int N, int Nk, int D, int dtype, float scale,
+                        const long long* strides, fa2_stream_t stream);
+int fa2_bwd_strided_f32(const void* q, const void* k, const void* v, const void* dout,
+                        const float* rowstats,
+                        float* dq, float* dk, float* dv, void* workspace, size_t workspace_bytes,
+                        int B, int H, int N, int Nk, int D, int dtype, float scale,
+                        int deterministic, const long long* strides, fa2_stream_t stream);
+
+/*
  * Diagnostics for benchmarks: the next fa2_bwd call of the calling thread that runs two kernels
  * (deterministic == 1: dK/dV kernel, dQ kernel; deterministic == 2 at D <= 128: dK/dV kernel,
  * dQ consumer kernel; the first chunk when the call is chunked) records `event`, a cudaEvent_t, on

@@ -151,6 +151,42 @@ def test_narrow_heads_at_the_edges_of_64_row_steps(nq, nk, d, dtype, mode, monke
     check_against(naive_attention(q, k, v, do), run_api(q, k, v, do, None, mode != "atomic"), dtype)
 
 
+@pytest.mark.parametrize("mode", ["spill", "recompute", "atomic"])
+@pytest.mark.parametrize("d", [8, 32, 40, 64, 96, 128, 192, 256])
+def test_fp32_results_are_the_unrounded_16_bit_ones(d, mode, monkeypatch):
+    """fp32 tensors are computed in fp16 and come back as fp32 straight from the accumulators:
+    rounding them gives the bits of the same call on fp16 tensors (dq of the atomic mode, whose
+    summation order is free, to rounding).  Ragged and tiny lengths, fewer and more keys than
+    queries, strided inputs, several chunks of the spill mode."""
+    monkeypatch.setenv("FA2_B200_BWD_MODE", mode)
+    lib = _lib.lib()
+    previous = lib.fa2_set_spill_budget(4 << 20)
+    try:
+        for nq, nk, strided in ((1, 1, False), (200, 200, True), (257, 129, False), (128, 300, False)):
+            g = torch.Generator(device=DEV).manual_seed(d + nq)
+            shape = lambda n: (2, n, 3, d) if strided else (2, 3, n, d)
+            q, k, v, do = (torch.randn(shape(n), device=DEV, generator=g).half() for n in (nq, nk, nk, nq))
+            if strided:
+                q, k, v, do = (t.transpose(1, 2) for t in (q, k, v, do))
+            want_leaves = [t.detach().requires_grad_(True) for t in (q, k, v)]
+            got_leaves = [t.detach().float().requires_grad_(True) for t in (q, k, v)]
+            want = flash_attention_v2(*want_leaves)
+            got = flash_attention_v2(*got_leaves)
+            assert got.dtype == torch.float32 and torch.equal(got.half(), want)
+            want_grads = torch.autograd.grad(want, want_leaves, do)
+            got_grads = torch.autograd.grad(got, got_leaves, do.float())
+            for name, a, b in zip(("dq", "dk", "dv"), got_grads, want_grads):
+                assert a.dtype == torch.float32
+                if name == "dq" and mode == "atomic" and d <= 128:
+                    # one ulp of fp16 at most between two summation orders in fp32
+                    assert ((a - b.float()).abs() <= 2e-3 * b.float().abs() + 1e-5).all()
+                else:
+                    assert torch.equal(a.half(), b), (name, nq, nk)
+    finally:
+        lib.fa2_set_spill_budget(previous)
+    assert _lib.device_status() == 0
+
+
 def test_spill_mode_chunks_change_no_bit(monkeypatch):
     """With a scratch bound of 3 MiB the spill mode works through [3, 5, 700, 64] (0.7 MiB per
     head) in chunks of 3 + 2 heads per batch entry; with 8 MiB in chunks of 2 + 1 batch

@@ -152,8 +152,8 @@ def test_native_host_path_refuses_what_is_not_a_tensor():
     from flash_attention_triton_b200 import _lib
 
     t = torch.zeros(1, 1, 8, 8, dtype=torch.float16)
-    for call in (lambda h: h.forward(t, t, None, 0.1), lambda h: h.forward(t, t, t), lambda h: h.forward(t, t, t, "x"),
-                 lambda h: h.gradients(t, 1, t), lambda h: h.preprocess(t, t[0, 0], t), lambda h: h.readable_in_place(2),
+    for call in (lambda h: h.forward(t, t, None, 0.1, False), lambda h: h.forward(t, t, t),
+                 lambda h: h.forward(t, t, t, "x", False), lambda h: h.gradients(t, 1, t, False), lambda h: h.preprocess(t, t[0, 0], t), lambda h: h.readable_in_place(2),
                  lambda h: h.backward(*([t] * 7), None, None, 0.1, 0), lambda h: h.backward(t)):
         with pytest.raises(TypeError):
             call(_lib.host())
