@@ -504,6 +504,172 @@ __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, 1)
 }
 
 // =========================================================================================
+// The same for two adjacent output tiles of head dim 256 per CTA.  One tile per CTA reads 32 KiB of
+// scratch and 64 KiB of operand for every 1024 cycles of tensor work, and the L2 cannot deliver 96 KiB
+// an SM in that time (2 000 - 2 175 cycles measured); two tiles share the operand, 64 KiB a product,
+// and come close to what reading the scratch from HBM takes.  Both accumulators fill the tensor
+// memory.  Shared memory: a ring of two stages of both scratch tiles (64 KiB each) and a ring of three
+// half operand tiles (64 reduction rows, 32 KiB each).  Every output tile adds the same products in the
+// same order as above, so the two kernels give the same bits.
+// warps 0-3 and 4-7 epilogue of the first and the second tile, warp 8 producer, warp 9 MMA issue.
+// Measured on the whole backward of [2,16,8192,256] bf16: 3517 -> 3015 us.
+// =========================================================================================
+struct ConsumePairCfg {
+  using T = Tile<256>;
+  static constexpr int kThreads = 320;
+  static constexpr int kLoadWarp = 8;
+  static constexpr int kMmaWarp = 9;
+  static constexpr int kAStages = 2, kAStageBytes = 2 * 32768;
+  static constexpr int kBStages = 3, kBStageBytes = T::kTileBytes / 2;
+  static constexpr int kOffA = 0;
+  static constexpr int kOffB = kAStages * kAStageBytes;
+  static constexpr int kOffBar = kOffB + kBStages * kBStageBytes;
+  static constexpr int kBarAFull = 0;
+  static constexpr int kBarAEmpty = kBarAFull + kAStages;
+  static constexpr int kBarBFull = kBarAEmpty + kAStages;
+  static constexpr int kBarBEmpty = kBarBFull + kBStages;
+  static constexpr int kBarDone = kBarBEmpty + kBStages;
+  static constexpr int kNumBars = kBarDone + 1;
+  static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;
+  static_assert(kSmemBytes <= 232448, "shared memory budget of one CTA");
+  static_assert(kAStages * kAStageBytes >= 2 * T::kTileBytes, "the scratch ring stages both outputs at the end");
+};
+
+template <bool BF16, int FORM>
+__global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
+    bwd_consume_pair_kernel(const uint4* __restrict__ scratch, const __grid_constant__ CUtensorMap tb,
+                            const __grid_constant__ CUtensorMap tout, const __grid_constant__ F32Out out32,
+                            int cols, const unsigned* __restrict__ tile_amax, int N, int Nk, int num_bh,
+                            int num_heads, int group, int* status) {
+  using C = ConsumePairCfg;
+  using T = Tile<256>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t smem_base = smem_u32(smem);
+  if (smem_base & 1023u) {
+    if (threadIdx.x == 0) atomicCAS(status, 0, 0x20000 | kBSiteAlign);
+    return;
+  }
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kOffBar);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::kNumBars);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  auto bar = [&](int i) { return smem_base + C::kOffBar + 8u * i; };
+
+  const int ntiles = (N + 127) >> 7;    // Q tiles
+  const int nktiles = (Nk + 127) >> 7;  // KV tiles
+  const int out_tiles = FORM == 2 ? ntiles : nktiles;
+  const int out_rows = FORM == 2 ? N : Nk;
+  const int npairs = (out_tiles + 1) >> 1;
+  const HeadTile ht = grouped_order(blockIdx.x, num_bh, npairs, group);
+  const int bh = ht.bh;
+  const HeadCoord hc{bh % num_heads, bh / num_heads};
+  const size_t head_tile0 = static_cast<size_t>(bh) * dstile_count(ntiles, nktiles);
+  // the last Q tiles (form 2) and the first KV tiles (forms 0, 1) are summed over the most tiles
+  const int ot0 = 2 * (FORM == 2 ? npairs - 1 - ht.rank : ht.rank);
+  // Range of tiles of the other kind each output tile is summed over: [begin, end).  Both start at 0
+  // (form 2) or both end at ntiles (forms 0, 1); a missing second tile has an empty range.
+  int begin[2], end[2];
+#pragma unroll
+  for (int o = 0; o < 2; ++o) {
+    const int ot = ot0 + o;
+    begin[o] = FORM == 2 ? 0 : ot;
+    end[o] = ot >= out_tiles ? begin[o] : (FORM == 2 ? min(ot + 1, nktiles) : ntiles);
+  }
+  const int first = begin[0], last = max(end[0], end[1]);
+  auto wanted = [&](int o, int x) { return x >= begin[o] && x < end[o]; };
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < C::kNumBars; ++i) mbar_init(bar(i), 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    fence_proxy_async_smem();
+  }
+  if (warp == C::kMmaWarp) {
+    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const WaitCtx w{abort_flag, status};
+
+  if (warp == C::kLoadWarp) {
+    const uint32_t elected = elect_one();
+    if (elected) prefetch_tensormap(&tb);
+    bool ok = true;
+    for (int x = first, n = 0; ok && x < last; ++x, ++n) {
+      const int st = n % C::kAStages, ph = (n / C::kAStages) & 1;
+      if (!(ok = mbar_wait_warp(bar(C::kBarAEmpty + st), ph ^ 1, w, kBSiteLoadQ))) break;
+      if (elected) {
+        mbar_arrive_expect_tx(bar(C::kBarAFull + st), 32768u * (wanted(0, x) + wanted(1, x)));
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+          if (!wanted(o, x)) continue;
+          const int jt = FORM == 2 ? x : ot0 + o, qt = FORM == 2 ? ot0 + o : x;
+          const size_t tile = head_tile0 + dstile_count(ntiles, jt) + (qt - jt);
+          bulk_load_1d(smem_base + C::kOffA + st * C::kAStageBytes + o * 32768, scratch + tile * 2048, 32768,
+                       bar(C::kBarAFull + st));
+        }
+      }
+      for (int half = 0; half < 2; ++half) {
+        const int m = 2 * n + half, bs = m % C::kBStages, bph = (m / C::kBStages) & 1;
+        if (!(ok = mbar_wait_warp(bar(C::kBarBEmpty + bs), bph ^ 1, w, kBSiteLoadDO))) break;
+        if (elected) {
+          mbar_arrive_expect_tx(bar(C::kBarBFull + bs), C::kBStageBytes);
+#pragma unroll
+          for (int ch = 0; ch < T::kChunks; ++ch)
+            tma_load_4d(smem_base + C::kOffB + bs * C::kBStageBytes + ch * (C::kBStageBytes / T::kChunks), &tb,
+                        ch * T::kChunkElems, x * 128 + half * 64, hc, bar(C::kBarBFull + bs));
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == C::kMmaWarp) {
+    const uint32_t elected = elect_one();
+    bool ok = true;
+    for (int x = first, n = 0; ok && x < last; ++x, ++n) {
+      const int st = n % C::kAStages, ph = (n / C::kAStages) & 1;
+      if (!(ok = mbar_wait(bar(C::kBarAFull + st), ph, w, kBSiteMmaKV))) break;
+      for (int half = 0; half < 2; ++half) {
+        const int m = 2 * n + half, bs = m % C::kBStages, bph = (m / C::kBStages) & 1;
+        if (!(ok = mbar_wait(bar(C::kBarBFull + bs), bph, w, kBSiteMmaQ))) break;
+#pragma unroll
+        for (int o = 0; o < 2; ++o)
+          if (wanted(o, x))
+            issue_pieces_x_half_tile<256, BF16, FORM == 2>(
+                elected, tmem_base + o * 256, smem_base + C::kOffA + st * C::kAStageBytes + o * 32768, half,
+                smem_base + C::kOffB + bs * C::kBStageBytes, half > 0 || x > begin[o]);
+        if (elected) mma_commit(bar(C::kBarBEmpty + bs));
+      }
+      if (ok && elected) mma_commit(bar(C::kBarAEmpty + st));
+    }
+    if (ok && elected) mma_commit(bar(C::kBarDone));
+    __syncwarp();
+  } else {
+    const int o = warp >> 2, w4 = warp & 3, ot = ot0 + o;
+    float inv_dscale = 1.0f;  // dS tiles carry the head's power-of-two factor (head_dscale); P tiles do not
+    if (FORM != 0) head_dscale<BF16>(tile_amax + static_cast<size_t>(bh) * ntiles, ntiles, lane, &inv_dscale);
+    if (mbar_wait_warp(bar(C::kBarDone), 0, w, kBSiteCmpDone) && ot < out_tiles) {
+      tc_fence_after();
+      const uint32_t acc = tmem_base + o * 256 + (static_cast<uint32_t>(w4 * 32) << 16);
+      if (out32.p != nullptr)
+        store_rows_f32<256>(acc, out32, cols, ot * 128 + w4 * 32 + lane, hc, out_rows, inv_dscale);
+      else  // every product has completed, so the scratch ring is idle
+        store_rows_16bit<256, BF16>(acc, smem + C::kOffA + o * T::kTileBytes, w4, lane, &tout, ot * 128, hc,
+                                    out_rows, inv_dscale);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == C::kMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// =========================================================================================
 // Head dim 256: scores only.  dK and dV alone would fill the 512 tensor-memory columns, so the
 // backward is split: this kernel forms P^T and dS^T for every (KV tile, Q tile) pair and writes
 // both as 16-bit piece-major tiles to two scratch tensors; bwd_consume_kernel then forms dV, dK
@@ -823,6 +989,22 @@ cudaError_t launch_consume_t(const AttnShape& s, const void* scratch, const CUte
   return cudaGetLastError();
 }
 
+template <bool BF16, int FORM>
+cudaError_t launch_consume_pair_t(const AttnShape& s, const void* scratch, const CUtensorMap& tb,
+                                  const CUtensorMap& tout, const F32Out& out32, const RowStats& rowstats,
+                                  int* status, cudaStream_t stream) {
+  using C = ConsumePairCfg;
+  auto kern = bwd_consume_pair_kernel<BF16, FORM>;
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  const unsigned out_tiles = static_cast<unsigned>(((FORM == 2 ? s.N : s.Nk) + 127) / 128);
+  kern<<<(out_tiles + 1) / 2 * s.B * s.H, C::kThreads, C::kSmemBytes, stream>>>(
+      static_cast<const uint4*>(scratch), tb, tout, out32, s.Dg, rowstats.tile_amax, s.N, s.Nk, s.B * s.H, s.H,
+      heads_per_group(s), status);
+  return cudaGetLastError();
+}
+
 template <int D, bool BF16>
 cudaError_t launch_dq_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                         const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
@@ -899,19 +1081,19 @@ cudaError_t launch_bwd_scores_wide(const AttnShape& s, const CUtensorMap& tq, co
 
 cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch,
                                const CUtensorMap& tb, const CUtensorMap& tout, const F32Out& out32,
-                               const RowStats& rowstats, int* status, cudaStream_t stream) {
+                               const RowStats& rowstats, bool two_tiles, int* status, cudaStream_t stream) {
 #define FA2_ARGS s, scratch, tb, tout, out32, rowstats, status, stream
 #define FA2_CASE(DD)                                                      \
   case DD:                                                                \
     return s.dtype ? launch_consume_t<DD, true, 2>(FA2_ARGS)              \
                    : launch_consume_t<DD, false, 2>(FA2_ARGS);
-  if (s.D == 256) {
-    if (form == 0)
-      return s.dtype ? launch_consume_t<256, true, 0>(FA2_ARGS) : launch_consume_t<256, false, 0>(FA2_ARGS);
-    if (form == 1)
-      return s.dtype ? launch_consume_t<256, true, 1>(FA2_ARGS) : launch_consume_t<256, false, 1>(FA2_ARGS);
-    return s.dtype ? launch_consume_t<256, true, 2>(FA2_ARGS) : launch_consume_t<256, false, 2>(FA2_ARGS);
-  }
+#define FA2_WIDE(FORM)                                                                        \
+  (two_tiles ? (s.dtype ? launch_consume_pair_t<true, FORM>(FA2_ARGS)                         \
+                        : launch_consume_pair_t<false, FORM>(FA2_ARGS))                       \
+             : (s.dtype ? launch_consume_t<256, true, FORM>(FA2_ARGS)                         \
+                        : launch_consume_t<256, false, FORM>(FA2_ARGS)))
+  if (s.D == 256) return form == 0 ? FA2_WIDE(0) : (form == 1 ? FA2_WIDE(1) : FA2_WIDE(2));
+#undef FA2_WIDE
   if (form != 2) return cudaErrorInvalidValue;
   switch (s.D) {
     FA2_CASE(32)

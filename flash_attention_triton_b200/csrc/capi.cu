@@ -449,17 +449,23 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
       cudaError_t ce = launch_bwd_scores_wide(s, tq, tk, tv, tdo, rs, p_scratch, ds_scratch,
                                               d->status, st);
       if (ce != cudaSuccess) return static_cast<int>(ce);
-      if ((ce = launch_bwd_consume(s, 0, p_scratch, tdo, tdv, dv32, rs, d->status, st)) != cudaSuccess)
+      const bool two = consume_two_tiles(s, d->num_sms);
+      if (two) {  // operands in half tiles
+        if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, 64)) return e;
+        if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, 64)) return e;
+        if (int e = make_map_of(&tdo, dout, strides, 3, dtype, B, H, N, D, 64)) return e;
+      }
+      if ((ce = launch_bwd_consume(s, 0, p_scratch, tdo, tdv, dv32, rs, two, d->status, st)) != cudaSuccess)
         return static_cast<int>(ce);
-      if ((ce = launch_bwd_consume(s, 1, ds_scratch, tq, tdk, dk32, rs, d->status, st)) != cudaSuccess)
+      if ((ce = launch_bwd_consume(s, 1, ds_scratch, tq, tdk, dk32, rs, two, d->status, st)) != cudaSuccess)
         return static_cast<int>(ce);
-      return static_cast<int>(launch_bwd_consume(s, 2, ds_scratch, tk, tdq, dq32, rs, d->status, st));
+      return static_cast<int>(launch_bwd_consume(s, 2, ds_scratch, tk, tdq, dq32, rs, two, d->status, st));
     }
     cudaError_t ce =
         launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, scratch, 2, d->status, st);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     record_mark_between(st);
-    return static_cast<int>(launch_bwd_consume(s, 2, scratch, tk, tdq, dq32, rs, d->status, st));
+    return static_cast<int>(launch_bwd_consume(s, 2, scratch, tk, tdq, dq32, rs, false, d->status, st));
   }
   float* dq_accum = static_cast<float*>(workspace);
   cudaError_t ce = cudaMemsetAsync(dq_accum, 0, fa2_bwd_workspace_bytes(B, H, N, D, 0), st);

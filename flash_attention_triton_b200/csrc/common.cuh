@@ -173,9 +173,20 @@ cudaError_t launch_bwd_scores_wide(const AttnShape& s, const CUtensorMap& tq, co
 //   form 2: dQ(qt) = sum_j dS(j, qt) K_j     (scratch = dS tiles, tb = K, tout = dQ)
 //   form 0: dV(jt) = sum_i P(jt, i)^T dO_i   (scratch = P tiles,  tb = dO, tout = dV)  head dim 256
 //   form 1: dK(jt) = sum_i dS(jt, i)^T Q_i   (scratch = dS tiles, tb = Q,  tout = dK)  head dim 256
+// At head dim 256, with two_tiles, a CTA forms two adjacent output tiles (tb then has boxes of 64 rows).
 cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch,
                                const CUtensorMap& tb, const CUtensorMap& tout, const F32Out& out32,
-                               const RowStats& rowstats, int* status, cudaStream_t stream);
+                               const RowStats& rowstats, bool two_tiles, int* status, cudaStream_t stream);
+
+// Whether the consumers of head dim 256 take two output tiles per CTA: when there are CTAs for one and a
+// half times the SMs.  Fewer, longer CTAs leave SMs idle.  Whole bf16 backward, microseconds, one tile
+// against two: 1024 pairs [2,16,8192,256] 3517 / 3015, 256 pairs
+// [1,16,4096,256] 506 / 456 and [1,32,2048,256] 312 / 283; 128 pairs [1,4,8192,256] 460 / 552, 64 pairs
+// [1,8,2048,256] 124 / 142.
+inline bool consume_two_tiles(const AttnShape& s, int num_sms) {
+  const long long tiles = (s.Nk + 127) / 128;
+  return s.D == 256 && 2 * ((tiles + 1) / 2 * s.B * s.H) >= 3ll * num_sms;
+}
 
 // (KV tile, Q tile) pairs of one head: KV tile t < nktiles meets Q tiles t .. ntiles-1.
 inline long long dstile_pairs(int N, int Nk) {

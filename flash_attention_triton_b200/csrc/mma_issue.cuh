@@ -136,4 +136,24 @@ __device__ __forceinline__ void issue_pieces_x_tile(uint32_t elected, uint32_t d
              k > 0 ? 1u : accumulate);
 }
 
+// Half of either product above: the four 16-row reduction steps of half `half` of the piece-major tile,
+// against a staged [64, D] half tile of the operand.  TRANSPOSED selects issue_piecesT_x_tile's use
+// of A.
+template <int D, bool BF16, bool TRANSPOSED>
+__device__ __forceinline__ void issue_pieces_x_half_tile(uint32_t elected, uint32_t d_tmem, uint32_t a_addr,
+                                                         int half, uint32_t b_addr, uint32_t accumulate) {
+  using T = Tile<D>;
+  constexpr uint32_t idesc = make_idesc_ab(128, D, kInterBF16<BF16>, BF16, TRANSPOSED, true);
+  constexpr uint32_t a_hi = desc_hi_word(TRANSPOSED ? kPiecesT_Sbo : kPieces_Sbo, 0u);
+  constexpr uint32_t b_hi = desc_hi_word(T::kAtomBytes, T::kSwizzleMode);
+  constexpr uint32_t kStep = TRANSPOSED ? 256 : 4096;  // bytes of A per reduction step
+  const uint32_t a_lo = desc_lo_word(a_addr + half * 4 * kStep, TRANSPOSED ? kPiecesT_Lbo : kPieces_Lbo);
+  const uint32_t b_lo = desc_lo_word(b_addr, T::kChunkTileBytes / 2);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (elected)
+      mma_ss(d_tmem, desc_from_words(a_lo + ((k * kStep) >> 4), a_hi),
+             desc_from_words(b_lo + ((k * 2 * T::kAtomBytes) >> 4), b_hi), idesc, k > 0 ? 1u : accumulate);
+}
+
 }  // namespace fa2

@@ -187,6 +187,36 @@ def test_fp32_results_are_the_unrounded_16_bit_ones(d, mode, monkeypatch):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("d,nq,nk", [(256, 257, 257), (192, 300, 129), (160, 128, 128), (256, 640, 640), (136, 130, 1)])
+def test_wide_head_consumers_with_two_output_tiles(d, nq, nk, monkeypatch):
+    """Head dims above 128 with enough heads form two output tiles per CTA; with one head per chunk of
+    the scratch they form one.  Same bits, and parity with the oracle on one head; odd and even tile
+    counts, a single tile, fewer keys than queries."""
+    b, h = 4, 75
+    g = torch.Generator(device=DEV).manual_seed(d + nq)
+    q, do = (torch.randn(b, h, nq, d, device=DEV, generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(b, h, nk, d, device=DEV, generator=g).bfloat16() for _ in range(2))
+
+    def run():
+        leaves = [t.detach().requires_grad_(True) for t in (q, k, v)]
+        out = flash_attention_v2(*leaves)
+        return dict(zip(("o", "dq", "dk", "dv"), (out.detach(), *torch.autograd.grad(out, leaves, do))))
+
+    lib = _lib.lib()
+    previous = lib.fa2_set_spill_budget(1 << 40)
+    try:
+        pairs = run()
+        lib.fa2_set_spill_budget(1)
+        single = run()
+    finally:
+        lib.fa2_set_spill_budget(previous)
+    assert _lib.device_status() == 0
+    for key in pairs:
+        assert torch.equal(pairs[key], single[key]), key
+    at = lambda t: t[2:3, 40:41].cpu()
+    check_against(naive_attention(at(q), at(k), at(v), at(do)), {key: at(t) for key, t in pairs.items()}, torch.bfloat16)
+
+
 def test_spill_mode_chunks_change_no_bit(monkeypatch):
     """With a scratch bound of 3 MiB the spill mode works through [3, 5, 700, 64] (0.7 MiB per
     head) in chunks of 3 + 2 heads per batch entry; with 8 MiB in chunks of 2 + 1 batch
