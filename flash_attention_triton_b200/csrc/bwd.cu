@@ -429,23 +429,29 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
 // One output tile per CTA from spilled 16-bit tiles (head dim 256: dV, dK and dQ; see
 // consume_roles).  warps 0-3 epilogue, warp 4 producer, warp 5 MMA issue.
 // =========================================================================================
+#ifndef FA2_CONSUME_CTAS
+#define FA2_CONSUME_CTAS 2
+#endif
 template <int D>
 struct ConsumeCfg {
   using T = Tile<D>;
-  static constexpr int kStages = D == 256 ? 2 : (D == 128 ? 3 : 4);
+  static constexpr int kCtasPerSm = D == 256 ? 1 : FA2_CONSUME_CTAS;
   static constexpr int kThreads = 192;
   static constexpr int kLoadWarp = 4;
   static constexpr int kMmaWarp = 5;
-  static constexpr int kStageBytes = 32768 + T::kTileBytes;  // scratch tile, then the operand tile
+  // scratch tile, then the operand tile (halves of them up to head dim 128)
+  static constexpr int kStageBytes = (32768 + T::kTileBytes) / consume_parts(D);
+  static constexpr int kStages = (228 * 1024 / kCtasPerSm - 2048) / kStageBytes;
   static constexpr int kOffBar = kStages * kStageBytes;
   static constexpr int kNumBars = 2 * kStages + 1;
   static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;
   static constexpr int kTmemCols = D < 32 ? 32 : D;
-  static_assert(kSmemBytes <= 232448, "shared memory budget of one CTA");
+  static_assert(kSmemBytes <= 232448 && kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "shared memory");
+  static_assert(kStages * kStageBytes >= T::kTileBytes, "the ring stages the output at the end");
 };
 
 template <int D, bool BF16, int FORM>
-__global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, 1)
+__global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, ConsumeCfg<D>::kCtasPerSm)
     bwd_consume_kernel(const uint4* __restrict__ scratch, const __grid_constant__ CUtensorMap tb,
                        const __grid_constant__ CUtensorMap tout, const __grid_constant__ F32Out out32, int cols,
                        const unsigned* __restrict__ tile_amax, int N, int Nk, int num_bh,

@@ -578,16 +578,16 @@ __device__ __forceinline__ void dkdv_roles(
       if constexpr (kPairs == 16) tmem_st_x16(tDpt, dsk); else tmem_st_x32(tDpt, dsk);
       if constexpr (SPILL) {
         // This thread's 64 values of dS^T(jt, qt) (kv row r, q columns wg*64 ..) straight to pair
-        // `tile0 + (qt - jt)` of the scratch tensor.  A tile is stored piece-major: the 16-byte
-        // piece (kv row r, q columns 8g .. 8g+7) at byte g * 2048 + r * 16, so one warp
-        // instruction writes 512 contiguous bytes, and the tile can later be copied linearly
-        // into shared memory as an unswizzled tensor-core operand.  Going through registers
+        // `tile0 + (qt - jt)` of the scratch tensor.  Each half of 64 kv rows is stored piece-major:
+        // the 16-byte piece (kv row r, q columns 8g .. 8g+7) at byte (r / 64) * 16384 + g * 1024 +
+        // (r % 64) * 16, so one warp instruction writes 512 contiguous bytes, and a half can later
+        // be copied linearly into shared memory as an unswizzled tensor-core operand.  Going through registers
         // keeps the copy out of shared memory, whose bandwidth the operand reads already use up.
         uint4* dst = reinterpret_cast<uint4*>(dq_accum) +
-                     ((item.tile0 + static_cast<size_t>(qt - jt)) * 2048 + wg * 1024 + r);
+                     ((item.tile0 + static_cast<size_t>(qt - jt)) * 2048 + (r >> 6) * 1024 + wg * 512 + (r & 63));
 #pragma unroll
         for (int pc = 0; pc < 8; ++pc)
-          dst[pc * 128] = make_uint4(dsk[4 * pc], dsk[4 * pc + 1], dsk[4 * pc + 2], dsk[4 * pc + 3]);
+          dst[pc * 64] = make_uint4(dsk[4 * pc], dsk[4 * pc + 1], dsk[4 * pc + 2], dsk[4 * pc + 3]);
       }
       if constexpr (FUSE) {
         const int col = (row & 127) + wg * kCols;  // first q column inside the Q tile
@@ -627,9 +627,13 @@ __device__ __forceinline__ void dkdv_roles(
 //   FORM 0: dV(jt) = sum_i P(jt, i)^T dO_i    A = P^T tile as stored   (K-major pieces)
 //   FORM 1: dK(jt) = sum_i dS(jt, i)^T Q_i    A = dS^T tile as stored  (K-major pieces)
 // (forms 0 and 1 serve head dim 256, where dK and dV do not fit next to the scores in tensor
-// memory.)  Roles: one producer warp (ring of kStages x (scratch tile + operand tile)), one
+// memory.)  Up to head dim 128 a stage is half of a product, 64 reduction rows (the scratch tile is stored
+// in halves then), so that two CTAs fit an SM: the start and the end of one are covered by the other.
+// Roles: one producer warp (ring of kStages x (scratch tile + operand tile)), one
 // MMA-issuing warp, four epilogue warps (tensor memory -> 16 bit -> TMA store).
 // =========================================================================================
+constexpr int consume_parts(int d) { return d <= 128 ? 2 : 1; }
+
 template <int STAGES>
 __device__ __forceinline__ void consume_init_barriers(uint32_t bar0) {
   for (int i = 0; i < 2 * STAGES; ++i) mbar_init(bar0 + 8u * i, 1);  // full[STAGES], empty[STAGES]
@@ -654,7 +658,9 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
                                               const F32Out& out32, int cols, int N,
                                               int Nk, const WaitCtx& w, const ConsumeItem& item) {
   using T = Tile<D>;
-  constexpr int kStageBytes = 32768 + T::kTileBytes;  // scratch tile, then the operand tile
+  constexpr int PARTS = consume_parts(D);  // stages per product
+  constexpr int kScratchBytes = 32768 / PARTS, kOperandBytes = T::kTileBytes / PARTS;
+  constexpr int kStageBytes = kScratchBytes + kOperandBytes;
   auto full = [&](int i) { return bar0 + 8u * i; };
   auto empty = [&](int i) { return bar0 + 8u * (STAGES + i); };
   const uint32_t done = bar0 + 8u * (2 * STAGES);
@@ -669,8 +675,9 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
   if (is_load_warp) {
     const uint32_t elected = elect_one();
     if (elected) prefetch_tensormap(tb);
-    for (int n = 0; n < count; ++n) {
-      const int st = n % STAGES, ph = (n / STAGES) & 1;
+    for (int m = 0; m < PARTS * count; ++m) {
+      const int n = m / PARTS, part = m % PARTS;
+      const int st = m % STAGES, ph = (m / STAGES) & 1;
       if (!mbar_wait_warp(empty(st), ph ^ 1, w, kBSiteLoadQ)) break;
       if (elected) {
         const uint32_t dst = ring_base + st * kStageBytes;
@@ -679,23 +686,26 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
         const size_t tile = item.head_tile0 + (FORM == 2 ? dstile_count(ntiles, other) + (ot - other)
                                                          : dstile_count(ntiles, ot) + n);
         mbar_arrive_expect_tx(full(st), kStageBytes);
-        bulk_load_1d(dst, scratch + tile * 2048, 32768, full(st));  // 32 KiB, stored as it is used
+        // stored as it is used
+        bulk_load_1d(dst, scratch + tile * 2048 + part * (2048 / PARTS), kScratchBytes, full(st));
 #pragma unroll
         for (int ch = 0; ch < T::kChunks; ++ch)
-          tma_load_4d(dst + 32768 + ch * T::kChunkTileBytes, tb, ch * T::kChunkElems, other * 128,
-                      item.hc, full(st));
+          tma_load_4d(dst + kScratchBytes + ch * (kOperandBytes / T::kChunks), tb, ch * T::kChunkElems,
+                      other * 128 + part * (128 / PARTS), item.hc, full(st));
       }
     }
     __syncwarp();
   } else if (is_mma_warp) {
     const uint32_t elected = elect_one();
     bool ok = true;
-    for (int n = 0; ok && n < count; ++n) {
+    for (int n = 0; ok && n < PARTS * count; ++n) {
       const int st = n % STAGES, ph = (n / STAGES) & 1;
       if (!(ok = mbar_wait(full(st), ph, w, kBSiteMmaKV))) break;
       const uint32_t src = ring_base + st * kStageBytes;
       // out[128, D] += A * B; B = the operand tile (d contiguous, MN-major)
-      if constexpr (FORM == 2)
+      if constexpr (PARTS == 2)
+        issue_piecesT_half_x_half_tile<D, BF16>(elected, tmem_acc, src, src + kScratchBytes, n > 0);
+      else if constexpr (FORM == 2)
         issue_piecesT_x_tile<D, BF16>(elected, tmem_acc, src, src + 32768, n > 0);
       else
         issue_pieces_x_tile<D, BF16>(elected, tmem_acc, src, src + 32768, n > 0);

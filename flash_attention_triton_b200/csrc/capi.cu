@@ -465,6 +465,7 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
         launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, scratch, 2, d->status, st);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     record_mark_between(st);
+    if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, 64)) return e;  // half tiles of K
     return static_cast<int>(launch_bwd_consume(s, 2, scratch, tk, tdq, dq32, rs, false, d->status, st));
   }
   float* dq_accum = static_cast<float*>(workspace);

@@ -136,6 +136,24 @@ __device__ __forceinline__ void issue_pieces_x_tile(uint32_t elected, uint32_t d
              k > 0 ? 1u : accumulate);
 }
 
+// Half of issue_piecesT_x_tile (64 reduction rows) with A as the spill mode of head dims up to 128
+// stores it, in halves: element (reduction row r, column c) of a half at byte (c / 8) * 1024 + r * 16 +
+// (c % 8) * 2; B a staged [64, D] half tile.
+template <int D, bool BF16>
+__device__ __forceinline__ void issue_piecesT_half_x_half_tile(uint32_t elected, uint32_t d_tmem, uint32_t a_addr,
+                                                               uint32_t b_addr, uint32_t accumulate) {
+  using T = Tile<D>;
+  constexpr uint32_t idesc = make_idesc_ab(128, D, kInterBF16<BF16>, BF16, true, true);
+  constexpr uint32_t a_hi = desc_hi_word(kPiecesT_Sbo / 2, 0u);  // no swizzle
+  constexpr uint32_t b_hi = desc_hi_word(T::kAtomBytes, T::kSwizzleMode);
+  const uint32_t a_lo = desc_lo_word(a_addr, kPiecesT_Lbo), b_lo = desc_lo_word(b_addr, T::kChunkTileBytes / 2);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (elected)
+      mma_ss(d_tmem, desc_from_words(a_lo + ((k * 256) >> 4), a_hi),
+             desc_from_words(b_lo + ((k * 2 * T::kAtomBytes) >> 4), b_hi), idesc, k > 0 ? 1u : accumulate);
+}
+
 // Half of either product above: the four 16-row reduction steps of half `half` of the piece-major tile,
 // against a staged [64, D] half tile of the operand.  TRANSPOSED selects issue_piecesT_x_tile's use
 // of A.
