@@ -29,7 +29,7 @@ namespace {
 // =========================================================================================
 // dK / dV (+ fused dQ) kernel: one CTA per KV tile of one (batch, head); see dkdv_roles.
 // =========================================================================================
-template <int D, bool BF16, int MODE>
+template <int D, bool BF16, int MODE, int KD = D>
 __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::kCtasPerSm)
     bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
 
-  dkdv_roles<D, BF16, MODE>(smem, smem_base, tmem_base, warp, lane, &tq, &tk, &tv, &tdo, &tdk, &tdv,
+  dkdv_roles<D, BF16, MODE, KD>(smem, smem_base, tmem_base, warp, lane, &tq, &tk, &tv, &tdo, &tdk, &tdv,
                             dk32, dv32, cols, rowstats, dq_accum, N, Nk, scale, scale_log2, w, item);
 
   tc_fence_before();
@@ -150,7 +150,7 @@ struct DqCfg {
   static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "shared memory of one SM");
 };
 
-template <int D, bool BF16>
+template <int D, bool BF16, int KD = D>
 __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
     bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                   const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
           tc_fence_after();
         }
         if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kBSiteMmaDO))) break;
-        issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColDp, doa,
+        issue_rows_x_rows<D, BF16, W, KD>(elected, tmem_base + C::kColDp, doa,
                                    smem_base + C::kOffV + vs * C::kKvBytes);
         commit(C::kBarDpFull);
         commit(C::kBarVEmpty + vs);  // V is free once dP has read it
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
           tc_fence_after();
         }
         if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kBSiteMmaKV))) break;
-        issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColS + (j & 1) * W, qa,
+        issue_rows_x_rows<D, BF16, W, KD>(elected, tmem_base + C::kColS + (j & 1) * W, qa,
                                    smem_base + C::kOffK + ks * C::kKvBytes);
         commit(C::kBarSFull + (j & 1));
         commit(C::kBarKEmpty + ks);
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
         if (!(ok = mbar_wait(bar(C::kBarDsReady), j & 1, w, kBSiteMmaDs))) break;
         tc_fence_after();
         // A = 16-bit dS over score buffer j%2, B = K_j as MN-major tile
-        issue_tmem_x_tile<D, BF16, W>(elected, tmem_base + C::kColDQ, tmem_base + C::kColS + (j & 1) * W,
+        issue_tmem_x_tile<D, BF16, W, KD>(elected, tmem_base + C::kColDQ, tmem_base + C::kColS + (j & 1) * W,
                                    kHalf, smem_base + C::kOffK + ks * C::kKvBytes, j > 0);
         commit(C::kBarDqDone + (j & 1));
         commit(C::kBarKEmpty + ks);
@@ -410,9 +410,9 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
     if (ok && wg == 0 && mbar_wait_warp(bar(C::kBarDone), 0, w, kBSiteCmpDone)) {
       tc_fence_after();
       if (dq32.p != nullptr)
-        store_rows_f32<D>(tmem_base + lane_base + C::kColDQ, dq32, cols, qt * 128 + r, hc, N, inv_dscale);
+        store_rows_f32<KD>(tmem_base + lane_base + C::kColDQ, dq32, cols, qt * 128 + r, hc, N, inv_dscale);
       else
-        store_rows_16bit<D, BF16>(tmem_base + lane_base + C::kColDQ, smem + C::kOffDO, w4, lane, &tdq,
+        store_rows_16bit<D, BF16, KD>(tmem_base + lane_base + C::kColDQ, smem + C::kOffDO, w4, lane, &tdq,
                                 qt * 128, hc, N, inv_dscale);
     }
   }
@@ -429,13 +429,16 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
 // One output tile per CTA from spilled 16-bit tiles (head dim 256: dV, dK and dQ; see
 // consume_roles).  warps 0-3 epilogue, warp 4 producer, warp 5 MMA issue.
 // =========================================================================================
-#ifndef FA2_CONSUME_CTAS
-#define FA2_CONSUME_CTAS 2
-#endif
+// Up to head dim 128 two CTAs run on an SM (rings of three 32 KiB stages at head dim 128).  With one,
+// the SM reads nothing while its CTA sets up (tensor memory, barriers, first loads) and stores its
+// result, some 6 us beside the few products of a short sum; two cover each other.  Whole backward,
+// microseconds, one CTA with whole tiles against two: [2,32,8192,128] bf16 3105 -> 2971, [32,20,1024,96]
+// fp16 868 -> 786, [1,32,4096,128] 467 -> 438, [8,32,512,128] 143 -> 133, [1,2,32768,128] 1409 / 1431 ->
+// 1450 / 1343 in two runs; three CTAs with two stages each measured the same within 1 %.
 template <int D>
 struct ConsumeCfg {
   using T = Tile<D>;
-  static constexpr int kCtasPerSm = D == 256 ? 1 : FA2_CONSUME_CTAS;
+  static constexpr int kCtasPerSm = D == 256 ? 1 : 2;
   static constexpr int kThreads = 192;
   static constexpr int kLoadWarp = 4;
   static constexpr int kMmaWarp = 5;
@@ -450,7 +453,7 @@ struct ConsumeCfg {
   static_assert(kStages * kStageBytes >= T::kTileBytes, "the ring stages the output at the end");
 };
 
-template <int D, bool BF16, int FORM>
+template <int D, bool BF16, int FORM, int KD = D>
 __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, ConsumeCfg<D>::kCtasPerSm)
     bwd_consume_kernel(const uint4* __restrict__ scratch, const __grid_constant__ CUtensorMap tb,
                        const __grid_constant__ CUtensorMap tout, const __grid_constant__ F32Out out32, int cols,
@@ -496,7 +499,7 @@ __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, ConsumeCfg<D>::kCtasP
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
 
-  consume_roles<D, BF16, FORM, C::kStages>(smem, smem_base, smem_base + C::kOffBar, tmem_base,
+  consume_roles<D, BF16, FORM, C::kStages, KD>(smem, smem_base, smem_base + C::kOffBar, tmem_base,
                                            warp == C::kLoadWarp, warp == C::kMmaWarp,
                                            warp < 4 ? warp : -1, lane, scratch, &tb, &tout, out32, cols, N, Nk, w,
                                            item);
@@ -960,14 +963,14 @@ cudaError_t launch_scores_wide_t(const AttnShape& s, const CUtensorMap& tq, cons
   return cudaGetLastError();
 }
 
-template <int D, bool BF16, int MODE>
+template <int D, bool BF16, int MODE, int KD = D>
 cudaError_t launch_dkdv_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                           const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdk,
                           const CUtensorMap& tdv, const F32Out& dk32, const F32Out& dv32,
                           const RowStats& rowstats, float* dq_accum,
                           int* status, cudaStream_t stream) {
   using C = DkdvCfg<D, MODE>;
-  auto kern = bwd_dkdv_kernel<D, BF16, MODE>;
+  auto kern = bwd_dkdv_kernel<D, BF16, MODE, KD>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
@@ -978,12 +981,12 @@ cudaError_t launch_dkdv_t(const AttnShape& s, const CUtensorMap& tq, const CUten
   return cudaGetLastError();
 }
 
-template <int D, bool BF16, int FORM>
+template <int D, bool BF16, int FORM, int KD = D>
 cudaError_t launch_consume_t(const AttnShape& s, const void* scratch, const CUtensorMap& tb,
                              const CUtensorMap& tout, const F32Out& out32, const RowStats& rowstats, int* status,
                              cudaStream_t stream) {
   using C = ConsumeCfg<D>;
-  auto kern = bwd_consume_kernel<D, BF16, FORM>;
+  auto kern = bwd_consume_kernel<D, BF16, FORM, KD>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
@@ -1011,12 +1014,12 @@ cudaError_t launch_consume_pair_t(const AttnShape& s, const void* scratch, const
   return cudaGetLastError();
 }
 
-template <int D, bool BF16>
+template <int D, bool BF16, int KD = D>
 cudaError_t launch_dq_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                         const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
                         const F32Out& dq32, const RowStats& rowstats, int* status, cudaStream_t stream) {
   using C = DqCfg<D>;
-  auto kern = bwd_dq_kernel<D, BF16>;
+  auto kern = bwd_dq_kernel<D, BF16, KD>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
@@ -1037,6 +1040,12 @@ cudaError_t launch_bwd_dkdv(const AttnShape& s, const CUtensorMap& tq, const CUt
   // modes: 0 dK/dV only, 1 fused atomic dQ (dq_accum = fp32 accumulator), 2 spill dS tiles
   // (dq_accum = the 16-bit scratch tensor)
 #define FA2_ARGS s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rowstats, dq_accum, status, stream
+  if (s.D == 128 && s.Dg <= kShortDim128 && mode == 2)
+    return s.dtype ? launch_dkdv_t<128, true, 2, kShortDim128>(FA2_ARGS)
+                   : launch_dkdv_t<128, false, 2, kShortDim128>(FA2_ARGS);
+  if (s.D == 128 && s.Dg <= kShortDim128 && mode == 0)
+    return s.dtype ? launch_dkdv_t<128, true, 0, kShortDim128>(FA2_ARGS)
+                   : launch_dkdv_t<128, false, 0, kShortDim128>(FA2_ARGS);
 #define FA2_CASE(DD)                                                                        \
   case DD:                                                                                  \
     if (mode == 1)                                                                          \
@@ -1061,6 +1070,9 @@ cudaError_t launch_bwd_dq(const AttnShape& s, const CUtensorMap& tq, const CUten
                           const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
                           const F32Out& dq32, const RowStats& rowstats, int* status, cudaStream_t stream) {
 #define FA2_ARGS s, tq, tk, tv, tdo, tdq, dq32, rowstats, status, stream
+  if (s.D == 128 && s.Dg <= kShortDim128)
+    return s.dtype ? launch_dq_t<128, true, kShortDim128>(FA2_ARGS)
+                   : launch_dq_t<128, false, kShortDim128>(FA2_ARGS);
 #define FA2_CASE(DD)                                                   \
   case DD:                                                             \
     return s.dtype ? launch_dq_t<DD, true>(FA2_ARGS)                   \
@@ -1101,6 +1113,9 @@ cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch
   if (s.D == 256) return form == 0 ? FA2_WIDE(0) : (form == 1 ? FA2_WIDE(1) : FA2_WIDE(2));
 #undef FA2_WIDE
   if (form != 2) return cudaErrorInvalidValue;
+  if (s.D == 128 && s.Dg <= kShortDim128)
+    return s.dtype ? launch_consume_t<128, true, 2, kShortDim128>(FA2_ARGS)
+                   : launch_consume_t<128, false, 2, kShortDim128>(FA2_ARGS);
   switch (s.D) {
     FA2_CASE(32)
     FA2_CASE(64)

@@ -70,14 +70,14 @@ __device__ __forceinline__ void mask_row(float2 (&p)[PAIRS], int first_column, i
 // Epilogue helper: one warp multiplies its 32 rows of a [128, D] fp32 accumulator by `mul` (a power
 // of two, see head_dscale), converts them to 16 bits, stages them swizzled in `stage` (a free
 // tile buffer) and stores them with one TMA per chunk.
-template <int D, bool BF16>
+template <int D, bool BF16, int KD = D>
 __device__ __forceinline__ void store_rows_16bit(uint32_t tmem_row_addr, uint8_t* stage, int warp4,
                                                  int lane, const CUtensorMap* map, int row_base,
                                                  HeadCoord hc, int N, float mul = 1.0f) {
   using T = Tile<D>;
   const int r = warp4 * 32 + lane;
 #pragma unroll
-  for (int c0 = 0; c0 < D; c0 += 32) {
+  for (int c0 = 0; c0 < KD; c0 += 32) {
     uint32_t v[32];
     tmem_ld_x32(tmem_row_addr + c0, v);
     tmem_wait_ld();
@@ -300,7 +300,7 @@ __device__ __forceinline__ void dkdv_init_barriers(uint32_t bar0) {
 //                                           workspace with vector atomics
 // -lse*log2(e) and -delta of a Q tile arrive in shared memory as one 1 KiB bulk copy from the
 // tile-blocked rowstats array; padded rows carry -lse = -inf, which makes their P exactly 0.
-template <int D, bool BF16, int MODE>
+template <int D, bool BF16, int MODE, int KD = D>
 __device__ __forceinline__ void dkdv_roles(
     uint8_t* smem, uint32_t smem_base, uint32_t tmem_base, int warp, int lane,
     const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, const CUtensorMap* tdo,
@@ -394,7 +394,7 @@ __device__ __forceinline__ void dkdv_roles(
       if (warp == C::kMmaWarp) {
         // ------------------------------------------------------------ warp X
         if (ok && (ok = mbar_wait(bar(C::kBarQFull + 0), 0, w, kBSiteMmaQ))) {
-          issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColSt, ka, smem_base + C::kOffQ);
+          issue_rows_x_rows<D, BF16, W, KD>(elected, tmem_base + C::kColSt, ka, smem_base + C::kOffQ);
           commit(C::kBarStFull);
           commit(C::kBarQEmpty + 0);
         }
@@ -404,12 +404,12 @@ __device__ __forceinline__ void dkdv_roles(
           if (!(ok = mbar_wait(bar(C::kBarDOFull + s), ph, w, kBSiteMmaDO))) break;
           if (!(ok = mbar_wait(bar(C::kBarPtReady), t & 1, w, kBSiteMmaPt))) break;
           tc_fence_after();
-          issue_tmem_x_tile<D, BF16, W>(elected, tmem_base + C::kColDV, tmem_base + C::kColSt, kHalf,
+          issue_tmem_x_tile<D, BF16, W, KD>(elected, tmem_base + C::kColDV, tmem_base + C::kColSt, kHalf,
                                         doa, t > 0);  // dV += Pt dO_t
           commit(C::kBarDOEmpty + s);
           if (t + 1 < nsteps) {
             if (!(ok = mbar_wait(bar(C::kBarQFull + s1), ph1, w, kBSiteMmaQ))) break;
-            issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColSt, ka,
+            issue_rows_x_rows<D, BF16, W, KD>(elected, tmem_base + C::kColSt, ka,
                                           smem_base + C::kOffQ + s1 * C::kStepBytes);  // St(t+1)
             commit(C::kBarStFull);
             commit(C::kBarQEmpty + s1);
@@ -421,7 +421,7 @@ __device__ __forceinline__ void dkdv_roles(
       } else {
         // ------------------------------------------------------------ warp Y
         if (ok && (ok = mbar_wait(bar(C::kBarDOFull + 0), 0, w, kBSiteMmaDO))) {
-          issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColDpt, va, smem_base + C::kOffDO);
+          issue_rows_x_rows<D, BF16, W, KD>(elected, tmem_base + C::kColDpt, va, smem_base + C::kOffDO);
           commit(C::kBarDptFull);
           commit(C::kBarDOEmpty + 0);
         }
@@ -439,7 +439,7 @@ __device__ __forceinline__ void dkdv_roles(
             }
           }
           tc_fence_after();
-          issue_tmem_x_tile<D, BF16, W>(elected, tmem_base + C::kColDK, tmem_base + C::kColDpt, kHalf,
+          issue_tmem_x_tile<D, BF16, W, KD>(elected, tmem_base + C::kColDK, tmem_base + C::kColDpt, kHalf,
                                         qa, t > 0);  // dK += dSt Q_t
           commit(C::kBarQEmpty + s);
           if constexpr (FUSE) {
@@ -458,7 +458,7 @@ __device__ __forceinline__ void dkdv_roles(
               }
             }
             if (!(ok = mbar_wait(bar(C::kBarDOFull + s1), ph1, w, kBSiteMmaDO))) break;
-            issue_rows_x_rows<D, BF16, W>(elected, tmem_base + C::kColDpt, va,
+            issue_rows_x_rows<D, BF16, W, KD>(elected, tmem_base + C::kColDpt, va,
                                           smem_base + C::kOffDO + s1 * C::kStepBytes);  // dPt(t+1)
             commit(C::kBarDptFull);
             commit(C::kBarDOEmpty + s1);
@@ -607,13 +607,13 @@ __device__ __forceinline__ void dkdv_roles(
     if (ok && mbar_wait_warp(bar(C::kBarDone), 0, w, kBSiteCmpDone)) {
       tc_fence_after();
       if (dk32.p != nullptr)
-        store_rows_f32<D>(tmem_base + lane_base + (wg == 0 ? C::kColDV : C::kColDK), wg == 0 ? dv32 : dk32,
+        store_rows_f32<KD>(tmem_base + lane_base + (wg == 0 ? C::kColDV : C::kColDK), wg == 0 ? dv32 : dk32,
                           cols, jt * 128 + r, hc, Nk, wg == 0 ? 1.0f : inv_dscale);
       else if (wg == 0)
-        store_rows_16bit<D, BF16>(tmem_base + lane_base + C::kColDV, smem + C::kOffDO, w4, lane,
+        store_rows_16bit<D, BF16, KD>(tmem_base + lane_base + C::kColDV, smem + C::kOffDO, w4, lane,
                                   tdv, jt * 128, hc, Nk);
       else
-        store_rows_16bit<D, BF16>(tmem_base + lane_base + C::kColDK, smem + C::kOffQ, w4, lane,
+        store_rows_16bit<D, BF16, KD>(tmem_base + lane_base + C::kColDK, smem + C::kOffQ, w4, lane,
                                   tdk, jt * 128, hc, Nk, inv_dscale);
     }
   }
@@ -650,7 +650,7 @@ struct ConsumeItem {
 
 // epi_warp: 0..3 for the four epilogue warps (warp e owns tensor-memory lanes 32e .. 32e+31),
 // -1 for every other warp.
-template <int D, bool BF16, int FORM, int STAGES>
+template <int D, bool BF16, int FORM, int STAGES, int KD = D>
 __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base, uint32_t bar0,
                                               uint32_t tmem_acc, bool is_load_warp, bool is_mma_warp,
                                               int epi_warp, int lane, const uint4* __restrict__ scratch,
@@ -704,7 +704,7 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
       const uint32_t src = ring_base + st * kStageBytes;
       // out[128, D] += A * B; B = the operand tile (d contiguous, MN-major)
       if constexpr (PARTS == 2)
-        issue_piecesT_half_x_half_tile<D, BF16>(elected, tmem_acc, src, src + kScratchBytes, n > 0);
+        issue_piecesT_half_x_half_tile<D, BF16, KD>(elected, tmem_acc, src, src + kScratchBytes, n > 0);
       else if constexpr (FORM == 2)
         issue_piecesT_x_tile<D, BF16>(elected, tmem_acc, src, src + 32768, n > 0);
       else
@@ -721,10 +721,10 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
       const uint32_t lane_base = static_cast<uint32_t>(epi_warp * 32) << 16;
       // every product has completed, so the ring is idle: stage through its first buffer
       if (out32.p != nullptr)
-        store_rows_f32<D>(tmem_acc + lane_base, out32, cols, ot * 128 + epi_warp * 32 + lane, item.hc, out_rows,
+        store_rows_f32<KD>(tmem_acc + lane_base, out32, cols, ot * 128 + epi_warp * 32 + lane, item.hc, out_rows,
                           inv_dscale);
       else
-        store_rows_16bit<D, BF16>(tmem_acc + lane_base, ring, epi_warp, lane, tout, ot * 128, item.hc,
+        store_rows_16bit<D, BF16, KD>(tmem_acc + lane_base, ring, epi_warp, lane, tout, ot * 128, item.hc,
                                 out_rows, inv_dscale);
     }
   }

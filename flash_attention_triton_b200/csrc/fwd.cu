@@ -107,7 +107,7 @@ enum FwdSite {
   kSiteAlign
 };
 
-template <int D, bool BF16>
+template <int D, bool BF16, int KD = D>
 __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtasPerSm)
     fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap to,
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
             // S = Q_lo K_lo^T + Q_hi K_hi^T: the Q slots hold the halves, K arrives half by half
             for (int half = 0; ok && half < 2; ++half) {
               if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
-              issue_rows_x_rows<DT, BF16, W>(elected, tmem_base + C::kColS,
+              issue_rows_x_rows<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColS,
                                           smem_base + C::kOffQ + half * T::kTileBytes,
                                           smem_base + C::kOffK + ks * C::kKvBytes, half);
               if (elected) mma_commit(bar(C::kBarKEmpty + ks));
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
             }
             if (!ok) break;
           } else {
-            issue_rows_x_rows<DT, BF16, W>(elected, tmem_base + C::kColS,
+            issue_rows_x_rows<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColS,
                                         smem_base + C::kOffQ + i * T::kTileBytes,
                                         smem_base + C::kOffK + ks * C::kKvBytes);
           }
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
             // O_lo += P V_lo, O_hi += P V_hi: the O0 / O1 columns hold the two halves of O
             for (int half = 0; ok && half < 2; ++half) {
               if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
-              issue_tmem_x_tile<DT, BF16, W>(elected, tmem_base + C::kColO + half * DT,
+              issue_tmem_x_tile<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColO + half * DT,
                                           tmem_base + C::kColP, W / 4,
                                           smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
               if (elected) mma_commit(bar(C::kBarVEmpty + vs));
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
             }
             if (!ok) break;
           } else {
-            issue_tmem_x_tile<DT, BF16, W>(elected, tmem_base + C::kColO + i * DT,
+            issue_tmem_x_tile<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColO + i * DT,
                                         tmem_base + C::kColP + i * (W / 2), W / 4,
                                         smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
           }
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
           pv_waited = true;
           constexpr int kStep = W == 64 ? 16 : 32;  // the score row stays in registers meanwhile
 #pragma unroll
-          for (int c0 = 0; c0 < D; c0 += kStep) {
+          for (int c0 = 0; c0 < KD; c0 += kStep) {
             uint32_t orr[kStep];
             if constexpr (kStep == 16) tmem_ld_x16(tO + c0, orr); else tmem_ld_x32(tO + c0, orr);
             tmem_wait_ld();
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
       float* const dst32 =
           o32.p != nullptr && row < N ? o32.p + hc.b * o32.st.b + hc.h * o32.st.h + row * o32.st.n : nullptr;
 #pragma unroll
-      for (int c0 = 0; c0 < D; c0 += 32) {
+      for (int c0 = 0; c0 < KD; c0 += 32) {
         uint32_t orr[32];
         tmem_ld_x32(tO + c0, orr);
         tmem_wait_ld();
@@ -518,12 +518,12 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
   }
 }
 
-template <int D, bool BF16>
+template <int D, bool BF16, int KD = D>
 cudaError_t launch_fwd_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                          const CUtensorMap& tv, const CUtensorMap& to, const F32Out& o32, float* lse,
                          const LaunchCtx& ctx, cudaStream_t stream) {
   using C = FwdCfg<D == 256 ? 128 : D>;  // head dim 256 runs on the plan of head dim 128
-  auto kern = fwd_kernel<D, BF16>;
+  auto kern = fwd_kernel<D, BF16, KD>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
@@ -548,6 +548,9 @@ cudaError_t launch_fwd(const AttnShape& s, const CUtensorMap& tq, const CUtensor
   case DD:                                                                           \
     return s.dtype ? launch_fwd_t<DD, true>(s, tq, tk, tv, to, o32, lse, ctx, stream)     \
                    : launch_fwd_t<DD, false>(s, tq, tk, tv, to, o32, lse, ctx, stream);
+  if (s.D == 128 && s.Dg <= kShortDim128)
+    return s.dtype ? launch_fwd_t<128, true, kShortDim128>(s, tq, tk, tv, to, o32, lse, ctx, stream)
+                   : launch_fwd_t<128, false, kShortDim128>(s, tq, tk, tv, to, o32, lse, ctx, stream);
   switch (s.D) {
     FA2_CASE(32)
     FA2_CASE(64)
