@@ -81,6 +81,8 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
+  grid_wait_previous();
+  grid_allow_next();
 
   dkdv_roles<D, BF16, MODE, KD>(smem, smem_base, tmem_base, warp, lane, &tq, &tk, &tv, &tdo, &tdk, &tdv,
                             dk32, dv32, cols, rowstats, dq_accum, N, Nk, scale, scale_log2, w, item);
@@ -215,6 +217,9 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
+  // Nothing here depends on the dK/dV kernel before it; what that one waited for has completed.  The
+  // wait for it stands at the end.
+  grid_allow_next();
 
   if (warp >= C::kMmaWarp) {
     reg_dec<C::kProducerRegs>();
@@ -417,6 +422,7 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
     }
   }
 
+  grid_wait_previous();
   tc_fence_before();
   __syncthreads();
   if (warp == C::kMmaWarp) {
@@ -498,12 +504,18 @@ __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, ConsumeCfg<D>::kCtasP
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
+  // Forms 1 (dK) and 2 (dQ) of head dim 256 do not depend on the consumer before them, only on what that
+  // one waited for; their wait stands at the end.
+  constexpr bool kIndependent = D == 256 && FORM != 0;
+  if constexpr (!kIndependent) grid_wait_previous();
+  grid_allow_next();
 
   consume_roles<D, BF16, FORM, C::kStages, KD>(smem, smem_base, smem_base + C::kOffBar, tmem_base,
                                            warp == C::kLoadWarp, warp == C::kMmaWarp,
                                            warp < 4 ? warp : -1, lane, scratch, &tb, &tout, out32, cols, N, Nk, w,
                                            item);
 
+  if constexpr (kIndependent) grid_wait_previous();
   tc_fence_before();
   __syncthreads();
   if (warp == C::kMmaWarp) {
@@ -602,6 +614,9 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
+  constexpr bool kIndependent = FORM != 0;  // as in bwd_consume_kernel
+  if constexpr (!kIndependent) grid_wait_previous();
+  grid_allow_next();
 
   if (warp == C::kLoadWarp) {
     const uint32_t elected = elect_one();
@@ -670,6 +685,7 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
     }
   }
 
+  if constexpr (kIndependent) grid_wait_previous();
   tc_fence_before();
   __syncthreads();
   if (warp == C::kMmaWarp) {
@@ -777,6 +793,8 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
+  grid_wait_previous();
+  grid_allow_next();
 
   if (warp >= C::kMmaWarp) {
     reg_dec<72>();
@@ -956,11 +974,10 @@ cudaError_t launch_scores_wide_t(const AttnShape& s, const CUtensorMap& tq, cons
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
   const unsigned grid = static_cast<unsigned>((s.Nk + 127) / 128) * s.B * s.H;  // one CTA per KV tile
-  kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(
+  return launch_dependent(kern, grid, C::kThreads, C::kSmemBytes, stream,
       tq, tk, tv, tdo, rowstats.stats, rowstats.tile_amax, static_cast<uint4*>(p_scratch),
       static_cast<uint4*>(ds_scratch), s.N, s.Nk, s.B * s.H, s.H, heads_per_group(s), s.scale,
       s.scale * 1.4426950408889634f, status);
-  return cudaGetLastError();
 }
 
 template <int D, bool BF16, int MODE, int KD = D>
@@ -975,10 +992,10 @@ cudaError_t launch_dkdv_t(const AttnShape& s, const CUtensorMap& tq, const CUten
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
   const unsigned grid = static_cast<unsigned>((s.Nk + 127) / 128) * s.B * s.H;  // one CTA per KV tile
-  kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(
-      tq, tk, tv, tdo, tdk, tdv, dk32, dv32, s.Dg, rowstats.stats, rowstats.tile_amax, dq_accum, s.N, s.Nk, s.B * s.H,
+  return launch_dependent(kern, grid, C::kThreads, C::kSmemBytes, stream,
+      tq, tk, tv, tdo, tdk, tdv, dk32, dv32, s.Dg, rowstats.stats, rowstats.tile_amax, dq_accum, s.N,
+      s.Nk, s.B * s.H,
       s.H, heads_per_group(s), s.scale, s.scale * 1.4426950408889634f, status);
-  return cudaGetLastError();
 }
 
 template <int D, bool BF16, int FORM, int KD = D>
@@ -992,10 +1009,10 @@ cudaError_t launch_consume_t(const AttnShape& s, const void* scratch, const CUte
   if (e != cudaSuccess) return e;
   const unsigned grid =
       static_cast<unsigned>(((FORM == 2 ? s.N : s.Nk) + 127) / 128) * s.B * s.H;  // one CTA per output tile
-  kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(static_cast<const uint4*>(scratch), tb, tout, out32, s.Dg,
+  return launch_dependent(kern, grid, C::kThreads, C::kSmemBytes, stream,
+      static_cast<const uint4*>(scratch), tb, tout, out32, s.Dg,
                                                      rowstats.tile_amax, s.N, s.Nk, s.B * s.H, s.H,
                                                      heads_per_group(s), status);
-  return cudaGetLastError();
 }
 
 template <bool BF16, int FORM>
@@ -1008,10 +1025,10 @@ cudaError_t launch_consume_pair_t(const AttnShape& s, const void* scratch, const
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
   const unsigned out_tiles = static_cast<unsigned>(((FORM == 2 ? s.N : s.Nk) + 127) / 128);
-  kern<<<(out_tiles + 1) / 2 * s.B * s.H, C::kThreads, C::kSmemBytes, stream>>>(
-      static_cast<const uint4*>(scratch), tb, tout, out32, s.Dg, rowstats.tile_amax, s.N, s.Nk, s.B * s.H, s.H,
+  return launch_dependent(kern, (out_tiles + 1) / 2 * s.B * s.H, C::kThreads, C::kSmemBytes, stream,
+      static_cast<const uint4*>(scratch), tb, tout, out32, s.Dg, rowstats.tile_amax, s.N, s.Nk, s.B * s.H,
+      s.H,
       heads_per_group(s), status);
-  return cudaGetLastError();
 }
 
 template <int D, bool BF16, int KD = D>
@@ -1024,10 +1041,9 @@ cudaError_t launch_dq_t(const AttnShape& s, const CUtensorMap& tq, const CUtenso
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
   const unsigned grid = static_cast<unsigned>((s.N + 127) / 128) * s.B * s.H;  // one CTA per Q tile
-  kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(
+  return launch_dependent(kern, grid, C::kThreads, C::kSmemBytes, stream,
       tq, tk, tv, tdo, tdq, dq32, s.Dg, rowstats.stats, rowstats.tile_amax, s.N, s.Nk, s.B * s.H, s.H,
       heads_per_group(s), s.scale, s.scale * 1.4426950408889634f, status);
-  return cudaGetLastError();
 }
 
 }  // namespace

@@ -66,6 +66,8 @@ __global__ void __launch_bounds__(kPreThreads)
   constexpr int kPasses = 128 / kRowsPerPass;               // 2, 4, 8 or 16
   constexpr int kBatch = kPasses < kPreMaxInFlight ? kPasses : kPreMaxInFlight;
   __shared__ unsigned warp_max[kPreThreads / 32];
+  grid_wait_previous();
+  grid_allow_next();
   const long long tile = blockIdx.x;  // = bh * ntiles + t
   const long long bh = tile / ntiles;
   const int t = static_cast<int>(tile - bh * ntiles);
@@ -198,6 +200,8 @@ __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
     fence_mbar_init();
   }
   __syncthreads();
+  grid_wait_previous();
+  grid_allow_next();
   const uint32_t row_bytes = static_cast<uint32_t>(d8) * 16u;
 
   if (warp == R::kConsumers / 32) {
@@ -337,6 +341,8 @@ template <int D, bool BF16>
 __global__ void __launch_bounds__(256)
     dq_convert_kernel(const float4* __restrict__ acc, uint4* __restrict__ dq, F32Out dq32, int N, int ntiles,
                       long long total, int d8, int H, Strides sdq) {
+  grid_wait_previous();
+  grid_allow_next();
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   // idx = ((tile_global * 4 + w) * (D/8) + k8) * 32 + lane
@@ -384,15 +390,16 @@ cudaError_t launch_pre_t(const AttnShape& s, const void* o, const Strides& so, c
         kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::kSmemBytes);
     if (attr != cudaSuccess) return attr;
     const unsigned grid = static_cast<unsigned>(tiles < num_sms ? tiles : num_sms);
-    kernel<<<grid, R::kThreads, R::kSmemBytes, stream>>>(
-        static_cast<const uint4*>(o), static_cast<const uint4*>(dout), lse, rowstats, tile_amax,
+    return launch_dependent(
+        kernel, grid, R::kThreads, R::kSmemBytes, stream,
+      static_cast<const uint4*>(o), static_cast<const uint4*>(dout), lse, rowstats, tile_amax,
         s.N, ntiles, tiles, s.Dg / 8, s.H, in_vec8(so), in_vec8(sdo), status);
   } else {
-    bwd_preprocess_kernel<D, BF16><<<static_cast<unsigned>(tiles), kPreThreads, 0, stream>>>(
+    return launch_dependent(
+        bwd_preprocess_kernel<D, BF16>, static_cast<unsigned>(tiles), kPreThreads, 0, stream,
         static_cast<const uint4*>(o), static_cast<const uint4*>(dout), lse, rowstats, tile_amax,
         s.N, ntiles, s.Dg / 8, s.H, in_vec8(so), in_vec8(sdo));
   }
-  return cudaGetLastError();
 }
 
 template <int D, bool BF16>
@@ -401,10 +408,10 @@ cudaError_t launch_cvt_t(const AttnShape& s, const float* dq_accum, void* dq, co
   const int ntiles = (s.N + 127) / 128;
   const long long total = static_cast<long long>(s.B) * s.H * ntiles * 128 * (D / 8);
   const long long blocks = (total + 255) / 256;
-  dq_convert_kernel<D, BF16><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
+  return launch_dependent(
+      dq_convert_kernel<D, BF16>, static_cast<unsigned>(blocks), 256, 0, stream,
       reinterpret_cast<const float4*>(dq_accum), static_cast<uint4*>(dq), dq32, s.N, ntiles, total,
       s.Dg / 8, s.H, in_vec8(sdq));
-  return cudaGetLastError();
 }
 
 }  // namespace

@@ -157,6 +157,8 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
+  grid_wait_previous();
+  grid_allow_next();
 
   // One or two CTAs per SM; work items (one Q-tile pair of one (batch, head)) are fetched from a
   // global counter in head-major, heavy-pair-first order, like a hardware block scheduler
@@ -533,10 +535,10 @@ cudaError_t launch_fwd_t(const AttnShape& s, const CUtensorMap& tq, const CUtens
   const long long slots = static_cast<long long>(ctx.num_sms) * C::kCtasPerSm;
   const unsigned grid = static_cast<unsigned>(items < slots ? items : slots);
   const float scale_log2 = s.scale * 1.4426950408889634f;
-  kern<<<grid, kFwdThreads, C::kSmemBytes, stream>>>(tq, tk, tv, to, o32, s.Dg, lse, s.N, s.Nk, s.B * s.H, s.H,
+  return launch_dependent(kern, grid, kFwdThreads, C::kSmemBytes, stream,
+      tq, tk, tv, to, o32, s.Dg, lse, s.N, s.Nk, s.B * s.H, s.H,
                                                      heads_per_group(s), scale_log2, ctx.status,
                                                      ctx.work_counter);
-  return cudaGetLastError();
 }
 
 }  // namespace

@@ -116,6 +116,18 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, co
 }
 
 // ----------------------------------------------------------------------------------------
+// Programmatic dependent launch (every kernel is launched with it, see launch_dependent).  A kernel may
+// start while its predecessor on the stream is still running; it sets up barriers and tensor memory
+// and then waits here, before its first access to global memory, until the predecessor has completed
+// and its writes are visible.  grid_allow_next lets the successor start once every CTA of this grid has
+// called it, which is after its own wait and after its tensor memory has been allocated: a successor's
+// CTA can therefore never hold the tensor memory that a CTA of this grid still needs, and when it
+// starts, everything before this grid has completed.
+// ----------------------------------------------------------------------------------------
+__device__ __forceinline__ void grid_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ----------------------------------------------------------------------------------------
 // Proxy fences and named barriers
 // ----------------------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {
