@@ -91,8 +91,8 @@ NCU_BWD_DRAM_MB_PER_24 = {0: 381.8 + 209.7 + 100.7 + 20.1, 1: 208.6 + 74.7 + 204
 NCU_DKDV_DRAM_MB_PER_24 = {1: 208.6 + 74.7, 2: 329.6 + 1679.5}  # the dK/dV kernel alone
 
 # Polynomial share of the exponentials (of every 8 column pairs) the kernels are built with
-# (FA2_FWD_POLY_PAIRS_PER_8 in csrc/fwd.cu, FA2_BWD_POLY_PAIRS_PER_8 in csrc/bwd_roles.cuh).
-POLY_SHARE = {"fwd": 3 / 8, "bwd": 2 / 8}  # at the head dims the ceiling is reported for (<= 64)
+# (FwdCfg::kPolyShare in csrc/fwd.cu, kPolyShareT in csrc/bwd_roles.cuh).
+POLY_SHARE = {"fwd": 0.0, "bwd": 2 / 8}  # at the head dims the ceiling is reported for (<= 64)
 
 
 def softmax_ceiling(d, which):

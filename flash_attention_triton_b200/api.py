@@ -105,12 +105,13 @@ def _backward_mode(deterministic: bool, headdim: int, seqlen_q: int) -> int:
 
     ``True`` must give the same bits whatever the batch / head partitioning, so the choice
     depends on the head dim and the sequence length only.  Head dims above 64: the spill mode
-    (fastest there, 12-15 % ahead of the recompute mode) unless one head's scratch is too
-    large, then the recompute mode.  Head dims up to 64: the recompute mode, which measures
-    within 4 % of the spill mode either way there (the 32 KiB dS tile does not shrink with the
-    head dim, the tensor work does) and needs no scratch, like the reference's O(N) backward.
+    (fastest there, 10-25 % ahead of the recompute mode) unless one head's scratch is too
+    large, then the recompute mode.  Head dims up to 64: the recompute mode, which is
+    4-14 % ahead of the spill mode there (the 32 KiB dS tile does not shrink with the head dim, the
+    tensor work does) and needs no scratch, like the reference's O(N) backward.
     ``False`` (the reference's default, atomics there) means "fastest": the atomic kernel at
-    head dims up to 64 (15-25 % ahead), the deterministic choice above.  ``FA2_B200_BWD_MODE`` =
+    head dims up to 64 (14-21 % ahead of the recompute mode from 4096 rows, the same at 2048), the
+    deterministic choice above.  ``FA2_B200_BWD_MODE`` =
     ``atomic`` / ``recompute`` / ``spill`` overrides both (for experiments).
     """
     if headdim > 128:  # one (deterministic) backward exists there: scores + three consumers

@@ -116,7 +116,7 @@ inline int heads_per_group(const AttnShape& s) {
   return static_cast<int>(g < 1 ? 1 : (g > bh ? bh : g));
 }
 
-// Per-launch context of the forward kernel.  It runs one CTA per SM; each CTA fetches work
+// Per-launch context of the forward kernel.  It runs one or two CTAs per SM; each CTA fetches work
 // items (pairs of Q tiles) from `work_counter` until none are left, so tensor memory is
 // allocated once and no SM idles between items.  The counter is zero before the launch and the kernel
 // leaves it at zero (see fetch_work_item), so no memset sits between launches.
