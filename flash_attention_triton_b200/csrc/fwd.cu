@@ -424,7 +424,10 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
       }
       // p = 2^(s*c - m*c) with packed fp32x2 FMAs; row sum in four independent packed chains.
       const float2 sc2 = make_float2(scale_log2, scale_log2);
-      const float2 nm2 = make_float2(-m_run * scale_log2, -m_run * scale_log2);
+      // A row whose scores so far are all -inf (infinite inputs) has weights 0 and not -inf + inf: half as
+      // many columns as before decide a row's first maximum with 64-row tiles.
+      const float neg_m = W == 64 && m_run == -INFINITY ? 0.f : -m_run * scale_log2;
+      const float2 nm2 = make_float2(neg_m, neg_m);
       float2 acc[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
       uint32_t pk[W / 2];
 #pragma unroll

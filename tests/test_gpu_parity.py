@@ -217,6 +217,23 @@ def test_wide_head_consumers_with_two_output_tiles(d, nq, nk, monkeypatch):
     check_against(naive_attention(at(q), at(k), at(v), at(do)), {key: at(t) for key, t in pairs.items()}, torch.bfloat16)
 
 
+@pytest.mark.parametrize("d", [32, 64])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_keys_with_scores_of_minus_infinity_have_no_weight(d, dtype):
+    """The first 64 keys score -inf against every query: rows beyond them attend to the others
+    only, whatever tile the first finite score falls into."""
+    g = torch.Generator().manual_seed(d)
+    q, k, v = (torch.randn(1, 2, 200, d, generator=g).to(dtype) for _ in range(3))
+    q[..., 0] = 1.0
+    k[:, :, :64, 0] = -math.inf
+    out = flash_attention_v2(q.to(DEV), k.to(DEV), v.to(DEV)).cpu().double()
+    scores = (q.double() @ k.double().transpose(-1, -2)) / math.sqrt(d)
+    scores.masked_fill_(torch.ones(200, 200, dtype=torch.bool).triu(1), -math.inf)
+    want = (scores.softmax(-1)[:, :, 64:, 64:] @ v.double()[:, :, 64:])
+    assert (out[:, :, 64:] - want).abs().max() <= BASE_TOL[dtype]
+    assert _lib.device_status() == 0
+
+
 def test_spill_mode_chunks_change_no_bit(monkeypatch):
     """With a scratch bound of 3 MiB the spill mode works through [3, 5, 700, 64] (0.7 MiB per
     head) in chunks of 3 + 2 heads per batch entry; with 8 MiB in chunks of 2 + 1 batch
