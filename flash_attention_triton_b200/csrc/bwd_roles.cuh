@@ -192,6 +192,11 @@ struct DkdvCfg {
   static constexpr int kCols = kW / kGroups;     // score columns of a compute thread
   static constexpr int kStepBytes = T::kTileBytes / 128 * kW;
   static constexpr int kStages = kW == 64 && !FUSE ? 4 : 2;  // Q (+rowstats) ring and dO ring
+  // Barriers of St, step t on barrier t % kStBars.  Warp Y waits for St(t+1) only to let it into the tensor
+  // pipe first, so nothing but the Q ring keeps warp X from completing St(t+2) before Y has looked: with two
+  // stages Q(t+2) needs the slot that Y's dK(t) gives back, with more stages it does not, and Y would
+  // find the phase it waits for gone.  On two barriers the next completion is St(t+3), which needs dPt(t+2), Y's own.
+  static constexpr int kStBars = kStages > 2 ? 2 : 1;
   static constexpr int kRedWarp = 4 * kGroups;   // first reduction warp (FUSE)
   static constexpr int kMmaWarp = kRedWarp + (FUSE ? 4 : 0);
   static constexpr int kThreads = 32 * (kMmaWarp + 4);
@@ -218,7 +223,7 @@ struct DkdvCfg {
   static constexpr int kBarDOFull = kBarQEmpty + kStages;  // kStages
   static constexpr int kBarDOEmpty = kBarDOFull + kStages;
   static constexpr int kBarStFull = kBarDOEmpty + kStages;
-  static constexpr int kBarDptFull = kBarStFull + 1;
+  static constexpr int kBarDptFull = kBarStFull + kStBars;
   static constexpr int kBarPtReady = kBarDptFull + 1;   // one arrival per compute warp
   static constexpr int kBarDsReady = kBarPtReady + 1;   // one arrival per compute warp
   static constexpr int kBarDqFull = kBarDsReady + 1;
@@ -273,7 +278,7 @@ __device__ __forceinline__ void dkdv_init_barriers(uint32_t bar0) {
     mbar_init(bar(C::kBarDOFull + i), 1);
     mbar_init(bar(C::kBarDOEmpty + i), 2);  // dV (warp X) and dPt (warp Y) both done
   }
-  mbar_init(bar(C::kBarStFull), 1);
+  for (int i = 0; i < C::kStBars; ++i) mbar_init(bar(C::kBarStFull + i), 1);
   mbar_init(bar(C::kBarDptFull), 1);
   mbar_init(bar(C::kBarPtReady), 4 * C::kGroups);
   mbar_init(bar(C::kBarDsReady), 4 * C::kGroups);
@@ -395,7 +400,7 @@ __device__ __forceinline__ void dkdv_roles(
         // ------------------------------------------------------------ warp X
         if (ok && (ok = mbar_wait(bar(C::kBarQFull + 0), 0, w, kBSiteMmaQ))) {
           issue_rows_x_rows<D, BF16, W, KD>(elected, tmem_base + C::kColSt, ka, smem_base + C::kOffQ);
-          commit(C::kBarStFull);
+          commit(C::kBarStFull + 0);
           commit(C::kBarQEmpty + 0);
         }
         for (int t = 0; ok && t < nsteps; ++t) {
@@ -411,7 +416,7 @@ __device__ __forceinline__ void dkdv_roles(
             if (!(ok = mbar_wait(bar(C::kBarQFull + s1), ph1, w, kBSiteMmaQ))) break;
             issue_rows_x_rows<D, BF16, W, KD>(elected, tmem_base + C::kColSt, ka,
                                           smem_base + C::kOffQ + s1 * C::kStepBytes);  // St(t+1)
-            commit(C::kBarStFull);
+            commit(C::kBarStFull + (t + 1) % C::kStBars);
             commit(C::kBarQEmpty + s1);
           }
           s = s1;
@@ -435,7 +440,9 @@ __device__ __forceinline__ void dkdv_roles(
             // St(t+1) sits on the critical chain St -> Pt -> dV -> St; let warp X get it into
             // the in-order pipe first, dK and dPt(t+1) then run under the next exponentials.
             if (t + 1 < nsteps) {
-              if (!(ok = mbar_wait(bar(C::kBarStFull), (t + 1) & 1, w, kBSiteMmaQ))) break;
+              if (!(ok = mbar_wait(bar(C::kBarStFull + (t + 1) % C::kStBars), ((t + 1) / C::kStBars) & 1, w,
+                                   kBSiteMmaQ)))
+                break;
             }
           }
           tc_fence_after();
@@ -527,7 +534,7 @@ __device__ __forceinline__ void dkdv_roles(
       const float4* nlse = reinterpret_cast<const float4*>(stats + wg * kCols);      // -lse*log2e
       const float4* ndlt = reinterpret_cast<const float4*>(stats + W + wg * kCols);  // -delta
       if (!(ok = mbar_wait_warp(bar(C::kBarQFull + s), ph, w, kBSiteCmpQ))) break;
-      if (!(ok = mbar_wait_warp(bar(C::kBarStFull), t & 1, w, kBSiteCmpSt))) break;
+      if (!(ok = mbar_wait_warp(bar(C::kBarStFull + t % C::kStBars), (t / C::kStBars) & 1, w, kBSiteCmpSt))) break;
       tc_fence_after();
       float2 p[kPairs];  // P^T for this thread's kv row, q columns wg*kCols ..
       {

@@ -1,0 +1,165 @@
+// Runs the kernels' warp roles on the CPU, one coroutine per warp, under many schedules: random priorities,
+// re-drawn now and then, decide which warp, copy or tensor-pipe arrival goes on at every barrier
+// operation, so one or the other is held back for as long as the rest can go on without it.  A schedule
+// fails when nothing can go on (deadlock), when a warp arrives twice in one phase of a barrier (it has
+// stood in for another one), or when a wait returns on a phase its warp has already seen.  One CTA runs
+// at a time, one lane of each warp; data does not exist.
+#include "cuda_runtime.h"
+#include <ucontext.h>
+#include <unistd.h>
+#include <cstdio>
+#include <cstdlib>
+#include <deque>
+#include <map>
+#include <memory>
+#include <random>
+#include <set>
+#include <vector>
+
+dim3 threadIdx, blockIdx, gridDim;
+namespace fa2 { namespace { alignas(1024) uint8_t smem[232448]; } }
+uint8_t* sim_smem = fa2::smem;
+
+namespace {
+struct Barrier {
+  unsigned count = 0, pending = 0, completed = 0;
+  std::map<int, unsigned> seen;  // warp -> completed phases at its last successful wait, plus one
+  std::set<int> arrived;         // in the current phase
+};
+std::map<uint32_t, Barrier> barriers;
+struct Arrival { uint32_t bar; int warp; };
+std::vector<Arrival> copies;
+std::deque<Arrival> pipe_queue;
+struct Warp {
+  ucontext_t ctx;
+  std::unique_ptr<char[]> stack;
+  bool done = false, at_sync = false;
+  uint32_t bar = 0, parity = 0;
+  int site = -1;  // >= 0: waiting
+};
+std::vector<Warp> warps;
+ucontext_t scheduler;
+int current;
+std::mt19937 rng;
+
+[[noreturn]] void fail(const char* what, uint32_t bar, int warp, int site) {
+  printf("%s: block %u, hardware warp %d, barrier +%u, wait site %d\n", what, blockIdx.x, warp, bar, site);
+  fflush(stdout);
+  _exit(1);
+}
+void arrive(Arrival a) {
+  Barrier& b = barriers[a.bar];
+  if (!b.arrived.insert(a.warp).second) fail("second arrival in one phase", a.bar, a.warp, -1);
+  if (--b.pending == 0) b.pending = b.count, ++b.completed, b.arrived.clear();
+}
+bool passes(uint32_t bar, uint32_t parity) { return (barriers[bar].completed & 1u) != parity; }
+void yield() { swapcontext(&warps[current].ctx, &scheduler); }
+void (*body_fn)(void*);
+void* body_arg;
+void entry() {
+  body_fn(body_arg);
+  warps[current].done = true;
+  yield();
+}
+}  // namespace
+
+void sim_init(uint32_t bar, uint32_t count) { barriers[bar] = Barrier{count, count, 0, {}, {}}; }
+void sim_arrive(uint32_t bar) { yield(); arrive({bar, current}); }
+void sim_arrive_later(uint32_t bar) { yield(); copies.push_back({bar, current}); }
+void sim_arrive_after_mma(uint32_t bar) { yield(); pipe_queue.push_back({bar, current}); }
+void sim_wait(uint32_t bar, uint32_t parity, int site) {
+  Warp& w = warps[current];
+  w.bar = bar, w.parity = parity, w.site = site;
+  yield();  // resumed only when the wait passes
+  w.site = -1;
+  Barrier& b = barriers[bar];
+  unsigned& seen = b.seen[current];
+  if (seen >= b.completed + 1) fail("wait returned on a phase already seen", bar, current, site);
+  seen = b.completed + 1;
+}
+void __syncthreads() {
+  warps[current].at_sync = true;
+  yield();
+}
+void sim_run(unsigned n, void (*body)(void*), void* arg) {
+  body_fn = body, body_arg = arg;
+  barriers.clear(), copies.clear(), pipe_queue.clear();
+  warps = std::vector<Warp>(n);
+  for (unsigned i = 0; i < n; ++i) {
+    Warp& w = warps[i];
+    w.stack.reset(new char[1 << 17]);
+    getcontext(&w.ctx);
+    w.ctx.uc_stack.ss_sp = w.stack.get(), w.ctx.uc_stack.ss_size = 1 << 17, w.ctx.uc_link = nullptr;
+    makecontext(&w.ctx, entry, 0);
+  }
+  std::vector<unsigned> priority(n + 2);  // warps, copies, tensor pipe
+  auto draw = [&] { for (auto& p : priority) p = rng(); };
+  draw();
+  for (;;) {
+    if (rng() % 64 == 0) draw();
+    int best = -1;
+    auto offer = [&](int i) { if (best < 0 || priority[i] > priority[best]) best = i; };
+    unsigned done = 0, synced = 0;
+    for (unsigned i = 0; i < n; ++i) {
+      done += warps[i].done, synced += warps[i].at_sync;
+      if (!warps[i].done && !warps[i].at_sync && (warps[i].site < 0 || passes(warps[i].bar, warps[i].parity))) offer(i);
+    }
+    if (done == n) return;
+    if (done + synced == n) {
+      for (auto& w : warps) w.at_sync = false;
+      continue;
+    }
+    if (!copies.empty()) offer(n);
+    if (!pipe_queue.empty()) offer(n + 1);
+    if (best < 0)
+      for (unsigned i = 0; i < n; ++i)
+        if (warps[i].site >= 0) fail("deadlock", warps[i].bar, i, warps[i].site);
+    if (best == int(n)) {
+      const size_t k = rng() % copies.size();
+      const Arrival a = copies[k];
+      copies.erase(copies.begin() + k);
+      arrive(a);
+    } else if (best == int(n) + 1) {
+      const Arrival a = pipe_queue.front();
+      pipe_queue.pop_front();
+      arrive(a);
+    } else {
+      current = best;
+      threadIdx = dim3(32 * best, 0, 0);
+      swapcontext(&scheduler, &warps[best].ctx);
+    }
+  }
+}
+
+#include "bwd.cu"
+#include "fwd.cu"
+
+// main <kernel> <head dim> <rows> <keys> <schedules>
+int main(int, char** argv) {
+  using namespace fa2;
+  const std::string kernel = argv[1];
+  const int d = atoi(argv[2]), n = atoi(argv[3]), nk = atoi(argv[4]);
+  const AttnShape s{1, 1, n, padded_head_dim(d), 1, 1.f, d, nk};
+  std::vector<unsigned> amax((n + 127) / 128);
+  std::vector<float> scratch(dstile_pairs(n, nk) * 16384), lse(n), stats(amax.size() * 256);
+  CUtensorMap m{};
+  const F32Out none{nullptr, {}};
+  const RowStats rs{stats.data(), amax.data()};
+  int status = 0;
+  unsigned counter = 0;
+  const LaunchCtx ctx{&status, &counter, 1};
+  for (int seed = 0; seed < atoi(argv[5]); ++seed) {
+    rng.seed(seed);
+    if (kernel == "fwd") launch_fwd(s, m, m, m, m, none, lse.data(), ctx, nullptr);
+    if (kernel == "dkdv") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, nullptr, 0, &status, nullptr);
+    if (kernel == "dkdv_atomic") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 1, &status, nullptr);
+    if (kernel == "dkdv_spill") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 2, &status, nullptr);
+    if (kernel == "dq") launch_bwd_dq(s, m, m, m, m, m, none, rs, &status, nullptr);
+    if (kernel == "scores") launch_bwd_scores_wide(s, m, m, m, m, rs, scratch.data(), scratch.data(), &status, nullptr);
+    for (int form = 0; form < 3; ++form) {
+      if (kernel == "consume" && (d > 128 || form == 2)) launch_bwd_consume(s, form, scratch.data(), m, m, none, rs, false, &status, nullptr);
+      if (kernel == "consume_pair") launch_bwd_consume(s, form, scratch.data(), m, m, none, rs, true, &status, nullptr);
+    }
+  }
+  return 0;
+}

@@ -1,0 +1,42 @@
+"""The warp roles of the attention kernels under adversarial schedules, on the CPU.
+
+``tests/schedules`` compiles the kernel sources as they are with a host compiler: barriers, copies and
+the tensor pipe are simulated, arithmetic and data movement are left out, and the order in which warps go
+on is drawn at random with some of them held back for long.  No schedule may deadlock, let a warp
+arrive twice in one phase of a barrier, or let a wait return on a phase that it has already seen.
+"""
+
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+HERE = Path(__file__).resolve().parent
+CSRC = HERE.parent / "flash_attention_triton_b200" / "csrc"
+
+
+@pytest.fixture(scope="module")
+def simulator(tmp_path_factory):
+    build = tmp_path_factory.mktemp("schedules")
+    for source in (*(CSRC / n for n in ("common.cuh", "mma_issue.cuh", "bwd_roles.cuh", "bwd.cu", "fwd.cu")),
+                   *(HERE / "schedules").iterdir()):
+        shutil.copy(source, build)
+    for stand_in in ("cuda.h", "ptx.cuh"):
+        (build / stand_in).write_text('#include "cuda_runtime.h"\n')
+    subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-I.", "main.cpp", "-o", "simulator"], cwd=build, check=True,
+                   capture_output=True, text=True)
+    return build / "simulator"
+
+
+def check(simulator, kernel, headdim, rows, keys, schedules=60):
+    run = subprocess.run([simulator, kernel, str(headdim), str(rows), str(keys), str(schedules)],
+                         capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stdout + run.stderr
+
+
+@pytest.mark.parametrize("rows,keys", [(1, 1), (128, 64), (449, 300), (640, 640)])
+@pytest.mark.parametrize("kernel", ["dkdv", "dkdv_atomic", "dkdv_spill"])
+@pytest.mark.parametrize("headdim", [32, 64, 96, 128])
+def test_dk_dv_roles(simulator, kernel, headdim, rows, keys):
+    check(simulator, kernel, headdim, rows, keys)
