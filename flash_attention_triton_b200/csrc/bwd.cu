@@ -139,8 +139,12 @@ struct DqCfg {
   static constexpr int kBarSFull = kBarVEmpty + kVStages;  // 2 (one per score buffer)
   static constexpr int kBarDpFull = kBarSFull + 2;
   static constexpr int kBarDpConsumed = kBarDpFull + 1;  // one arrival per compute warp
-  static constexpr int kBarDsReady = kBarDpConsumed + 1;  // one arrival per compute warp
-  static constexpr int kBarDqDone = kBarDsReady + 1;      // 2: dQ += dS(j) K_j completed, by j%2
+  // 2, by j%2, one arrival per compute warp.  With S(j+1) in the other score buffer, a warp can be through with
+  // step j+1 before another one, held up after it has read dP(j), is through with step j; on one barrier
+  // it would arrive in that one's place, or complete a phase that the MMA warp has not looked at yet.
+  // Step j+2 needs S(j+2), which needs dQ += dS(j) K_j.
+  static constexpr int kBarDsReady = kBarDpConsumed + 1;
+  static constexpr int kBarDqDone = kBarDsReady + 2;      // 2: dQ += dS(j) K_j completed, by j%2
   static constexpr int kBarDone = kBarDqDone + 2;
   static constexpr int kNumBars = kBarDone + 1;
   static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;
@@ -200,7 +204,8 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
     mbar_init(bar(C::kBarSFull + 1), 1);
     mbar_init(bar(C::kBarDpFull), 1);
     mbar_init(bar(C::kBarDpConsumed), 4 * C::kGroups);
-    mbar_init(bar(C::kBarDsReady), 4 * C::kGroups);
+    mbar_init(bar(C::kBarDsReady + 0), 4 * C::kGroups);
+    mbar_init(bar(C::kBarDsReady + 1), 4 * C::kGroups);
     mbar_init(bar(C::kBarDqDone + 0), 1);
     mbar_init(bar(C::kBarDqDone + 1), 1);
     mbar_init(bar(C::kBarDone), 1);
@@ -327,7 +332,7 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
       int ks = 0, kph = 0;
       for (int j = 0; ok && j < nkv; ++j) {
         if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kBSiteMmaKV))) break;
-        if (!(ok = mbar_wait(bar(C::kBarDsReady), j & 1, w, kBSiteMmaDs))) break;
+        if (!(ok = mbar_wait(bar(C::kBarDsReady + (j & 1)), (j >> 1) & 1, w, kBSiteMmaDs))) break;
         tc_fence_after();
         // A = 16-bit dS over score buffer j%2, B = K_j as MN-major tile
         issue_tmem_x_tile<D, BF16, W, KD>(elected, tmem_base + C::kColDQ, tmem_base + C::kColS + (j & 1) * W,
@@ -410,7 +415,7 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(C::kBarDsReady));
+      if (lane == 0) mbar_arrive(bar(C::kBarDsReady + (j & 1)));
     }
     if (ok && wg == 0 && mbar_wait_warp(bar(C::kBarDone), 0, w, kBSiteCmpDone)) {
       tc_fence_after();

@@ -40,3 +40,9 @@ def check(simulator, kernel, headdim, rows, keys, schedules=60):
 @pytest.mark.parametrize("headdim", [32, 64, 96, 128])
 def test_dk_dv_roles(simulator, kernel, headdim, rows, keys):
     check(simulator, kernel, headdim, rows, keys)
+
+
+@pytest.mark.parametrize("rows,keys", [(1, 1), (128, 64), (449, 300), (640, 640)])
+@pytest.mark.parametrize("headdim", [32, 64, 96, 128])
+def test_dq_roles(simulator, headdim, rows, keys):
+    check(simulator, "dq", headdim, rows, keys)
