@@ -164,7 +164,8 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
   // global counter in head-major, heavy-pair-first order, like a hardware block scheduler
   // would hand them out, but without the launch gap and with tensor memory kept allocated.
   // Between items all roles meet at a barrier and the mbarriers are re-initialised, so each
-  // item starts from phase 0.
+  // item starts from phase 0.  Nothing may still be on its way to an mbarrier then: the MMA warps commit
+  // only what another role waits for, no release of a ring stage that is not filled again.
   for (bool first = true;; first = false) {
     __syncthreads();  // every role has finished the previous item
     if (threadIdx.x == 0) {
@@ -269,7 +270,10 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
       bool ok = mbar_wait(bar(C::kBarQFull), 0, w, kSiteMmaQ);
       int ks = 0, kph = 0;          // K ring position of tile j
       int prev_i = -1, prev_ph = 0;  // group and phase of the previous score product
-      auto next_k = [&]() {
+      int k_left = nkv * HALVES;  // staged tiles of this item not released yet
+      auto release_k = [&]() {
+        if (elected && k_left > C::kKStages) mma_commit(bar(C::kBarKEmpty + ks));
+        --k_left;
         if (++ks == C::kKStages) {
           ks = 0;
           kph ^= 1;
@@ -293,8 +297,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
               issue_rows_x_rows<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColS,
                                           smem_base + C::kOffQ + half * T::kTileBytes,
                                           smem_base + C::kOffK + ks * C::kKvBytes, half);
-              if (elected) mma_commit(bar(C::kBarKEmpty + ks));
-              next_k();
+              release_k();
             }
             if (!ok) break;
           } else {
@@ -307,17 +310,17 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
           prev_ph = j & 1;
         }
         if (!ok) break;
-        if constexpr (!WIDE) {
-          if (elected) mma_commit(bar(C::kBarKEmpty + ks));  // both products that read K_j issued
-          next_k();
-        }
+        if constexpr (!WIDE) release_k();  // both products that read K_j issued
       }
     } else if (warp == 10) {
       // ---------------------------------------------------------------- O_i += P_i V_j issuer
       const uint32_t elected = elect_one();
       bool ok = true;
       int vs = 0, vph = 0;  // V ring position of tile j
-      auto next_v = [&]() {
+      int v_left = nkv * HALVES;
+      auto release_v = [&]() {
+        if (elected && v_left > C::kVStages) mma_commit(bar(C::kBarVEmpty + vs));
+        --v_left;
         if (++vs == C::kVStages) {
           vs = 0;
           vph ^= 1;
@@ -339,8 +342,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
               issue_tmem_x_tile<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColO + half * DT,
                                           tmem_base + C::kColP, W / 4,
                                           smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
-              if (elected) mma_commit(bar(C::kBarVEmpty + vs));
-              next_v();
+              release_v();
             }
             if (!ok) break;
           } else {
@@ -351,10 +353,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
           if (elected) mma_commit(bar(C::kBarPvDone + i));
         }
         if (!ok) break;
-        if constexpr (!WIDE) {
-          if (elected) mma_commit(bar(C::kBarVEmpty + vs));
-          next_v();
-        }
+        if constexpr (!WIDE) release_v();
       }
     }
     __syncwarp();

@@ -46,3 +46,17 @@ def test_dk_dv_roles(simulator, kernel, headdim, rows, keys):
 @pytest.mark.parametrize("headdim", [32, 64, 96, 128])
 def test_dq_roles(simulator, headdim, rows, keys):
     check(simulator, "dq", headdim, rows, keys)
+
+
+@pytest.mark.parametrize("rows,keys", [(1, 1), (128, 64), (449, 300), (1200, 1200)])
+@pytest.mark.parametrize("headdim", [32, 64, 96, 128, 256])
+def test_forward_roles(simulator, headdim, rows, keys):
+    """One CTA takes every work item: what an item leaves on its way to a barrier meets the next one."""
+    check(simulator, "fwd", headdim, rows, keys)
+
+
+@pytest.mark.parametrize("rows,keys", [(1, 1), (128, 64), (449, 300), (640, 640)])
+@pytest.mark.parametrize("kernel,headdim", [("scores", 256), ("consume", 64), ("consume", 128), ("consume", 256),
+                                            ("consume_pair", 256)])
+def test_spill_roles(simulator, kernel, headdim, rows, keys):
+    check(simulator, kernel, headdim, rows, keys)
