@@ -222,8 +222,7 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
-  // Nothing here depends on the dK/dV kernel before it; what that one waited for has completed.  The
-  // wait for it stands at the end.
+  grid_wait_previous();
   grid_allow_next();
 
   if (warp >= C::kMmaWarp) {
@@ -427,7 +426,6 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
     }
   }
 
-  grid_wait_previous();
   tc_fence_before();
   __syncthreads();
   if (warp == C::kMmaWarp) {
@@ -509,10 +507,7 @@ __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, ConsumeCfg<D>::kCtasP
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
-  // Forms 1 (dK) and 2 (dQ) of head dim 256 do not depend on the consumer before them, only on what that
-  // one waited for; their wait stands at the end.
-  constexpr bool kIndependent = D == 256 && FORM != 0;
-  if constexpr (!kIndependent) grid_wait_previous();
+  grid_wait_previous();
   grid_allow_next();
 
   consume_roles<D, BF16, FORM, C::kStages, KD>(smem, smem_base, smem_base + C::kOffBar, tmem_base,
@@ -520,7 +515,6 @@ __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, ConsumeCfg<D>::kCtasP
                                            warp < 4 ? warp : -1, lane, scratch, &tb, &tout, out32, cols, N, Nk, w,
                                            item);
 
-  if constexpr (kIndependent) grid_wait_previous();
   tc_fence_before();
   __syncthreads();
   if (warp == C::kMmaWarp) {
@@ -619,8 +613,7 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtx w{abort_flag, status};
-  constexpr bool kIndependent = FORM != 0;  // as in bwd_consume_kernel
-  if constexpr (!kIndependent) grid_wait_previous();
+  grid_wait_previous();
   grid_allow_next();
 
   if (warp == C::kLoadWarp) {
@@ -690,7 +683,6 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
     }
   }
 
-  if constexpr (kIndependent) grid_wait_previous();
   tc_fence_before();
   __syncthreads();
   if (warp == C::kMmaWarp) {

@@ -143,8 +143,7 @@ __device__ __forceinline__ int fetch_work_item(unsigned int* work_counter, int t
 // whole kernel.  Launch, set-up and the last wave of a kernel are what this covers; microseconds, plain
 // launches against these: backward [4,16,2048,64] recompute 172 / 185 -> 167 / 171, atomic 173 -> 166,
 // [8,16,1000,64] 113 -> 107, [8,12,4095,32] 757 -> 736, [32,20,1024,96] 782 -> 764, [2,16,8192,256] 3175
-// -> 3065 (of that 2 % from the consumers that wait at their end only); forward [4,16,2048,64] 64.5 ->
-// 59; [2,32,8192,128] unchanged.
+// -> 3065; forward [4,16,2048,64] 64.5 -> 59; [2,32,8192,128] unchanged.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, int threads, int smem_bytes,
                                     cudaStream_t stream, Args&&... args) {

@@ -96,6 +96,8 @@ size_t fa2_rowstats_bytes(int B, int H, int N);
  * its Q tiles from the last one down to the diagonal); the modes differ in how dQ is formed and
  * in the workspace they need (`workspace`, 256-byte aligned, `workspace_bytes` long; the call
  * never writes beyond it and returns FA2_ERR_WORKSPACE when it is below the mode's minimum).
+ * dq may be the memory of q or of dout (16-bit dq with their strides): its rows are written after their last
+ * reader has ended, in every mode.  No other output may overlap an input or another output.
  *   deterministic == 1 ("recompute"): dK/dV kernel + a separate dQ kernel that recomputes S and
  *     dP; every output tile has one owner and a fixed accumulation order, so results are
  *     bit-identical across runs, SM counts and (batch, head) partitionings.  No workspace

@@ -54,6 +54,8 @@ void sim_arrive_after_mma(uint32_t bar);  // behind everything in the in-order t
 void sim_init(uint32_t bar, uint32_t count);
 void sim_wait(uint32_t bar, uint32_t parity, int site);
 void __syncthreads();
+void sim_wait_previous();
+void sim_access();  // of global memory: not before the kernel has waited for its predecessor
 void sim_run(unsigned warps, void (*body)(void*), void* arg);
 
 template <typename... Params, typename... Args>
@@ -70,7 +72,7 @@ cudaError_t cudaLaunchKernelEx(const cudaLaunchConfig_t* cfg, void (*kernel)(Par
 inline void __syncwarp() {}
 inline bool __any_sync(unsigned, bool x) { return x; }
 inline unsigned __reduce_max_sync(unsigned, unsigned x) { return x; }
-template <typename T> T __ldg(const T* p) { return *p; }
+template <typename T> T __ldg(const T* p) { return sim_access(), *p; }
 template <typename T> T atomicAdd(T* p, T v) { T old = *p; *p += v; return old; }
 template <typename T> T atomicExch(T* p, T v) { T old = *p; *p = v; return old; }
 template <typename T> T atomicCAS(T* p, T cmp, T v) { T old = *p; if (old == cmp) *p = v; return old; }
@@ -98,7 +100,7 @@ inline uint32_t elect_one() { return 1; }
 inline void mbar_init(uint32_t bar, uint32_t count) { sim_init(bar, count); }
 inline void mbar_inval(uint32_t) {}
 inline void mbar_arrive(uint32_t bar) { sim_arrive(bar); }
-inline void mbar_arrive_expect_tx(uint32_t bar, uint32_t) { sim_arrive_later(bar); }
+inline void mbar_arrive_expect_tx(uint32_t bar, uint32_t) { sim_access(), sim_arrive_later(bar); }
 inline void mma_commit(uint32_t bar) { sim_arrive_after_mma(bar); }
 inline bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx&, int site) { return sim_wait(bar, parity, site), true; }
 inline bool mbar_wait_warp(uint32_t bar, uint32_t parity, const WaitCtx&, int site) { return sim_wait(bar, parity, site), true; }
@@ -115,7 +117,8 @@ FA2_NOTHING(tma_store_4d) FA2_NOTHING(tma_store_commit) FA2_NOTHING(tma_store_wa
 FA2_NOTHING(prefetch_tensormap) FA2_NOTHING(tmem_alloc) FA2_NOTHING(tmem_relinquish) FA2_NOTHING(tmem_dealloc)
 FA2_NOTHING(tc_fence_before) FA2_NOTHING(tc_fence_after) FA2_NOTHING(tmem_wait_ld) FA2_NOTHING(tmem_wait_st)
 FA2_NOTHING(tmem_st_x32) FA2_NOTHING(tmem_st_x16) FA2_NOTHING(mma_ss) FA2_NOTHING(mma_ts) FA2_NOTHING(st_global_8)
-FA2_NOTHING(grid_wait_previous) FA2_NOTHING(grid_allow_next)
+FA2_NOTHING(grid_allow_next)
+inline void grid_wait_previous() { sim_wait_previous(); }
 template <int N> void reg_inc() {}
 template <int N> void reg_dec() {}
 }  // namespace fa2

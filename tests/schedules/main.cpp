@@ -2,8 +2,9 @@
 // re-drawn now and then, decide which warp, copy or tensor-pipe arrival goes on at every barrier
 // operation, so one or the other is held back for as long as the rest can go on without it.  A schedule
 // fails when nothing can go on (deadlock), when a warp arrives twice in one phase of a barrier (it has
-// stood in for another one), or when a wait returns on a phase its warp has already seen.  One CTA runs
-// at a time, one lane of each warp; data does not exist.
+// stood in for another one), when a wait returns on a phase its warp has already seen, or when a warp
+// starts a copy from global memory before it has waited for the kernel before its own.  One CTA runs at a
+// time, one lane of each warp; data does not exist.
 #include "cuda_runtime.h"
 #include <ucontext.h>
 #include <unistd.h>
@@ -33,7 +34,7 @@ std::deque<Arrival> pipe_queue;
 struct Warp {
   ucontext_t ctx;
   std::unique_ptr<char[]> stack;
-  bool done = false, at_sync = false;
+  bool done = false, at_sync = false, waited_previous = false;
   uint32_t bar = 0, parity = 0;
   int site = -1;  // >= 0: waiting
 };
@@ -76,6 +77,10 @@ void sim_wait(uint32_t bar, uint32_t parity, int site) {
   unsigned& seen = b.seen[current];
   if (seen >= b.completed + 1) fail("wait returned on a phase already seen", bar, current, site);
   seen = b.completed + 1;
+}
+void sim_wait_previous() { warps[current].waited_previous = true; }
+void sim_access() {
+  if (!warps[current].waited_previous) fail("access before the wait for the previous kernel", 0, current, -1);
 }
 void __syncthreads() {
   warps[current].at_sync = true;

@@ -3,7 +3,8 @@
 ``tests/schedules`` compiles the kernel sources as they are with a host compiler: barriers, copies and
 the tensor pipe are simulated, arithmetic and data movement are left out, and the order in which warps go
 on is drawn at random with some of them held back for long.  No schedule may deadlock, let a warp
-arrive twice in one phase of a barrier, or let a wait return on a phase that it has already seen.
+arrive twice in one phase of a barrier, or let a wait return on a phase that it has already seen; and no
+warp may read global memory before it has waited for the kernel before its own.
 """
 
 import shutil

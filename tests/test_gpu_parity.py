@@ -477,6 +477,43 @@ def test_packed_qkv_through_the_strided_c_abi(det):
     assert not torch.isnan(dqkv).any()  # every element of the packed gradient was written
 
 
+@pytest.mark.parametrize("mode,d", [(0, 64), (1, 32), (1, 64), (1, 128), (2, 64), (2, 128), (2, 256)])
+@pytest.mark.parametrize("heads", [3, 80])  # at head dim 256: one and two output tiles per CTA
+@pytest.mark.parametrize("target", ["q", "dout"])
+def test_dq_may_take_the_memory_of_q_or_dout(target, heads, mode, d):
+    b, n = 2, 700
+    g = torch.Generator(device=DEV).manual_seed(d)
+    q, k, v, do = (torch.randn(b, heads, n, d, device=DEV, generator=g).half() for _ in range(4))
+    lib = _lib.lib()
+    st = torch.cuda.current_stream().cuda_stream
+    scale = 1.0 / math.sqrt(d)
+    o, lse = torch.empty_like(q), torch.empty(b, heads, n, device=DEV)
+    rs = torch.empty(lib.fa2_rowstats_bytes(b, heads, n) // 4, device=DEV)
+    wsb = lib.fa2_bwd_workspace_bytes(b, heads, n, d, mode)
+    ws = torch.empty(max(wsb, 256), device=DEV, dtype=torch.uint8)
+
+    def backward(q, do, dq):
+        dk, dv = torch.empty_like(k), torch.empty_like(v)
+        assert lib.fa2_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
+                           b, heads, n, d, 0, scale, st) == 0
+        assert lib.fa2_bwd_preprocess(o.data_ptr(), do.data_ptr(), lse.data_ptr(), rs.data_ptr(),
+                                      b, heads, n, d, 0, st) == 0
+        assert lib.fa2_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), do.data_ptr(), rs.data_ptr(), dq.data_ptr(),
+                           dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), wsb, b, heads, n, d, 0, scale, mode, st) == 0
+        return dq, dk, dv
+
+    want = backward(q, do, torch.empty_like(q))
+    for _ in range(3):
+        q2, do2 = q.clone(), do.clone()
+        got = backward(q2, do2, q2 if target == "q" else do2)
+        for name, x, y in zip(("dq", "dk", "dv"), got, want):
+            if name == "dq" and mode == 0:  # one ulp of fp16 at most between two summation orders in fp32
+                assert ((x.float() - y.float()).abs() <= 2e-3 * y.float().abs() + 1e-5).all()
+            else:
+                assert torch.equal(x, y), name
+    assert _lib.device_status() == 0
+
+
 def test_unsupported_head_dim_raises():
     q = torch.randn(1, 1, 64, 264, device=DEV, dtype=torch.float16)
     with pytest.raises(ValueError, match="head dimension"):
