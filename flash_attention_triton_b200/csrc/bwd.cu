@@ -35,8 +35,8 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                     const __grid_constant__ CUtensorMap tdk,
                     const __grid_constant__ CUtensorMap tdv, const __grid_constant__ F32Out dk32,
-                    const __grid_constant__ F32Out dv32, int cols, const float* __restrict__ rowstats,
-                    const unsigned* __restrict__ tile_amax, float* __restrict__ dq_accum, int N,
+                    const __grid_constant__ F32Out dv32, int cols, const float* rowstats,
+                    const unsigned* tile_amax, float* __restrict__ dq_accum, int N,
                     int Nk, int num_bh, int num_heads, int group, float scale, float scale_log2,
                     int* status) {
   using C = DkdvCfg<D, MODE>;
@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
     bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                   const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                   const __grid_constant__ CUtensorMap tdq, const __grid_constant__ F32Out dq32, int cols,
-                  const float* __restrict__ rowstats,
-                  const unsigned* __restrict__ tile_amax, int N, int Nk, int num_bh, int num_heads,
+                  const float* rowstats,
+                  const unsigned* tile_amax, int N, int Nk, int num_bh, int num_heads,
                   int group, float scale, float scale_log2, int* status) {
   using C = DqCfg<D>;
   using T = Tile<D>;
@@ -464,9 +464,9 @@ struct ConsumeCfg {
 
 template <int D, bool BF16, int FORM, int KD = D>
 __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, ConsumeCfg<D>::kCtasPerSm)
-    bwd_consume_kernel(const uint4* __restrict__ scratch, const __grid_constant__ CUtensorMap tb,
+    bwd_consume_kernel(const uint4* scratch, const __grid_constant__ CUtensorMap tb,
                        const __grid_constant__ CUtensorMap tout, const __grid_constant__ F32Out out32, int cols,
-                       const unsigned* __restrict__ tile_amax, int N, int Nk, int num_bh,
+                       const unsigned* tile_amax, int N, int Nk, int num_bh,
                        int num_heads, int group, int* status) {
   using C = ConsumeCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -557,9 +557,9 @@ struct ConsumePairCfg {
 
 template <bool BF16, int FORM>
 __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
-    bwd_consume_pair_kernel(const uint4* __restrict__ scratch, const __grid_constant__ CUtensorMap tb,
+    bwd_consume_pair_kernel(const uint4* scratch, const __grid_constant__ CUtensorMap tb,
                             const __grid_constant__ CUtensorMap tout, const __grid_constant__ F32Out out32,
-                            int cols, const unsigned* __restrict__ tile_amax, int N, int Nk, int num_bh,
+                            int cols, const unsigned* tile_amax, int N, int Nk, int num_bh,
                             int num_heads, int group, int* status) {
   using C = ConsumePairCfg;
   using T = Tile<256>;
@@ -734,8 +734,8 @@ template <bool BF16>
 __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
     bwd_scores_wide_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                            const __grid_constant__ CUtensorMap tv,
-                           const __grid_constant__ CUtensorMap tdo, const float* __restrict__ rowstats,
-                           const unsigned* __restrict__ tile_amax, uint4* __restrict__ p_scratch,
+                           const __grid_constant__ CUtensorMap tdo, const float* rowstats,
+                           const unsigned* tile_amax, uint4* __restrict__ p_scratch,
                            uint4* __restrict__ ds_scratch, int N, int Nk, int num_bh,
                            int num_heads, int group, float scale, float scale_log2, int* status) {
   using C = ScoresCfg;

@@ -137,10 +137,10 @@ __device__ __forceinline__ void store_rows_f32(uint32_t tmem_row_addr, const F32
 // |dO| as its 16-bit pattern with the sign cleared (written by the preprocess kernel); called by
 // a whole warp.  Returns 2^k and stores 2^-k in *inverse; 1 for an all-zero or non-finite head.
 template <bool BF16>
-__device__ __forceinline__ float head_dscale(const unsigned* __restrict__ tile_amax, int ntiles,
+__device__ __forceinline__ float head_dscale(const unsigned* tile_amax, int ntiles,
                                              int lane, float* inverse) {
   unsigned m = 0;
-  for (int t = lane; t < ntiles; t += 32) m = max(m, __ldg(tile_amax + t));
+  for (int t = lane; t < ntiles; t += 32) m = max(m, ld_global(tile_amax + t));
   m = __reduce_max_sync(0xffffffffu, m);
   int k = 0;
   if constexpr (BF16) {
@@ -310,7 +310,7 @@ __device__ __forceinline__ void dkdv_roles(
     uint8_t* smem, uint32_t smem_base, uint32_t tmem_base, int warp, int lane,
     const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, const CUtensorMap* tdo,
     const CUtensorMap* tdk, const CUtensorMap* tdv, const F32Out& dk32, const F32Out& dv32, int cols,
-    const float* __restrict__ rowstats, float* __restrict__ dq_accum, int N, int Nk, float scale, float scale_log2, const WaitCtx& w,
+    const float* rowstats, float* __restrict__ dq_accum, int N, int Nk, float scale, float scale_log2, const WaitCtx& w,
     const DkdvItem& item) {
   using C = DkdvCfg<D, MODE>;
   constexpr bool FUSE = C::FUSE;
@@ -660,7 +660,7 @@ struct ConsumeItem {
 template <int D, bool BF16, int FORM, int STAGES, int KD = D>
 __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base, uint32_t bar0,
                                               uint32_t tmem_acc, bool is_load_warp, bool is_mma_warp,
-                                              int epi_warp, int lane, const uint4* __restrict__ scratch,
+                                              int epi_warp, int lane, const uint4* scratch,
                                               const CUtensorMap* tb, const CUtensorMap* tout,
                                               const F32Out& out32, int cols, int N,
                                               int Nk, const WaitCtx& w, const ConsumeItem& item) {

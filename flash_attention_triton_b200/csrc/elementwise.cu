@@ -33,14 +33,6 @@ __device__ __forceinline__ float dot8(const uint4& a, const uint4& b) {
   return acc;
 }
 
-__device__ __forceinline__ uint4 ld_stream(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
-
 constexpr int kPreThreads = 256;
 constexpr int kPreMaxInFlight = 8;  // rows a thread group has in flight at once (2 x 16 bytes each)
 constexpr float kLog2e = 1.4426950408889634f;
@@ -57,8 +49,8 @@ constexpr float kLog2e = 1.4426950408889634f;
 // 16-bit pattern with the sign cleared, in tile_amax[tile] (see head_dscale in bwd_roles.cuh).
 template <int D, bool BF16>
 __global__ void __launch_bounds__(kPreThreads)
-    bwd_preprocess_kernel(const uint4* __restrict__ o, const uint4* __restrict__ dout,
-                          const float* __restrict__ lse, float* __restrict__ rowstats,
+    bwd_preprocess_kernel(const uint4* o, const uint4* dout,
+                          const float* lse, float* __restrict__ rowstats,
                           unsigned* __restrict__ tile_amax, int N, int ntiles, int d8, int H,
                           Strides so, Strides sdo) {
   constexpr int kLanesPerRow = D / 8;
@@ -87,8 +79,8 @@ __global__ void __launch_bounds__(kPreThreads)
       const int r = (p0 + i) * kRowsPerPass + row_in_pass;  // row inside the tile
       const long long row = static_cast<long long>(t) * 128 + r;
       if (row < N && sub < d8) {
-        a[i] = ld_stream(o_head + row * so.n + sub);
-        b[i] = ld_stream(do_head + row * sdo.n + sub);
+        a[i] = ld_global_once(o_head + row * so.n + sub);
+        b[i] = ld_global_once(do_head + row * sdo.n + sub);
       } else {
         a[i] = make_uint4(0, 0, 0, 0);
         b[i] = make_uint4(0, 0, 0, 0);
@@ -108,7 +100,7 @@ __global__ void __launch_bounds__(kPreThreads)
       if (sub == 0) {
         const long long row = static_cast<long long>(t) * 128 + r;
         const bool valid = row < N;
-        out[r] = valid ? -lse[bh * N + row] * kLog2e : -INFINITY;
+        out[r] = valid ? -ld_global(lse + bh * N + row) * kLog2e : -INFINITY;
         out[128 + r] = valid ? -acc : 0.f;
       }
     }
@@ -173,8 +165,8 @@ __device__ __forceinline__ bool consumers_all(bool ok, int nthreads) {
 
 template <int D, bool BF16>
 __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
-    bwd_preprocess_ring_kernel(const uint4* __restrict__ o, const uint4* __restrict__ dout,
-                               const float* __restrict__ lse, float* __restrict__ rowstats,
+    bwd_preprocess_ring_kernel(const uint4* o, const uint4* dout,
+                               const float* lse, float* __restrict__ rowstats,
                                unsigned* __restrict__ tile_amax, int N, int ntiles,
                                long long tiles, int d8, int H, Strides so, Strides sdo,
                                int* status) {
@@ -246,7 +238,7 @@ __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
 #pragma unroll
     for (int i = 0; i < kPasses; ++i) {
       const int row = t * 128 + i * kRowsPerPass + row_in_pass;
-      dst[i] = (sub == 0 && tile < tiles && row < N) ? __ldg(lse + bh * N + row) : INFINITY;
+      dst[i] = (sub == 0 && tile < tiles && row < N) ? ld_global(lse + bh * N + row) : INFINITY;
     }
   };
   fetch_lse(blockIdx.x, lse_cur);
@@ -339,7 +331,7 @@ __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
 // (the layout the fused backward kernel accumulates into).
 template <int D, bool BF16>
 __global__ void __launch_bounds__(256)
-    dq_convert_kernel(const float4* __restrict__ acc, uint4* __restrict__ dq, F32Out dq32, int N, int ntiles,
+    dq_convert_kernel(const float4* acc, uint4* __restrict__ dq, F32Out dq32, int N, int ntiles,
                       long long total, int d8, int H, Strides sdq) {
   grid_wait_previous();
   grid_allow_next();
@@ -357,8 +349,8 @@ __global__ void __launch_bounds__(256)
   const int row = tile * 128 + w * 32 + lane;
   if (row >= N || k8 >= d8) return;  // padding rows / padding columns of the accumulator
   const long long blk = (tile_global * 4 + w) * (D / 4);  // in units of [32 lanes][float4]
-  const float4 x = acc[(blk + 2 * k8) * 32 + lane];
-  const float4 y = acc[(blk + 2 * k8 + 1) * 32 + lane];
+  const float4 x = ld_global(acc + (blk + 2 * k8) * 32 + lane);
+  const float4 y = ld_global(acc + (blk + 2 * k8 + 1) * 32 + lane);
   const long long bb = bh / H, hh = bh - bb * H;
   if (dq32.p != nullptr) {
     const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};

@@ -127,6 +127,34 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, co
 __device__ __forceinline__ void grid_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Loads of what an earlier kernel of the stream wrote, which may still be running when this one starts.  The
+// read-only path (__ldg, ld.global.nc, what the compiler makes of a const __restrict__ parameter) is for
+// memory that nobody writes while the kernel lives, and such a load may be moved above
+// grid_wait_previous; these are coherent and stay behind it.
+__device__ __forceinline__ float ld_global(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned ld_global(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 ld_global(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+// Read once: not kept in L1.
+__device__ __forceinline__ uint4 ld_global_once(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+
 // ----------------------------------------------------------------------------------------
 // Proxy fences and named barriers
 // ----------------------------------------------------------------------------------------

@@ -72,7 +72,6 @@ cudaError_t cudaLaunchKernelEx(const cudaLaunchConfig_t* cfg, void (*kernel)(Par
 inline void __syncwarp() {}
 inline bool __any_sync(unsigned, bool x) { return x; }
 inline unsigned __reduce_max_sync(unsigned, unsigned x) { return x; }
-template <typename T> T __ldg(const T* p) { return sim_access(), *p; }
 template <typename T> T atomicAdd(T* p, T v) { T old = *p; *p += v; return old; }
 template <typename T> T atomicExch(T* p, T v) { T old = *p; *p = v; return old; }
 template <typename T> T atomicCAS(T* p, T cmp, T v) { T old = *p; if (old == cmp) *p = v; return old; }
@@ -104,6 +103,7 @@ inline void mbar_arrive_expect_tx(uint32_t bar, uint32_t) { sim_access(), sim_ar
 inline void mma_commit(uint32_t bar) { sim_arrive_after_mma(bar); }
 inline bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx&, int site) { return sim_wait(bar, parity, site), true; }
 inline bool mbar_wait_warp(uint32_t bar, uint32_t parity, const WaitCtx&, int site) { return sim_wait(bar, parity, site), true; }
+template <typename T> T ld_global(const T* p) { return sim_access(), *p; }
 inline void tmem_ld_x32(uint32_t, uint32_t* r) { memset(r, 0, 128); }
 inline void tmem_ld_x16(uint32_t, uint32_t* r) { memset(r, 0, 64); }
 template <bool BF16> uint32_t pack2(float, float) { return 0; }

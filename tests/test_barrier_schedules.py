@@ -7,6 +7,7 @@ arrive twice in one phase of a barrier, or let a wait return on a phase that it 
 warp may read global memory before it has waited for the kernel before its own.
 """
 
+import re
 import shutil
 import subprocess
 from pathlib import Path
@@ -34,6 +35,16 @@ def check(simulator, kernel, headdim, rows, keys, schedules=60):
     run = subprocess.run([simulator, kernel, str(headdim), str(rows), str(keys), str(schedules)],
                          capture_output=True, text=True, timeout=300)
     assert run.returncode == 0, run.stdout + run.stderr
+
+
+def test_no_kernel_takes_the_read_only_path_to_global_memory():
+    """A kernel starts while the one before it still writes: what it reads must neither come through the
+    non-coherent path nor be open to the compiler's use of it (const __restrict__ parameters)."""
+    for source in CSRC.glob("*.cu*"):
+        if source.name == "selftest.cu":  # an ordinary launch
+            continue
+        code = re.sub(r"//.*", "", source.read_text())
+        assert not re.search(r"__ldg|\.nc\b|const \w+\* ?__restrict__", code), source.name
 
 
 @pytest.mark.parametrize("rows,keys", [(1, 1), (128, 64), (449, 300), (640, 640)])
