@@ -401,7 +401,8 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
       const bool need = (m_new - m_run) * scale_log2 > threshold;
       bool pv_waited = false;
       if (__any_sync(0xffffffffu, need)) {
-        const float alpha = ex2((m_run - m_new) * scale_log2);
+        // A neighbour's rescale must not touch a row without a finite score so far: -inf - -inf is no factor.
+        const float alpha = W == 64 && m_new == -INFINITY ? 1.0f : ex2((m_run - m_new) * scale_log2);
         l_run *= alpha;
         m_run = m_new;
         if (j > 0) {

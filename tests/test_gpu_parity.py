@@ -234,6 +234,32 @@ def test_keys_with_scores_of_minus_infinity_have_no_weight(d, dtype):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("dtype,key,queries", [
+    (torch.float16, -math.inf, (1.0, -1.0)),  # every second row scores +inf there (and is NaN itself)
+    (torch.bfloat16, -math.inf, (1.0, -1.0)),
+    (torch.bfloat16, -3e38, (2.0, 0.5)),  # finite inputs: 2 q k overflows to -inf, q k / 2 does not
+])
+def test_rows_of_minus_infinity_beside_rows_that_rescale(d, dtype, key, queries):
+    """Rows whose scores against the first 64 keys are all -inf share a warp with rows that have a maximum
+    there: they attend to the other keys, whatever their neighbours do."""
+    n = 330
+    g = torch.Generator().manual_seed(d)
+    q, k, v = (torch.randn(1, 2, n, d, generator=g).to(dtype) for _ in range(3))
+    q[..., 0::2, 0], q[..., 1::2, 0] = queries
+    k[:, :, :64, 0] = key
+    k[:, :, 64:, 0] = 0.0
+    out = flash_attention_v2(q.to(DEV), k.to(DEV), v.to(DEV)).cpu().double()
+    scores = (q.double() @ k.double().transpose(-1, -2)) / math.sqrt(d)
+    scores.masked_fill_(torch.ones(n, n, dtype=torch.bool).triu(1), -math.inf)
+    want = scores[..., 64::2, 64:].softmax(-1) @ v.double()[:, :, 64:]
+    assert (out[:, :, 64::2] - want).abs().max() <= BASE_TOL[dtype]
+    if math.isfinite(key):  # these rows have finite scores everywhere, and no weight on the first 64 keys
+        want = scores[..., 65::2, 64:].softmax(-1) @ v.double()[:, :, 64:]
+        assert (out[:, :, 65::2] - want).abs().max() <= BASE_TOL[dtype]
+    assert _lib.device_status() == 0
+
+
 def test_spill_mode_chunks_change_no_bit(monkeypatch):
     """With a scratch bound of 3 MiB the spill mode works through [3, 5, 700, 64] (0.7 MiB per
     head) in chunks of 3 + 2 heads per batch entry; with 8 MiB in chunks of 2 + 1 batch
