@@ -40,13 +40,14 @@ _MAX_HEAD_DIM = 256  # the reference's max_headdim on B200 (line 533)
 _COMPUTE_DTYPES = (torch.float16, torch.bfloat16)
 
 
-def _check_status_if_asked(fn: str) -> None:
+def _check_status_if_asked(fn: str, device: torch.device) -> None:
     """Kernels that give up on a bounded wait leave their outputs unwritten and only set the
     device status word; reading it synchronises the device, so it is not read by default.
-    ``FA2_B200_CHECK_STATUS=1`` makes every forward / backward call read it and raise
-    ``Fa2Error`` (``FA2_ERR_DEVICE_STATUS``) when it is non-zero."""
+    ``FA2_B200_CHECK_STATUS=1`` makes every forward / backward call read that of the tensors' device and
+    raise ``Fa2Error`` (``FA2_ERR_DEVICE_STATUS``) when it is non-zero."""
     if os.environ.get("FA2_B200_CHECK_STATUS") == "1":
-        word = _lib.device_status()
+        with torch.cuda.device(device):  # the library reads the current device's word
+            word = _lib.device_status()
         if word:
             raise _lib.Fa2Error(fn, -7, f"{_lib.lib().fa2_strerror(-7).decode()} (status {word:#x})")
 
@@ -83,7 +84,7 @@ def _flash_attention_forward(
     # output and LSE are dense, like the reference's
     code, output, lse, output32 = _lib.host().forward(q, k, v, float(softmax_scale), f32)
     _lib.check("fa2_fwd_strided", code)
-    _check_status_if_asked("fa2_fwd_strided")
+    _check_status_if_asked("fa2_fwd_strided", q.device)
     return (output, lse, softmax_scale, output32) if f32 else (output, lse, softmax_scale)
 
 
@@ -195,7 +196,7 @@ def _flash_attention_backward(
         _lib.lib(), q.device, batch, nheads, seqlen_q, headdim, mode)
     _lib.check("fa2_bwd_strided", host.backward(
         q, k, v, d_output, dq, dk, dv, rowstats, workspace, float(softmax_scale), mode))
-    _check_status_if_asked("fa2_bwd_strided")
+    _check_status_if_asked("fa2_bwd_strided", q.device)
 
 
 # ------------------------------------------------------------------ autograd integration

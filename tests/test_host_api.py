@@ -157,3 +157,37 @@ def test_native_host_path_refuses_what_is_not_a_tensor():
                  lambda h: h.backward(*([t] * 7), None, None, 0.1, 0), lambda h: h.backward(t)):
         with pytest.raises(TypeError):
             call(_lib.host())
+
+
+def test_status_check_reads_the_word_of_the_tensors_device(monkeypatch):
+    """Tensors on cuda:1 while cuda:0 is current, on a fake library: the word read, and reported, is cuda:1's."""
+    from contextlib import contextmanager
+    from types import SimpleNamespace
+
+    from flash_attention_triton_b200 import _lib, api
+
+    current = [torch.device("cuda:0")]
+
+    @contextmanager
+    def device(d):
+        current.append(d)
+        yield
+        current.pop()
+
+    words = {torch.device("cuda:0"): 0, torch.device("cuda:1"): 0x10003}
+    fake = SimpleNamespace(forward=lambda *a: (0, "o", "lse", None), readable_in_place=lambda t: True,
+                           preprocess=lambda o, do, lse: (0, "rowstats", do), backward=lambda *a: 0)
+    monkeypatch.setattr(_lib, "host", lambda: fake)
+    monkeypatch.setattr(_lib, "device_status", lambda: words[current[-1]])
+    monkeypatch.setattr(torch.cuda, "device", device)
+    t = SimpleNamespace(shape=torch.Size((1, 2, 8, 64)), dtype=torch.float16, is_cuda=True,
+                        device=torch.device("cuda:1"), is_contiguous=lambda: True)
+    lse = SimpleNamespace(shape=torch.Size((1, 2, 8)))
+    calls = (lambda: api._flash_attention_forward(t, t, t, None),
+             lambda: api._flash_attention_backward(t, t, t, t, lse, t, t, t, t, 0.1, True))
+    for call in calls:
+        call()  # not asked: not read
+    monkeypatch.setenv("FA2_B200_CHECK_STATUS", "1")
+    for call in calls:
+        with pytest.raises(_lib.Fa2Error, match="0x10003"):
+            call()
