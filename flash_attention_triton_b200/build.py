@@ -68,11 +68,9 @@ def _compile(src: Path, verbose: bool) -> Path:
 
 def _build_host(verbose: bool) -> None:
     """The Python module with the host path (``csrc/host.cpp``), against torch's C++ headers and the
-    library next to it."""
+    library next to it.  Rebuilt when its sources, the command, torch or the interpreter have changed."""
     src = CSRC / "host.cpp"
     newest = max(src.stat().st_mtime, (INCLUDE / "fa2_b200.h").stat().st_mtime)
-    if HOST_PATH.exists() and HOST_PATH.stat().st_mtime >= newest:
-        return
     import torch
 
     root = Path(torch.__file__).resolve().parent
@@ -84,9 +82,15 @@ def _build_host(verbose: bool) -> None:
            *(f"-I{p}" for p in includes), str(src), "-o", str(HOST_PATH),
            f"-L{PKG_DIR}", f"-l:{LIB_PATH.name}", "-Wl,-rpath,$ORIGIN", f"-L{root / 'lib'}",
            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]  # already loaded by `import torch`
+    key = "\n".join([torch.__version__, sys.version, *cmd])
+    stamp = BUILD_DIR / "host.key"
+    if (HOST_PATH.exists() and HOST_PATH.stat().st_mtime >= newest
+            and stamp.exists() and stamp.read_text() == key):
+        return
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed for {src.name}:\n{res.stderr[-4000:]}")
+    stamp.write_text(key)
     if verbose:
         print(f"[build] compiled {src.name}")
 

@@ -191,3 +191,24 @@ def test_status_check_reads_the_word_of_the_tensors_device(monkeypatch):
     for call in calls:
         with pytest.raises(_lib.Fa2Error, match="0x10003"):
             call()
+
+
+def test_host_module_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    from types import SimpleNamespace
+
+    from flash_attention_triton_b200 import build
+
+    runs = []
+
+    def compile_(cmd, **kwargs):
+        runs.append(cmd)
+        (tmp_path / "_host.so").touch()
+        return SimpleNamespace(returncode=0)
+
+    monkeypatch.setattr(build, "HOST_PATH", tmp_path / "_host.so")
+    monkeypatch.setattr(build, "BUILD_DIR", tmp_path)
+    monkeypatch.setattr(build.subprocess, "run", compile_)
+    for version, expected in (("1", 1), ("1", 1), ("2", 2), ("2", 2)):
+        monkeypatch.setattr(torch, "__version__", version)
+        build._build_host(False)
+        assert len(runs) == expected
