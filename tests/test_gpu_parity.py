@@ -363,6 +363,45 @@ def test_calls_on_two_streams_do_not_disturb_each_other():
                 assert torch.equal(got[key], want[key]), key
 
 
+@pytest.mark.parametrize("d,dtype,det", [(64, torch.float16, False), (64, torch.float16, True), (40, torch.bfloat16, False),
+                                         (96, torch.float32, False), (128, torch.bfloat16, False),
+                                         (256, torch.bfloat16, False)])
+def test_forward_and_backward_in_a_cuda_graph(d, dtype, det):
+    """Dependent launches under capture, a memset between them in the atomic mode: replays on other inputs
+    give the bits of plain calls (dq of the atomic mode, whose summation order is free, to rounding)."""
+    g = torch.Generator(device=DEV).manual_seed(d)
+    draw = lambda: [torch.randn(2, 40, 450, d, device=DEV, generator=g, dtype=dtype) for _ in range(4)]
+    *leaves, do = draw()
+    for t in leaves:
+        t.requires_grad_(True)
+
+    def step():
+        out = flash_attention_v2(*leaves, None, det)
+        return [out.detach(), *torch.autograd.grad(out, leaves, do)]
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step()
+    for _ in range(3):
+        with torch.no_grad():
+            for t, new in zip((*leaves, do), draw()):
+                t.copy_(new)
+        graph.replay()
+        got = [t.clone() for t in captured]
+        for name, x, y in zip(("o", "dq", "dk", "dv"), got, step()):
+            if name == "dq" and d <= 64 and not det:
+                # one ulp of bf16 / fp16 at most between two summation orders in fp32
+                assert ((x.float() - y.float()).abs() <= (1.6e-2 if dtype == torch.bfloat16 else 2e-3) * y.float().abs() + 1e-5).all()
+            else:
+                assert torch.equal(x, y), name
+    assert _lib.device_status() == 0
+
+
 def test_lse_and_rowstats_through_the_c_abi():
     """fa2_fwd's LSE and fa2_bwd_preprocess's tile-blocked (-lse*log2e, -delta) array, ragged N."""
     b, h, n, d = 2, 3, 300, 64
