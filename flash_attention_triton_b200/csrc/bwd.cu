@@ -6,21 +6,10 @@
 //     S = Q K^T, P = exp(scale*S - lse), dP = dO V^T, dS = P o (dP - delta) * scale,
 //     dV += P^T dO, dK += dS^T Q, dQ += dS K.
 //
-// bwd_dkdv_kernel (one CTA per KV tile) works on the TRANSPOSED score tile so that everything
-// a later MMA consumes as its A operand already sits in tensor memory with kv rows on lanes:
-//     St  = K  Q_i^T      (smem x smem)  -> tensor memory, 128 columns
-//     dPt = V  dO_i^T     (smem x smem)  -> tensor memory, 128 columns
-//     dV += Pt  dO_i      (tmem x smem)     Pt  = 16-bit P^T written over St by the compute warps
-//     dK += dSt Q_i       (tmem x smem)     dSt = 16-bit dS^T written over dPt
-//     dQ_i = dS K         (smem x smem)     fused variant only: dS^T also goes to shared memory,
-//                                           the tile lands over dPt and is added to the fp32
-//                                           workspace with vector atomics
+// bwd_dkdv_kernel (one CTA per KV tile) works on the TRANSPOSED score tile; see dkdv_roles.
 // bwd_dq_kernel (one CTA per Q tile, deterministic path) recomputes S and dP untransposed and
 // accumulates dQ_i over ascending j in tensor memory, so each dQ tile has one owner and one
 // summation order.
-//
-// -lse*log2(e) and -delta of a Q tile arrive in shared memory as one 1 KiB bulk copy from the
-// tile-blocked rowstats array; padded rows carry -lse = -inf, which makes their P exactly 0.
 #include "bwd_roles.cuh"
 
 namespace fa2 {
@@ -1007,9 +996,8 @@ cudaError_t launch_consume_t(const AttnShape& s, const void* scratch, const CUte
   const unsigned grid =
       static_cast<unsigned>(((FORM == 2 ? s.N : s.Nk) + 127) / 128) * s.B * s.H;  // one CTA per output tile
   return launch_dependent(kern, grid, C::kThreads, C::kSmemBytes, stream,
-      static_cast<const uint4*>(scratch), tb, tout, out32, s.Dg,
-                                                     rowstats.tile_amax, s.N, s.Nk, s.B * s.H, s.H,
-                                                     heads_per_group(s), status);
+      static_cast<const uint4*>(scratch), tb, tout, out32, s.Dg, rowstats.tile_amax, s.N, s.Nk, s.B * s.H,
+      s.H, heads_per_group(s), status);
 }
 
 template <bool BF16, int FORM>
@@ -1024,8 +1012,7 @@ cudaError_t launch_consume_pair_t(const AttnShape& s, const void* scratch, const
   const unsigned out_tiles = static_cast<unsigned>(((FORM == 2 ? s.N : s.Nk) + 127) / 128);
   return launch_dependent(kern, (out_tiles + 1) / 2 * s.B * s.H, C::kThreads, C::kSmemBytes, stream,
       static_cast<const uint4*>(scratch), tb, tout, out32, s.Dg, rowstats.tile_amax, s.N, s.Nk, s.B * s.H,
-      s.H,
-      heads_per_group(s), status);
+      s.H, heads_per_group(s), status);
 }
 
 template <int D, bool BF16, int KD = D>

@@ -39,9 +39,9 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
 }
 
 // The transposed-score kernels (bwd_dkdv_kernel, bwd_scores_wide_kernel) give each thread one kv
-// row and 64 q columns of a tile.  probabilities_of_row: p = 2^(s * c - lse2[q]) from the raw
-// scores `sr` and the negated, log2-scaled row statistics of the 64 columns (`nlse`, read with
-// warp-wide broadcasts).  mask_row: keep only the q columns >= `first` (128 keeps nothing).
+// row and 2 * PAIRS q columns of a tile: 64, or 32 in steps of 64 rows.  probabilities_of_row:
+// p = 2^(s * c - lse2[q]) from the raw scores `sr` and the negated, log2-scaled row statistics of
+// these columns (`nlse`, read with warp-wide broadcasts).  mask_row: keep only the q columns >= `first` (128 keeps nothing).
 template <int SHARE = FA2_BWD_POLY_PAIRS_PER_8, int PAIRS>
 __device__ __forceinline__ void probabilities_of_row(const uint32_t (&sr)[2 * PAIRS], const float4* nlse,
                                                      float2 sc2, float2 (&p)[PAIRS]) {
@@ -296,15 +296,16 @@ __device__ __forceinline__ void dkdv_init_barriers(uint32_t bar0) {
 //
 // It works on the TRANSPOSED score tile so that everything a later MMA consumes as its A operand
 // already sits in tensor memory with kv rows on lanes:
-//     St  = K  Q_i^T      (smem x smem)  -> tensor memory, 128 columns
-//     dPt = V  dO_i^T     (smem x smem)  -> tensor memory, 128 columns
+//     St  = K  Q_i^T      (smem x smem)  -> tensor memory, kW columns (128, or 64 up to head dim 64)
+//     dPt = V  dO_i^T     (smem x smem)  -> tensor memory, kW columns
 //     dV += Pt  dO_i      (tmem x smem)     Pt  = 16-bit P^T written over St by the compute warps
 //     dK += dSt Q_i       (tmem x smem)     dSt = 16-bit dS^T written over dPt
 //     dQ_i = dS K         (smem x smem)     fused variant only: dS^T also goes to shared memory,
 //                                           the tile lands over dPt and is added to the fp32
 //                                           workspace with vector atomics
 // -lse*log2(e) and -delta of a Q tile arrive in shared memory as one 1 KiB bulk copy from the
-// tile-blocked rowstats array; padded rows carry -lse = -inf, which makes their P exactly 0.
+// tile-blocked rowstats array, or two of 256 bytes for each step of 64 rows; padded rows carry
+// -lse = -inf, which makes their P exactly 0.
 template <int D, bool BF16, int MODE, int KD = D>
 __device__ __forceinline__ void dkdv_roles(
     uint8_t* smem, uint32_t smem_base, uint32_t tmem_base, int warp, int lane,

@@ -218,7 +218,7 @@ const char* fa2_strerror(int code) {
     case FA2_ERR_NULL_POINTER: return "a required pointer is NULL";
     case FA2_ERR_HEAD_DIM: return "head dimension must be a multiple of 8 between 8 and 256";
     case FA2_ERR_DTYPE: return "dtype must be 0 (fp16) or 1 (bf16)";
-    case FA2_ERR_MISALIGNED: return "tensor pointers must be 16-byte aligned";
+    case FA2_ERR_MISALIGNED: return "tensor pointers must be 16-byte aligned, fp32 outputs 32-byte aligned";
     case FA2_ERR_SHAPE: return "B, H, N must be positive, B*H <= 65535, N <= 2^24, 1 <= Nk <= N";
     case FA2_ERR_ARCH: return "the current device is not compute capability 10.x (B200)";
     case FA2_ERR_DEVICE_STATUS: return "a kernel abandoned a bounded wait (see fa2_device_status)";

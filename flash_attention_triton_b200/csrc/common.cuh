@@ -44,7 +44,7 @@ __host__ __device__ __forceinline__ uint32_t swizzled_offset_128B(uint32_t row, 
 
 // ----------------------------------------------------------------------------------------
 // Host launchers (one per kernel family), defined in the .cu files of this directory.
-// Tensor maps describe [B, H, N, D] tensors with box (CH, 128 or 32, 1, 1).
+// Tensor maps describe [B, H, N, D] tensors with box (CH, 128, 64 or 32, 1, 1).
 // ----------------------------------------------------------------------------------------
 struct AttnShape {
   int B, H;

@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(kPreThreads)
 // copy per row), so the bytes in flight per SM stay near the ring size (128 - 192 KiB) whatever
 // the eight consumer warps are doing; the block-per-tile kernel above has nothing in flight while
 // a block reduces and stores, and reaches less than half of the HBM rate.  Consumers read their
-// pieces from shared memory with the row / lane assignment of the kernel above, free the stage as
-// soon as the pieces are in registers, and hand the tile's 256 results to the next iteration,
+// pieces from shared memory with the row / lane assignment of the kernel above, free the stage
+// once every piece has been used, and hand the tile's 256 results to the next iteration,
 // which stores them with one coalesced 1 KiB write.  lse of the next tile is fetched one
 // iteration ahead.  Rows in shared memory are packed at their true width (d8 pieces).
 // ----------------------------------------------------------------------------------------

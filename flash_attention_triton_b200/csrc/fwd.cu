@@ -111,8 +111,8 @@ template <int D, bool BF16, int KD = D>
 __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtasPerSm)
     fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap to,
-               const __grid_constant__ F32Out o32, int cols, float* __restrict__ lse, int N, int Nk, int num_bh, int num_heads, int group,
-               float scale_log2, int* status, unsigned int* work_counter) {
+               const __grid_constant__ F32Out o32, int cols, float* __restrict__ lse, int N, int Nk,
+               int num_bh, int num_heads, int group, float scale_log2, int* status, unsigned int* work_counter) {
   // Head dim 256 ("wide") runs on the staging and tensor-memory plan of head dim 128 with ONE
   // Q tile per work item: the two Q slots hold the two 128-column halves of that tile, K and V
   // tiles stream through their rings as half tiles, S = Q_lo K_lo^T + Q_hi K_hi^T accumulates
@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
   using C = FwdCfg<DT>;
   using T = Tile<DT>;
   constexpr int W = C::kW;  // rows of a KV tile
+  constexpr int KT = WIDE ? DT : KD;  // columns of a staged tile that the products run over
   extern __shared__ __align__(1024) uint8_t smem[];
 
   // Role index: hardware warps 0-3 take roles 8-11 (MMA, TMA, idle, idle) and hardware warps
@@ -294,14 +295,14 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
             // S = Q_lo K_lo^T + Q_hi K_hi^T: the Q slots hold the halves, K arrives half by half
             for (int half = 0; ok && half < 2; ++half) {
               if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
-              issue_rows_x_rows<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColS,
+              issue_rows_x_rows<DT, BF16, W, KT>(elected, tmem_base + C::kColS,
                                           smem_base + C::kOffQ + half * T::kTileBytes,
                                           smem_base + C::kOffK + ks * C::kKvBytes, half);
               release_k();
             }
             if (!ok) break;
           } else {
-            issue_rows_x_rows<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColS,
+            issue_rows_x_rows<DT, BF16, W, KT>(elected, tmem_base + C::kColS,
                                         smem_base + C::kOffQ + i * T::kTileBytes,
                                         smem_base + C::kOffK + ks * C::kKvBytes);
           }
@@ -339,14 +340,14 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
             // O_lo += P V_lo, O_hi += P V_hi: the O0 / O1 columns hold the two halves of O
             for (int half = 0; ok && half < 2; ++half) {
               if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
-              issue_tmem_x_tile<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColO + half * DT,
+              issue_tmem_x_tile<DT, BF16, W, KT>(elected, tmem_base + C::kColO + half * DT,
                                           tmem_base + C::kColP, W / 4,
                                           smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
               release_v();
             }
             if (!ok) break;
           } else {
-            issue_tmem_x_tile<DT, BF16, W, WIDE ? DT : KD>(elected, tmem_base + C::kColO + i * DT,
+            issue_tmem_x_tile<DT, BF16, W, KT>(elected, tmem_base + C::kColO + i * DT,
                                         tmem_base + C::kColP + i * (W / 2), W / 4,
                                         smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
           }
@@ -539,9 +540,8 @@ cudaError_t launch_fwd_t(const AttnShape& s, const CUtensorMap& tq, const CUtens
   const unsigned grid = static_cast<unsigned>(items < slots ? items : slots);
   const float scale_log2 = s.scale * 1.4426950408889634f;
   return launch_dependent(kern, grid, kFwdThreads, C::kSmemBytes, stream,
-      tq, tk, tv, to, o32, s.Dg, lse, s.N, s.Nk, s.B * s.H, s.H,
-                                                     heads_per_group(s), scale_log2, ctx.status,
-                                                     ctx.work_counter);
+      tq, tk, tv, to, o32, s.Dg, lse, s.N, s.Nk, s.B * s.H, s.H, heads_per_group(s), scale_log2, ctx.status,
+      ctx.work_counter);
 }
 
 }  // namespace

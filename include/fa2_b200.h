@@ -43,7 +43,7 @@ extern "C" {
 #define FA2_ERR_NULL_POINTER (-1)      /* a required pointer is NULL */
 #define FA2_ERR_HEAD_DIM (-2)          /* D not a multiple of 8 in [8, 256] */
 #define FA2_ERR_DTYPE (-3)             /* dtype not FA2_DTYPE_FP16 / FA2_DTYPE_BF16 */
-#define FA2_ERR_MISALIGNED (-4)        /* a tensor pointer is not 16-byte aligned */
+#define FA2_ERR_MISALIGNED (-4)        /* a tensor pointer is not 16-byte aligned (fp32 outputs: 32) */
 #define FA2_ERR_SHAPE (-5)             /* B, H or N <= 0, B*H > 65535, N too large, Nk not in [1, N] */
 #define FA2_ERR_ARCH (-6)              /* current device is not compute capability 10.x */
 #define FA2_ERR_DEVICE_STATUS (-7)     /* a kernel gave up on a bounded wait */
@@ -65,8 +65,8 @@ const char* fa2_strerror(int code);
  * Forward: O = softmax_causal(scale * Q K^T) V, lse[b,h,i] = log sum_j exp(scale * s_ij)
  * (natural log).  Replaces _flash_attention_forward / _forward_kernel; unlike the
  * reference (flash_attention_2.py:98-100) lse is not padded and no scratch buffer is used.
- * The kernel runs one CTA per SM (two up to head dim 64); the CTAs draw their work items from a device counter that
- * the library takes from a ring of 1024 (a new one per call, so calls on different streams do
+ * The kernel runs one CTA per SM (two up to head dim 64); the CTAs draw their work items from a device
+ * counter that the library takes from a ring of 1024 (a new one per call, so calls on different streams do
  * not share one).  A call captured into a CUDA graph keeps its counter: replays of that graph
  * must not overlap each other.
  */
