@@ -18,8 +18,8 @@ namespace {
 // =========================================================================================
 // dK / dV (+ fused dQ) kernel: one CTA per KV tile of one (batch, head); see dkdv_roles.
 // =========================================================================================
-template <int D, bool BF16, int MODE, int KD = D>
-__global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::kCtasPerSm)
+template <int D, bool BF16, int MODE, int KD, int W>
+__global__ void __launch_bounds__(DkdvCfg<D, MODE, W>::kThreads, DkdvCfg<D, MODE, W>::kCtasPerSm)
     bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                     const __grid_constant__ CUtensorMap tdk,
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::
                     const unsigned* tile_amax, float* __restrict__ dq_accum, int N,
                     int Nk, int num_bh, int num_heads, int group, float scale, float scale_log2,
                     int* status) {
-  using C = DkdvCfg<D, MODE>;
+  using C = DkdvCfg<D, MODE, W>;
   extern __shared__ __align__(1024) uint8_t smem[];
   // Role index: the producer / MMA group takes hardware warps 0-3 (lowest ids on their
   // schedulers), the compute and reduction groups follow; shifts are multiples of 4, so
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::
   item.tile_amax = tile_amax + static_cast<size_t>(item.bh) * ntiles;
 
   if (threadIdx.x == 0) {
-    dkdv_init_barriers<D, MODE>(smem_base + C::kOffBar);
+    dkdv_init_barriers<D, MODE, W>(smem_base + C::kOffBar);
     *abort_flag = 0;
     fence_mbar_init();
     fence_proxy_async_smem();
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::
   grid_wait_previous();
   grid_allow_next();
 
-  dkdv_roles<D, BF16, MODE, KD>(smem, smem_base, tmem_base, warp, lane, &tq, &tk, &tv, &tdo, &tdk, &tdv,
+  dkdv_roles<D, BF16, MODE, KD, W>(smem, smem_base, tmem_base, warp, lane, &tq, &tk, &tv, &tdo, &tdk, &tdv,
                             dk32, dv32, cols, rowstats, dq_accum, N, Nk, scale, scale_log2, w, item);
 
   tc_fence_before();
@@ -93,12 +93,13 @@ __global__ void __launch_bounds__(DkdvCfg<D, MODE>::kThreads, DkdvCfg<D, MODE>::
 // buffer they just read, and the MMA warp then issues dQ += dS(j) K_j followed by S(j+2) into
 // the same buffer.  S(j+1) is already in the other buffer, so the tensor pipe and the compute
 // warps overlap instead of alternating.
-// Head dims up to 64 walk the KV tiles in steps of 64 rows with two CTAs per SM, for the reasons given
-// at DkdvCfg; the polynomial's share of the exponentials is that of the dK/dV kernel.
-template <int D>
+// Head dims up to 64 walk the KV tiles in steps of 64 rows with two CTAs per SM where bwd_step_rows says so, for the
+// reasons given at DkdvCfg; the polynomial's share of the exponentials is that of the dK/dV kernel.
+template <int D, int W>
 struct DqCfg {
   using T = Tile<D>;
-  static constexpr int kW = bwd_step_rows(D);  // rows of a KV tile = score columns of a step
+  static constexpr int kW = W;  // rows of a KV tile = score columns of a step
+  static_assert(W == 128 || (W == 64 && D <= 64), "bwd_step_rows");
   static constexpr int kCtasPerSm = kW == 64 ? 2 : 1;
   static constexpr int kGroups = 2;           // compute groups of four warps
   static constexpr int kCols = kW / kGroups;  // score columns of a compute thread
@@ -145,17 +146,16 @@ struct DqCfg {
   static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "shared memory of one SM");
 };
 
-template <int D, bool BF16, int KD = D>
-__global__ void __launch_bounds__(DqCfg<D>::kThreads, DqCfg<D>::kCtasPerSm)
+template <int D, bool BF16, int KD, int W>
+__global__ void __launch_bounds__(DqCfg<D, W>::kThreads, DqCfg<D, W>::kCtasPerSm)
     bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                   const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                   const __grid_constant__ CUtensorMap tdq, const __grid_constant__ F32Out dq32, int cols,
                   const float* rowstats,
                   const unsigned* tile_amax, int N, int Nk, int num_bh, int num_heads,
                   int group, float scale, float scale_log2, int* status) {
-  using C = DqCfg<D>;
+  using C = DqCfg<D, W>;
   using T = Tile<D>;
-  constexpr int W = C::kW;  // rows of a KV tile
   constexpr int kCols = C::kCols, kPairs = kCols / 2;
   constexpr uint32_t kHalf = kCols;  // columns between the two groups' halves of dS
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -966,14 +966,14 @@ cudaError_t launch_scores_wide_t(const AttnShape& s, const CUtensorMap& tq, cons
       s.scale * 1.4426950408889634f, status);
 }
 
-template <int D, bool BF16, int MODE, int KD = D>
+template <int D, bool BF16, int MODE, int KD = D, int W = 128>
 cudaError_t launch_dkdv_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                           const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdk,
                           const CUtensorMap& tdv, const F32Out& dk32, const F32Out& dv32,
                           const RowStats& rowstats, float* dq_accum,
                           int* status, cudaStream_t stream) {
-  using C = DkdvCfg<D, MODE>;
-  auto kern = bwd_dkdv_kernel<D, BF16, MODE, KD>;
+  using C = DkdvCfg<D, MODE, W>;
+  auto kern = bwd_dkdv_kernel<D, BF16, MODE, KD, W>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
@@ -1015,12 +1015,12 @@ cudaError_t launch_consume_pair_t(const AttnShape& s, const void* scratch, const
       s.H, heads_per_group(s), status);
 }
 
-template <int D, bool BF16, int KD = D>
+template <int D, bool BF16, int KD = D, int W = 128>
 cudaError_t launch_dq_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                         const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
                         const F32Out& dq32, const RowStats& rowstats, int* status, cudaStream_t stream) {
-  using C = DqCfg<D>;
-  auto kern = bwd_dq_kernel<D, BF16, KD>;
+  using C = DqCfg<D, W>;
+  auto kern = bwd_dq_kernel<D, BF16, KD, W>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
@@ -1035,8 +1035,8 @@ cudaError_t launch_dq_t(const AttnShape& s, const CUtensorMap& tq, const CUtenso
 cudaError_t launch_bwd_dkdv(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                             const CUtensorMap& tv, const CUtensorMap& tdo,
                             const CUtensorMap& tdk, const CUtensorMap& tdv, const F32Out& dk32,
-                            const F32Out& dv32, const RowStats& rowstats, float* dq_accum, int mode, int* status,
-                            cudaStream_t stream) {
+                            const F32Out& dv32, const RowStats& rowstats, float* dq_accum, int mode, int step_rows,
+                            int* status, cudaStream_t stream) {
   // modes: 0 dK/dV only, 1 fused atomic dQ (dq_accum = fp32 accumulator), 2 spill dS tiles
   // (dq_accum = the 16-bit scratch tensor)
 #define FA2_ARGS s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rowstats, dq_accum, status, stream
@@ -1046,6 +1046,17 @@ cudaError_t launch_bwd_dkdv(const AttnShape& s, const CUtensorMap& tq, const CUt
   if (s.D == 128 && s.Dg <= kShortDim128 && mode == 0)
     return s.dtype ? launch_dkdv_t<128, true, 0, kShortDim128>(FA2_ARGS)
                    : launch_dkdv_t<128, false, 0, kShortDim128>(FA2_ARGS);
+  if (step_rows == 64) {
+    if (s.D == 64 && mode == 1)
+      return s.dtype ? launch_dkdv_t<64, true, 1, 64, 64>(FA2_ARGS) : launch_dkdv_t<64, false, 1, 64, 64>(FA2_ARGS);
+    if (s.D == 64 && mode == 0)
+      return s.dtype ? launch_dkdv_t<64, true, 0, 64, 64>(FA2_ARGS) : launch_dkdv_t<64, false, 0, 64, 64>(FA2_ARGS);
+    if (s.D == 32 && mode == 1)
+      return s.dtype ? launch_dkdv_t<32, true, 1, 32, 64>(FA2_ARGS) : launch_dkdv_t<32, false, 1, 32, 64>(FA2_ARGS);
+    if (s.D == 32 && mode == 0)
+      return s.dtype ? launch_dkdv_t<32, true, 0, 32, 64>(FA2_ARGS) : launch_dkdv_t<32, false, 0, 32, 64>(FA2_ARGS);
+    return cudaErrorInvalidValue;
+  }
 #define FA2_CASE(DD)                                                                        \
   case DD:                                                                                  \
     if (mode == 1)                                                                          \
@@ -1068,11 +1079,17 @@ cudaError_t launch_bwd_dkdv(const AttnShape& s, const CUtensorMap& tq, const CUt
 
 cudaError_t launch_bwd_dq(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                           const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
-                          const F32Out& dq32, const RowStats& rowstats, int* status, cudaStream_t stream) {
+                          const F32Out& dq32, const RowStats& rowstats, int step_rows, int* status,
+                          cudaStream_t stream) {
 #define FA2_ARGS s, tq, tk, tv, tdo, tdq, dq32, rowstats, status, stream
   if (s.D == 128 && s.Dg <= kShortDim128)
     return s.dtype ? launch_dq_t<128, true, kShortDim128>(FA2_ARGS)
                    : launch_dq_t<128, false, kShortDim128>(FA2_ARGS);
+  if (step_rows == 64) {
+    if (s.D == 64) return s.dtype ? launch_dq_t<64, true, 64, 64>(FA2_ARGS) : launch_dq_t<64, false, 64, 64>(FA2_ARGS);
+    if (s.D == 32) return s.dtype ? launch_dq_t<32, true, 32, 64>(FA2_ARGS) : launch_dq_t<32, false, 32, 64>(FA2_ARGS);
+    return cudaErrorInvalidValue;
+  }
 #define FA2_CASE(DD)                                                   \
   case DD:                                                             \
     return s.dtype ? launch_dq_t<DD, true>(FA2_ARGS)                   \

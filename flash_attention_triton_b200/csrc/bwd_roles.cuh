@@ -170,7 +170,7 @@ __host__ __device__ __forceinline__ int dstile_count(int ntiles, int jt) {
 // 16-bit dS^T tile to a scratch tensor, from which a consumer forms dQ with one product per tile
 // pair instead of recomputing S, P, dP.
 //
-// Modes 0 and 1 take head dims up to 64 in steps of 64 Q rows (kW).  The products of a 128 x 128 tile
+// Modes 0 and 1 take head dims up to 64 in steps of 64 Q rows (kW) where bwd_step_rows says so.  The products of a 128 x 128 tile
 // pair are short there and a step is a chain of latencies: score product, copy-out, exponentials,
 // copy-in, dP product, ...; all eight compute warps of a CTA stand at the same link of it.  With 64
 // score columns a CTA needs half of the tensor memory and registers, so two CTAs run on an SM and
@@ -181,12 +181,13 @@ __host__ __device__ __forceinline__ int dstile_count(int ntiles, int jt) {
 // mode 1 124 -> 115; [2,16,8192,64] mode 0 1258 -> 1149, mode 1 986 -> 997 (bound by the fp32
 // reductions in L2, 2.2 TB/s: without them it takes 791).  One compute group of 64 columns per thread
 // instead of two of 32 was 2-6 % slower.
-template <int D, int MODE>
+template <int D, int MODE, int W>
 struct DkdvCfg {
   using T = Tile<D>;
   static constexpr bool FUSE = MODE == 1;
   static constexpr bool SPILL = MODE == 2;
-  static constexpr int kW = SPILL ? 128 : bwd_step_rows(D);  // Q rows of a step = score columns
+  static constexpr int kW = W;  // Q rows of a step = score columns
+  static_assert(W == 128 || (W == 64 && D <= 64 && !SPILL), "bwd_step_rows");
   static constexpr int kCtasPerSm = kW == 64 ? 2 : 1;
   static constexpr int kGroups = 2;  // compute groups of four warps
   static constexpr int kCols = kW / kGroups;     // score columns of a compute thread
@@ -267,9 +268,9 @@ struct DkdvItem {
   size_t tile0;         // spill modes: scratch index of the item's first pair (jt, jt)
 };
 
-template <int D, int MODE>
+template <int D, int MODE, int W>
 __device__ __forceinline__ void dkdv_init_barriers(uint32_t bar0) {
-  using C = DkdvCfg<D, MODE>;
+  using C = DkdvCfg<D, MODE, W>;
   auto bar = [&](int i) { return bar0 + 8u * i; };
   mbar_init(bar(C::kBarKV), 1);
   for (int i = 0; i < C::kStages; ++i) {
@@ -306,14 +307,14 @@ __device__ __forceinline__ void dkdv_init_barriers(uint32_t bar0) {
 // -lse*log2(e) and -delta of a Q tile arrive in shared memory as one 1 KiB bulk copy from the
 // tile-blocked rowstats array, or two of 256 bytes for each step of 64 rows; padded rows carry
 // -lse = -inf, which makes their P exactly 0.
-template <int D, bool BF16, int MODE, int KD = D>
+template <int D, bool BF16, int MODE, int KD, int W>
 __device__ __forceinline__ void dkdv_roles(
     uint8_t* smem, uint32_t smem_base, uint32_t tmem_base, int warp, int lane,
     const CUtensorMap* tq, const CUtensorMap* tk, const CUtensorMap* tv, const CUtensorMap* tdo,
     const CUtensorMap* tdk, const CUtensorMap* tdv, const F32Out& dk32, const F32Out& dv32, int cols,
     const float* rowstats, float* __restrict__ dq_accum, int N, int Nk, float scale, float scale_log2, const WaitCtx& w,
     const DkdvItem& item) {
-  using C = DkdvCfg<D, MODE>;
+  using C = DkdvCfg<D, MODE, W>;
   constexpr bool FUSE = C::FUSE;
   constexpr bool SPILL = C::SPILL;
   using T = Tile<D>;
@@ -326,7 +327,6 @@ __device__ __forceinline__ void dkdv_roles(
   const bool kv_ragged = jt * 128 + 128 > Nk;  // this KV tile has rows beyond the last key
   // A Q tile is worked through in kSub steps of W rows, first rows first, so that dK and dV add the
   // same products in the same order whatever W is.
-  constexpr int W = C::kW;
   constexpr int kSub = 128 / W;
   const int nsteps = nq * kSub;
   auto q_row = [&](int t) { return (ntiles - 1 - t / kSub) * 128 + (t % kSub) * W; };

@@ -406,8 +406,9 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
   CUtensorMap tq, tk, tv, tdo;
   CUtensorMap tdq{}, tdk{}, tdv{};  // of 16-bit gradients
   F32Out dq32{nullptr, {}}, dk32{nullptr, {}}, dv32{nullptr, {}};
+  const AttnShape s = make_shape(B, H, N, Nk, D, dtype, scale);
   // boxes of the resident tiles are 128 rows high, those of the tiles a kernel walks step_rows
-  const int step_rows = deterministic == 2 ? 128 : bwd_step_rows(padded_head_dim(D));
+  const int step_rows = deterministic == 2 ? 128 : bwd_step_rows(s, Nk, deterministic == 0, d->num_sms);
   if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, step_rows)) return e;
   if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, 128)) return e;
   if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, 128)) return e;
@@ -423,21 +424,24 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
     if (deterministic != 0)
       if (int e = make_map(&tdq, dq, dtype, B, H, N, D, sdq, 32)) return e;
   }
-  const AttnShape s = make_shape(B, H, N, Nk, D, dtype, scale);
   const RowStats rs{rowstats, tile_amax};
 
   if (deterministic == 1) {
     cudaError_t ce =
-        launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, nullptr, 0, d->status, st);
+        launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, nullptr, 0, step_rows, d->status, st);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     record_mark_between(st);
-    if (step_rows != 128) {  // here Q and dO are resident, K and V are walked
+    // here Q and dO are resident, K and V are walked
+    const int kv_rows = bwd_step_rows(s, N, false, d->num_sms);
+    if (step_rows != 128) {
       if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, 128)) return e;
-      if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, step_rows)) return e;
-      if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, step_rows)) return e;
       if (int e = make_map_of(&tdo, dout, strides, 3, dtype, B, H, N, D, 128)) return e;
     }
-    return static_cast<int>(launch_bwd_dq(s, tq, tk, tv, tdo, tdq, dq32, rs, d->status, st));
+    if (kv_rows != 128) {
+      if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, kv_rows)) return e;
+      if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, kv_rows)) return e;
+    }
+    return static_cast<int>(launch_bwd_dq(s, tq, tk, tv, tdo, tdq, dq32, rs, kv_rows, d->status, st));
   }
   if (deterministic == 2) {
     float* scratch = static_cast<float*>(workspace);
@@ -462,7 +466,7 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
       return static_cast<int>(launch_bwd_consume(s, 2, ds_scratch, tk, tdq, dq32, rs, two, d->status, st));
     }
     cudaError_t ce =
-        launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, scratch, 2, d->status, st);
+        launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, scratch, 2, step_rows, d->status, st);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     record_mark_between(st);
     if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, 64)) return e;  // half tiles of K
@@ -471,7 +475,7 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
   float* dq_accum = static_cast<float*>(workspace);
   cudaError_t ce = cudaMemsetAsync(dq_accum, 0, fa2_bwd_workspace_bytes(B, H, N, D, 0), st);
   if (ce != cudaSuccess) return static_cast<int>(ce);
-  ce = launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, dq_accum, 1, d->status, st);
+  ce = launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, dq_accum, 1, step_rows, d->status, st);
   if (ce != cudaSuccess) return static_cast<int>(ce);
   return static_cast<int>(launch_dq_convert(s, dq_accum, dq, sdq, dq32, st));
 }

@@ -84,9 +84,22 @@ inline int padded_head_dim(int d) { return d <= 32 ? 32 : (d <= 64 ? 64 : (d <= 
 // Rows of the KV tiles the forward kernel walks (its K and V tensor maps use boxes of this height).
 __host__ __device__ constexpr int fwd_kv_rows(int padded_d) { return padded_d <= 64 ? 64 : 128; }
 
-// Rows of the tiles the backward kernels walk past their resident tile: Q and dO tiles of the dK/dV
-// kernel (its spill mode always takes 128), K and V tiles of the dQ kernel.
-__host__ __device__ constexpr int bwd_step_rows(int padded_d) { return padded_d <= 64 ? 64 : 128; }
+// Rows of the tiles a backward kernel walks past its resident tile, one CTA per resident tile of the `rows` of a
+// head: Q and dO tiles of the dK/dV kernel (its spill mode always takes 128), K and V tiles of the dQ kernel.
+// Up to head dim 64 steps of 64 rows with two CTAs on an SM win once there are CTAs to pair: a CTA that has its SM
+// to itself takes 1.2 to 1.5 times as long in them, and so does the longest CTA of a launch that is not
+// many times longer, which is why the line rises with the tiles a head has.  Both give the same bits.
+// Whole backward, fp16, head dim 64, microseconds in steps of 64 / 128 rows, recompute and atomic mode:
+//     512 rows: 160 CTAs 24.3 / 23.6 and 24.9 / 24.1, 192 CTAs 25.3 / 26.6 and 26.9 / 26.9, 512 CTAs 43 / 57 and 45 / 52
+//    2048 rows: 320 CTAs 69.4 / 68.9 and 62.9 / 61.4, 384 CTAs 73.7 / 79.3 and 65.8 / 69.9, 144 CTAs 67.6 / 46.5 and 49.6 / 43.4
+//    8192 rows: 384 CTAs 271 / 229 and 211 / 202, 512 CTAs 301 / 309 and 249 / 260, 128 CTAs 217 / 146 and 155 / 127
+//   32768 rows: 256 CTAs 872 / 552 and 680 / 461, 512 CTAs 1145 / 1141 and 935 / 963, 1024 CTAs 2191 / 2271 and 1843 / 1898
+// (head dim 32, 8192 rows, 512 CTAs: 263 / 251 and 189 / 203).
+inline int bwd_step_rows(const AttnShape& s, int rows, bool atomic, int num_sms) {
+  const int tiles = (rows + 127) / 128;
+  const int percent = tiles <= 4 ? 125 : (tiles <= 16 ? 240 : (atomic ? 330 : 360));  // CTAs a hundred SMs
+  return s.D <= 64 && 100ll * tiles * s.B * s.H >= static_cast<long long>(percent) * num_sms ? 64 : 128;
+}
 
 // Order in which the causal kernels take their (head, tile) work items.  A tile's work shrinks
 // with its rank (rank 0 is the tile that meets the most tiles of the other kind), so for an even
@@ -180,8 +193,8 @@ cudaError_t launch_bwd_preprocess(const AttnShape& s, const void* o, const Strid
 cudaError_t launch_bwd_dkdv(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                             const CUtensorMap& tv, const CUtensorMap& tdo,
                             const CUtensorMap& tdk, const CUtensorMap& tdv, const F32Out& dk32,
-                            const F32Out& dv32, const RowStats& rowstats, float* dq_accum, int mode, int* status,
-                            cudaStream_t stream);
+                            const F32Out& dv32, const RowStats& rowstats, float* dq_accum, int mode, int step_rows,
+                            int* status, cudaStream_t stream);
 
 // Head dim 256: P^T and dS^T of every (KV tile, Q tile) pair as 16-bit piece-major tiles into two
 // scratch tensors (pair numbering as in the spill mode); launch_bwd_consume forms 0, 1 and 2 then
@@ -220,7 +233,8 @@ inline long long dstile_pairs(int N, int Nk) {
 // dQ per Q tile, ascending KV order (deterministic path).
 cudaError_t launch_bwd_dq(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                           const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdq,
-                          const F32Out& dq32, const RowStats& rowstats, int* status, cudaStream_t stream);
+                          const F32Out& dq32, const RowStats& rowstats, int step_rows, int* status,
+                          cudaStream_t stream);
 
 // dq = convert(dq_accum) (non-deterministic path); into dq32 when that is given.
 cudaError_t launch_dq_convert(const AttnShape& s, const float* dq_accum, void* dq,

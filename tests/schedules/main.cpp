@@ -139,7 +139,7 @@ void sim_run(unsigned n, void (*body)(void*), void* arg) {
 #include "bwd.cu"
 #include "fwd.cu"
 
-// main <kernel> <head dim> <rows> <keys> <schedules>
+// main <kernel> <head dim> <rows> <keys> <schedules> <rows of a step>
 int main(int, char** argv) {
   using namespace fa2;
   const std::string kernel = argv[1];
@@ -153,13 +153,14 @@ int main(int, char** argv) {
   int status = 0;
   unsigned counter = 0;
   const LaunchCtx ctx{&status, &counter, 1};
+  const int step = atoi(argv[6]);
   for (int seed = 0; seed < atoi(argv[5]); ++seed) {
     rng.seed(seed);
     if (kernel == "fwd") launch_fwd(s, m, m, m, m, none, lse.data(), ctx, nullptr);
-    if (kernel == "dkdv") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, nullptr, 0, &status, nullptr);
-    if (kernel == "dkdv_atomic") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 1, &status, nullptr);
-    if (kernel == "dkdv_spill") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 2, &status, nullptr);
-    if (kernel == "dq") launch_bwd_dq(s, m, m, m, m, m, none, rs, &status, nullptr);
+    if (kernel == "dkdv") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, nullptr, 0, step, &status, nullptr);
+    if (kernel == "dkdv_atomic") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 1, step, &status, nullptr);
+    if (kernel == "dkdv_spill") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 2, step, &status, nullptr);
+    if (kernel == "dq") launch_bwd_dq(s, m, m, m, m, m, none, rs, step, &status, nullptr);
     if (kernel == "scores") launch_bwd_scores_wide(s, m, m, m, m, rs, scratch.data(), scratch.data(), &status, nullptr);
     for (int form = 0; form < 3; ++form) {
       if (kernel == "consume" && (d > 128 || form == 2)) launch_bwd_consume(s, form, scratch.data(), m, m, none, rs, false, &status, nullptr);

@@ -714,6 +714,34 @@ def test_deterministic_mode_is_bit_identical_across_partitionings():
             assert torch.equal(torch.cat(parts[key], dim=1).view_as(full[key]), full[key]), (key, world)
 
 
+@pytest.mark.parametrize("mode", ["recompute", "atomic"])
+@pytest.mark.parametrize("d,dtype", [(64, torch.float16), (40, torch.bfloat16), (32, torch.float16)])
+@pytest.mark.parametrize("nq,nk", [(1, 1), (63, 63), (64, 64), (65, 65), (128, 64), (129, 65), (191, 191), (192, 192),
+                                   (193, 129), (257, 257), (320, 191), (449, 449), (1153, 385)])
+def test_narrow_heads_give_the_same_bits_few_and_many_at_a_time(nq, nk, d, dtype, mode, monkeypatch):
+    """640 heads fill the GPU and go through the backward in 64-row steps, a single one in 128-row steps: same
+    bits (dq of the atomic mode, whose summation order is free, to rounding), and parity with the oracle."""
+    monkeypatch.setenv("FA2_B200_BWD_MODE", mode)
+    g = torch.Generator().manual_seed(nq * 1000 + nk + d)
+    q, do = (torch.randn(2, 320, nq, d, generator=g).to(dtype) for _ in range(2))
+    k, v = (torch.randn(2, 320, nk, d, generator=g).to(dtype) for _ in range(2))
+    many = run_api(q, k, v, do, None, mode != "atomic")
+    for b, h in ((0, 0), (1, 41), (1, 319)):
+        one = [t[b : b + 1, h : h + 1] for t in (q, k, v, do)]
+        few = run_api(*one, None, mode != "atomic")
+        part = {key: t[b : b + 1, h : h + 1] for key, t in many.items()}
+        ref = naive_attention(*one)
+        check_against(ref, few, dtype)
+        check_against(ref, part, dtype)
+        for key in few:
+            x, y = few[key], part[key]
+            if key == "dq" and mode == "atomic":  # one ulp at most between two summation orders in fp32
+                ulp = 2e-3 if dtype == torch.float16 else 1.6e-2
+                assert ((x.float() - y.float()).abs() <= ulp * y.float().abs() + 1e-5).all()
+            else:
+                assert torch.equal(x, y), key
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs at least two GPUs")
 def test_deterministic_mode_is_bit_identical_across_gpus():
     """Each GPU of the node computes its slab of (batch, head) problems; gathered, the results
