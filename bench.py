@@ -92,7 +92,7 @@ NCU_DKDV_DRAM_MB_PER_24 = {1: 208.6 + 74.7, 2: 329.6 + 1679.5}  # the dK/dV kern
 
 # Polynomial share of the exponentials (of every 8 column pairs) the kernels are built with
 # (FwdCfg::kPolyShare in csrc/fwd.cu, kPolyShareT in csrc/bwd_roles.cuh).
-POLY_SHARE = {"fwd": 0.0, "bwd": 2 / 8}  # at the head dims the ceiling is reported for (<= 64)
+POLY_SHARE = {"fwd": 3 / 8, "bwd": 2 / 8}  # head dims <= 64 and more than 1024 rows, as the workloads here
 
 
 def softmax_ceiling(d, which):

@@ -254,16 +254,16 @@ static int fwd_strided(const void* q, const void* k, const void* v, void* o, flo
   DeviceState* d = nullptr;
   if (int e = device_state(&d)) return e;
   CUtensorMap tq, tk, tv, to;
-  const int kv_rows = fwd_kv_rows(padded_head_dim(D));
+  const AttnShape s = make_shape(B, H, N, Nk, D, dtype, scale);
+  const int kv_rows = fwd_kv_rows(s);
   if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, 128)) return e;
   if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, kv_rows)) return e;
   if (int e = make_map_of(&tv, v, strides, 2, dtype, B, H, Nk, D, kv_rows)) return e;
   if (int e = make_map_of(&to, o, strides, 3, dtype, B, H, N, D, 32)) return e;
-  const AttnShape s = make_shape(B, H, N, Nk, D, dtype, scale);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LaunchCtx ctx;
   make_ctx(d, &ctx);
-  return static_cast<int>(launch_fwd(s, tq, tk, tv, to, out32, lse, ctx, st));
+  return static_cast<int>(launch_fwd(s, kv_rows, tq, tk, tv, to, out32, lse, ctx, st));
 }
 
 int fa2_fwd_strided(const void* q, const void* k, const void* v, void* o, float* lse, int B, int H,

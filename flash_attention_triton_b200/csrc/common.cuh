@@ -81,9 +81,6 @@ struct RowStats {
 // Smallest instantiated head dim that holds `d` columns.
 inline int padded_head_dim(int d) { return d <= 32 ? 32 : (d <= 64 ? 64 : (d <= 128 ? 128 : 256)); }
 
-// Rows of the KV tiles the forward kernel walks (its K and V tensor maps use boxes of this height).
-__host__ __device__ constexpr int fwd_kv_rows(int padded_d) { return padded_d <= 64 ? 64 : 128; }
-
 // Rows of the tiles a backward kernel walks past its resident tile, one CTA per resident tile of the `rows` of a
 // head: Q and dO tiles of the dK/dV kernel (its spill mode always takes 128), K and V tiles of the dQ kernel.
 // Up to head dim 64 steps of 64 rows with two CTAs on an SM win once there are CTAs to pair: a CTA that has its SM
@@ -99,6 +96,30 @@ inline int bwd_step_rows(const AttnShape& s, int rows, bool atomic, int num_sms)
   const int tiles = (rows + 127) / 128;
   const int percent = tiles <= 4 ? 125 : (tiles <= 16 ? 240 : (atomic ? 330 : 360));  // CTAs a hundred SMs
   return s.D <= 64 && 100ll * tiles * s.B * s.H >= static_cast<long long>(percent) * num_sms ? 64 : 128;
+}
+
+// Rows of the KV tiles the forward kernel walks (its K and V tensor maps use boxes of this height): 64, with two
+// CTAs on an SM, up to head dim 64 and 1024 rows.  The two forms round differently (other rescale points,
+// other exponentials), so the rule looks at nothing but the head dim and the rows: O, and with it every
+// gradient, keeps its bits however a batch is split.  Where the work fills the GPU 64 rows win up to about 4096
+// rows at head dim 64 and everywhere at 32; where it does not they lose, the more the longer the rows.
+// fp16, head dim 64, microseconds with 64 / 128 rows (single-tile items below where they are taken):
+//     512 rows: 256 heads 27.9 / 34.4, 128: 18.5 / 18.4, 64: 13.5 / 11.7, 8: 12.3 / 12.2
+//    1000 rows: 256 heads 68.3 / 85.4, 128: 35.9 / 43.6, 64: 26.1 / 24.2, 16: 19.5 / 18.2
+//    2048 rows: 48 heads 53.2 / 49.0, 32: 50.7 (38.9) / 32.7, 8: 33.6 (29.9) / 27.2
+//    4096 rows: 64 heads 203 / 210, 32: 104 / 100, 16: 91.6 (66.5) / 51.2, 4: 61.1 (54.7) / 48.2
+//   16384 rows: 16 heads 766 / 721, 4: 337 (246) / 177;   32768 rows: 8 heads 1500 / 1385, 2: 669 (486) / 347
+// (head dim 32: 4096 rows, 64 heads 172 / 187; 32768 rows, 8 heads 1199 / 1215).  Up to 1024 rows the loss
+// with few heads stays at 2 us of a call that takes some 20 us on the host.
+inline int fwd_kv_rows(const AttnShape& s) { return s.D <= 64 && s.N <= 1024 ? 64 : 128; }
+
+// Q tiles of a work item of the 64-row form: two that share every K and V tile, or one where there are few, so that
+// they spread over more CTAs and no CTA is left with a long pair.  Microseconds, one / two, head dim 64: 1000
+// rows: 16 heads 19.5 / 21.5, 64: 26.1 / 29.8, 128: 47.7 / 35.9; 512 rows: 80 heads 13.7 / 17.9, 128: 18.8 / 18.5,
+// 256: 34.7 / 27.9; 300 rows: 64 heads 10.3 / 10.2, 128: 15.1 / 12.9.  Same bits.
+inline int fwd_tiles_per_item(const AttnShape& s, int num_sms) {
+  const long long tiles = (s.N + 127) / 128;
+  return 2 * tiles * s.B * s.H <= (tiles <= 3 ? 4 : 7) * static_cast<long long>(num_sms) ? 1 : 2;
 }
 
 // Order in which the causal kernels take their (head, tile) work items.  A tile's work shrinks
@@ -173,7 +194,7 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, in
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-cudaError_t launch_fwd(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
+cudaError_t launch_fwd(const AttnShape& s, int kv_rows, const CUtensorMap& tq, const CUtensorMap& tk,
                        const CUtensorMap& tv, const CUtensorMap& to, const F32Out& o32, float* lse,
                        const LaunchCtx& ctx, cudaStream_t stream);
 

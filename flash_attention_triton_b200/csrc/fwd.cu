@@ -2,7 +2,7 @@
 //
 // Replaces _forward_kernel (src/flash_attention_triton/_triton_kernels_v2.py:11-189 of the
 // reference).  One CTA owns two adjacent 128-row Q tiles of one (batch, head) and walks the KV
-// tiles 0..diagonal.  (What follows describes head dims above 64; the last paragraph the others.)  Warp roles:
+// tiles 0..diagonal.  (What follows describes 128-row KV tiles, the last paragraph 64-row ones.)  Warp roles:
 //   warps 0-3   softmax for Q tile 0   (thread = one score row = one tensor-memory lane)
 //   warps 4-7   softmax for Q tile 1
 //   warp  8     issues S = Q_i K_j^T          } one elected lane each; two warps so that neither
@@ -25,20 +25,21 @@
 // polynomial on the FMA pipe because the MUFU rate (16 / clk / SM) would otherwise bound the
 // kernel: 2 x 128 x 128 exponentials per KV step cost as many cycles as the four MMAs.
 //
-// Head dims up to 64: the MMAs of a tile are short (512 cycles or less per 128 x 128 scores) and the
+// Head dims up to 64, rows up to fwd_kv_rows' line: the MMAs of a tile are short (512 cycles or less per 128 x 128 scores) and the
 // softmax instruction stream is what takes the time; with two softmax warps per scheduler it issues
 // in half of the cycles only, the rest is latency of dependent instructions.  So the KV tiles are
 // 64 rows there: a thread holds 64 instead of 128 scores, 96 registers do instead of 208, 256
 // columns of tensor memory instead of 512, and TWO CTAs run on an SM, four softmax warps per
 // scheduler.  The exponentials then all go to the MUFU, which has time (the polynomial costs five
-// times the issue slots).  Measured against 128-row tiles and one CTA, microseconds:
-// [4,16,2048,64] 70.5 -> 61.6, [8,12,4095,32] 296 -> 269, [2,16,8192,64] 388 -> 382.
+// times the issue slots).  Measured against 128-row tiles and one CTA, fp16, head dim 64, microseconds:
+// [1,256,1000,64] 85.4 -> 68.3, [1,128,1000,64] 43.6 -> 35.9, [1,256,512,64] 34.4 -> 27.9; where there are too
+// few CTAs to pair, or the rows are long, 128-row tiles win (figures at fwd_kv_rows).
 #include "common.cuh"
 #include "mma_issue.cuh"
 #include "ptx.cuh"
 
 #ifndef FA2_FWD_POLY_PAIRS_PER_8
-#define FA2_FWD_POLY_PAIRS_PER_8 3  // of every 8 column pairs, this many use ex2_poly2 (D > 64)
+#define FA2_FWD_POLY_PAIRS_PER_8 3  // of every 8 column pairs, this many use ex2_poly2 (128-row KV tiles)
 #endif
 
 namespace fa2 {
@@ -47,10 +48,11 @@ namespace {
 constexpr int kFwdThreads = 384;
 constexpr float kLn2 = 0.6931471805599453f;
 
-template <int D>
+template <int D, int W>
 struct FwdCfg {
   using T = Tile<D>;
-  static constexpr int kW = fwd_kv_rows(D);  // rows of a KV tile = columns of a score tile
+  static constexpr int kW = W;  // rows of a KV tile = columns of a score tile
+  static_assert(W == 128 || (W == 64 && D <= 64), "fwd_kv_rows");
   static constexpr int kPolyShare = kW == 64 ? 0 : FA2_FWD_POLY_PAIRS_PER_8;
   static constexpr int kCtasPerSm = kW == 64 ? 2 : 1;
   // O is rescaled when the running maximum has moved by more than this (log2 units).  A row's
@@ -107,12 +109,13 @@ enum FwdSite {
   kSiteAlign
 };
 
-template <int D, bool BF16, int KD = D>
-__global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtasPerSm)
+template <int D, bool BF16, int KD, int W>
+__global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kCtasPerSm)
     fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap to,
                const __grid_constant__ F32Out o32, int cols, float* __restrict__ lse, int N, int Nk,
-               int num_bh, int num_heads, int group, float scale_log2, int* status, unsigned int* work_counter) {
+               int num_bh, int num_heads, int group, float scale_log2, int tiles_per_item, int* status,
+               unsigned int* work_counter) {
   // Head dim 256 ("wide") runs on the staging and tensor-memory plan of head dim 128 with ONE
   // Q tile per work item: the two Q slots hold the two 128-column halves of that tile, K and V
   // tiles stream through their rings as half tiles, S = Q_lo K_lo^T + Q_hi K_hi^T accumulates
@@ -120,9 +123,8 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
   constexpr bool WIDE = D == 256;
   constexpr int DT = WIDE ? 128 : D;    // columns of one staged tile
   constexpr int HALVES = WIDE ? 2 : 1;  // staged tiles per 128 rows
-  using C = FwdCfg<DT>;
+  using C = FwdCfg<DT, W>;
   using T = Tile<DT>;
-  constexpr int W = C::kW;  // rows of a KV tile
   constexpr int KT = WIDE ? DT : KD;  // columns of a staged tile that the products run over
   extern __shared__ __align__(1024) uint8_t smem[];
 
@@ -145,7 +147,8 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
 
   const int ntiles = (N + 127) >> 7;
   const int nktiles = (Nk + W - 1) / W;  // KV tiles of W rows
-  const int npairs = WIDE ? ntiles : (ntiles + 1) >> 1;  // work items per (batch, head)
+  const int per_item = WIDE ? 1 : (W == 128 ? 2 : tiles_per_item);  // Q tiles of a work item
+  const int npairs = per_item == 1 ? ntiles : (ntiles + 1) >> 1;    // work items per (batch, head)
   const int total_items = npairs * num_bh;
 
   if (threadIdx.x == 0) *abort_flag = 0;
@@ -202,8 +205,8 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
     const int bh = ht.bh;
     const HeadCoord hc{bh % num_heads, bh / num_heads};
     const int pair = npairs - 1 - ht.rank;  // the last pair of Q tiles meets the most KV tiles
-    const int qt0 = WIDE ? pair : 2 * pair, qt1 = qt0 + 1;
-    const bool has1 = !WIDE && qt1 < ntiles;
+    const int qt0 = per_item * pair, qt1 = qt0 + 1;
+    const bool has1 = per_item == 2 && qt1 < ntiles;
     // KV tiles of Q tile i: those up to its diagonal, or to the last key  (N = query rows,
     // Nk <= N = key rows)
     constexpr int kPerQ = 128 / W;
@@ -524,31 +527,36 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D>::kCtas
   }
 }
 
-template <int D, bool BF16, int KD = D>
+template <int D, bool BF16, int KD = D, int W = 128>
 cudaError_t launch_fwd_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                          const CUtensorMap& tv, const CUtensorMap& to, const F32Out& o32, float* lse,
                          const LaunchCtx& ctx, cudaStream_t stream) {
-  using C = FwdCfg<D == 256 ? 128 : D>;  // head dim 256 runs on the plan of head dim 128
-  auto kern = fwd_kernel<D, BF16, KD>;
+  using C = FwdCfg<D == 256 ? 128 : D, W>;  // head dim 256 runs on the plan of head dim 128
+  auto kern = fwd_kernel<D, BF16, KD, W>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
   const int ntiles = (s.N + 127) / 128;
-  const int npairs = D == 256 ? ntiles : (ntiles + 1) / 2;
-  const long long items = static_cast<long long>(npairs) * s.B * s.H;
+  const int tiles_per_item = D == 256 ? 1 : (W == 128 ? 2 : fwd_tiles_per_item(s, ctx.num_sms));
+  const long long items = static_cast<long long>((ntiles + tiles_per_item - 1) / tiles_per_item) * s.B * s.H;
   const long long slots = static_cast<long long>(ctx.num_sms) * C::kCtasPerSm;
   const unsigned grid = static_cast<unsigned>(items < slots ? items : slots);
   const float scale_log2 = s.scale * 1.4426950408889634f;
   return launch_dependent(kern, grid, kFwdThreads, C::kSmemBytes, stream,
-      tq, tk, tv, to, o32, s.Dg, lse, s.N, s.Nk, s.B * s.H, s.H, heads_per_group(s), scale_log2, ctx.status,
-      ctx.work_counter);
+      tq, tk, tv, to, o32, s.Dg, lse, s.N, s.Nk, s.B * s.H, s.H, heads_per_group(s), scale_log2,
+      tiles_per_item, ctx.status, ctx.work_counter);
 }
 
 }  // namespace
 
-cudaError_t launch_fwd(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
+cudaError_t launch_fwd(const AttnShape& s, int kv_rows, const CUtensorMap& tq, const CUtensorMap& tk,
                        const CUtensorMap& tv, const CUtensorMap& to, const F32Out& o32, float* lse,
                        const LaunchCtx& ctx, cudaStream_t stream) {
+  if (kv_rows == 64)
+    return s.D == 64 ? (s.dtype ? launch_fwd_t<64, true, 64, 64>(s, tq, tk, tv, to, o32, lse, ctx, stream)
+                                : launch_fwd_t<64, false, 64, 64>(s, tq, tk, tv, to, o32, lse, ctx, stream))
+                     : (s.dtype ? launch_fwd_t<32, true, 32, 64>(s, tq, tk, tv, to, o32, lse, ctx, stream)
+                                : launch_fwd_t<32, false, 32, 64>(s, tq, tk, tv, to, o32, lse, ctx, stream));
 #define FA2_CASE(DD)                                                                 \
   case DD:                                                                           \
     return s.dtype ? launch_fwd_t<DD, true>(s, tq, tk, tv, to, o32, lse, ctx, stream)     \

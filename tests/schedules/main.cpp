@@ -152,11 +152,12 @@ int main(int, char** argv) {
   const RowStats rs{stats.data(), amax.data()};
   int status = 0;
   unsigned counter = 0;
-  const LaunchCtx ctx{&status, &counter, 1};
+  LaunchCtx ctx{&status, &counter, 1};
   const int step = atoi(argv[6]);
   for (int seed = 0; seed < atoi(argv[5]); ++seed) {
     rng.seed(seed);
-    if (kernel == "fwd") launch_fwd(s, m, m, m, m, none, lse.data(), ctx, nullptr);
+    ctx.num_sms = 1 + seed % 2 * 63;  // work items of two Q tiles and of one
+    if (kernel == "fwd") launch_fwd(s, step, m, m, m, m, none, lse.data(), ctx, nullptr);
     if (kernel == "dkdv") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, nullptr, 0, step, &status, nullptr);
     if (kernel == "dkdv_atomic") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 1, step, &status, nullptr);
     if (kernel == "dkdv_spill") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 2, step, &status, nullptr);

@@ -69,7 +69,7 @@ def test_dq_roles(simulator, headdim, rows, keys):
 @pytest.mark.parametrize("headdim", [32, 64, 96, 128, 256])
 def test_forward_roles(simulator, headdim, rows, keys):
     """One CTA takes every work item: what an item leaves on its way to a barrier meets the next one."""
-    check(simulator, "fwd", headdim, rows, keys)
+    check(simulator, "fwd", headdim, rows, keys, steps_of(headdim))
 
 
 @pytest.mark.parametrize("rows,keys", [(1, 1), (128, 64), (449, 300), (640, 640)])
