@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
       bool pv_waited = false;
       if (__any_sync(0xffffffffu, need)) {
         // A neighbour's rescale must not touch a row without a finite score so far: -inf - -inf is no factor.
-        const float alpha = W == 64 && m_new == -INFINITY ? 1.0f : ex2((m_run - m_new) * scale_log2);
+        const float alpha = m_new == -INFINITY ? 1.0f : ex2((m_run - m_new) * scale_log2);
         l_run *= alpha;
         m_run = m_new;
         if (j > 0) {
@@ -428,9 +428,9 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
       }
       // p = 2^(s*c - m*c) with packed fp32x2 FMAs; row sum in four independent packed chains.
       const float2 sc2 = make_float2(scale_log2, scale_log2);
-      // A row whose scores so far are all -inf (infinite inputs) has weights 0 and not -inf + inf: half as
-      // many columns as before decide a row's first maximum with 64-row tiles.
-      const float neg_m = W == 64 && m_run == -INFINITY ? 0.f : -m_run * scale_log2;
+      // A row whose scores so far are all -inf (infinite inputs, or finite ones whose product overflows) has
+      // weights 0 (2^-126 from the polynomial) and not -inf + inf; its first finite score rescales them away.
+      const float neg_m = m_run == -INFINITY ? 0.f : -m_run * scale_log2;
       const float2 nm2 = make_float2(neg_m, neg_m);
       float2 acc[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
       uint32_t pk[W / 2];
@@ -461,7 +461,8 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
     }
     if (ok && nj > 0 && mbar_wait_warp(bar(C::kBarPvDone + wg), (nj - 1) & 1, w, kSiteSoftO)) {
       tc_fence_after();
-      const float inv_l = 1.0f / l_run;
+      // a row without any finite score has no softmax, whatever weights it was left with
+      const float inv_l = m_run == -INFINITY ? __uint_as_float(0x7fffffffu) : 1.0f / l_run;
       // Stage the tile through the (now idle) Q buffer in the swizzled layout the output
       // tensor map expects; each warp stores its own 32 rows.
       uint8_t* sO = smem + C::kOffQ + wg * T::kTileBytes;

@@ -260,6 +260,34 @@ def test_rows_of_minus_infinity_beside_rows_that_rescale(d, dtype, key, queries)
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("d", [32, 64, 96, 128, 256])
+@pytest.mark.parametrize("n", [330, 1025])
+@pytest.mark.parametrize("first", [128, 200])  # a whole first tile, and one tile and part of the next
+@pytest.mark.parametrize("dtype,key,queries", [
+    (torch.float16, -math.inf, (1.0, 1.0)),
+    (torch.bfloat16, -math.inf, (1.0, -1.0)),  # every second row scores +inf there (and is NaN itself)
+    (torch.bfloat16, -3e38, (2.0, 0.5)),  # finite inputs: 2 q k overflows to -inf, q k / 2 does not
+])
+def test_rows_of_minus_infinity_over_whole_tiles(d, n, first, dtype, key, queries):
+    """As above with the first `first` keys, in either form of the kernel (the rows decide): rows beyond them
+    attend to the other keys, and rows with no other key have no softmax."""
+    g = torch.Generator().manual_seed(d)
+    q, k, v = (torch.randn(1, 2, n, d, generator=g).to(dtype) for _ in range(3))
+    q[..., 0::2, 0], q[..., 1::2, 0] = queries
+    k[:, :, :first, 0] = key
+    k[:, :, first:, 0] = 0.0
+    out = flash_attention_v2(q.to(DEV), k.to(DEV), v.to(DEV)).cpu().double()
+    scores = (q.double() @ k.double().transpose(-1, -2)) / math.sqrt(d)
+    scores.masked_fill_(torch.ones(n, n, dtype=torch.bool).triu(1), -math.inf)
+    want = scores[..., first::2, first:].softmax(-1) @ v.double()[:, :, first:]
+    assert (out[:, :, first::2] - want).abs().max() <= BASE_TOL[dtype]
+    assert out[:, :, 0:first:2].isnan().all()
+    if math.isfinite(key):  # these rows have finite scores everywhere, and no weight on the first keys
+        want = scores[..., first + 1::2, first:].softmax(-1) @ v.double()[:, :, first:]
+        assert (out[:, :, first + 1::2] - want).abs().max() <= BASE_TOL[dtype]
+    assert _lib.device_status() == 0
+
+
 def test_spill_mode_chunks_change_no_bit(monkeypatch):
     """With a scratch bound of 3 MiB the spill mode works through [3, 5, 700, 64] (0.7 MiB per
     head) in chunks of 3 + 2 heads per batch entry; with 8 MiB in chunks of 2 + 1 batch
