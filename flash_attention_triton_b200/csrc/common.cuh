@@ -235,14 +235,14 @@ cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch
                                const CUtensorMap& tb, const CUtensorMap& tout, const F32Out& out32,
                                const RowStats& rowstats, bool two_tiles, int* status, cudaStream_t stream);
 
-// Whether the consumers of head dim 256 take two output tiles per CTA: when there are CTAs for one and a
-// half times the SMs.  Fewer, longer CTAs leave SMs idle.  Whole bf16 backward, microseconds, one tile
-// against two: 1024 pairs [2,16,8192,256] 3517 / 3015, 256 pairs
-// [1,16,4096,256] 506 / 456 and [1,32,2048,256] 312 / 283; 128 pairs [1,4,8192,256] 460 / 552, 64 pairs
-// [1,8,2048,256] 124 / 142.
+// Whether the consumers of head dim 256 take two output tiles per CTA: when that still gives every SM a CTA.
+// Below, fewer and longer CTAs leave SMs idle.  Whole bf16 backward, microseconds, one tile against two:
+//     1024 rows: 128 pairs of tiles 111 / 111, 160: 153 / 139, 192: 164 / 158, 256: 200 / 184, 512: 367 / 342
+//     2048 rows: 128 pairs 148 / 160, 160: 227 / 207, 208: 242 / 225, 256: 276 / 252, 320: 352 / 348
+//     8192 rows: 128 pairs 406 / 481, 160: 680 / 616, 192: 680 / 629, 256: 827 / 749, 320: 1133 / 1137
 inline bool consume_two_tiles(const AttnShape& s, int num_sms) {
   const long long tiles = (s.Nk + 127) / 128;
-  return s.D == 256 && 2 * ((tiles + 1) / 2 * s.B * s.H) >= 3ll * num_sms;
+  return s.D == 256 && (tiles + 1) / 2 * s.B * s.H > num_sms;
 }
 
 // (KV tile, Q tile) pairs of one head: KV tile t < nktiles meets Q tiles t .. ntiles-1.
