@@ -176,11 +176,11 @@ __host__ __device__ __forceinline__ int dstile_count(int ntiles, int jt) {
 // score columns a CTA needs half of the tensor memory and registers, so two CTAs run on an SM and
 // fill each other's waits, at the price of score products that read their A operand twice as often
 // (shared-memory bound: 384 instead of 256 cycles per tile pair at head dim 64).  Measured, whole
-// backward call, microseconds, 128- against 64-row steps: [4,16,2048,64] mode 0 207 -> 171, mode 1
-// 178 -> 169; [8,12,4095,32] mode 0 850 -> 743, mode 1 638 -> 576; [8,16,1000,64] mode 0 147 -> 120,
-// mode 1 124 -> 115; [2,16,8192,64] mode 0 1258 -> 1149, mode 1 986 -> 997 (bound by the fp32
-// reductions in L2, 2.2 TB/s: without them it takes 791).  One compute group of 64 columns per thread
-// instead of two of 32 was 2-6 % slower.
+// backward call through autograd, fp16, microseconds, 128- against 64-row steps: [4,16,2048,64] mode 0
+// 216 -> 185, mode 1 181 -> 171; [8,12,4095,32] mode 0 900 -> 830, mode 1 734 -> 685; [8,16,1024,64] mode 0
+// 153 -> 124, mode 1 130 -> 117; [2,16,8192,64] mode 0 1112 -> 1016, mode 1 927 -> 890 (bound by the fp32
+// reductions in L2); [1,16,8192,64], whose last wave of pairs is short, mode 1 519 -> 525.  One compute
+// group of 64 columns per thread instead of two of 32 was 2-6 % slower.
 template <int D, int MODE, int W>
 struct DkdvCfg {
   using T = Tile<D>;
