@@ -18,7 +18,7 @@ __device__ int g_status_word;
 // launches that overlap on the device do not share a counter (unless more than
 // kWorkCounterSlots of them are in flight at once).  No launch zeroes its slot: the slots are
 // zero at module load and every kernel puts its counter back to zero when it draws its last
-// number (fetch_work_item), so a slot is only left non-zero by a kernel that did not run to
+// number, so a slot is only left non-zero by a kernel that did not run to
 // its end.
 constexpr int kWorkCounterSlots = 1024;
 __device__ unsigned int g_work_counters[kWorkCounterSlots];

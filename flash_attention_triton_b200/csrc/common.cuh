@@ -150,27 +150,16 @@ inline int heads_per_group(const AttnShape& s) {
   return static_cast<int>(g < 1 ? 1 : (g > bh ? bh : g));
 }
 
-// Per-launch context of the forward kernel.  It runs one or two CTAs per SM; each CTA fetches work
-// items (pairs of Q tiles) from `work_counter` until none are left, so tensor memory is
-// allocated once and no SM idles between items.  The counter is zero before the launch and the kernel
-// leaves it at zero (see fetch_work_item), so no memset sits between launches.
+// Per-launch context of the forward kernel.  It runs one or two CTAs per SM; a CTA takes work item blockIdx.x
+// and then draws items (pairs of Q tiles) from `work_counter` until none are left, so tensor memory is
+// allocated once and no SM idles between items.  The counter is zero before the launch; a launch draws
+// total_items numbers in all (one with every item), and whoever draws the last one puts the counter back to zero,
+// so no memset sits between launches.
 struct LaunchCtx {
   int* status;                 // device status word (bounded-wait failures)
   unsigned int* work_counter;  // device word, 0 at kernel start and again at kernel end
   int num_sms;
 };
-
-// Next work item of this CTA (called by one thread).  With a counter, CTAs draw items in launch
-// order until the counter passes `total_items`; the launch draws total_items + gridDim.x numbers
-// in all, and whoever draws the last one puts the counter back to zero for the next launch that
-// uses it.  Without a counter every CTA handles the single item blockIdx.x.
-__device__ __forceinline__ int fetch_work_item(unsigned int* work_counter, int total_items,
-                                               bool first) {
-  if (work_counter == nullptr) return first ? static_cast<int>(blockIdx.x) : total_items;
-  const unsigned int next = atomicAdd(work_counter, 1u);
-  if (next == static_cast<unsigned int>(total_items) + gridDim.x - 1u) atomicExch(work_counter, 0u);
-  return next < static_cast<unsigned int>(total_items) ? static_cast<int>(next) : total_items;
-}
 
 // Launches a kernel that may overlap the end of its predecessor on the stream (grid_wait_previous and
 // grid_allow_next in ptx.cuh).  A successor without the attribute, a memset or an event still waits for the

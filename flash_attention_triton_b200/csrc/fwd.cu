@@ -7,7 +7,7 @@
 //   warps 4-7   softmax for Q tile 1
 //   warp  8     issues S = Q_i K_j^T          } one elected lane each; two warps so that neither
 //   warp  10    issues O_i += P_i V_j         } MMA stream waits behind the other's barriers
-//   warp  9     TMA producer: Q once, then a K ring and a V ring
+//   warp  9     draws the work items; TMA producer: Q once an item, then a K ring and a V ring
 //   warp  11    idle; warps 8-11 give registers to the softmax groups (setmaxnreg)
 // (role numbers; hardware warps 0-3 take roles 8-11, see below)
 //
@@ -38,10 +38,6 @@
 #include "mma_issue.cuh"
 #include "ptx.cuh"
 
-#ifndef FA2_FWD_POLY_PAIRS_PER_8
-#define FA2_FWD_POLY_PAIRS_PER_8 3  // of every 8 column pairs, this many use ex2_poly2 (128-row KV tiles)
-#endif
-
 namespace fa2 {
 namespace {
 
@@ -53,7 +49,7 @@ struct FwdCfg {
   using T = Tile<D>;
   static constexpr int kW = W;  // rows of a KV tile = columns of a score tile
   static_assert(W == 128 || (W == 64 && D <= 64), "fwd_kv_rows");
-  static constexpr int kPolyShare = kW == 64 ? 0 : FA2_FWD_POLY_PAIRS_PER_8;
+  static constexpr int kPolyShare = kW == 64 ? 0 : 3;  // of every 8 column pairs, this many use ex2_poly2
   static constexpr int kCtasPerSm = kW == 64 ? 2 : 1;
   // O is rescaled when the running maximum has moved by more than this (log2 units).  A row's
   // largest P is exactly 1, without rounding error, when its maximum is fresh: 64-row tiles, whose
@@ -65,18 +61,28 @@ struct FwdCfg {
   // kLaunchRegs (the launch bounds' limit, rounded down to a multiple of 8)
   static constexpr int kLaunchRegs = 65536 / (kFwdThreads * kCtasPerSm) / 8 * 8;
   static constexpr int kProducerRegs = kW == 64 ? 48 : 72;
-  static constexpr int kSoftmaxRegs = kW == 64 ? 96 : 208;
+  static constexpr int kSoftmaxRegs = kW == 64 ? 96 : 216;
   static_assert(128 * kProducerRegs + 256 * kSoftmaxRegs <= kFwdThreads * kLaunchRegs,
                 "setmaxnreg.inc waits for registers that setmaxnreg.dec has released");
-  static constexpr int kKStages = D == 128 ? 3 : 4;
-  static constexpr int kVStages = D == 128 ? 2 : 4;
+  // At head dim 128 a third K stage measured the same as two; the output staging takes its place.
+  static constexpr int kKStages = D == 128 ? 2 : 4;
+  static constexpr int kVStages = kKStages;
+  // O is staged in its own memory, 32 rows of one chunk for each softmax warp, so that the next item's Q can be
+  // loaded under the epilogue; in the 64-row form, where the other CTA of the SM fills the gap, in the Q
+  // tiles (with own memory the rings lose a stage: [8,16,1000,64] 35.6 -> 37.8 us).
+  static constexpr bool kStageInQ = kW == 64;
+  static constexpr int kStageBytes = 32 * T::kRowBytes;
   static constexpr int kOffQ = 0;
   static constexpr int kOffK = kOffQ + 2 * T::kTileBytes;
   static constexpr int kOffV = kOffK + kKStages * kKvBytes;
-  static constexpr int kOffBar = kOffV + kVStages * kKvBytes;
+  static constexpr int kOffStage = kOffV + kVStages * kKvBytes;  // one piece for each softmax warp
+  static constexpr int kOffBar = kOffStage + (kStageInQ ? 0 : 8 * kStageBytes);
   // barrier slots
-  static constexpr int kBarQFull = 0;
-  static constexpr int kBarKFull = 1;
+  static constexpr int kBarItemFull = 0;   // 2: the work item in slot n % 2 may be read
+  static constexpr int kBarItemEmpty = 2;  // 2: every role but the producer has read it (10 arrivals)
+  static constexpr int kBarQFull = 4;
+  static constexpr int kBarQEmpty = 5;     // the item's last score product, or its last store, has read the Q tiles
+  static constexpr int kBarKFull = 6;
   static constexpr int kBarKEmpty = kBarKFull + kKStages;
   static constexpr int kBarVFull = kBarKEmpty + kKStages;
   static constexpr int kBarVEmpty = kBarVFull + kVStages;
@@ -85,7 +91,8 @@ struct FwdCfg {
   static constexpr int kBarPFull = kBarSFree + 2;    // 2: P_i written, O_i rescaled (4 arrivals)
   static constexpr int kBarPvDone = kBarPFull + 2;   // 2: O_i += P_i V completed
   static constexpr int kNumBars = kBarPvDone + 2;
-  static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;  // + tmem slot, abort, work slot
+  static constexpr int kOffItems = (kOffBar + kNumBars * 8 + 15) / 16 * 16;  // 2 x WorkItem
+  static constexpr int kSmemBytes = kOffItems + 2 * 16 + 16;  // + tmem slot, abort flag, next item
   // tensor-memory columns
   static constexpr int kColS = 0;
   static constexpr int kColP = kW;      // P0, then P1 (kW / 2 columns of 16-bit pairs each)
@@ -93,6 +100,12 @@ struct FwdCfg {
   static constexpr int kTmemCols = 512 / kCtasPerSm;
   static_assert(kColO + 2 * D <= kTmemCols, "tensor memory of one CTA");
   static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "shared memory of one SM");
+};
+
+// What the producer leaves in an item slot: one Q tile, or two adjacent ones, of one (batch, head).
+struct WorkItem {
+  int pair;  // -1: no more items
+  int bh, h, b;
 };
 
 enum FwdSite {
@@ -106,7 +119,9 @@ enum FwdSite {
   kSiteSoftS,
   kSiteSoftPv,
   kSiteSoftO,
-  kSiteAlign
+  kSiteAlign,
+  kSiteItem,
+  kSiteLoadQ
 };
 
 template <int D, bool BF16, int KD, int W>
@@ -139,10 +154,9 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
     if (threadIdx.x == 0) atomicCAS(status, 0, 0x20000 | kSiteAlign);
     return;
   }
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kOffBar);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::kNumBars);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::kOffItems + 2 * sizeof(WorkItem));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* work_slot = reinterpret_cast<volatile int*>(tmem_slot + 2);
+  volatile int* next_slot = reinterpret_cast<volatile int*>(tmem_slot + 2);
   auto bar = [&](int i) { return smem_base + C::kOffBar + 8u * i; };
 
   const int ntiles = (N + 127) >> 7;
@@ -150,8 +164,38 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
   const int per_item = WIDE ? 1 : (W == 128 ? 2 : tiles_per_item);  // Q tiles of a work item
   const int npairs = per_item == 1 ? ntiles : (ntiles + 1) >> 1;    // work items per (batch, head)
   const int total_items = npairs * num_bh;
+  // KV tiles of an item's Q tile i: those up to its diagonal, or to the last key (N = query rows, Nk <= N = key
+  // rows); 0 for a second tile that does not exist
+  auto second_tile = [&](const WorkItem& item) { return per_item == 2 && 2 * item.pair + 1 < ntiles; };
+  auto kv_tiles = [&](const WorkItem& item, int i) {
+    return i == 1 && !second_tile(item) ? 0 : min((per_item * item.pair + i + 1) * (128 / W), nktiles);
+  };
 
-  if (threadIdx.x == 0) *abort_flag = 0;
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(C::kBarItemFull + i), 1);
+      mbar_init(bar(C::kBarItemEmpty + i), 10);
+    }
+    mbar_init(bar(C::kBarQFull), 1);
+    mbar_init(bar(C::kBarQEmpty), C::kStageInQ ? 8 : 1);
+    for (int i = 0; i < C::kKStages; ++i) {
+      mbar_init(bar(C::kBarKFull + i), 1);
+      mbar_init(bar(C::kBarKEmpty + i), 1);
+    }
+    for (int i = 0; i < C::kVStages; ++i) {
+      mbar_init(bar(C::kBarVFull + i), 1);
+      mbar_init(bar(C::kBarVEmpty + i), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(C::kBarSFull + i), 1);
+      mbar_init(bar(C::kBarSFree + i), 4);
+      mbar_init(bar(C::kBarPFull + i), 4);
+      mbar_init(bar(C::kBarPvDone + i), 1);
+    }
+    fence_mbar_init();
+    fence_proxy_async_smem();
+  }
   if (warp == 8) {
     tmem_alloc(smem_u32(tmem_slot), C::kTmemCols);
     tmem_relinquish();
@@ -164,55 +208,24 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
   grid_wait_previous();
   grid_allow_next();
 
-  // One or two CTAs per SM; work items (one Q-tile pair of one (batch, head)) are fetched from a
-  // global counter in head-major, heavy-pair-first order, like a hardware block scheduler
-  // would hand them out, but without the launch gap and with tensor memory kept allocated.
-  // Between items all roles meet at a barrier and the mbarriers are re-initialised, so each
-  // item starts from phase 0.  Nothing may still be on its way to an mbarrier then: the MMA warps commit
-  // only what another role waits for, no release of a ring stage that is not filled again.
-  for (bool first = true;; first = false) {
-    __syncthreads();  // every role has finished the previous item
-    if (threadIdx.x == 0) {
-      const int next = fetch_work_item(work_counter, total_items, first);
-      *work_slot = next;
-      if (next < total_items && !*abort_flag) {
-        if (!first)
-          for (int i = 0; i < C::kNumBars; ++i) mbar_inval(bar(i));
-        mbar_init(bar(C::kBarQFull), 1);
-        for (int i = 0; i < C::kKStages; ++i) {
-          mbar_init(bar(C::kBarKFull + i), 1);
-          mbar_init(bar(C::kBarKEmpty + i), 1);
-        }
-        for (int i = 0; i < C::kVStages; ++i) {
-          mbar_init(bar(C::kBarVFull + i), 1);
-          mbar_init(bar(C::kBarVEmpty + i), 1);
-        }
-        for (int i = 0; i < 2; ++i) {
-          mbar_init(bar(C::kBarSFull + i), 1);
-          mbar_init(bar(C::kBarSFree + i), 4);
-          mbar_init(bar(C::kBarPFull + i), 4);
-          mbar_init(bar(C::kBarPvDone + i), 1);
-        }
-        fence_mbar_init();
-        fence_proxy_async_smem();
-      }
-    }
-    __syncthreads();
-    const int item = *work_slot;
-    if (item >= total_items) break;
-    if (*abort_flag) continue;  // keep drawing so that the counter is left at zero
-    const HeadTile ht = grouped_order(item, num_bh, npairs, group);
-    const int bh = ht.bh;
-    const HeadCoord hc{bh % num_heads, bh / num_heads};
-    const int pair = npairs - 1 - ht.rank;  // the last pair of Q tiles meets the most KV tiles
-    const int qt0 = per_item * pair, qt1 = qt0 + 1;
-    const bool has1 = per_item == 2 && qt1 < ntiles;
-    // KV tiles of Q tile i: those up to its diagonal, or to the last key  (N = query rows,
-    // Nk <= N = key rows)
-    constexpr int kPerQ = 128 / W;
-    const int n0 = min((qt0 + 1) * kPerQ, nktiles);
-    const int n1 = has1 ? min((qt1 + 1) * kPerQ, nktiles) : 0;
-    const int nkv = n1 > n0 ? n1 : n0;
+  // One or two CTAs per SM.  A CTA starts with work item blockIdx.x and draws the others from a global counter,
+  // heaviest first within a group of heads (grouped_order).  The roles run through the items without
+  // meeting: the producer draws the next item while the last tiles of the one before are in
+  // flight, and loads its first K tile and, once the last score product has read Q, its Q tiles, so that
+  // the next item's scores are formed while the softmax groups finish this one.  Every barrier keeps
+  // its phase from item to item.  What bounds short rows is this boundary; with all roles meeting there it took
+  // some 4 us an item (Q and K loads, first scores, epilogue, one after the other).  Microseconds before and after,
+  // passes in a loop: [32,20,1024,96] fp16 246 -> 223, [4,16,2048,64] fp16 63.4 -> 56.1, [8,12,4095,32] fp16 282 ->
+  // 258, [4,16,1000,64] bf16 25.7 -> 23.9, [2,32,8192,128] bf16 973 -> 974, [1,2,32768,128] 463 -> 471.
+  //
+  // Slot of the n-th item of this CTA, for every role but the producer; false: there is none, or the CTA gives up.
+  auto take_item = [&](int n, WorkItem& item) {
+    if (!mbar_wait_warp(bar(C::kBarItemFull + (n & 1)), (n >> 1) & 1, w, kSiteItem)) return false;
+    item = reinterpret_cast<const WorkItem*>(smem + C::kOffItems)[n & 1];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(C::kBarItemEmpty + (n & 1)));
+    return item.pair >= 0;
+  };
 
   if (warp >= 8) {
     reg_dec<C::kProducerRegs>();  // whole warpgroup (warps 8-11) gives registers to the softmax groups
@@ -224,43 +237,80 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
         prefetch_tensormap(&tq);
         prefetch_tensormap(&tk);
         prefetch_tensormap(&tv);
-        const int nslots = (WIDE || has1) ? 2 : 1;
-        mbar_arrive_expect_tx(bar(C::kBarQFull), nslots * T::kTileBytes);
-        for (int i = 0; i < nslots; ++i)
-          for (int ch = 0; ch < T::kChunks; ++ch)
-            tma_load_4d(smem_base + C::kOffQ + i * T::kTileBytes + ch * T::kChunkTileBytes, &tq,
-                        (WIDE ? i * 128 : 0) + ch * T::kChunkElems, (WIDE ? qt0 : qt0 + i) * 128, hc,
-                        bar(C::kBarQFull));
       }
-      // K runs one KV tile ahead of V: S(j+1) is issued during KV step j.  Ring entries are
-      // staged tiles: entry t holds columns (t % HALVES) * 128 .. of KV tile t / HALVES.
-      const int nsub = nkv * HALVES;
-      for (int t = 0; t < nsub + HALVES; ++t) {
-        if (t < nsub) {
-          const int ks = t % C::kKStages, kph = (t / C::kKStages) & 1;
-          if (!mbar_wait_warp(bar(C::kBarKEmpty + ks), kph ^ 1, w, kSiteLoadK)) break;
-          if (elected) {
-            mbar_arrive_expect_tx(bar(C::kBarKFull + ks), C::kKvBytes);
+      bool ok = true;
+      int ks = 0, kph = 0, vs = 0, vph = 0;  // ring positions
+      unsigned drawn = 0;
+      for (int n = 0, id = blockIdx.x;; ++n) {
+        WorkItem item{-1, 0, 0, 0};
+        if (id < total_items) {
+          const HeadTile ht = grouped_order(id, num_bh, npairs, group);
+          // the last pair of Q tiles meets the most KV tiles
+          item = WorkItem{npairs - 1 - ht.rank, ht.bh, ht.bh % num_heads, ht.bh / num_heads};
+        }
+        if (ok) ok = mbar_wait_warp(bar(C::kBarItemEmpty + (n & 1)), ((n >> 1) & 1) ^ 1, w, kSiteItem);
+        if (ok && lane == 0) {
+          reinterpret_cast<WorkItem*>(smem + C::kOffItems)[n & 1] = item;
+          mbar_arrive(bar(C::kBarItemFull + (n & 1)));
+        }
+        if (item.pair < 0) break;
+        const HeadCoord hc{item.h, item.b};
+        const int nkv = max(kv_tiles(item, 0), kv_tiles(item, 1));
+        const int qt0 = per_item * item.pair;
+        // K runs one KV tile ahead of V: S(j+1) is issued during KV step j.  Ring entries are
+        // staged tiles: entry t holds columns (t % HALVES) * 128 .. of KV tile t / HALVES.
+        const int nsub = nkv * HALVES;
+        for (int t = 0; ok && t < nsub + HALVES; ++t) {
+          if (t < nsub) {
+            if (!(ok = mbar_wait_warp(bar(C::kBarKEmpty + ks), kph ^ 1, w, kSiteLoadK))) break;
+            if (elected) {
+              mbar_arrive_expect_tx(bar(C::kBarKFull + ks), C::kKvBytes);
 #pragma unroll
-            for (int ch = 0; ch < T::kChunks; ++ch)
-              tma_load_4d(smem_base + C::kOffK + ks * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tk,
-                          (t % HALVES) * 128 + ch * T::kChunkElems, (t / HALVES) * W, hc,
-                          bar(C::kBarKFull + ks));
+              for (int ch = 0; ch < T::kChunks; ++ch)
+                tma_load_4d(smem_base + C::kOffK + ks * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tk,
+                            (t % HALVES) * 128 + ch * T::kChunkElems, (t / HALVES) * W, hc,
+                            bar(C::kBarKFull + ks));
+            }
+            if (++ks == C::kKStages) ks = 0, kph ^= 1;
+          }
+          if (t == 0) {
+            if (!(ok = mbar_wait_warp(bar(C::kBarQEmpty), (n & 1) ^ 1, w, kSiteLoadQ))) break;
+            if (elected) {
+              const int nslots = (WIDE || second_tile(item)) ? 2 : 1;
+              mbar_arrive_expect_tx(bar(C::kBarQFull), nslots * T::kTileBytes);
+              for (int i = 0; i < nslots; ++i)
+                for (int ch = 0; ch < T::kChunks; ++ch)
+                  tma_load_4d(smem_base + C::kOffQ + i * T::kTileBytes + ch * T::kChunkTileBytes, &tq,
+                              (WIDE ? i * 128 : 0) + ch * T::kChunkElems, (WIDE ? qt0 : qt0 + i) * 128, hc,
+                              bar(C::kBarQFull));
+            }
+          }
+          if (t >= HALVES) {
+            const int tv_ = t - HALVES;
+            // the number of the next item is on its way while the last V tile waits for its stage
+            if (tv_ == nsub - 1 && lane == 0) drawn = atomicAdd(work_counter, 1u);
+            if (!(ok = mbar_wait_warp(bar(C::kBarVEmpty + vs), vph ^ 1, w, kSiteLoadV))) break;
+            if (elected) {
+              mbar_arrive_expect_tx(bar(C::kBarVFull + vs), C::kKvBytes);
+#pragma unroll
+              for (int ch = 0; ch < T::kChunks; ++ch)
+                tma_load_4d(smem_base + C::kOffV + vs * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tv,
+                            (tv_ % HALVES) * 128 + ch * T::kChunkElems, (tv_ / HALVES) * W, hc,
+                            bar(C::kBarVFull + vs));
+            }
+            if (++vs == C::kVStages) vs = 0, vph ^= 1;
+            if (tv_ == nsub - 1) break;
           }
         }
-        if (t >= HALVES) {
-          const int tv_ = t - HALVES;
-          const int vs = tv_ % C::kVStages, vph = (tv_ / C::kVStages) & 1;
-          if (!mbar_wait_warp(bar(C::kBarVEmpty + vs), vph ^ 1, w, kSiteLoadV)) break;
-          if (elected) {
-            mbar_arrive_expect_tx(bar(C::kBarVFull + vs), C::kKvBytes);
-#pragma unroll
-            for (int ch = 0; ch < T::kChunks; ++ch)
-              tma_load_4d(smem_base + C::kOffV + vs * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tv,
-                          (tv_ % HALVES) * 128 + ch * T::kChunkElems, (tv_ / HALVES) * W, hc,
-                          bar(C::kBarVFull + vs));
-          }
+        // A CTA that gives up goes on drawing, so that the counter is left at zero.
+        if (lane == 0) {
+          if (!ok) drawn = atomicAdd(work_counter, 1u);
+          if (drawn == static_cast<unsigned>(total_items) - 1u) atomicExch(work_counter, 0u);
+          *next_slot = static_cast<int>(drawn + gridDim.x);
         }
+        __syncwarp();
+        id = *next_slot;
+        __syncwarp();
       }
     } else if (warp == 8) {
       // ---------------------------------------------------------------- S = Q_i K_j^T issuer
@@ -269,95 +319,103 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
       // 10): they touch disjoint tensor-memory columns and are ordered against each other
       // only through the softmax groups, so neither stream waits behind the other's barriers.
       // Order: S0(0) S1(0) S0(1) S1(1) ...; each product waits until the previous one has
-      // been copied out of the single score buffer.
+      // been copied out of the single score buffer.  Releases are committed before the product's own
+      // barrier, so that nothing is on its way to a barrier when the last item's outputs have been formed.
       const uint32_t elected = elect_one();
-      bool ok = mbar_wait(bar(C::kBarQFull), 0, w, kSiteMmaQ);
-      int ks = 0, kph = 0;          // K ring position of tile j
-      int prev_i = -1, prev_ph = 0;  // group and phase of the previous score product
-      int k_left = nkv * HALVES;  // staged tiles of this item not released yet
-      auto release_k = [&]() {
-        if (elected && k_left > C::kKStages) mma_commit(bar(C::kBarKEmpty + ks));
-        --k_left;
-        if (++ks == C::kKStages) {
-          ks = 0;
-          kph ^= 1;
-        }
+      auto commit = [&](int b) {
+        if (elected) mma_commit(bar(b));
       };
-      for (int j = 0; ok && j < nkv; ++j) {
-        if constexpr (!WIDE) {
-          if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
-        }
+      bool ok = true;
+      int ks = 0, kph = 0;           // K ring position
+      int prev_i = -1, prev_ph = 0;  // group and phase of the previous score product
+      int count[2] = {0, 0};         // score products of either group so far
+      auto release_k = [&]() {
+        commit(C::kBarKEmpty + ks);
+        if (++ks == C::kKStages) ks = 0, kph ^= 1;
+      };
+      WorkItem item;
+      for (int n = 0; ok && take_item(n, item); ++n) {
+        const int n0 = kv_tiles(item, 0), n1 = kv_tiles(item, 1), nkv = max(n0, n1);
+        if (!(ok = mbar_wait(bar(C::kBarQFull), n & 1, w, kSiteMmaQ))) break;
+        for (int j = 0; ok && j < nkv; ++j) {
+          if constexpr (!WIDE) {
+            if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
+          }
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          if (j >= (i == 0 ? n0 : n1)) continue;
-          if (prev_i >= 0) {
-            if (!(ok = mbar_wait(bar(C::kBarSFree + prev_i), prev_ph, w, kSiteMmaSFree))) break;
-            tc_fence_after();
-          }
-          if constexpr (WIDE) {
-            // S = Q_lo K_lo^T + Q_hi K_hi^T: the Q slots hold the halves, K arrives half by half
-            for (int half = 0; ok && half < 2; ++half) {
-              if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
-              issue_rows_x_rows<DT, BF16, W, KT>(elected, tmem_base + C::kColS,
-                                          smem_base + C::kOffQ + half * T::kTileBytes,
-                                          smem_base + C::kOffK + ks * C::kKvBytes, half);
-              release_k();
+          for (int i = 0; i < 2; ++i) {
+            if (j >= (i == 0 ? n0 : n1)) continue;
+            if (prev_i >= 0) {
+              if (!(ok = mbar_wait(bar(C::kBarSFree + prev_i), prev_ph, w, kSiteMmaSFree))) break;
+              tc_fence_after();
             }
-            if (!ok) break;
-          } else {
-            issue_rows_x_rows<DT, BF16, W, KT>(elected, tmem_base + C::kColS,
-                                        smem_base + C::kOffQ + i * T::kTileBytes,
-                                        smem_base + C::kOffK + ks * C::kKvBytes);
+            const bool last_of_tile = i == 1 || n1 == 0;
+            if constexpr (WIDE) {
+              // S = Q_lo K_lo^T + Q_hi K_hi^T: the Q slots hold the halves, K arrives half by half
+              for (int half = 0; ok && half < 2; ++half) {
+                if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
+                issue_rows_x_rows<DT, BF16, W, KT>(elected, tmem_base + C::kColS,
+                                            smem_base + C::kOffQ + half * T::kTileBytes,
+                                            smem_base + C::kOffK + ks * C::kKvBytes, half);
+                release_k();
+              }
+              if (!ok) break;
+            } else {
+              issue_rows_x_rows<DT, BF16, W, KT>(elected, tmem_base + C::kColS,
+                                          smem_base + C::kOffQ + i * T::kTileBytes,
+                                          smem_base + C::kOffK + ks * C::kKvBytes);
+              if (last_of_tile) release_k();  // both products that read K_j issued
+            }
+            if (!C::kStageInQ && last_of_tile && j == nkv - 1) commit(C::kBarQEmpty);
+            commit(C::kBarSFull + i);
+            prev_i = i;
+            prev_ph = count[i]++ & 1;
           }
-          if (elected) mma_commit(bar(C::kBarSFull + i));
-          prev_i = i;
-          prev_ph = j & 1;
         }
-        if (!ok) break;
-        if constexpr (!WIDE) release_k();  // both products that read K_j issued
       }
     } else if (warp == 10) {
       // ---------------------------------------------------------------- O_i += P_i V_j issuer
       const uint32_t elected = elect_one();
-      bool ok = true;
-      int vs = 0, vph = 0;  // V ring position of tile j
-      int v_left = nkv * HALVES;
-      auto release_v = [&]() {
-        if (elected && v_left > C::kVStages) mma_commit(bar(C::kBarVEmpty + vs));
-        --v_left;
-        if (++vs == C::kVStages) {
-          vs = 0;
-          vph ^= 1;
-        }
+      auto commit = [&](int b) {
+        if (elected) mma_commit(bar(b));
       };
-      for (int j = 0; ok && j < nkv; ++j) {
-        if constexpr (!WIDE) {
-          if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          if (j >= (i == 0 ? n0 : n1)) continue;
-          if (!(ok = mbar_wait(bar(C::kBarPFull + i), j & 1, w, kSiteMmaP))) break;
-          tc_fence_after();
-          if constexpr (WIDE) {
-            // O_lo += P V_lo, O_hi += P V_hi: the O0 / O1 columns hold the two halves of O
-            for (int half = 0; ok && half < 2; ++half) {
-              if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
-              issue_tmem_x_tile<DT, BF16, W, KT>(elected, tmem_base + C::kColO + half * DT,
-                                          tmem_base + C::kColP, W / 4,
-                                          smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
-              release_v();
-            }
-            if (!ok) break;
-          } else {
-            issue_tmem_x_tile<DT, BF16, W, KT>(elected, tmem_base + C::kColO + i * DT,
-                                        tmem_base + C::kColP + i * (W / 2), W / 4,
-                                        smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
+      bool ok = true;
+      int vs = 0, vph = 0;    // V ring position
+      int count[2] = {0, 0};  // products of either group so far
+      auto release_v = [&]() {
+        commit(C::kBarVEmpty + vs);
+        if (++vs == C::kVStages) vs = 0, vph ^= 1;
+      };
+      WorkItem item;
+      for (int n = 0; ok && take_item(n, item); ++n) {
+        const int n0 = kv_tiles(item, 0), n1 = kv_tiles(item, 1), nkv = max(n0, n1);
+        for (int j = 0; ok && j < nkv; ++j) {
+          if constexpr (!WIDE) {
+            if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
           }
-          if (elected) mma_commit(bar(C::kBarPvDone + i));
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            if (j >= (i == 0 ? n0 : n1)) continue;
+            if (!(ok = mbar_wait(bar(C::kBarPFull + i), count[i]++ & 1, w, kSiteMmaP))) break;
+            tc_fence_after();
+            if constexpr (WIDE) {
+              // O_lo += P V_lo, O_hi += P V_hi: the O0 / O1 columns hold the two halves of O
+              for (int half = 0; ok && half < 2; ++half) {
+                if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
+                issue_tmem_x_tile<DT, BF16, W, KT>(elected, tmem_base + C::kColO + half * DT,
+                                            tmem_base + C::kColP, W / 4,
+                                            smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
+                release_v();
+              }
+              if (!ok) break;
+            } else {
+              issue_tmem_x_tile<DT, BF16, W, KT>(elected, tmem_base + C::kColO + i * DT,
+                                          tmem_base + C::kColP + i * (W / 2), W / 4,
+                                          smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
+              if (i == 1 || n1 == 0) release_v();
+            }
+            commit(C::kBarPvDone + i);
+          }
         }
-        if (!ok) break;
-        if constexpr (!WIDE) release_v();
       }
     }
     __syncwarp();
@@ -365,17 +423,22 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
     // ------------------------------------------------------------------ softmax groups
     reg_inc<C::kSoftmaxRegs>();
     const int wg = warp >> 2;
-    const int qt = wg == 0 ? qt0 : qt1;
-    const int nj = wg == 0 ? n0 : n1;
     const int r = (warp & 3) * 32 + lane;  // row inside the Q tile = tensor-memory lane
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tS = tmem_base + lane_base + C::kColS;
     const uint32_t tP = tmem_base + lane_base + C::kColP + wg * (W / 2);
     const uint32_t tO = tmem_base + lane_base + C::kColO + wg * DT;  // wide: 256 columns, wg 0 only
-    float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
+    int done = 0;  // KV tiles of this group's earlier items
+    WorkItem item;
+    for (int n = 0; ok && take_item(n, item); ++n) {
+    const HeadCoord hc{item.h, item.b};
+    const int qt = per_item * item.pair + wg;
+    const int nj = kv_tiles(item, wg);
+    float m_run = -INFINITY, l_run = 0.f;
     for (int j = 0; j < nj; ++j) {
-      if (!(ok = mbar_wait_warp(bar(C::kBarSFull + wg), j & 1, w, kSiteSoftS))) break;
+      const int ph = (done + j) & 1;  // of this tile on the group's barriers
+      if (!(ok = mbar_wait_warp(bar(C::kBarSFull + wg), ph, w, kSiteSoftS))) break;
       tc_fence_after();
       uint32_t sr[W];
 #pragma unroll
@@ -411,7 +474,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
         m_run = m_new;
         if (j > 0) {
           // O_i must be at rest: wait for O_i += P_i(j-1) V_(j-1)
-          if (!(ok = mbar_wait_warp(bar(C::kBarPvDone + wg), (j - 1) & 1, w, kSiteSoftPv))) break;
+          if (!(ok = mbar_wait_warp(bar(C::kBarPvDone + wg), ph ^ 1, w, kSiteSoftPv))) break;
           tc_fence_after();
           pv_waited = true;
           constexpr int kStep = W == 64 ? 16 : 32;  // the score row stays in registers meanwhile
@@ -448,7 +511,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
       }
       if (j > 0 && !pv_waited) {
         // P_i still feeds O_i += P_i(j-1) V_(j-1) until that product has completed
-        if (!(ok = mbar_wait_warp(bar(C::kBarPvDone + wg), (j - 1) & 1, w, kSiteSoftPv))) break;
+        if (!(ok = mbar_wait_warp(bar(C::kBarPvDone + wg), ph ^ 1, w, kSiteSoftPv))) break;
       }
 #pragma unroll
       for (int c = 0; c < W / 2; c += 32) tmem_st_x32(tP + c, pk + c);
@@ -459,14 +522,14 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
       const float2 a01 = __fadd2_rn(acc[0], acc[1]), a23 = __fadd2_rn(acc[2], acc[3]);
       l_run += (a01.x + a01.y) + (a23.x + a23.y);
     }
-    if (ok && nj > 0 && mbar_wait_warp(bar(C::kBarPvDone + wg), (nj - 1) & 1, w, kSiteSoftO)) {
+    done += nj;
+    if (ok && nj > 0 && (ok = mbar_wait_warp(bar(C::kBarPvDone + wg), (done - 1) & 1, w, kSiteSoftO))) {
       tc_fence_after();
       // a row without any finite score has no softmax, whatever weights it was left with
       const float inv_l = m_run == -INFINITY ? __uint_as_float(0x7fffffffu) : 1.0f / l_run;
-      // Stage the tile through the (now idle) Q buffer in the swizzled layout the output
-      // tensor map expects; each warp stores its own 32 rows.
-      uint8_t* sO = smem + C::kOffQ + wg * T::kTileBytes;
-      const int row = qt * 128 + r;
+      // Each warp stages its own 32 rows, chunk by chunk, in the swizzled layout the output tensor map
+      // expects, and stores them while the other roles are at the next item.
+      const int row = qt * 128 + r, row0 = qt * 128 + (warp & 3) * 32;
       float* const dst32 =
           o32.p != nullptr && row < N ? o32.p + hc.b * o32.st.b + hc.h * o32.st.h + row * o32.st.n : nullptr;
 #pragma unroll
@@ -474,8 +537,15 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
         uint32_t orr[32];
         tmem_ld_x32(tO + c0, orr);
         tmem_wait_ld();
-        const int chunk = c0 / T::kChunkElems;
         const int piece0 = (c0 % T::kChunkElems) / 8;
+        uint8_t* const sO = C::kStageInQ ? smem + C::kOffQ + wg * T::kTileBytes + (warp & 3) * C::kStageBytes
+                                         : smem + C::kOffStage + warp * C::kStageBytes;
+        if (!C::kStageInQ && piece0 == 0) {
+          // the staging piece may be refilled once the store before has READ it; the write itself
+          // completes on its own before the grid does
+          if (lane == 0) tma_store_wait_read();
+          __syncwarp();
+        }
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
           uint4 val;
@@ -487,8 +557,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
                               __uint_as_float(orr[8 * p + 5]) * inv_l);
           val.w = pack2<BF16>(__uint_as_float(orr[8 * p + 6]) * inv_l,
                               __uint_as_float(orr[8 * p + 7]) * inv_l);
-          *reinterpret_cast<uint4*>(sO + chunk * T::kChunkTileBytes +
-                                    swizzled_offset<DT>(r, piece0 + p)) = val;
+          *reinterpret_cast<uint4*>(sO + swizzled_offset<DT>(lane, piece0 + p)) = val;
           // the unrounded row as well, for fp32 callers (see store_rows_f32 in bwd_roles.cuh)
           if (dst32 != nullptr && c0 + 8 * p < cols) {
             float x[8];
@@ -497,27 +566,27 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
             st_global_8(dst32 + c0 + 8 * p, x);
           }
         }
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        const int row0 = (warp & 3) * 32;
-        if (qt * 128 + row0 < N) {
-          for (int ch = 0; ch < D / T::kChunkElems; ++ch)
-            tma_store_4d(&to, ch * T::kChunkElems, qt * 128 + row0, hc,
-                         smem_u32(sO + ch * T::kChunkTileBytes + row0 * T::kRowBytes));
-          tma_store_commit();
-          // the staging buffer may be refilled once the store has READ it; the write itself
-          // completes on its own before the grid does
-          tma_store_wait_read();
+        if ((c0 + 32) % T::kChunkElems == 0 || c0 + 32 == KD) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && row0 < N) {
+            tma_store_4d(&to, c0 / T::kChunkElems * T::kChunkElems, row0, hc, smem_u32(sO));
+            tma_store_commit();
+          }
         }
       }
+      tc_fence_before();  // O_i is overwritten by the next item's first product, which this group's P lets in
       if (row < N)
-        lse[static_cast<size_t>(bh) * N + row] = (m_run * scale_log2 + lg2(l_run)) * kLn2;
+        lse[static_cast<size_t>(item.bh) * N + row] = (m_run * scale_log2 + lg2(l_run)) * kLn2;
     }
+    if constexpr (C::kStageInQ) {
+      // A group without a tile has waited for nothing yet: its arrival must not count for the item before.
+      if (ok && nj == 0) ok = mbar_wait_warp(bar(C::kBarQFull), n & 1, w, kSiteSoftO);
+      if (lane == 0) tma_store_wait_read(), mbar_arrive(bar(C::kBarQEmpty));
+    }
+    }  // items
+    if (lane == 0) tma_store_wait_read();
   }
-
-  }  // work-item loop
 
   // ---------------------------------------------------------------------- teardown
   tc_fence_before();

@@ -139,8 +139,8 @@ void sim_run(unsigned n, void (*body)(void*), void* arg) {
 #include "bwd.cu"
 #include "fwd.cu"
 
-// main <kernel> <head dim> <rows> <keys> <schedules> <rows of a step>
-int main(int, char** argv) {
+// main <kernel> <head dim> <rows> <keys> <schedules> <rows of a step> [<SMs>]
+int main(int argc, char** argv) {
   using namespace fa2;
   const std::string kernel = argv[1];
   const int d = atoi(argv[2]), n = atoi(argv[3]), nk = atoi(argv[4]);
@@ -156,7 +156,7 @@ int main(int, char** argv) {
   const int step = atoi(argv[6]);
   for (int seed = 0; seed < atoi(argv[5]); ++seed) {
     rng.seed(seed);
-    ctx.num_sms = 1 + seed % 2 * 63;  // work items of two Q tiles and of one
+    ctx.num_sms = argc > 7 ? atoi(argv[7]) : 1 + seed % 2 * 63;  // work items of two Q tiles and of one
     if (kernel == "fwd") launch_fwd(s, step, m, m, m, m, none, lse.data(), ctx, nullptr);
     if (kernel == "dkdv") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, nullptr, 0, step, &status, nullptr);
     if (kernel == "dkdv_atomic") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 1, step, &status, nullptr);

@@ -72,6 +72,19 @@ def test_forward_roles(simulator, headdim, rows, keys):
     check(simulator, "fwd", headdim, rows, keys, steps_of(headdim))
 
 
+@pytest.mark.parametrize("rows,keys", [(700, 300), (1200, 1200), (2200, 1000)])
+@pytest.mark.parametrize("headdim", [32, 64])
+def test_forward_roles_single_tile_items_one_after_the_other(simulator, headdim, rows, keys):
+    """So few SMs that a CTA takes several items of one Q tile each: the softmax group without a tile has nothing to
+    wait for and must not run ahead of the other one."""
+    tiles = (rows + 127) // 128
+    sms = (2 * tiles + 6) // 7  # fwd_tiles_per_item: the fewest that give single-tile items
+    assert tiles > 2 * sms
+    run = subprocess.run([simulator, "fwd", str(headdim), str(rows), str(keys), "60", "64", str(sms)],
+                         capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stdout + run.stderr
+
+
 @pytest.mark.parametrize("rows,keys", [(1, 1), (128, 64), (449, 300), (640, 640)])
 @pytest.mark.parametrize("kernel,headdim", [("scores", 256), ("consume", 64), ("consume", 128), ("consume", 256),
                                             ("consume_pair", 256)])

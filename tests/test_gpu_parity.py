@@ -928,3 +928,23 @@ def test_ragged_peaked_c5_shape_is_repeatable():
         # elements is a tail value quantised in fp16 ulps, so it gets a factor of two
         assert rms_ours <= 1.25 * rms_ref + 1e-5, f"{key}: rms ours {rms_ours:.3e}, reference {rms_ref:.3e}"
         assert e_ours <= max(5e-3, 2.0 * e_ref), f"{key}: ours {e_ours:.3e}, reference {e_ref:.3e}"
+
+
+@pytest.mark.parametrize("headdim", [32, 64, 96, 128, 256])
+@pytest.mark.parametrize("rows,keys,heads", [(128, 128, 650), (300, 300, 450), (700, 650, 180), (1100, 1100, 110)])
+def test_forward_items_do_not_see_each_other(headdim, rows, keys, heads):
+    """A CTA of the forward kernel walks through several work items, the next one's loads and scores under the end
+    of the one before.  Launched alone, a head has at most nine items, one for each CTA: its O must have the same
+    bits.  Strided (row-interleaved heads) inputs; rows of one tile, of a lone last tile, of more keys tiles
+    than the rings hold, and fewer keys than queries."""
+    g = torch.Generator(device=DEV).manual_seed(rows + headdim)
+    q = torch.randn(1, rows, heads, headdim, device=DEV, generator=g, dtype=torch.bfloat16).transpose(1, 2)
+    k, v = (torch.randn(1, keys, heads, headdim, device=DEV, generator=g, dtype=torch.bfloat16).transpose(1, 2)
+            for _ in range(2))
+    with torch.no_grad():
+        for _ in range(2):  # the second launch finds the work counter as the first one left it
+            together = flash_attention_v2(q, k, v)
+        for h in (0, 1, heads // 2, heads - 2, heads - 1):
+            alone = flash_attention_v2(*(t[:, h:h + 1] for t in (q, k, v)))
+            assert torch.equal(together[:, h:h + 1], alone), h
+    assert _lib.device_status() == 0
