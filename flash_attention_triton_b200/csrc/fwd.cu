@@ -21,17 +21,20 @@
 //
 // The online softmax works in the exp2 domain with the scale folded in, and rescales O only
 // when the running maximum has moved by more than kRescaleThreshold ("lazy rescale"); masking code runs on
-// the diagonal tile only.  A fixed fraction of the exponentials is evaluated with a
-// polynomial on the FMA pipe because the MUFU rate (16 / clk / SM) would otherwise bound the
-// kernel: 2 x 128 x 128 exponentials per KV step cost as many cycles as the four MMAs.
+// the diagonal tile only.  The exponentials go to the MUFU, although 2 x 128 x 128 of them a KV step cost as
+// many cycles there (16 / clk / SM) as the four products: under load the power limit sets the clock, and a
+// polynomial on the FMA pipe takes five times the instructions.  With 3 of 8 pairs in the polynomial against
+// none, passes in a loop, microseconds: [2,32,8192,128] bf16 974 -> 921, [1,32,4096,128] 138 -> 129.5,
+// [32,20,1024,96] fp16 223 -> 212, [2,16,8192,256] bf16 974 -> 926, [2,16,8192,64] fp16 373 -> 361.  At
+// head dim 32, where the products are shortest, 2 of 8 pairs measured best: [8,12,4095,32] 258 / 259 / 265
+// with 3, 2 and none.
 //
 // Head dims up to 64, rows up to fwd_kv_rows' line: the MMAs of a tile are short (512 cycles or less per 128 x 128 scores) and the
 // softmax instruction stream is what takes the time; with two softmax warps per scheduler it issues
 // in half of the cycles only, the rest is latency of dependent instructions.  So the KV tiles are
 // 64 rows there: a thread holds 64 instead of 128 scores, 96 registers do instead of 208, 256
 // columns of tensor memory instead of 512, and TWO CTAs run on an SM, four softmax warps per
-// scheduler.  The exponentials then all go to the MUFU, which has time (the polynomial costs five
-// times the issue slots).  Measured against 128-row tiles and one CTA, fp16, head dim 64, microseconds:
+// scheduler.  Measured against 128-row tiles and one CTA, fp16, head dim 64, microseconds:
 // [1,256,1000,64] 85.4 -> 68.3, [1,128,1000,64] 43.6 -> 35.9, [1,256,512,64] 34.4 -> 27.9; where there are too
 // few CTAs to pair, or the rows are long, 128-row tiles win (figures at fwd_kv_rows).
 #include "common.cuh"
@@ -49,7 +52,7 @@ struct FwdCfg {
   using T = Tile<D>;
   static constexpr int kW = W;  // rows of a KV tile = columns of a score tile
   static_assert(W == 128 || (W == 64 && D <= 64), "fwd_kv_rows");
-  static constexpr int kPolyShare = kW == 64 ? 0 : 3;  // of every 8 column pairs, this many use ex2_poly2
+  static constexpr int kPolyShare = kW == 128 && D == 32 ? 2 : 0;  // of every 8 column pairs, this many use ex2_poly2
   static constexpr int kCtasPerSm = kW == 64 ? 2 : 1;
   // O is rescaled when the running maximum has moved by more than this (log2 units).  A row's
   // largest P is exactly 1, without rounding error, when its maximum is fresh: 64-row tiles, whose
