@@ -38,6 +38,13 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
                : "memory");
 }
 
+// The same for `bytes` (a multiple of 16) of shared memory, by the copy engine.
+__device__ __forceinline__ void bulk_add_f32(float* dst, uint32_t src_smem, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src_smem),
+               "r"(bytes)
+               : "memory");
+}
+
 // The transposed-score kernels (bwd_dkdv_kernel, bwd_scores_wide_kernel) give each thread one kv
 // row and 2 * PAIRS q columns of a tile: 64, or 32 in steps of 64 rows.  probabilities_of_row:
 // p = 2^(s * c - lse2[q]) from the raw scores `sr` and the negated, log2-scaled row statistics of
@@ -229,10 +236,18 @@ struct DkdvCfg {
   static constexpr int kBarDsReady = kBarPtReady + 1;   // one arrival per compute warp
   static constexpr int kBarDqFull = kBarDsReady + 1;
   static constexpr int kBarDqDrained = kBarDqFull + 1;  // 4 arrivals
-  static constexpr int kBarDone = kBarDqDrained + 1;
+  static constexpr int kBarDqAdded = kBarDqDrained + 1;  // 4 arrivals (kBulkAdd)
+  static constexpr int kBarDone = kBarDqAdded + 1;
   static constexpr int kNumBars = kBarDone + 1;
   static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;
   static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "shared memory of one SM");
+  // In steps of 64 rows dQ goes to the fp32 workspace through the copy engine, staged in the half of the dS tile
+  // that the first step of the next Q tile does not write.  Red instructions hold the dQ columns, and with them
+  // dPt of the next step, for as long as the load/store unit takes to accept them.  Whole backward, microseconds,
+  // red against copies: [4,16,2048,64] 165 -> 159, [2,16,8192,64] 1001 -> 958, [8,16,1000,64] bf16 106.6 -> 104.4,
+  // [8,12,4095,32] 581 -> 574 (without any addition 137, 795, 97, 526: the L2 takes 5.6 TB/s of either form,
+  // more than twice what arrives here).
+  static constexpr bool kBulkAdd = FUSE && kW == 64;
   static_assert(kStages * kStepBytes >= T::kTileBytes, "the rings stage dK and dV at the end");
   static constexpr int kColSt = 0;
   static constexpr int kColDpt = kW;  // dQ (fused) reuses these columns
@@ -285,6 +300,7 @@ __device__ __forceinline__ void dkdv_init_barriers(uint32_t bar0) {
   mbar_init(bar(C::kBarDsReady), 4 * C::kGroups);
   mbar_init(bar(C::kBarDqFull), 1);
   mbar_init(bar(C::kBarDqDrained), 4);
+  mbar_init(bar(C::kBarDqAdded), 4);
   mbar_init(bar(C::kBarDone), 2);  // last dV (warp X) and last dK (warp Y)
 }
 
@@ -463,6 +479,9 @@ __device__ __forceinline__ void dkdv_roles(
               if (tile_end) {
                 if (!(ok = mbar_wait(bar(C::kBarDqDrained), (t / kSub) & 1, w, kBSiteMmaDrain))) break;
                 tc_fence_after();
+              } else if (C::kBulkAdd && t / kSub > 0) {
+                // the next step's dS goes where dQ of the tile before was staged
+                if (!(ok = mbar_wait(bar(C::kBarDqAdded), (t / kSub - 1) & 1, w, kBSiteMmaDrain))) break;
               }
             }
             if (!(ok = mbar_wait(bar(C::kBarDOFull + s1), ph1, w, kBSiteMmaDO))) break;
@@ -491,28 +510,61 @@ __device__ __forceinline__ void dkdv_roles(
       const int qt = ntiles - 1 - ii;
       float* dst = dq_accum + (((static_cast<size_t>(bh) * ntiles + qt) * 4 + w4) * (D / 4)) * 128 +
                    lane * 4;
-      // Whole dQ tile into registers first, so the MMA warp can reuse the columns at once;
-      // the atomics follow at leisure.
-      constexpr int kPart = C::kReduceRegs < 72 ? 32 : D;  // what the registers hold at a time
+      if constexpr (C::kBulkAdd) {
+        // 32 columns at a time through 4 KiB of this warp, laid out as the workspace is; the columns are given
+        // back before the first copy is started
+        const uint32_t stage = smem_base + C::kOffDS + 16384 + w4 * 4096;
+        float4* const mine = reinterpret_cast<float4*>(smem + C::kOffDS + 16384 + w4 * 4096) + lane;
+        uint32_t v[32];
+        auto load = [&](int d0) {
+          tmem_ld_x32(tmem_base + lane_base + C::kColDpt + d0, v);
+          tmem_wait_ld();
+        };
+        auto put = [&]() {
 #pragma unroll
-      for (int d0 = 0; d0 < D; d0 += kPart) {
-        uint32_t v[kPart];
-#pragma unroll
-        for (int c0 = 0; c0 < kPart; c0 += 32)
-          tmem_ld_x32(tmem_base + lane_base + C::kColDpt + d0 + c0, v + c0);
-        tmem_wait_ld();
-        if (d0 + kPart == D) {
-          tc_fence_before();
+          for (int k = 0; k < 8; ++k)
+            mine[k * 32] = float4{__uint_as_float(v[4 * k]) * inv_dscale, __uint_as_float(v[4 * k + 1]) * inv_dscale,
+                                  __uint_as_float(v[4 * k + 2]) * inv_dscale, __uint_as_float(v[4 * k + 3]) * inv_dscale};
+        };
+        auto add = [&](int d0) {
+          fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar(C::kBarDqDrained));
+          if (lane == 0) {
+            bulk_add_f32(dst - lane * 4 + d0 * 32, stage, 4096);
+            tma_store_commit();
+            tma_store_wait_read();
+          }
+          __syncwarp();
+        };
+        load(0);
+        put();
+        if constexpr (D == 64) load(32);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(C::kBarDqDrained));
+        add(0);
+        if constexpr (D == 64) {
+          put();
+          add(32);
         }
+        if (lane == 0) mbar_arrive(bar(C::kBarDqAdded));
+      } else {
+        // Whole dQ tile into registers first, so the MMA warp can reuse the columns at once;
+        // the atomics follow at leisure.
+        uint32_t v[D];
 #pragma unroll
-        for (int k = 0; k < kPart / 4; ++k)
-          red_add_v4(dst + (d0 / 4 + k) * 128, __uint_as_float(v[4 * k]) * inv_dscale,
-                     __uint_as_float(v[4 * k + 1]) * inv_dscale, __uint_as_float(v[4 * k + 2]) * inv_dscale,
-                     __uint_as_float(v[4 * k + 3]) * inv_dscale);
+        for (int c0 = 0; c0 < D; c0 += 32) tmem_ld_x32(tmem_base + lane_base + C::kColDpt + c0, v + c0);
+        tmem_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(C::kBarDqDrained));
+#pragma unroll
+        for (int k = 0; k < D / 4; ++k)
+          red_add_v4(dst + k * 128, __uint_as_float(v[4 * k]) * inv_dscale, __uint_as_float(v[4 * k + 1]) * inv_dscale,
+                     __uint_as_float(v[4 * k + 2]) * inv_dscale, __uint_as_float(v[4 * k + 3]) * inv_dscale);
       }
     }
+    if (C::kBulkAdd && lane == 0) tma_store_wait_all();
   } else {
     // ---------------------------------------------------------------- compute groups
     reg_inc<C::kComputeRegs>();
