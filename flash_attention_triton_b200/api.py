@@ -304,6 +304,17 @@ def _check_device(q: torch.Tensor) -> None:
         )
 
 
+def _attention(q, k, v, softmax_scale, deterministic):  # noqa: ANN001
+    """The call through the native autograd function where it serves it (plain fp16, bf16 or fp32 tensors, no
+    transform, trace or mode active), through :class:`FlashAttentionV2Function` otherwise: same kernels, same
+    results, same errors."""
+    if not torch.compiler.is_compiling():
+        output = _lib.host().attention(q, k, v, softmax_scale, deterministic)
+        if output is not None:
+            return output
+    return FlashAttentionV2Function.apply(q, k, v, softmax_scale, deterministic)
+
+
 def flash_attention_v2(
     q: torch.Tensor,
     k: torch.Tensor,
@@ -323,7 +334,7 @@ def flash_attention_v2(
         Attention output, same shape and dtype as ``q``.
     """
     _check_device(q)
-    return FlashAttentionV2Function.apply(q, k, v, softmax_scale, deterministic)
+    return _attention(q, k, v, softmax_scale, deterministic)
 
 
 def flash_attention_v2_custom(
@@ -346,4 +357,4 @@ def flash_attention_v2_custom(
             "KernelsConfig must be provided for the current GPU architecture"
         )
     deterministic = kernels_configs[cc].is_deterministic()
-    return FlashAttentionV2Function.apply(q, k, v, softmax_scale, deterministic)
+    return _attention(q, k, v, softmax_scale, deterministic)

@@ -948,3 +948,80 @@ def test_forward_items_do_not_see_each_other(headdim, rows, keys, heads):
             alone = flash_attention_v2(*(t[:, h:h + 1] for t in (q, k, v)))
             assert torch.equal(together[:, h:h + 1], alone), h
     assert _lib.device_status() == 0
+
+
+def _call_and_gradients(call, leaves, views, do, det):
+    out = call(*views(leaves), None, det)
+    return [out.detach(), *torch.autograd.grad(out, leaves, do)]
+
+
+@pytest.mark.parametrize("layout", ["dense", "rows", "packed"])
+@pytest.mark.parametrize("d,n,dtype,det", [(64, 300, torch.float16, True), (40, 200, torch.bfloat16, True),
+                                           (96, 260, torch.float32, False), (128, 257, torch.bfloat16, False),
+                                           (192, 129, torch.float16, False), (20, 70, torch.float16, True)])
+def test_native_call_and_python_function_give_the_same_bits(d, n, dtype, det, layout):
+    from flash_attention_triton_b200 import FlashAttentionV2Function
+
+    g = torch.Generator(device=DEV).manual_seed(d)
+    shape = {"dense": (2, 3, n, d), "rows": (2, n, 3, d), "packed": (2, n, 3, 3, d)}[layout]
+    leaves = [torch.randn(shape, device=DEV, generator=g, dtype=dtype).requires_grad_(True)
+              for _ in range(1 if layout == "packed" else 3)]
+    views = {"dense": lambda ts: ts, "rows": lambda ts: [t.transpose(1, 2) for t in ts],
+             "packed": lambda ts: ts[0].permute(2, 0, 3, 1, 4).unbind(0)}[layout]
+    do = torch.randn(2, 3, n, d, device=DEV, generator=g, dtype=dtype)
+    for dout in (do, do.transpose(1, 2).contiguous().transpose(1, 2)):
+        native = _call_and_gradients(flash_attention_v2, leaves, views, dout, det)
+        python = _call_and_gradients(FlashAttentionV2Function.apply, leaves, views, dout, det)
+        for x, y in zip(native, python):
+            assert x.dtype == y.dtype and x.shape == y.shape and torch.equal(x, y)
+    with torch.no_grad():
+        out = flash_attention_v2(*views(leaves), None, det)
+    assert torch.equal(out, native[0]) and not out.requires_grad
+
+
+def test_native_call_keeps_the_rules_of_autograd(monkeypatch):
+    from flash_attention_triton_b200 import FlashAttentionV2Function, api
+
+    q, k, v, do = (torch.randn(1, 2, 200, 64, device=DEV, dtype=torch.float16) for _ in range(4))
+    q.requires_grad_(True)
+    # saved-tensor hooks see the five saved tensors, and backward uses what they give back
+    packed, unpacked = [], []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t.cpu(),
+                                                  lambda t: unpacked.append(t.shape) or t.to(DEV)):
+        out = flash_attention_v2(q, k, v, None, True)
+    (dq,) = torch.autograd.grad(out, q, do, retain_graph=True)
+    assert len(packed) == len(unpacked) == 5
+    assert torch.equal(dq, torch.autograd.grad(FlashAttentionV2Function.apply(q, k, v, None, True), q, do)[0])
+    torch.autograd.grad(out, q, do)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(out, q, do)
+    # an input changed in place between forward and backward is noticed
+    k2 = k.clone()
+    out = flash_attention_v2(q, k2, v)
+    k2.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.backward(do)
+    # the output, another view of the one that is saved, is not changed in place at all
+    for call in (flash_attention_v2, FlashAttentionV2Function.apply):
+        with pytest.raises(RuntimeError, match="being modified inplace"):
+            call(q, k, v, None, False).mul_(2)
+    assert flash_attention_v2(k, k, v).grad_fn is None
+    # transforms and forward mode go to the Python function, which refuses them
+    plain = q.detach()
+    for transform in (lambda: torch.func.grad(lambda x: flash_attention_v2(x, k, v).float().sum())(plain),
+                      lambda: torch.func.vmap(lambda x: flash_attention_v2(x, x, x))(plain[None]),
+                      lambda: torch.func.jvp(lambda x: flash_attention_v2(x, k, v), (plain,), (do,))):
+        with pytest.raises(RuntimeError):
+            transform()
+    # the switches of the environment reach a backward whose forward ran without them
+    out = flash_attention_v2(q, k, v, None, False)
+    asked = []
+    monkeypatch.setattr(api, "_backward_mode", lambda *a: asked.append(a) or 1)
+    monkeypatch.setenv("FA2_B200_BWD_MODE", "recompute")
+    assert torch.equal(torch.autograd.grad(out, q, do)[0], dq) and asked
+    # an error in there is the caller's exception
+    monkeypatch.setattr(api, "_backward_mode", lambda *a: 1 / 0)
+    out = flash_attention_v2(q, k, v)
+    with pytest.raises(ZeroDivisionError):
+        torch.autograd.grad(out, q, do)
+    assert _lib.device_status() == 0
