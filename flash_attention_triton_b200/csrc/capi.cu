@@ -115,28 +115,32 @@ int get_strides(const long long* user, int idx, int B, int H, int N, int D, Stri
   return FA2_OK;
 }
 
-// Tensor map over a [B, H, N, D] 16-bit tensor with box (chunk, box_rows, 1, 1).  The chunk
-// follows the padded head dim, so for D = 48 or 96 the last box of a row hangs over the
-// tensor: those columns read as zeros and are not written.
-int make_map(CUtensorMap* m, const void* base, int dtype, int B, int H, int N, int D,
-             const Strides& st, int box_rows) {
+int encode_map(CUtensorMap* m, const void* base, int dtype, int B, int H, int N, int D, const Strides& st,
+               int box_columns, int box_rows, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return FA2_ERR_DRIVER;
-  const int chunk = padded_head_dim(D) >= 64 ? 64 : 32;
   const cuuint64_t gdim[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(N),
                               static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(B)};
   const cuuint64_t gstride[3] = {static_cast<cuuint64_t>(st.n) * 2,
                                  static_cast<cuuint64_t>(st.h) * 2,
                                  static_cast<cuuint64_t>(st.b) * 2};
-  const cuuint32_t box[4] = {static_cast<cuuint32_t>(chunk), static_cast<cuuint32_t>(box_rows), 1,
-                             1};
+  const cuuint32_t box[4] = {static_cast<cuuint32_t>(box_columns), static_cast<cuuint32_t>(box_rows), 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r =
       enc(m, dtype ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
-          const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-          chunk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+          const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? FA2_OK : FA2_ERR_DRIVER;
+}
+
+// Tensor map over a [B, H, N, D] 16-bit tensor with box (chunk, box_rows, 1, 1).  The chunk
+// follows the padded head dim, so for D = 48 or 96 the last box of a row hangs over the
+// tensor: those columns read as zeros and are not written.
+int make_map(CUtensorMap* m, const void* base, int dtype, int B, int H, int N, int D,
+             const Strides& st, int box_rows) {
+  const int chunk = padded_head_dim(D) >= 64 ? 64 : 32;
+  return encode_map(m, base, dtype, B, H, N, D, st, chunk, box_rows,
+                    chunk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -303,7 +307,13 @@ int fa2_bwd_preprocess_strided(const void* o, const void* dout, const float* lse
   DeviceState* d = nullptr;
   if (int e = device_state(&d)) return e;
   const AttnShape s = make_shape(B, H, N, N, D, dtype, 1.f);
-  return static_cast<int>(launch_bwd_preprocess(s, o, so, dout, sdo, lse, rowstats, d->status,
+  // whole rows, packed, of tensors that are not contiguous
+  CUtensorMap to{}, tdo{};
+  if (D <= 128 && so.n != D)
+    if (int e = encode_map(&to, o, dtype, B, H, N, D, so, D, 128, CU_TENSOR_MAP_SWIZZLE_NONE)) return e;
+  if (D <= 128 && sdo.n != D)
+    if (int e = encode_map(&tdo, dout, dtype, B, H, N, D, sdo, D, 128, CU_TENSOR_MAP_SWIZZLE_NONE)) return e;
+  return static_cast<int>(launch_bwd_preprocess(s, to, tdo, o, so, dout, sdo, lse, rowstats, d->status,
                                                 d->num_sms, static_cast<cudaStream_t>(stream)));
 }
 

@@ -122,15 +122,19 @@ __global__ void __launch_bounds__(kPreThreads)
 // The same computation as a persistent kernel fed by the copy engine (head dims up to 128).
 //
 // One CTA per SM walks the 128-row tiles blockIdx.x, blockIdx.x + gridDim.x, ...  A producer warp
-// keeps a ring of shared-memory stages full with untiled bulk copies (one stage = the o rows and
-// the dout rows of one tile; one copy per tensor when its rows are contiguous in memory, else one
-// copy per row), so the bytes in flight per SM stay near the ring size (128 - 192 KiB) whatever
+// keeps a ring of shared-memory stages full (one stage = the o rows and the dout rows of one tile; an
+// untiled bulk copy per tensor when its rows are contiguous in memory, else a tiled one through its
+// tensor map), so the bytes in flight per SM stay near the ring size (128 - 192 KiB) whatever
 // the eight consumer warps are doing; the block-per-tile kernel above has nothing in flight while
 // a block reduces and stores, and reaches less than half of the HBM rate.  Consumers read their
 // pieces from shared memory with the row / lane assignment of the kernel above, free the stage
 // once every piece has been used, and hand the tile's 256 results to the next iteration,
 // which stores them with one coalesced 1 KiB write.  lse of the next tile is fetched one
 // iteration ahead.  Rows in shared memory are packed at their true width (d8 pieces).
+// Rows apart from each other (dout as a projection behind it works on it, [B,N,H,d]) came in one bulk copy each,
+// 64 to 256 bytes at a time; as tiled copies they cost what contiguous rows do.  Microseconds, copies of a row /
+// tiled / contiguous rows: [8,16,1000,64] 37 / 13 / 12, [8,12,4095,32] 96 / 21 / 21, [32,20,1024,96] 162 / 49 / 49,
+// [2,32,8192,128] 135 / 50 / 49.
 // ----------------------------------------------------------------------------------------
 template <int D>
 struct PreRing {
@@ -165,8 +169,8 @@ __device__ __forceinline__ bool consumers_all(bool ok, int nthreads) {
 
 template <int D, bool BF16>
 __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
-    bwd_preprocess_ring_kernel(const uint4* o, const uint4* dout,
-                               const float* lse, float* __restrict__ rowstats,
+    bwd_preprocess_ring_kernel(const __grid_constant__ CUtensorMap to, const __grid_constant__ CUtensorMap tdo,
+                               const uint4* o, const uint4* dout, const float* lse, float* __restrict__ rowstats,
                                unsigned* __restrict__ tile_amax, int N, int ntiles,
                                long long tiles, int d8, int H, Strides so, Strides sdo,
                                int* status) {
@@ -207,21 +211,20 @@ __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
       const int t = static_cast<int>(tile - bh * ntiles);
       const long long bb = bh / H, hh = bh - bb * H;
       const int rows = min(128, N - t * 128);
-      if (lane == 0) mbar_arrive_expect_tx(full(s), 2u * rows * row_bytes);
-      __syncwarp();
-      const uint32_t dst = base + s * R::kStageBytes;
+      if (lane == 0) {
+        // a tiled copy delivers all 128 rows of its box, zeros beyond the last one
+        const uint32_t dense_bytes = rows * row_bytes, box_bytes = 128 * row_bytes;
+        mbar_arrive_expect_tx(full(s), (so.n == d8 ? dense_bytes : box_bytes) + (sdo.n == d8 ? dense_bytes : box_bytes));
 #pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        const Strides& st = which ? sdo : so;
-        const uint4* src = (which ? dout : o) + bb * st.b + hh * st.h +
-                           static_cast<long long>(t) * 128 * st.n;
-        const uint32_t d0 = dst + which * R::kTileBytes;
-        if (st.n == d8) {
-          if (lane == 0) bulk_load_1d(d0, src, rows * row_bytes, full(s));
-        } else {
-          for (int r = lane; r < rows; r += 32)
-            bulk_load_1d(d0 + r * row_bytes, src + static_cast<long long>(r) * st.n, row_bytes,
-                         full(s));
+        for (int which = 0; which < 2; ++which) {
+          const Strides& st = which ? sdo : so;
+          const uint32_t dst = base + s * R::kStageBytes + which * R::kTileBytes;
+          if (st.n == d8)
+            bulk_load_1d(dst, (which ? dout : o) + bb * st.b + hh * st.h + static_cast<long long>(t) * 128 * st.n,
+                         dense_bytes, full(s));
+          else
+            tma_load_4d(dst, which ? &tdo : &to, 0, t * 128, HeadCoord{static_cast<int>(hh), static_cast<int>(bb)},
+                        full(s));
         }
       }
     }
@@ -369,8 +372,8 @@ __global__ void __launch_bounds__(256)
 Strides in_vec8(const Strides& st) { return Strides{st.b / 8, st.h / 8, st.n / 8}; }
 
 template <int D, bool BF16>
-cudaError_t launch_pre_t(const AttnShape& s, const void* o, const Strides& so, const void* dout,
-                         const Strides& sdo, const float* lse, float* rowstats, int* status,
+cudaError_t launch_pre_t(const AttnShape& s, const CUtensorMap& to, const CUtensorMap& tdo, const void* o,
+                         const Strides& so, const void* dout, const Strides& sdo, const float* lse, float* rowstats, int* status,
                          int num_sms, cudaStream_t stream) {
   const int ntiles = (s.N + 127) / 128;
   const long long tiles = static_cast<long long>(s.B) * s.H * ntiles;
@@ -383,8 +386,8 @@ cudaError_t launch_pre_t(const AttnShape& s, const void* o, const Strides& so, c
     if (attr != cudaSuccess) return attr;
     const unsigned grid = static_cast<unsigned>(tiles < num_sms ? tiles : num_sms);
     return launch_dependent(
-        kernel, grid, R::kThreads, R::kSmemBytes, stream,
-      static_cast<const uint4*>(o), static_cast<const uint4*>(dout), lse, rowstats, tile_amax,
+        kernel, grid, R::kThreads, R::kSmemBytes, stream, to, tdo, static_cast<const uint4*>(o),
+        static_cast<const uint4*>(dout), lse, rowstats, tile_amax,
         s.N, ntiles, tiles, s.Dg / 8, s.H, in_vec8(so), in_vec8(sdo), status);
   } else {
     return launch_dependent(
@@ -408,16 +411,16 @@ cudaError_t launch_cvt_t(const AttnShape& s, const float* dq_accum, void* dq, co
 
 }  // namespace
 
-cudaError_t launch_bwd_preprocess(const AttnShape& s, const void* o, const Strides& so,
-                                  const void* dout, const Strides& sdo, const float* lse,
+cudaError_t launch_bwd_preprocess(const AttnShape& s, const CUtensorMap& to, const CUtensorMap& tdo,
+                                  const void* o, const Strides& so, const void* dout, const Strides& sdo, const float* lse,
                                   float* rowstats, int* status, int num_sms,
                                   cudaStream_t stream) {
 #define FA2_CASE(DD)                                                                          \
   case DD:                                                                                    \
     return s.dtype                                                                            \
-               ? launch_pre_t<DD, true>(s, o, so, dout, sdo, lse, rowstats, status, num_sms,  \
+               ? launch_pre_t<DD, true>(s, to, tdo, o, so, dout, sdo, lse, rowstats, status, num_sms,  \
                                         stream)                                               \
-               : launch_pre_t<DD, false>(s, o, so, dout, sdo, lse, rowstats, status, num_sms, \
+               : launch_pre_t<DD, false>(s, to, tdo, o, so, dout, sdo, lse, rowstats, status, num_sms, \
                                          stream);
   switch (s.D) {
     FA2_CASE(32)

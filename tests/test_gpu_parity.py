@@ -1025,3 +1025,23 @@ def test_native_call_keeps_the_rules_of_autograd(monkeypatch):
     with pytest.raises(ZeroDivisionError):
         torch.autograd.grad(out, q, do)
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 100, 128, 300, 1000])
+@pytest.mark.parametrize("d", [8, 32, 40, 64, 72, 96, 128])
+def test_preprocess_reads_rows_apart_from_each_other(d, rows):
+    """Strided o and dout, NaN between their rows, give the bits of contiguous ones (40 heads: several tiles an SM)."""
+    host = _lib.host()
+    o, do = (torch.randn(2, 40, rows, d, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    lse = torch.randn(2, 40, rows, device=DEV)
+    apart = []
+    for t in (o, do):
+        wide = torch.full((2, rows, 40, 3, d), float("nan"), device=DEV, dtype=torch.bfloat16)
+        wide[:, :, :, 1] = t.transpose(1, 2)
+        apart.append(wide[:, :, :, 1].transpose(1, 2))
+    code, want, _ = host.preprocess(o, do, lse)
+    assert code == 0
+    for a, b in ((apart[0], do), (o, apart[1]), apart):
+        code, got, used = host.preprocess(a, b, lse)
+        assert code == 0 and used.data_ptr() == b.data_ptr() and torch.equal(got, want)
+    assert _lib.device_status() == 0
