@@ -476,10 +476,9 @@ __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, ConsumeCfg<D>::kCtasP
   const int bh = ht.bh;
   item.hc = HeadCoord{bh % num_heads, bh / num_heads};
   item.head_tile0 = static_cast<size_t>(bh) * dstile_count(ntiles, nktiles);
-  // the last Q tile (form 2) and the first KV tile (forms 0, 1) are summed over the most tiles
+  // the last Q tile (form 2) and the first KV tile (form 1) are summed over the most tiles
   item.ot = FORM == 2 ? ntiles - 1 - ht.rank : ht.rank;
-  // dS tiles carry the head's power-of-two factor (head_dscale); P tiles (form 0) do not
-  item.tile_amax = FORM == 0 ? nullptr : tile_amax + static_cast<size_t>(bh) * ntiles;
+  item.tile_amax = tile_amax + static_cast<size_t>(bh) * ntiles;
 
   if (threadIdx.x == 0) {
     consume_init_barriers<C::kStages>(smem_base + C::kOffBar);
@@ -573,10 +572,10 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
   const int bh = ht.bh;
   const HeadCoord hc{bh % num_heads, bh / num_heads};
   const size_t head_tile0 = static_cast<size_t>(bh) * dstile_count(ntiles, nktiles);
-  // the last Q tiles (form 2) and the first KV tiles (forms 0, 1) are summed over the most tiles
+  // the last Q tiles (form 2) and the first KV tiles (form 1) are summed over the most tiles
   const int ot0 = 2 * (FORM == 2 ? npairs - 1 - ht.rank : ht.rank);
   // Range of tiles of the other kind each output tile is summed over: [begin, end).  Both start at 0
-  // (form 2) or both end at ntiles (forms 0, 1); a missing second tile has an empty range.
+  // (form 2) or both end at ntiles (form 1); a missing second tile has an empty range.
   int begin[2], end[2];
 #pragma unroll
   for (int o = 0; o < 2; ++o) {
@@ -659,8 +658,8 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
     __syncwarp();
   } else {
     const int o = warp >> 2, w4 = warp & 3, ot = ot0 + o;
-    float inv_dscale = 1.0f;  // dS tiles carry the head's power-of-two factor (head_dscale); P tiles do not
-    if (FORM != 0) head_dscale<BF16>(tile_amax + static_cast<size_t>(bh) * ntiles, ntiles, lane, &inv_dscale);
+    float inv_dscale;  // dS tiles carry the head's power-of-two factor
+    head_dscale<BF16>(tile_amax + static_cast<size_t>(bh) * ntiles, ntiles, lane, &inv_dscale);
     if (mbar_wait_warp(bar(C::kBarDone), 0, w, kBSiteCmpDone) && ot < out_tiles) {
       tc_fence_after();
       const uint32_t acc = tmem_base + o * 256 + (static_cast<uint32_t>(w4 * 32) << 16);
@@ -681,41 +680,52 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
 }
 
 // =========================================================================================
-// Head dim 256: scores only.  dK and dV alone would fill the 512 tensor-memory columns, so the
-// backward is split: this kernel forms P^T and dS^T for every (KV tile, Q tile) pair and writes
-// both as 16-bit piece-major tiles to two scratch tensors; bwd_consume_kernel then forms dV, dK
-// and dQ from them.  CTA = one KV tile.  K and V stay in shared memory as two half tiles each
-// (128 KiB); Q and dO stream through a ring of three half-tile slots; St and dPt are double
-// buffered in tensor memory (4 x 128 columns) and accumulate over the two halves of the head dim.
+// Head dims above 128: scores and dV.  dK and dV together would fill the 512 tensor-memory columns, so
+// the backward is split: this kernel forms P^T and dS^T for every (KV tile, Q tile) pair, accumulates
+// dV += P^T dO in tensor memory and writes dS^T as 16-bit piece-major tiles to a scratch tensor;
+// bwd_consume_kernel then forms dK and dQ from them.  CTA = one KV tile.  K and V stay in shared memory as
+// kChunks chunk tiles of 64 columns each (128 KiB together); Q and dO stream through a ring of six such chunks,
+// in the order Q(i), dO(i), Q(i+1), ...; dO(i) keeps its chunks until dV has been formed with them, which
+// leaves two for what comes next.  Tensor memory: St, dPt (128 columns each), dV (256).
 //   warps 0-7  compute (as in bwd_dkdv_kernel: kv row per thread, two groups of 64 q columns)
-//   warp  8    MMA issue: St(i) = K_lo Q_lo^T + K_hi Q_hi^T, dPt(i) = V_lo dO_lo^T + V_hi dO_hi^T
+//   warp  8    MMA issue, per step:  [Pt(i) ready]  dV += Pt(i) dO(i),  St(i+1) = K Q^T (over Pt(i)),
+//              [dPt(i) copied]  dPt(i+1) = V dO^T.  dPt(i+1) runs under the exponentials of St(i+1).
 //   warp  9    TMA producer
+// Bound by the power limit at long sequences (1.25 GHz under load, 4 500 cycles a pair against 3 072 of tensor and
+// 3 584 of shared-memory time; without the ring's loads 6 % less, without the dS stores 12 %).  The version before
+// wrote P^T to a second scratch tensor too, from which a third consumer formed dV: 4.4 of 10.9 GB on
+// [2,16,8192,256] bf16, forward and backward 4 148 -> 3 690 us in a loop.  Same bits.  Walking the Q tiles
+// from the last one, as bwd_dkdv_kernel does, measured the same.
 // =========================================================================================
 struct ScoresCfg {
   using T = Tile<128>;
   static constexpr int kThreads = 384;
   static constexpr int kMmaWarp = 8;
   static constexpr int kLoadWarp = 9;
-  static constexpr int kRing = 3;
-  static constexpr int kOffK = 0;                                   // K_lo, K_hi
-  static constexpr int kOffV = 2 * T::kTileBytes;                   // V_lo, V_hi
-  static constexpr int kOffRing = 4 * T::kTileBytes;                // Q_lo, Q_hi, dO_lo, dO_hi stream
-  static constexpr int kOffStats = kOffRing + kRing * T::kTileBytes;  // [2][256] fp32
+  static constexpr int kChunks = 4;  // of 64 columns: head dim 256
+  static constexpr int kChunkBytes = T::kChunkTileBytes;
+  static constexpr int kRing = 6;
+  static constexpr int kOffK = 0;
+  static constexpr int kOffV = kChunks * kChunkBytes;
+  static constexpr int kOffRing = 2 * kChunks * kChunkBytes;
+  static constexpr int kOffStats = kOffRing + kRing * kChunkBytes;  // [2][256] fp32
   static constexpr int kOffBar = kOffStats + 2 * 1024;
   static constexpr int kBarKV = 0;
   static constexpr int kBarRingFull = 1;
   static constexpr int kBarRingEmpty = kBarRingFull + kRing;
-  static constexpr int kBarStFull = kBarRingEmpty + kRing;  // 2
-  static constexpr int kBarStFree = kBarStFull + 2;         // 2, 8 arrivals
-  static constexpr int kBarDptFull = kBarStFree + 2;        // 2
-  static constexpr int kBarDptFree = kBarDptFull + 2;       // 2, 8 arrivals
-  static constexpr int kBarStatsFull = kBarDptFree + 2;     // 2
-  static constexpr int kBarStatsFree = kBarStatsFull + 2;   // 2, 8 arrivals
-  static constexpr int kNumBars = kBarStatsFree + 2;
+  static constexpr int kBarStFull = kBarRingEmpty + kRing;
+  static constexpr int kBarPtReady = kBarStFull + 1;     // 8 arrivals
+  static constexpr int kBarDptFull = kBarPtReady + 1;
+  static constexpr int kBarDptFree = kBarDptFull + 1;    // 8 arrivals
+  static constexpr int kBarStatsFull = kBarDptFree + 1;  // 2
+  static constexpr int kBarStatsFree = kBarStatsFull + 2;  // 2, 8 arrivals
+  static constexpr int kBarDone = kBarStatsFree + 2;
+  static constexpr int kNumBars = kBarDone + 1;
   static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;
   static_assert(kSmemBytes <= 232448, "shared memory budget of one CTA");
-  static constexpr int kColSt = 0;     // 2 x 128
-  static constexpr int kColDpt = 256;  // 2 x 128
+  static constexpr int kColSt = 0;  // Pt(i) is written over St(i)
+  static constexpr int kColDpt = 128;
+  static constexpr int kColDV = 256;
   static constexpr int kTmemCols = 512;
 };
 
@@ -723,9 +733,9 @@ template <bool BF16>
 __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
     bwd_scores_wide_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                            const __grid_constant__ CUtensorMap tv,
-                           const __grid_constant__ CUtensorMap tdo, const float* rowstats,
-                           const unsigned* tile_amax, uint4* __restrict__ p_scratch,
-                           uint4* __restrict__ ds_scratch, int N, int Nk, int num_bh,
+                           const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdv,
+                           const __grid_constant__ F32Out dv32, int cols, const float* rowstats,
+                           const unsigned* tile_amax, uint4* __restrict__ ds_scratch, int N, int Nk, int num_bh,
                            int num_heads, int group, float scale, float scale_log2, int* status) {
   using C = ScoresCfg;
   using T = Tile<128>;
@@ -753,18 +763,9 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
   const int tile0 = bh * dstile_count(ntiles, nktiles) + dstile_count(ntiles, jt);
 
   if (threadIdx.x == 0) {
-    mbar_init(bar(C::kBarKV), 1);
-    for (int i = 0; i < C::kRing; ++i) {
-      mbar_init(bar(C::kBarRingFull + i), 1);
-      mbar_init(bar(C::kBarRingEmpty + i), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(C::kBarStFull + i), 1);
-      mbar_init(bar(C::kBarStFree + i), 8);
-      mbar_init(bar(C::kBarDptFull + i), 1);
-      mbar_init(bar(C::kBarDptFree + i), 8);
-      mbar_init(bar(C::kBarStatsFull + i), 1);
-      mbar_init(bar(C::kBarStatsFree + i), 8);
+    for (int i = 0; i < C::kNumBars; ++i) {
+      const bool compute = i == C::kBarPtReady || i == C::kBarDptFree || i == C::kBarStatsFree || i == C::kBarStatsFree + 1;
+      mbar_init(bar(i), compute ? 8 : 1);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -791,16 +792,14 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
         prefetch_tensormap(&tk);
         prefetch_tensormap(&tv);
         prefetch_tensormap(&tdo);
-        mbar_arrive_expect_tx(bar(C::kBarKV), 4 * T::kTileBytes);
-        for (int half = 0; half < 2; ++half)
-          for (int ch = 0; ch < T::kChunks; ++ch) {
-            tma_load_4d(smem_base + C::kOffK + half * T::kTileBytes + ch * T::kChunkTileBytes, &tk,
-                        half * 128 + ch * T::kChunkElems, jt * 128, hc, bar(C::kBarKV));
-            tma_load_4d(smem_base + C::kOffV + half * T::kTileBytes + ch * T::kChunkTileBytes, &tv,
-                        half * 128 + ch * T::kChunkElems, jt * 128, hc, bar(C::kBarKV));
-          }
+        mbar_arrive_expect_tx(bar(C::kBarKV), 2 * C::kChunks * C::kChunkBytes);
+        for (int ch = 0; ch < C::kChunks; ++ch) {
+          tma_load_4d(smem_base + C::kOffK + ch * C::kChunkBytes, &tk, ch * T::kChunkElems, jt * 128, hc, bar(C::kBarKV));
+          tma_load_4d(smem_base + C::kOffV + ch * C::kChunkBytes, &tv, ch * T::kChunkElems, jt * 128, hc, bar(C::kBarKV));
+        }
       }
       bool ok = true;
+      int slot = 0, ph = 0;
       for (int i = 0; ok && i < nq; ++i) {
         const int qt = jt + i;
         // rowstats of Q tile qt -> stats buffer i % 2, once the compute warps are done with
@@ -813,17 +812,14 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
                        rowstats + (static_cast<size_t>(bh) * ntiles + qt) * 256, 1024,
                        bar(C::kBarStatsFull + (i & 1)));
         }
-        for (int sub = 0; sub < 4; ++sub) {  // Q_lo, Q_hi, dO_lo, dO_hi
-          const int t = 4 * i + sub, slot = t % C::kRing, ph = (t / C::kRing) & 1;
+        for (int sub = 0; sub < 2 * C::kChunks; ++sub) {  // the chunks of Q, then those of dO
           if (!(ok = mbar_wait_warp(bar(C::kBarRingEmpty + slot), ph ^ 1, w, kBSiteLoadDO))) break;
           if (elected) {
-            mbar_arrive_expect_tx(bar(C::kBarRingFull + slot), T::kTileBytes);
-#pragma unroll
-            for (int ch = 0; ch < T::kChunks; ++ch)
-              tma_load_4d(smem_base + C::kOffRing + slot * T::kTileBytes + ch * T::kChunkTileBytes,
-                          sub < 2 ? &tq : &tdo, (sub & 1) * 128 + ch * T::kChunkElems, qt * 128, hc,
-                          bar(C::kBarRingFull + slot));
+            mbar_arrive_expect_tx(bar(C::kBarRingFull + slot), C::kChunkBytes);
+            tma_load_4d(smem_base + C::kOffRing + slot * C::kChunkBytes, sub < C::kChunks ? &tq : &tdo,
+                        (sub % C::kChunks) * T::kChunkElems, qt * 128, hc, bar(C::kBarRingFull + slot));
           }
+          if (++slot == C::kRing) slot = 0, ph ^= 1;
         }
       }
     } else if (warp == C::kMmaWarp) {
@@ -832,28 +828,41 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
         if (elected) mma_commit(bar(b));
       };
       bool ok = mbar_wait(bar(C::kBarKV), 0, w, kBSiteMmaKV);
-      for (int i = 0; ok && i < nq; ++i) {
-        const int b = i & 1, u = i >> 1;  // tensor-memory buffer and its use count
-        for (int prod = 0; ok && prod < 2; ++prod) {  // 0: St(i), 1: dPt(i)
-          if (u > 0) {
-            // the compute warps have copied use u - 1 of this buffer into registers
-            if (!(ok = mbar_wait(bar((prod ? C::kBarDptFree : C::kBarStFree) + b), (u - 1) & 1, w,
-                                 kBSiteMmaDrain)))
-              break;
-            tc_fence_after();
-          }
-          for (int half = 0; ok && half < 2; ++half) {
-            const int t = 4 * i + 2 * prod + half, slot = t % C::kRing, ph = (t / C::kRing) & 1;
-            if (!(ok = mbar_wait(bar(C::kBarRingFull + slot), ph, w, kBSiteMmaQ))) break;
-            issue_rows_x_rows<128, BF16>(
-                elected, tmem_base + (prod ? C::kColDpt : C::kColSt) + b * 128,
-                smem_base + (prod ? C::kOffV : C::kOffK) + half * T::kTileBytes,
-                smem_base + C::kOffRing + slot * T::kTileBytes, half);
-            commit(C::kBarRingEmpty + slot);
-          }
-          if (ok) commit((prod ? C::kBarDptFull : C::kBarStFull) + b);
+      int slot = 0, ph = 0;  // of the next chunk
+      // St and dPt: 64 columns of the head dim after another, from the next chunks of the ring
+      auto scores = [&](int column, int resident, bool release) {
+        for (int ch = 0; ok && ch < C::kChunks; ++ch) {
+          if (!(ok = mbar_wait(bar(C::kBarRingFull + slot), ph, w, kBSiteMmaQ))) break;
+          issue_rows_x_rows<64, BF16>(elected, tmem_base + column, smem_base + resident + ch * C::kChunkBytes,
+                                      smem_base + C::kOffRing + slot * C::kChunkBytes, ch > 0);
+          if (release) commit(C::kBarRingEmpty + slot);
+          if (++slot == C::kRing) slot = 0, ph ^= 1;
         }
+      };
+      for (int i = 0; ok && i <= nq; ++i) {
+        if (i > 0) {
+          int s = (slot + C::kRing - C::kChunks) % C::kRing;  // dO(i-1) lies in the last chunks taken
+          if (!(ok = mbar_wait(bar(C::kBarPtReady), (i - 1) & 1, w, kBSiteMmaPt))) break;
+          tc_fence_after();
+          for (int ch = 0; ch < C::kChunks; ++ch) {
+            issue_tmem_x_tile<64, BF16>(elected, tmem_base + C::kColDV + ch * 64, tmem_base + C::kColSt, 64,
+                                        smem_base + C::kOffRing + s * C::kChunkBytes, i > 1);
+            commit(C::kBarRingEmpty + s);
+            if (++s == C::kRing) s = 0;
+          }
+        }
+        if (i == nq) break;
+        scores(C::kColSt, C::kOffK, true);
+        if (!ok) break;
+        commit(C::kBarStFull);
+        if (i > 0) {
+          if (!(ok = mbar_wait(bar(C::kBarDptFree), (i - 1) & 1, w, kBSiteMmaDrain))) break;
+          tc_fence_after();
+        }
+        scores(C::kColDpt, C::kOffV, false);
+        if (ok) commit(C::kBarDptFull);
       }
+      if (ok) commit(C::kBarDone);
     }
     __syncwarp();
   } else {
@@ -862,6 +871,8 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
     const int w4 = warp & 3;
     const int r = w4 * 32 + lane;  // kv row in the tile = tensor-memory lane
     const uint32_t lane_base = static_cast<uint32_t>(w4 * 32) << 16;
+    const uint32_t tSt = tmem_base + lane_base + C::kColSt + wg * 64;
+    const uint32_t tDpt = tmem_base + lane_base + C::kColDpt + wg * 64;
     const float2 sc2 = make_float2(scale_log2, scale_log2);
     float inv_dscale;
     const float dscale =
@@ -869,15 +880,12 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
     const float2 scale2 = make_float2(scale * dscale, scale * dscale);  // dS * 2^k, see head_dscale
     bool ok = true;
     for (int i = 0; i < nq; ++i) {
-      const int b = i & 1, u = i >> 1;
-      const uint32_t tSt = tmem_base + lane_base + C::kColSt + b * 128 + wg * 64;
-      const uint32_t tDpt = tmem_base + lane_base + C::kColDpt + b * 128 + wg * 64;
+      const int b = i & 1;
       const float* stats = reinterpret_cast<const float*>(smem + C::kOffStats + b * 1024);
       const float4* nlse = reinterpret_cast<const float4*>(stats + wg * 64);        // -lse*log2e
       const float4* ndlt = reinterpret_cast<const float4*>(stats + 128 + wg * 64);  // -delta
-      const size_t out_off = static_cast<size_t>(tile0 + i) * 2048 + wg * 1024 + r;
-      if (!(ok = mbar_wait_warp(bar(C::kBarStatsFull + b), u & 1, w, kBSiteCmpQ))) break;
-      if (!(ok = mbar_wait_warp(bar(C::kBarStFull + b), u & 1, w, kBSiteCmpSt))) break;
+      if (!(ok = mbar_wait_warp(bar(C::kBarStatsFull + b), (i >> 1) & 1, w, kBSiteCmpQ))) break;
+      if (!(ok = mbar_wait_warp(bar(C::kBarStFull), i & 1, w, kBSiteCmpSt))) break;
       tc_fence_after();
       float2 p[32];  // P^T for this thread's kv row, q columns wg*64 .. wg*64+63
       {
@@ -885,9 +893,6 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
         tmem_ld_x32(tSt, sr);
         tmem_ld_x32(tSt + 32, sr + 32);
         tmem_wait_ld();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(C::kBarStFree + b));  // St(i + 2) may overwrite the buffer
         probabilities_of_row(sr, nlse, sc2, p);
       }
       if (i == 0 || kv_ragged) {
@@ -895,16 +900,17 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
         mask_row(p, (jt * 128 + r >= Nk) ? 128 : (i == 0 ? r : 0), wg * 64);
       }
       {
-        // P^T rounded to 16 bits, piece-major (see bwd_dkdv_kernel's spill store)
-        uint4* dst = p_scratch + out_off;
+        uint32_t pk[32];
 #pragma unroll
-        for (int pc = 0; pc < 8; ++pc)
-          dst[pc * 128] = make_uint4(pack2<kInterBF16<BF16>>(p[4 * pc].x, p[4 * pc].y),
-                                     pack2<kInterBF16<BF16>>(p[4 * pc + 1].x, p[4 * pc + 1].y),
-                                     pack2<kInterBF16<BF16>>(p[4 * pc + 2].x, p[4 * pc + 2].y),
-                                     pack2<kInterBF16<BF16>>(p[4 * pc + 3].x, p[4 * pc + 3].y));
+        for (int c = 0; c < 32; ++c) pk[c] = pack2<kInterBF16<BF16>>(p[c].x, p[c].y);
+        tmem_st_x32(tSt, pk);
+        tmem_wait_st();
       }
-      if (!(ok = mbar_wait_warp(bar(C::kBarDptFull + b), u & 1, w, kBSiteCmpDpt))) break;
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(C::kBarPtReady));
+
+      if (!(ok = mbar_wait_warp(bar(C::kBarDptFull), i & 1, w, kBSiteCmpDpt))) break;
       tc_fence_after();
       uint32_t dp[64];
       tmem_ld_x32(tDpt, dp);
@@ -912,7 +918,7 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(C::kBarDptFree + b));
+      if (lane == 0) mbar_arrive(bar(C::kBarDptFree));
       uint32_t dsk[32];
 #pragma unroll
       for (int c4 = 0; c4 < 16; ++c4) {
@@ -928,7 +934,8 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
         dsk[2 * c4 + 1] = pack2<kInterBF16<BF16>>(u1.x, u1.y);
       }
       {
-        uint4* dst = ds_scratch + out_off;
+        // piece-major, see bwd_dkdv_kernel's spill store
+        uint4* dst = ds_scratch + (static_cast<size_t>(tile0 + i) * 2048 + wg * 1024 + r);
 #pragma unroll
         for (int pc = 0; pc < 8; ++pc)
           dst[pc * 128] = make_uint4(dsk[4 * pc], dsk[4 * pc + 1], dsk[4 * pc + 2], dsk[4 * pc + 3]);
@@ -938,6 +945,16 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
       // the copy engine then refills the buffer under it (seen as four wrong q columns of a tile).
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(C::kBarStatsFree + b));
+    }
+    // dV: group 0 stores columns 0..127, group 1 the others, staged through the idle K tile
+    if (ok && mbar_wait_warp(bar(C::kBarDone), 0, w, kBSiteCmpDone)) {
+      tc_fence_after();
+      const uint32_t acc = tmem_base + lane_base + C::kColDV + wg * 128;
+      if (dv32.p != nullptr)
+        store_rows_f32<128>(acc, F32Out{dv32.p + wg * 128, dv32.st}, cols - wg * 128, jt * 128 + r, hc, Nk);
+      else
+        store_rows_16bit<128, BF16>(acc, smem + C::kOffK + wg * T::kTileBytes, w4, lane, &tdv, jt * 128, hc, Nk, 1.0f,
+                                    wg * T::kChunks);
     }
   }
 
@@ -951,8 +968,8 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
 
 template <bool BF16>
 cudaError_t launch_scores_wide_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
-                                 const CUtensorMap& tv, const CUtensorMap& tdo, const RowStats& rowstats,
-                                 void* p_scratch, void* ds_scratch, int* status,
+                                 const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdv,
+                                 const F32Out& dv32, const RowStats& rowstats, void* ds_scratch, int* status,
                                  cudaStream_t stream) {
   using C = ScoresCfg;
   auto kern = bwd_scores_wide_kernel<BF16>;
@@ -961,8 +978,7 @@ cudaError_t launch_scores_wide_t(const AttnShape& s, const CUtensorMap& tq, cons
   if (e != cudaSuccess) return e;
   const unsigned grid = static_cast<unsigned>((s.Nk + 127) / 128) * s.B * s.H;  // one CTA per KV tile
   return launch_dependent(kern, grid, C::kThreads, C::kSmemBytes, stream,
-      tq, tk, tv, tdo, rowstats.stats, rowstats.tile_amax, static_cast<uint4*>(p_scratch),
-      static_cast<uint4*>(ds_scratch), s.N, s.Nk, s.B * s.H, s.H, heads_per_group(s), s.scale,
+      tq, tk, tv, tdo, tdv, dv32, s.Dg, rowstats.stats, rowstats.tile_amax, static_cast<uint4*>(ds_scratch), s.N, s.Nk, s.B * s.H, s.H, heads_per_group(s), s.scale,
       s.scale * 1.4426950408889634f, status);
 }
 
@@ -1105,13 +1121,11 @@ cudaError_t launch_bwd_dq(const AttnShape& s, const CUtensorMap& tq, const CUten
 }
 
 cudaError_t launch_bwd_scores_wide(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
-                                   const CUtensorMap& tv, const CUtensorMap& tdo,
-                                   const RowStats& rowstats, void* p_scratch, void* ds_scratch,
-                                   int* status, cudaStream_t stream) {
-  return s.dtype ? launch_scores_wide_t<true>(s, tq, tk, tv, tdo, rowstats, p_scratch, ds_scratch,
-                                              status, stream)
-                 : launch_scores_wide_t<false>(s, tq, tk, tv, tdo, rowstats, p_scratch, ds_scratch,
-                                               status, stream);
+                                   const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdv,
+                                   const F32Out& dv32, const RowStats& rowstats, void* ds_scratch, int* status,
+                                   cudaStream_t stream) {
+  return s.dtype ? launch_scores_wide_t<true>(s, tq, tk, tv, tdo, tdv, dv32, rowstats, ds_scratch, status, stream)
+                 : launch_scores_wide_t<false>(s, tq, tk, tv, tdo, tdv, dv32, rowstats, ds_scratch, status, stream);
 }
 
 cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch,
@@ -1127,7 +1141,8 @@ cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch
                         : launch_consume_pair_t<false, FORM>(FA2_ARGS))                       \
              : (s.dtype ? launch_consume_t<256, true, FORM>(FA2_ARGS)                         \
                         : launch_consume_t<256, false, FORM>(FA2_ARGS)))
-  if (s.D == 256) return form == 0 ? FA2_WIDE(0) : (form == 1 ? FA2_WIDE(1) : FA2_WIDE(2));
+  if (s.D == 256 && form == 1) return FA2_WIDE(1);
+  if (s.D == 256 && form == 2) return FA2_WIDE(2);
 #undef FA2_WIDE
   if (form != 2) return cudaErrorInvalidValue;
   if (s.D == 128 && s.Dg <= kShortDim128)

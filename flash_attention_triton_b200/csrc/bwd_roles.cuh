@@ -76,11 +76,12 @@ __device__ __forceinline__ void mask_row(float2 (&p)[PAIRS], int first_column, i
 
 // Epilogue helper: one warp multiplies its 32 rows of a [128, D] fp32 accumulator by `mul` (a power
 // of two, see head_dscale), converts them to 16 bits, stages them swizzled in `stage` (a free
-// tile buffer) and stores them with one TMA per chunk.
+// tile buffer) and stores them with one TMA per chunk, into the tensor's columns from chunk `chunk0` on.
 template <int D, bool BF16, int KD = D>
 __device__ __forceinline__ void store_rows_16bit(uint32_t tmem_row_addr, uint8_t* stage, int warp4,
                                                  int lane, const CUtensorMap* map, int row_base,
-                                                 HeadCoord hc, int N, float mul = 1.0f) {
+                                                 HeadCoord hc, int N, float mul = 1.0f,
+                                                 int chunk0 = 0) {
   using T = Tile<D>;
   const int r = warp4 * 32 + lane;
 #pragma unroll
@@ -105,7 +106,7 @@ __device__ __forceinline__ void store_rows_16bit(uint32_t tmem_row_addr, uint8_t
   __syncwarp();
   if (lane == 0 && row_base + warp4 * 32 < N) {
     for (int ch = 0; ch < T::kChunks; ++ch)
-      tma_store_4d(map, ch * T::kChunkElems, row_base + warp4 * 32, hc,
+      tma_store_4d(map, (chunk0 + ch) * T::kChunkElems, row_base + warp4 * 32, hc,
                    smem_u32(stage + ch * T::kChunkTileBytes + warp4 * 32 * T::kRowBytes));
     tma_store_commit();
     tma_store_wait_all();
@@ -684,9 +685,8 @@ __device__ __forceinline__ void dkdv_roles(
 // pair in ascending order, no exponentials; its cost is reading the 32 KiB scratch tile (and the
 // operand tile) per product.
 //   FORM 2: dQ(qt) = sum_j dS(j, qt) K_j      A = dS^T tile transposed (MN-major pieces)
-//   FORM 0: dV(jt) = sum_i P(jt, i)^T dO_i    A = P^T tile as stored   (K-major pieces)
 //   FORM 1: dK(jt) = sum_i dS(jt, i)^T Q_i    A = dS^T tile as stored  (K-major pieces)
-// (forms 0 and 1 serve head dim 256, where dK and dV do not fit next to the scores in tensor
+// (form 1 serves head dim 256, where dK and dV do not fit next to the scores in tensor
 // memory.)  Up to head dim 128 a stage is half of a product, 64 reduction rows (the scratch tile is stored
 // in halves then), so that two CTAs fit an SM: the start and the end of one are covered by the other.
 // Roles: one producer warp (ring of kStages x (scratch tile + operand tile)), one
@@ -704,8 +704,7 @@ struct ConsumeItem {
   int ot;             // output tile
   HeadCoord hc;
   size_t head_tile0;  // scratch index of the head's first pair
-  const unsigned* tile_amax;  // forms 1, 2: largest |dO| per Q tile of the head (the tiles are dS * 2^k,
-                              // see head_dscale); nullptr for form 0 (P tiles)
+  const unsigned* tile_amax;  // largest |dO| per Q tile of the head (the tiles are dS * 2^k, see head_dscale)
 };
 
 // epi_warp: 0..3 for the four epilogue warps (warp e owns tensor-memory lanes 32e .. 32e+31),
@@ -741,7 +740,7 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
       if (!mbar_wait_warp(empty(st), ph ^ 1, w, kBSiteLoadQ)) break;
       if (elected) {
         const uint32_t dst = ring_base + st * kStageBytes;
-        const int other = first + n;  // the KV tile (form 2) or Q tile (forms 0, 1) of this product
+        const int other = first + n;  // the KV tile (form 2) or Q tile (form 1) of this product
         // pair (KV tile, Q tile) -> scratch tile: pairs of a head are numbered KV tile by KV tile
         const size_t tile = item.head_tile0 + (FORM == 2 ? dstile_count(ntiles, other) + (ot - other)
                                                          : dstile_count(ntiles, ot) + n);
@@ -774,8 +773,8 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
     if (ok && elected) mma_commit(done);
     __syncwarp();
   } else if (epi_warp >= 0) {
-    float inv_dscale = 1.0f;
-    if (item.tile_amax != nullptr) head_dscale<BF16>(item.tile_amax, ntiles, lane, &inv_dscale);
+    float inv_dscale;
+    head_dscale<BF16>(item.tile_amax, ntiles, lane, &inv_dscale);
     if (mbar_wait_warp(done, 0, w, kBSiteCmpDone)) {
       tc_fence_after();
       const uint32_t lane_base = static_cast<uint32_t>(epi_warp * 32) << 16;

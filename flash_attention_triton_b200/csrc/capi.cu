@@ -172,8 +172,8 @@ int check_shape(int B, int H, int N, int D, int dtype) {
   return FA2_OK;
 }
 
-// Scratch of the spilling backward modes: one 32 KiB dS tile per (KV tile, Q tile) pair of a
-// head, and a P tile as well for head dims above 128.
+// Scratch of the spilling backward modes: one 32 KiB dS tile per (KV tile, Q tile) pair of a head.  Callers are
+// asked for twice that for head dims above 128, which kept a P tile too once; it goes into larger chunks there.
 long long spill_bytes_per_head(int N, int Nk, int D) {
   return dstile_pairs(N, Nk) * 32768 * (D > 128 ? 2 : 1);
 }
@@ -385,7 +385,7 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
   if (deterministic == 2) {
-    const SpillPlan plan = spill_plan(B, H, per_head, ws);
+    const SpillPlan plan = spill_plan(B, H, dstile_pairs(N, Nk) * 32768, ws);
     if (plan.nb < B || plan.nh < H) {
       // more than one chunk: the same call on sub-ranges, one after the other on the stream
       // (they share the scratch), with the caller's strides spelled out
@@ -456,24 +456,16 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
   if (deterministic == 2) {
     float* scratch = static_cast<float*>(workspace);
     if (D > 128) {
-      // P tiles first, dS tiles behind them
-      const long long pairs = BH * dstile_pairs(N, Nk);
-      char* p_scratch = static_cast<char*>(workspace);
-      char* ds_scratch = p_scratch + static_cast<size_t>(pairs) * 32768;
-      cudaError_t ce = launch_bwd_scores_wide(s, tq, tk, tv, tdo, rs, p_scratch, ds_scratch,
-                                              d->status, st);
+      cudaError_t ce = launch_bwd_scores_wide(s, tq, tk, tv, tdo, tdv, dv32, rs, scratch, d->status, st);
       if (ce != cudaSuccess) return static_cast<int>(ce);
       const bool two = consume_two_tiles(s, d->num_sms);
       if (two) {  // operands in half tiles
         if (int e = make_map_of(&tq, q, strides, 0, dtype, B, H, N, D, 64)) return e;
         if (int e = make_map_of(&tk, k, strides, 1, dtype, B, H, Nk, D, 64)) return e;
-        if (int e = make_map_of(&tdo, dout, strides, 3, dtype, B, H, N, D, 64)) return e;
       }
-      if ((ce = launch_bwd_consume(s, 0, p_scratch, tdo, tdv, dv32, rs, two, d->status, st)) != cudaSuccess)
+      if ((ce = launch_bwd_consume(s, 1, scratch, tq, tdk, dk32, rs, two, d->status, st)) != cudaSuccess)
         return static_cast<int>(ce);
-      if ((ce = launch_bwd_consume(s, 1, ds_scratch, tq, tdk, dk32, rs, two, d->status, st)) != cudaSuccess)
-        return static_cast<int>(ce);
-      return static_cast<int>(launch_bwd_consume(s, 2, ds_scratch, tk, tdq, dq32, rs, two, d->status, st));
+      return static_cast<int>(launch_bwd_consume(s, 2, scratch, tk, tdq, dq32, rs, two, d->status, st));
     }
     cudaError_t ce =
         launch_bwd_dkdv(s, tq, tk, tv, tdo, tdk, tdv, dk32, dv32, rs, scratch, 2, step_rows, d->status, st);

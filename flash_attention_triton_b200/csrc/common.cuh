@@ -207,19 +207,17 @@ cudaError_t launch_bwd_dkdv(const AttnShape& s, const CUtensorMap& tq, const CUt
                             const F32Out& dv32, const RowStats& rowstats, float* dq_accum, int mode, int step_rows,
                             int* status, cudaStream_t stream);
 
-// Head dim 256: P^T and dS^T of every (KV tile, Q tile) pair as 16-bit piece-major tiles into two
-// scratch tensors (pair numbering as in the spill mode); launch_bwd_consume forms 0, 1 and 2 then
-// give dV, dK and dQ.
+// Head dims above 128: dV per KV tile, and dS^T of every (KV tile, Q tile) pair as 16-bit piece-major tiles into a
+// scratch tensor (pair numbering as in the spill mode); launch_bwd_consume forms 1 and 2 then give dK and dQ.
 cudaError_t launch_bwd_scores_wide(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
-                                   const CUtensorMap& tv, const CUtensorMap& tdo,
-                                   const RowStats& rowstats, void* p_scratch, void* ds_scratch,
-                                   int* status, cudaStream_t stream);
+                                   const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdv,
+                                   const F32Out& dv32, const RowStats& rowstats, void* ds_scratch, int* status,
+                                   cudaStream_t stream);
 
-// One output tile per CTA from spilled 16-bit score-gradient / probability tiles, one product
+// One output tile per CTA from spilled 16-bit score-gradient tiles, one product
 // per tile pair in ascending order (deterministic):
-//   form 2: dQ(qt) = sum_j dS(j, qt) K_j     (scratch = dS tiles, tb = K, tout = dQ)
-//   form 0: dV(jt) = sum_i P(jt, i)^T dO_i   (scratch = P tiles,  tb = dO, tout = dV)  head dim 256
-//   form 1: dK(jt) = sum_i dS(jt, i)^T Q_i   (scratch = dS tiles, tb = Q,  tout = dK)  head dim 256
+//   form 2: dQ(qt) = sum_j dS(j, qt) K_j     (tb = K, tout = dQ)
+//   form 1: dK(jt) = sum_i dS(jt, i)^T Q_i   (tb = Q, tout = dK)  head dim 256
 // At head dim 256, with two_tiles, a CTA forms two adjacent output tiles (tb then has boxes of 64 rows).
 cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch,
                                const CUtensorMap& tb, const CUtensorMap& tout, const F32Out& out32,

@@ -162,8 +162,8 @@ int main(int argc, char** argv) {
     if (kernel == "dkdv_atomic") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 1, step, &status, nullptr);
     if (kernel == "dkdv_spill") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 2, step, &status, nullptr);
     if (kernel == "dq") launch_bwd_dq(s, m, m, m, m, m, none, rs, step, &status, nullptr);
-    if (kernel == "scores") launch_bwd_scores_wide(s, m, m, m, m, rs, scratch.data(), scratch.data(), &status, nullptr);
-    for (int form = 0; form < 3; ++form) {
+    if (kernel == "scores") launch_bwd_scores_wide(s, m, m, m, m, m, none, rs, scratch.data(), &status, nullptr);
+    for (int form = 1; form < 3; ++form) {
       if (kernel == "consume" && (d > 128 || form == 2)) launch_bwd_consume(s, form, scratch.data(), m, m, none, rs, false, &status, nullptr);
       if (kernel == "consume_pair") launch_bwd_consume(s, form, scratch.data(), m, m, none, rs, true, &status, nullptr);
     }

@@ -217,6 +217,20 @@ def test_wide_head_consumers_with_two_output_tiles(d, nq, nk, monkeypatch):
     check_against(naive_attention(at(q), at(k), at(v), at(do)), {key: at(t) for key, t in pairs.items()}, torch.bfloat16)
 
 
+@pytest.mark.parametrize("d", [136, 256])
+@pytest.mark.parametrize("nq,nk", [(1, 1), (130, 127), (384, 384), (900, 900), (1025, 640)])
+def test_wide_head_dv_over_the_chunk_ring(d, nq, nk):
+    """1 to 9 steps of eight chunks through a ring of six; rows beyond the last key; 16-bit and fp32 outputs."""
+    g = torch.Generator().manual_seed(nq)
+    q, do = (torch.randn(1, 2, nq, d, generator=g).half() for _ in range(2))
+    k, v = (torch.randn(1, 2, nk, d, generator=g).half() for _ in range(2))
+    ref = naive_attention(q, k, v, do)
+    got = run_api(q, k, v, do, None, True)
+    check_against(ref, got, torch.float16)
+    wide = run_api(q.float(), k.float(), v.float(), do.float(), None, True)
+    assert torch.equal(wide["dv"].half(), got["dv"])
+
+
 @pytest.mark.parametrize("d", [32, 64])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_keys_with_scores_of_minus_infinity_have_no_weight(d, dtype):
