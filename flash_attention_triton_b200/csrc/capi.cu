@@ -300,7 +300,7 @@ int fa2_bwd_preprocess_strided(const void* o, const void* dout, const float* lse
   if (!o || !dout || !lse || !rowstats) return FA2_ERR_NULL_POINTER;
   if (int e = check_shape(B, H, N, D, dtype)) return e;
   if (!aligned16(o) || !aligned16(dout) || !aligned16(rowstats)) return FA2_ERR_MISALIGNED;
-  if (static_cast<long long>(B) * H * ((N + 127) / 128) > 0x7fffffffll) return FA2_ERR_SHAPE;  // one block per tile (head dim 256)
+  if (static_cast<long long>(B) * H * ((N + 127) / 128) > 0x7fffffffll) return FA2_ERR_SHAPE;
   Strides so, sdo;
   if (int e = get_strides(strides, 0, B, H, N, D, &so)) return e;
   if (int e = get_strides(strides, 1, B, H, N, D, &sdo)) return e;
@@ -309,10 +309,11 @@ int fa2_bwd_preprocess_strided(const void* o, const void* dout, const float* lse
   const AttnShape s = make_shape(B, H, N, N, D, dtype, 1.f);
   // whole rows, packed, of tensors that are not contiguous
   CUtensorMap to{}, tdo{};
-  if (D <= 128 && so.n != D)
-    if (int e = encode_map(&to, o, dtype, B, H, N, D, so, D, 128, CU_TENSOR_MAP_SWIZZLE_NONE)) return e;
-  if (D <= 128 && sdo.n != D)
-    if (int e = encode_map(&tdo, dout, dtype, B, H, N, D, sdo, D, 128, CU_TENSOR_MAP_SWIZZLE_NONE)) return e;
+  const int box_rows = D <= 128 ? 128 : 64;
+  if (so.n != D)
+    if (int e = encode_map(&to, o, dtype, B, H, N, D, so, D, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE)) return e;
+  if (sdo.n != D)
+    if (int e = encode_map(&tdo, dout, dtype, B, H, N, D, sdo, D, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE)) return e;
   return static_cast<int>(launch_bwd_preprocess(s, to, tdo, o, so, dout, sdo, lse, rowstats, d->status,
                                                 d->num_sms, static_cast<cudaStream_t>(stream)));
 }

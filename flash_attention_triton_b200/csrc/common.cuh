@@ -190,7 +190,7 @@ cudaError_t launch_fwd(const AttnShape& s, int kv_rows, const CUtensorMap& tq, c
 // rowstats[bh][t][0][r] = -lse * log2(e) (-inf for padded rows), rowstats[bh][t][1][r] = -delta;
 // behind the last tile, one 32-bit word per tile: the largest |dout| of the tile's rows as its
 // 16-bit pattern with the sign cleared.  Tensors whose rows are not contiguous are read through `to` and `tdo`
-// (boxes of 128 whole rows, no swizzle; up to head dim 128), which need not be valid otherwise.
+// (boxes of 128 whole rows, 64 above head dim 128, no swizzle), which need not be valid otherwise.
 cudaError_t launch_bwd_preprocess(const AttnShape& s, const CUtensorMap& to, const CUtensorMap& tdo,
                                   const void* o, const Strides& so, const void* dout, const Strides& sdo, const float* lse,
                                   float* rowstats, int* status, int num_sms,

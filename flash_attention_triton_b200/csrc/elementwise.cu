@@ -1,6 +1,6 @@
 // Bandwidth-bound helpers of the backward pass.
 //
-//   bwd_preprocess_kernel  delta[row] = sum_d float(o[row,d]) * float(dout[row,d])
+//   bwd_preprocess_ring_kernel  delta[row] = sum_d float(o[row,d]) * float(dout[row,d])
 //       replaces _backward_preprocess_do_o_dot (_triton_kernels_v2.py:532-608 of the
 //       reference).  Algorithmic traffic per row: 2 * D * 2 bytes read + 4 bytes (lse) read +
 //       8 bytes written.
@@ -33,104 +33,25 @@ __device__ __forceinline__ float dot8(const uint4& a, const uint4& b) {
   return acc;
 }
 
-constexpr int kPreThreads = 256;
-constexpr int kPreMaxInFlight = 8;  // rows a thread group has in flight at once (2 x 16 bytes each)
 constexpr float kLog2e = 1.4426950408889634f;
 
-// One block per 128-row tile of one (batch, head).  A group of D/8 adjacent lanes owns a row: each
-// lane reads one 16-byte piece of o and of dout, multiplies, and the group reduces with shuffles
-// in a fixed order (deterministic).  The block's 256 threads cover 2048 / D rows per pass and a
-// thread issues the loads of up to kPreMaxInFlight passes (16 independent 16-byte loads) before it
-// uses the first one, which is what keeps enough bytes in flight to fill the HBM pipe.
-// D is the padded head dim; a row in memory has d8 <= D/8 pieces and the lanes beyond it
-// contribute zeros.  Rows beyond N are written too: -lse2 = -inf makes every probability of a
-// padded row exactly 0 downstream.  Both vectors are stored NEGATED so the consumers can use them
-// as FMA / ADD addends directly.  The block also leaves the largest |dout| of its rows, as the
-// 16-bit pattern with the sign cleared, in tile_amax[tile] (see head_dscale in bwd_roles.cuh).
-template <int D, bool BF16>
-__global__ void __launch_bounds__(kPreThreads)
-    bwd_preprocess_kernel(const uint4* o, const uint4* dout,
-                          const float* lse, float* __restrict__ rowstats,
-                          unsigned* __restrict__ tile_amax, int N, int ntiles, int d8, int H,
-                          Strides so, Strides sdo) {
-  constexpr int kLanesPerRow = D / 8;
-  constexpr int kRowsPerPass = kPreThreads / kLanesPerRow;  // 64, 32, 16 or 8
-  constexpr int kPasses = 128 / kRowsPerPass;               // 2, 4, 8 or 16
-  constexpr int kBatch = kPasses < kPreMaxInFlight ? kPasses : kPreMaxInFlight;
-  __shared__ unsigned warp_max[kPreThreads / 32];
-  grid_wait_previous();
-  grid_allow_next();
-  const long long tile = blockIdx.x;  // = bh * ntiles + t
-  const long long bh = tile / ntiles;
-  const int t = static_cast<int>(tile - bh * ntiles);
-  const long long bb = bh / H, hh = bh - bb * H;
-  const int sub = threadIdx.x % kLanesPerRow;
-  const int row_in_pass = threadIdx.x / kLanesPerRow;
-  // strides are in 16-byte units (the host divides the element strides by 8)
-  const uint4* o_head = o + bb * so.b + hh * so.h;
-  const uint4* do_head = dout + bb * sdo.b + hh * sdo.h;
-  float* out = rowstats + tile * 256;
-  unsigned amax2 = 0;  // two running maxima of 15-bit magnitudes, one per 16-bit half
-#pragma unroll
-  for (int p0 = 0; p0 < kPasses; p0 += kBatch) {
-    uint4 a[kBatch], b[kBatch];
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int r = (p0 + i) * kRowsPerPass + row_in_pass;  // row inside the tile
-      const long long row = static_cast<long long>(t) * 128 + r;
-      if (row < N && sub < d8) {
-        a[i] = ld_global_once(o_head + row * so.n + sub);
-        b[i] = ld_global_once(do_head + row * sdo.n + sub);
-      } else {
-        a[i] = make_uint4(0, 0, 0, 0);
-        b[i] = make_uint4(0, 0, 0, 0);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      float acc = dot8<BF16>(a[i], b[i]);
-#pragma unroll
-      for (int off = kLanesPerRow / 2; off > 0; off >>= 1)
-        acc += __shfl_xor_sync(0xffffffffu, acc, off);
-      amax2 = __vmaxu2(amax2, b[i].x & 0x7fff7fffu);
-      amax2 = __vmaxu2(amax2, b[i].y & 0x7fff7fffu);
-      amax2 = __vmaxu2(amax2, b[i].z & 0x7fff7fffu);
-      amax2 = __vmaxu2(amax2, b[i].w & 0x7fff7fffu);
-      const int r = (p0 + i) * kRowsPerPass + row_in_pass;
-      if (sub == 0) {
-        const long long row = static_cast<long long>(t) * 128 + r;
-        const bool valid = row < N;
-        out[r] = valid ? -ld_global(lse + bh * N + row) * kLog2e : -INFINITY;
-        out[128 + r] = valid ? -acc : 0.f;
-      }
-    }
-  }
-  // largest magnitude of the block: halves, warp, block (a NaN or inf pattern wins, which
-  // head_dscale treats as "do not scale")
-  unsigned m = max(amax2 & 0xffffu, amax2 >> 16);
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int i = 1; i < kPreThreads / 32; ++i) m = max(m, warp_max[i]);
-    tile_amax[tile] = m;
-  }
-}
-
 // ----------------------------------------------------------------------------------------
-// The same computation as a persistent kernel fed by the copy engine (head dims up to 128).
+// The preprocess: a persistent kernel fed by the copy engine.
 //
 // One CTA per SM walks the 128-row tiles blockIdx.x, blockIdx.x + gridDim.x, ...  A producer warp
-// keeps a ring of shared-memory stages full (one stage = the o rows and the dout rows of one tile; an
-// untiled bulk copy per tensor when its rows are contiguous in memory, else a tiled one through its
-// tensor map), so the bytes in flight per SM stay near the ring size (128 - 192 KiB) whatever
-// the eight consumer warps are doing; the block-per-tile kernel above has nothing in flight while
-// a block reduces and stores, and reaches less than half of the HBM rate.  Consumers read their
-// pieces from shared memory with the row / lane assignment of the kernel above, free the stage
-// once every piece has been used, and hand the tile's 256 results to the next iteration,
+// keeps a ring of shared-memory stages full (one stage = the o rows and the dout rows of one tile, or of half a tile
+// at head dims above 128; an untiled bulk copy per tensor when its rows are contiguous in memory, else a tiled one
+// through its tensor map), so the bytes in flight per SM stay near the ring size (128 - 192 KiB) whatever
+// the eight consumer warps are doing; a block per tile has nothing in flight while
+// it reduces and stores, and reaches less than half of the HBM rate ([2,16,8192,256] bf16, inside a step: 125 us, now 87).
+// A group of D/8 adjacent lanes owns a row: each lane multiplies one 16-byte piece of o and of dout, and the group
+// reduces with shuffles in a fixed order (deterministic).  The lanes beyond the d8 pieces of a row contribute zeros.
+// Consumers free the stage once every piece has been used, and hand the tile's 256 results to the next iteration,
 // which stores them with one coalesced 1 KiB write.  lse of the next tile is fetched one
-// iteration ahead.  Rows in shared memory are packed at their true width (d8 pieces).
+// iteration ahead.  Rows in shared memory are packed at their true width (d8 pieces).  Rows beyond N are written
+// too: -lse2 = -inf makes every probability of a padded row exactly 0 downstream.  Both vectors are stored NEGATED so
+// that the consumers can use them as FMA / ADD addends directly.  The largest |dout| of a tile goes, as the
+// 16-bit pattern with the sign cleared, to tile_amax[tile] (see head_dscale in bwd_roles.cuh).
 // Rows apart from each other (dout as a projection behind it works on it, [B,N,H,d]) came in one bulk copy each,
 // 64 to 256 bytes at a time; as tiled copies they cost what contiguous rows do.  Microseconds, copies of a row /
 // tiled / contiguous rows: [8,16,1000,64] 37 / 13 / 12, [8,12,4095,32] 96 / 21 / 21, [32,20,1024,96] 162 / 49 / 49,
@@ -138,9 +59,11 @@ __global__ void __launch_bounds__(kPreThreads)
 // ----------------------------------------------------------------------------------------
 template <int D>
 struct PreRing {
-  static constexpr int kTileBytes = 128 * D * 2;      // one tensor's rows at the padded width
-  static constexpr int kStageBytes = 2 * kTileBytes;  // o, then dout
-  static constexpr int kStages = D == 128 ? 3 : (D == 64 ? 6 : 8);
+  static constexpr int kRows = D == 256 ? 64 : 128;   // of a stage
+  static constexpr int kParts = 128 / kRows;          // stages of a tile
+  static constexpr int kPartBytes = kRows * D * 2;    // one tensor's rows at the padded width
+  static constexpr int kStageBytes = 2 * kPartBytes;  // o, then dout
+  static constexpr int kStages = D >= 128 ? 3 : (D == 64 ? 6 : 8);
   static constexpr int kConsumers = 256;
   static constexpr int kThreads = kConsumers + 32;
   // after the stages: full / empty barriers, two result buffers of 256 floats, two of 8 maxima
@@ -176,8 +99,9 @@ __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
                                int* status) {
   using R = PreRing<D>;
   constexpr int kLanesPerRow = D / 8;
-  constexpr int kRowsPerPass = R::kConsumers / kLanesPerRow;  // 64, 32 or 16
-  constexpr int kPasses = 128 / kRowsPerPass;                 // 2, 4 or 8
+  constexpr int kRowsPerPass = R::kConsumers / kLanesPerRow;  // 64, 32, 16 or 8
+  constexpr int kPasses = R::kRows / kRowsPerPass;            // of a stage: 2, 4 or 8
+  constexpr int kTilePasses = R::kParts * kPasses;
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t base = smem_u32(smem);
   auto full = [&](int s) { return base + R::kOffBars + 16u * s; };
@@ -202,30 +126,32 @@ __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
 
   if (warp == R::kConsumers / 32) {
     // ---------------- producer warp ----------------
-    int it = 0;
-    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
-      const int s = it % R::kStages;
-      const uint32_t ph = (it / R::kStages) & 1;
-      if (!mbar_wait_warp(empty(s), ph ^ 1, w, kPSiteProducer)) break;
+    int s = 0, ph = 0;
+    bool ok = true;
+    for (long long tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
       const long long bh = tile / ntiles;
       const int t = static_cast<int>(tile - bh * ntiles);
       const long long bb = bh / H, hh = bh - bb * H;
-      const int rows = min(128, N - t * 128);
-      if (lane == 0) {
-        // a tiled copy delivers all 128 rows of its box, zeros beyond the last one
-        const uint32_t dense_bytes = rows * row_bytes, box_bytes = 128 * row_bytes;
-        mbar_arrive_expect_tx(full(s), (so.n == d8 ? dense_bytes : box_bytes) + (sdo.n == d8 ? dense_bytes : box_bytes));
+      for (int row0 = t * 128; row0 < min(N, t * 128 + 128); row0 += R::kRows) {  // stages without a row are left out
+        if (!(ok = mbar_wait_warp(empty(s), ph ^ 1, w, kPSiteProducer))) break;
+        const int rows = min(R::kRows, N - row0);
+        if (lane == 0) {
+          // a tiled copy delivers all rows of its box, zeros beyond the last one
+          const uint32_t dense_bytes = rows * row_bytes, box_bytes = R::kRows * row_bytes;
+          mbar_arrive_expect_tx(full(s), (so.n == d8 ? dense_bytes : box_bytes) + (sdo.n == d8 ? dense_bytes : box_bytes));
 #pragma unroll
-        for (int which = 0; which < 2; ++which) {
-          const Strides& st = which ? sdo : so;
-          const uint32_t dst = base + s * R::kStageBytes + which * R::kTileBytes;
-          if (st.n == d8)
-            bulk_load_1d(dst, (which ? dout : o) + bb * st.b + hh * st.h + static_cast<long long>(t) * 128 * st.n,
-                         dense_bytes, full(s));
-          else
-            tma_load_4d(dst, which ? &tdo : &to, 0, t * 128, HeadCoord{static_cast<int>(hh), static_cast<int>(bb)},
-                        full(s));
+          for (int which = 0; which < 2; ++which) {
+            const Strides& st = which ? sdo : so;
+            const uint32_t dst = base + s * R::kStageBytes + which * R::kPartBytes;
+            if (st.n == d8)
+              bulk_load_1d(dst, (which ? dout : o) + bb * st.b + hh * st.h + static_cast<long long>(row0) * st.n,
+                           dense_bytes, full(s));
+            else
+              tma_load_4d(dst, which ? &tdo : &to, 0, row0, HeadCoord{static_cast<int>(hh), static_cast<int>(bb)},
+                          full(s));
+          }
         }
+        if (++s == R::kStages) s = 0, ph ^= 1;
       }
     }
     return;
@@ -234,86 +160,96 @@ __global__ void __launch_bounds__(PreRing<D>::kThreads, 1)
   // ---------------- consumer warps ----------------
   const int sub = threadIdx.x % kLanesPerRow;
   const int row_in_pass = threadIdx.x / kLanesPerRow;
-  float lse_cur[kPasses], lse_nxt[kPasses];
+  float lse_cur[kTilePasses], lse_nxt[kTilePasses];
   auto fetch_lse = [&](long long tile, float* dst) {
     const long long bh = tile / ntiles;
     const int t = static_cast<int>(tile - bh * ntiles);
 #pragma unroll
-    for (int i = 0; i < kPasses; ++i) {
+    for (int i = 0; i < kTilePasses; ++i) {
       const int row = t * 128 + i * kRowsPerPass + row_in_pass;
       dst[i] = (sub == 0 && tile < tiles && row < N) ? ld_global(lse + bh * N + row) : INFINITY;
     }
   };
   fetch_lse(blockIdx.x, lse_cur);
-  int it = 0;
+  int it = 0, s = 0, ph = 0;
   long long prev_tile = -1;
   for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
-    const int s = it % R::kStages;
-    const uint32_t ph = (it / R::kStages) & 1;
     fetch_lse(tile + gridDim.x, lse_nxt);
-    const bool ok = mbar_wait(full(s), ph, w, kPSiteConsumer);
-    if (!consumers_all(ok, R::kConsumers)) return;
-    // the previous tile's results are complete in shared memory: one coalesced store
-    if (prev_tile >= 0) {
-      const int pb = (it - 1) & 1;
-      rowstats[prev_tile * 256 + threadIdx.x] = stat[pb * 256 + threadIdx.x];
-      if (threadIdx.x == 0) {
-        unsigned m = wmax[pb * 8];
-#pragma unroll
-        for (int i = 1; i < 8; ++i) m = max(m, wmax[pb * 8 + i]);
-        tile_amax[prev_tile] = m;
-      }
-    }
     const int t = static_cast<int>(tile % ntiles);
-    const int rows = min(128, N - t * 128);
-    const uint4* so_ = reinterpret_cast<const uint4*>(smem + s * R::kStageBytes);
-    const uint4* sdo_ = reinterpret_cast<const uint4*>(smem + s * R::kStageBytes + R::kTileBytes);
-    uint4 a[kPasses], b[kPasses];
-#pragma unroll
-    for (int i = 0; i < kPasses; ++i) {
-      const int r = i * kRowsPerPass + row_in_pass;
-      if (r < rows && sub < d8) {
-        a[i] = so_[r * d8 + sub];
-        b[i] = sdo_[r * d8 + sub];
-      } else {
-        a[i] = make_uint4(0, 0, 0, 0);
-        b[i] = make_uint4(0, 0, 0, 0);
-      }
-    }
-    // Products and maxima first: the stage is given back once every piece has been used, not when
-    // its load has been issued (an arrive can overtake a load that is still in flight).
-    float dot[kPasses];
-    unsigned amax2 = 0;
-#pragma unroll
-    for (int i = 0; i < kPasses; ++i) {
-      dot[i] = dot8<BF16>(a[i], b[i]);
-      amax2 = __vmaxu2(amax2, b[i].x & 0x7fff7fffu);
-      amax2 = __vmaxu2(amax2, b[i].y & 0x7fff7fffu);
-      amax2 = __vmaxu2(amax2, b[i].z & 0x7fff7fffu);
-      amax2 = __vmaxu2(amax2, b[i].w & 0x7fff7fffu);
-      dot[i] += __shfl_xor_sync(0xffffffffu, dot[i], kLanesPerRow / 2);
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty(s));
+    const int tile_rows = min(128, N - t * 128);
     const int cb = it & 1;
+    unsigned amax2 = 0;  // two running maxima of 15-bit magnitudes, one per 16-bit half
 #pragma unroll
-    for (int i = 0; i < kPasses; ++i) {
-      float acc = dot[i];
+    for (int part = 0; part < R::kParts; ++part) {
+      const int rows = tile_rows - part * R::kRows;  // of this stage, as far as it goes
+      const bool staged = part == 0 || rows > 0;
+      if (staged) {
+        const bool ok = mbar_wait(full(s), ph, w, kPSiteConsumer);
+        if (!consumers_all(ok, R::kConsumers)) return;
+      }
+      // the previous tile's results are complete in shared memory: one coalesced store
+      if (part == 0 && prev_tile >= 0) {
+        const int pb = (it - 1) & 1;
+        rowstats[prev_tile * 256 + threadIdx.x] = stat[pb * 256 + threadIdx.x];
+        if (threadIdx.x == 0) {
+          unsigned m = wmax[pb * 8];
 #pragma unroll
-      for (int off = kLanesPerRow / 4; off > 0; off >>= 1)
-        acc += __shfl_xor_sync(0xffffffffu, acc, off);
-      const int r = i * kRowsPerPass + row_in_pass;
-      if (sub == 0) {
-        const bool valid = r < rows;
-        stat[cb * 256 + r] = valid ? -lse_cur[i] * kLog2e : -INFINITY;
-        stat[cb * 256 + 128 + r] = valid ? -acc : 0.f;
+          for (int i = 1; i < 8; ++i) m = max(m, wmax[pb * 8 + i]);
+          tile_amax[prev_tile] = m;
+        }
+      }
+      const uint4* so_ = reinterpret_cast<const uint4*>(smem + s * R::kStageBytes);
+      const uint4* sdo_ = reinterpret_cast<const uint4*>(smem + s * R::kStageBytes + R::kPartBytes);
+      uint4 a[kPasses], b[kPasses];
+#pragma unroll
+      for (int i = 0; i < kPasses; ++i) {
+        const int r = i * kRowsPerPass + row_in_pass;
+        if (r < rows && sub < d8) {
+          a[i] = so_[r * d8 + sub];
+          b[i] = sdo_[r * d8 + sub];
+        } else {
+          a[i] = make_uint4(0, 0, 0, 0);
+          b[i] = make_uint4(0, 0, 0, 0);
+        }
+      }
+      // Products and maxima first: the stage is given back once every piece has been used, not when
+      // its load has been issued (an arrive can overtake a load that is still in flight).
+      float dot[kPasses];
+#pragma unroll
+      for (int i = 0; i < kPasses; ++i) {
+        dot[i] = dot8<BF16>(a[i], b[i]);
+        amax2 = __vmaxu2(amax2, b[i].x & 0x7fff7fffu);
+        amax2 = __vmaxu2(amax2, b[i].y & 0x7fff7fffu);
+        amax2 = __vmaxu2(amax2, b[i].z & 0x7fff7fffu);
+        amax2 = __vmaxu2(amax2, b[i].w & 0x7fff7fffu);
+        dot[i] += __shfl_xor_sync(0xffffffffu, dot[i], kLanesPerRow / 2);
+      }
+      __syncwarp();
+      if (staged) {
+        if (lane == 0) mbar_arrive(empty(s));
+        if (++s == R::kStages) s = 0, ph ^= 1;
+      }
+#pragma unroll
+      for (int i = 0; i < kPasses; ++i) {
+        float acc = dot[i];
+#pragma unroll
+        for (int off = kLanesPerRow / 4; off > 0; off >>= 1)
+          acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        const int r = i * kRowsPerPass + row_in_pass;
+        if (sub == 0) {
+          const bool valid = r < rows;
+          stat[cb * 256 + part * R::kRows + r] = valid ? -lse_cur[part * kPasses + i] * kLog2e : -INFINITY;
+          stat[cb * 256 + 128 + part * R::kRows + r] = valid ? -acc : 0.f;
+        }
       }
     }
+    // largest magnitude of the tile: halves, warp, block (a NaN or inf pattern wins, which
+    // head_dscale treats as "do not scale")
     unsigned m = max(amax2 & 0xffffu, amax2 >> 16);
     m = __reduce_max_sync(0xffffffffu, m);
     if (lane == 0) wmax[cb * 8 + warp] = m;
 #pragma unroll
-    for (int i = 0; i < kPasses; ++i) lse_cur[i] = lse_nxt[i];
+    for (int i = 0; i < kTilePasses; ++i) lse_cur[i] = lse_nxt[i];
     prev_tile = tile;
   }
   if (prev_tile >= 0) {
@@ -378,23 +314,16 @@ cudaError_t launch_pre_t(const AttnShape& s, const CUtensorMap& to, const CUtens
   const int ntiles = (s.N + 127) / 128;
   const long long tiles = static_cast<long long>(s.B) * s.H * ntiles;
   unsigned* tile_amax = reinterpret_cast<unsigned*>(rowstats + tiles * 256);  // behind the last tile
-  if constexpr (D <= 128) {
-    using R = PreRing<D>;
-    auto* kernel = bwd_preprocess_ring_kernel<D, BF16>;
-    const cudaError_t attr = cudaFuncSetAttribute(
-        kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::kSmemBytes);
-    if (attr != cudaSuccess) return attr;
-    const unsigned grid = static_cast<unsigned>(tiles < num_sms ? tiles : num_sms);
-    return launch_dependent(
-        kernel, grid, R::kThreads, R::kSmemBytes, stream, to, tdo, static_cast<const uint4*>(o),
-        static_cast<const uint4*>(dout), lse, rowstats, tile_amax,
-        s.N, ntiles, tiles, s.Dg / 8, s.H, in_vec8(so), in_vec8(sdo), status);
-  } else {
-    return launch_dependent(
-        bwd_preprocess_kernel<D, BF16>, static_cast<unsigned>(tiles), kPreThreads, 0, stream,
-        static_cast<const uint4*>(o), static_cast<const uint4*>(dout), lse, rowstats, tile_amax,
-        s.N, ntiles, s.Dg / 8, s.H, in_vec8(so), in_vec8(sdo));
-  }
+  using R = PreRing<D>;
+  auto* kernel = bwd_preprocess_ring_kernel<D, BF16>;
+  const cudaError_t attr = cudaFuncSetAttribute(
+      kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::kSmemBytes);
+  if (attr != cudaSuccess) return attr;
+  const unsigned grid = static_cast<unsigned>(tiles < num_sms ? tiles : num_sms);
+  return launch_dependent(
+      kernel, grid, R::kThreads, R::kSmemBytes, stream, to, tdo, static_cast<const uint4*>(o),
+      static_cast<const uint4*>(dout), lse, rowstats, tile_amax,
+      s.N, ntiles, tiles, s.Dg / 8, s.H, in_vec8(so), in_vec8(sdo), status);
 }
 
 template <int D, bool BF16>

@@ -146,14 +146,6 @@ __device__ __forceinline__ float4 ld_global(const float4* p) {
   asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
   return v;
 }
-// Read once: not kept in L1.
-__device__ __forceinline__ uint4 ld_global_once(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
 
 // ----------------------------------------------------------------------------------------
 // Proxy fences and named barriers

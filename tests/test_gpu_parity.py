@@ -511,6 +511,11 @@ def test_preprocess_over_many_tiles_per_sm(d, strided):
     assert torch.equal(tile_amax, want_amax)
 
 
+@pytest.mark.parametrize("d, strided", [(136, True), (192, False), (256, True)])
+def test_preprocess_of_wide_heads_in_half_tiles(d, strided):
+    test_preprocess_over_many_tiles_per_sm(d, strided)
+
+
 def test_fp32_inputs_follow_the_reference_dtype_policy():
     """fp32 in -> computed in fp16, output and grads returned as fp32 (flash_attention_2.py:316,339);
     the reference's own tests use fp32 inputs with atol 1e-2 on O (tests/test_flash_attention_2.py:297)."""
