@@ -423,13 +423,13 @@ def main():
         def launches_per_step(self):
             """Kernels of this library per step: forward, preprocess and the backward-main kernels
             of the mode (atomic: memset + fused kernel + convert; recompute: dK/dV + dQ; spill:
-            dK/dV + dQ per chunk of the workspace; head dims above 128: scores + three consumers
+            dK/dV + dQ per chunk of the workspace; head dims above 128: scores with dV + two consumers
             per chunk)."""
             if self.mode == 2 or self.d > 128:
                 tiles = (self.n + 127) // 128
-                per_head = tiles * (tiles + 1) // 2 * 32768 * (2 if self.d > 128 else 1)
+                per_head = tiles * (tiles + 1) // 2 * 32768
                 chunks = -(-self.lb * self.lh * per_head // max(self.wsb, 1))
-                return 2 + chunks * (4 if self.d > 128 else 2)
+                return 2 + chunks * (3 if self.d > 128 else 2)
             return 4
 
         def timed(self, steps, warmup, split=False):

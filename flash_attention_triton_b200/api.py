@@ -115,7 +115,7 @@ def _backward_mode(deterministic: bool, headdim: int, seqlen_q: int) -> int:
     deterministic choice above.  ``FA2_B200_BWD_MODE`` =
     ``atomic`` / ``recompute`` / ``spill`` overrides both (for experiments).
     """
-    if headdim > 128:  # one (deterministic) backward exists there: scores + three consumers
+    if headdim > 128:  # one (deterministic) backward exists there: scores with dV + two consumers
         return _MODE_SPILL
     forced = os.environ.get("FA2_B200_BWD_MODE")
     if forced:
