@@ -543,7 +543,7 @@ struct ConsumePairCfg {
   static_assert(kAStages * kAStageBytes >= 2 * T::kTileBytes, "the scratch ring stages both outputs at the end");
 };
 
-template <bool BF16, int FORM>
+template <bool BF16, int FORM, int KD>
 __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
     bwd_consume_pair_kernel(const uint4* scratch, const __grid_constant__ CUtensorMap tb,
                             const __grid_constant__ CUtensorMap tout, const __grid_constant__ F32Out out32,
@@ -626,9 +626,9 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
         const int m = 2 * n + half, bs = m % C::kBStages, bph = (m / C::kBStages) & 1;
         if (!(ok = mbar_wait_warp(bar(C::kBarBEmpty + bs), bph ^ 1, w, kBSiteLoadDO))) break;
         if (elected) {
-          mbar_arrive_expect_tx(bar(C::kBarBFull + bs), C::kBStageBytes);
+          mbar_arrive_expect_tx(bar(C::kBarBFull + bs), C::kBStageBytes / T::kChunks * (KD / T::kChunkElems));
 #pragma unroll
-          for (int ch = 0; ch < T::kChunks; ++ch)
+          for (int ch = 0; ch < KD / T::kChunkElems; ++ch)
             tma_load_4d(smem_base + C::kOffB + bs * C::kBStageBytes + ch * (C::kBStageBytes / T::kChunks), &tb,
                         ch * T::kChunkElems, x * 128 + half * 64, hc, bar(C::kBarBFull + bs));
         }
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
 #pragma unroll
         for (int o = 0; o < 2; ++o)
           if (wanted(o, x))
-            issue_pieces_x_half_tile<256, BF16, FORM == 2>(
+            issue_pieces_x_half_tile<256, BF16, FORM == 2, KD>(
                 elected, tmem_base + o * 256, smem_base + C::kOffA + st * C::kAStageBytes + o * 32768, half,
                 smem_base + C::kOffB + bs * C::kBStageBytes, half > 0 || x > begin[o]);
         if (elected) mma_commit(bar(C::kBarBEmpty + bs));
@@ -664,9 +664,9 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
       tc_fence_after();
       const uint32_t acc = tmem_base + o * 256 + (static_cast<uint32_t>(w4 * 32) << 16);
       if (out32.p != nullptr)
-        store_rows_f32<256>(acc, out32, cols, ot * 128 + w4 * 32 + lane, hc, out_rows, inv_dscale);
+        store_rows_f32<KD>(acc, out32, cols, ot * 128 + w4 * 32 + lane, hc, out_rows, inv_dscale);
       else  // every product has completed, so the scratch ring is idle
-        store_rows_16bit<256, BF16>(acc, smem + C::kOffA + o * T::kTileBytes, w4, lane, &tout, ot * 128, hc,
+        store_rows_16bit<256, BF16, KD>(acc, smem + C::kOffA + o * T::kTileBytes, w4, lane, &tout, ot * 128, hc,
                                     out_rows, inv_dscale);
     }
   }
@@ -684,9 +684,9 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
 // the backward is split: this kernel forms P^T and dS^T for every (KV tile, Q tile) pair, accumulates
 // dV += P^T dO in tensor memory and writes dS^T as 16-bit piece-major tiles to a scratch tensor;
 // bwd_consume_kernel then forms dK and dQ from them.  CTA = one KV tile.  K and V stay in shared memory as
-// kChunks chunk tiles of 64 columns each (128 KiB together); Q and dO stream through a ring of six such chunks,
-// in the order Q(i), dO(i), Q(i+1), ...; dO(i) keeps its chunks until dV has been formed with them, which
-// leaves two for what comes next.  Tensor memory: St, dPt (128 columns each), dV (256).
+// kChunks chunk tiles of 64 columns each (128 KiB together at head dim 256); Q and dO stream through a ring of six such
+// chunks (eight up to head dim 192), in the order Q(i), dO(i), Q(i+1), ...; dO(i) keeps its chunks until dV has been formed
+// with them, which leaves two (five) for what comes next.  Tensor memory: St, dPt (128 columns each), dV (256).
 //   warps 0-7  compute (as in bwd_dkdv_kernel: kv row per thread, two groups of 64 q columns)
 //   warp  8    MMA issue, per step:  [Pt(i) ready]  dV += Pt(i) dO(i),  St(i+1) = K Q^T (over Pt(i)),
 //              [dPt(i) copied]  dPt(i+1) = V dO^T.  dPt(i+1) runs under the exponentials of St(i+1).
@@ -697,14 +697,20 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
 // [2,16,8192,256] bf16, forward and backward 4 148 -> 3 690 us in a loop.  Same bits.  Walking the Q tiles
 // from the last one, as bwd_dkdv_kernel does, measured the same.
 // =========================================================================================
+template <int N>
+struct Columns {
+  static constexpr int value = N;
+};
+
+template <int CH>
 struct ScoresCfg {
   using T = Tile<128>;
   static constexpr int kThreads = 384;
   static constexpr int kMmaWarp = 8;
   static constexpr int kLoadWarp = 9;
-  static constexpr int kChunks = 4;  // of 64 columns: head dim 256
+  static constexpr int kChunks = CH;  // of 64 columns: 4 at head dim 256, 3 up to 192
   static constexpr int kChunkBytes = T::kChunkTileBytes;
-  static constexpr int kRing = 6;
+  static constexpr int kRing = 14 - 2 * CH;
   static constexpr int kOffK = 0;
   static constexpr int kOffV = kChunks * kChunkBytes;
   static constexpr int kOffRing = 2 * kChunks * kChunkBytes;
@@ -729,15 +735,15 @@ struct ScoresCfg {
   static constexpr int kTmemCols = 512;
 };
 
-template <bool BF16>
-__global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
+template <bool BF16, int CH>
+__global__ void __launch_bounds__(ScoresCfg<CH>::kThreads, 1)
     bwd_scores_wide_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                            const __grid_constant__ CUtensorMap tv,
                            const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdv,
                            const __grid_constant__ F32Out dv32, int cols, const float* rowstats,
                            const unsigned* tile_amax, uint4* __restrict__ ds_scratch, int N, int Nk, int num_bh,
                            int num_heads, int group, float scale, float scale_log2, int* status) {
-  using C = ScoresCfg;
+  using C = ScoresCfg<CH>;
   using T = Tile<128>;
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int kWarps = C::kThreads / 32;
@@ -950,11 +956,14 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
     if (ok && mbar_wait_warp(bar(C::kBarDone), 0, w, kBSiteCmpDone)) {
       tc_fence_after();
       const uint32_t acc = tmem_base + lane_base + C::kColDV + wg * 128;
-      if (dv32.p != nullptr)
-        store_rows_f32<128>(acc, F32Out{dv32.p + wg * 128, dv32.st}, cols - wg * 128, jt * 128 + r, hc, Nk);
-      else
-        store_rows_16bit<128, BF16>(acc, smem + C::kOffK + wg * T::kTileBytes, w4, lane, &tdv, jt * 128, hc, Nk, 1.0f,
-                                    wg * T::kChunks);
+      auto store = [&](auto columns) {
+        if (dv32.p != nullptr)
+          store_rows_f32<columns.value>(acc, F32Out{dv32.p + wg * 128, dv32.st}, cols - wg * 128, jt * 128 + r, hc, Nk);
+        else
+          store_rows_16bit<128, BF16, columns.value>(acc, smem + C::kOffK + wg * T::kTileBytes, w4, lane, &tdv, jt * 128, hc,
+                                                     Nk, 1.0f, wg * T::kChunks);
+      };
+      if (wg == 0) store(Columns<128>{}); else store(Columns<CH * 64 - 128>{});
     }
   }
 
@@ -966,13 +975,13 @@ __global__ void __launch_bounds__(ScoresCfg::kThreads, 1)
   }
 }
 
-template <bool BF16>
+template <bool BF16, int CH>
 cudaError_t launch_scores_wide_t(const AttnShape& s, const CUtensorMap& tq, const CUtensorMap& tk,
                                  const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdv,
                                  const F32Out& dv32, const RowStats& rowstats, void* ds_scratch, int* status,
                                  cudaStream_t stream) {
-  using C = ScoresCfg;
-  auto kern = bwd_scores_wide_kernel<BF16>;
+  using C = ScoresCfg<CH>;
+  auto kern = bwd_scores_wide_kernel<BF16, CH>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
@@ -1016,12 +1025,12 @@ cudaError_t launch_consume_t(const AttnShape& s, const void* scratch, const CUte
       s.H, heads_per_group(s), status);
 }
 
-template <bool BF16, int FORM>
+template <bool BF16, int FORM, int KD>
 cudaError_t launch_consume_pair_t(const AttnShape& s, const void* scratch, const CUtensorMap& tb,
                                   const CUtensorMap& tout, const F32Out& out32, const RowStats& rowstats,
                                   int* status, cudaStream_t stream) {
   using C = ConsumePairCfg;
-  auto kern = bwd_consume_pair_kernel<BF16, FORM>;
+  auto kern = bwd_consume_pair_kernel<BF16, FORM, KD>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
@@ -1124,8 +1133,11 @@ cudaError_t launch_bwd_scores_wide(const AttnShape& s, const CUtensorMap& tq, co
                                    const CUtensorMap& tv, const CUtensorMap& tdo, const CUtensorMap& tdv,
                                    const F32Out& dv32, const RowStats& rowstats, void* ds_scratch, int* status,
                                    cudaStream_t stream) {
-  return s.dtype ? launch_scores_wide_t<true>(s, tq, tk, tv, tdo, tdv, dv32, rowstats, ds_scratch, status, stream)
-                 : launch_scores_wide_t<false>(s, tq, tk, tv, tdo, tdv, dv32, rowstats, ds_scratch, status, stream);
+#define FA2_ARGS s, tq, tk, tv, tdo, tdv, dv32, rowstats, ds_scratch, status, stream
+  if (s.Dg <= kShortDim256)
+    return s.dtype ? launch_scores_wide_t<true, 3>(FA2_ARGS) : launch_scores_wide_t<false, 3>(FA2_ARGS);
+  return s.dtype ? launch_scores_wide_t<true, 4>(FA2_ARGS) : launch_scores_wide_t<false, 4>(FA2_ARGS);
+#undef FA2_ARGS
 }
 
 cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch,
@@ -1136,13 +1148,18 @@ cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch
   case DD:                                                                \
     return s.dtype ? launch_consume_t<DD, true, 2>(FA2_ARGS)              \
                    : launch_consume_t<DD, false, 2>(FA2_ARGS);
-#define FA2_WIDE(FORM)                                                                        \
-  (two_tiles ? (s.dtype ? launch_consume_pair_t<true, FORM>(FA2_ARGS)                         \
-                        : launch_consume_pair_t<false, FORM>(FA2_ARGS))                       \
-             : (s.dtype ? launch_consume_t<256, true, FORM>(FA2_ARGS)                         \
-                        : launch_consume_t<256, false, FORM>(FA2_ARGS)))
-  if (s.D == 256 && form == 1) return FA2_WIDE(1);
-  if (s.D == 256 && form == 2) return FA2_WIDE(2);
+#define FA2_WIDE(FORM, KD)                                                                        \
+  (two_tiles ? (s.dtype ? launch_consume_pair_t<true, FORM, KD>(FA2_ARGS)                         \
+                        : launch_consume_pair_t<false, FORM, KD>(FA2_ARGS))                       \
+             : (s.dtype ? launch_consume_t<256, true, FORM, KD>(FA2_ARGS)                         \
+                        : launch_consume_t<256, false, FORM, KD>(FA2_ARGS)))
+  if (s.D == 256 && s.Dg <= kShortDim256) {
+    if (form == 1) return FA2_WIDE(1, kShortDim256);
+    if (form == 2) return FA2_WIDE(2, kShortDim256);
+  } else if (s.D == 256) {
+    if (form == 1) return FA2_WIDE(1, 256);
+    if (form == 2) return FA2_WIDE(2, 256);
+  }
 #undef FA2_WIDE
   if (form != 2) return cudaErrorInvalidValue;
   if (s.D == 128 && s.Dg <= kShortDim128)

@@ -105,7 +105,7 @@ __device__ __forceinline__ void store_rows_16bit(uint32_t tmem_row_addr, uint8_t
   fence_proxy_async_smem();
   __syncwarp();
   if (lane == 0 && row_base + warp4 * 32 < N) {
-    for (int ch = 0; ch < T::kChunks; ++ch)
+    for (int ch = 0; ch < (KD + T::kChunkElems - 1) / T::kChunkElems; ++ch)
       tma_store_4d(map, (chunk0 + ch) * T::kChunkElems, row_base + warp4 * 32, hc,
                    smem_u32(stage + ch * T::kChunkTileBytes + warp4 * 32 * T::kRowBytes));
     tma_store_commit();
@@ -719,6 +719,7 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
   using T = Tile<D>;
   constexpr int PARTS = consume_parts(D);  // stages per product
   constexpr int kScratchBytes = 32768 / PARTS, kOperandBytes = T::kTileBytes / PARTS;
+  constexpr int kChunks = D == 256 ? KD / T::kChunkElems : T::kChunks;  // staged (the last one may be short)
   constexpr int kStageBytes = kScratchBytes + kOperandBytes;
   auto full = [&](int i) { return bar0 + 8u * i; };
   auto empty = [&](int i) { return bar0 + 8u * (STAGES + i); };
@@ -744,11 +745,11 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
         // pair (KV tile, Q tile) -> scratch tile: pairs of a head are numbered KV tile by KV tile
         const size_t tile = item.head_tile0 + (FORM == 2 ? dstile_count(ntiles, other) + (ot - other)
                                                          : dstile_count(ntiles, ot) + n);
-        mbar_arrive_expect_tx(full(st), kStageBytes);
+        mbar_arrive_expect_tx(full(st), kScratchBytes + kOperandBytes / T::kChunks * kChunks);
         // stored as it is used
         bulk_load_1d(dst, scratch + tile * 2048 + part * (2048 / PARTS), kScratchBytes, full(st));
 #pragma unroll
-        for (int ch = 0; ch < T::kChunks; ++ch)
+        for (int ch = 0; ch < kChunks; ++ch)
           tma_load_4d(dst + kScratchBytes + ch * (kOperandBytes / T::kChunks), tb, ch * T::kChunkElems,
                       other * 128 + part * (128 / PARTS), item.hc, full(st));
       }
@@ -765,9 +766,9 @@ __device__ __forceinline__ void consume_roles(uint8_t* ring, uint32_t ring_base,
       if constexpr (PARTS == 2)
         issue_piecesT_half_x_half_tile<D, BF16, KD>(elected, tmem_acc, src, src + kScratchBytes, n > 0);
       else if constexpr (FORM == 2)
-        issue_piecesT_x_tile<D, BF16>(elected, tmem_acc, src, src + 32768, n > 0);
+        issue_piecesT_x_tile<D, BF16, KD>(elected, tmem_acc, src, src + 32768, n > 0);
       else
-        issue_pieces_x_tile<D, BF16>(elected, tmem_acc, src, src + 32768, n > 0);
+        issue_pieces_x_tile<D, BF16, KD>(elected, tmem_acc, src, src + 32768, n > 0);
       if (elected) mma_commit(empty(st));
     }
     if (ok && elected) mma_commit(done);

@@ -355,8 +355,8 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
   if (int e = check_shape(B, H, N, D, dtype)) return e;
   if (Nk < 1 || Nk > N) return FA2_ERR_SHAPE;
   if (deterministic < 0 || deterministic > 2) return FA2_ERR_SHAPE;
-  // Head dims above 128 have one backward (scores kernel + three consumer kernels over two
-  // scratch tensors, in chunks); it is deterministic and serves every value of `deterministic`.
+  // Head dims above 128 have one backward (scores kernel with dV + two consumer kernels over
+  // the scratch tensor, in chunks); it is deterministic and serves every value of `deterministic`.
   if (D > 128) deterministic = 2;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(dout) || !aligned16(dq) ||
       !aligned16(dk) || !aligned16(dv) || !aligned16(rowstats))

@@ -144,6 +144,8 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
   using C = FwdCfg<DT, W>;
   using T = Tile<DT>;
   constexpr int KT = WIDE ? DT : KD;  // columns of a staged tile that the products run over
+  constexpr int KT1 = WIDE ? KD - DT : KD;                            // and of the second half
+  constexpr int kChunks1 = WIDE ? KT1 / T::kChunkElems : T::kChunks;  // chunks staged of the second half
   extern __shared__ __align__(1024) uint8_t smem[];
 
   // Role index: hardware warps 0-3 take roles 8-11 (MMA, TMA, idle, idle) and hardware warps
@@ -267,10 +269,11 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
           if (t < nsub) {
             if (!(ok = mbar_wait_warp(bar(C::kBarKEmpty + ks), kph ^ 1, w, kSiteLoadK))) break;
             if (elected) {
-              mbar_arrive_expect_tx(bar(C::kBarKFull + ks), C::kKvBytes);
+              const int chunks = t % HALVES ? kChunks1 : T::kChunks;
+              mbar_arrive_expect_tx(bar(C::kBarKFull + ks), C::kKvBytes / T::kChunks * chunks);
 #pragma unroll
               for (int ch = 0; ch < T::kChunks; ++ch)
-                tma_load_4d(smem_base + C::kOffK + ks * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tk,
+                if (ch < chunks) tma_load_4d(smem_base + C::kOffK + ks * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tk,
                             (t % HALVES) * 128 + ch * T::kChunkElems, (t / HALVES) * W, hc,
                             bar(C::kBarKFull + ks));
             }
@@ -280,9 +283,10 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
             if (!(ok = mbar_wait_warp(bar(C::kBarQEmpty), (n & 1) ^ 1, w, kSiteLoadQ))) break;
             if (elected) {
               const int nslots = (WIDE || second_tile(item)) ? 2 : 1;
-              mbar_arrive_expect_tx(bar(C::kBarQFull), nslots * T::kTileBytes);
+              mbar_arrive_expect_tx(bar(C::kBarQFull),
+                                    WIDE ? T::kTileBytes + kChunks1 * T::kChunkTileBytes : nslots * T::kTileBytes);
               for (int i = 0; i < nslots; ++i)
-                for (int ch = 0; ch < T::kChunks; ++ch)
+                for (int ch = 0; ch < (WIDE && i ? kChunks1 : T::kChunks); ++ch)
                   tma_load_4d(smem_base + C::kOffQ + i * T::kTileBytes + ch * T::kChunkTileBytes, &tq,
                               (WIDE ? i * 128 : 0) + ch * T::kChunkElems, (WIDE ? qt0 : qt0 + i) * 128, hc,
                               bar(C::kBarQFull));
@@ -294,10 +298,11 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
             if (tv_ == nsub - 1 && lane == 0) drawn = atomicAdd(work_counter, 1u);
             if (!(ok = mbar_wait_warp(bar(C::kBarVEmpty + vs), vph ^ 1, w, kSiteLoadV))) break;
             if (elected) {
-              mbar_arrive_expect_tx(bar(C::kBarVFull + vs), C::kKvBytes);
+              const int chunks = tv_ % HALVES ? kChunks1 : T::kChunks;
+              mbar_arrive_expect_tx(bar(C::kBarVFull + vs), C::kKvBytes / T::kChunks * chunks);
 #pragma unroll
               for (int ch = 0; ch < T::kChunks; ++ch)
-                tma_load_4d(smem_base + C::kOffV + vs * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tv,
+                if (ch < chunks) tma_load_4d(smem_base + C::kOffV + vs * C::kKvBytes + ch * (C::kKvBytes / T::kChunks), &tv,
                             (tv_ % HALVES) * 128 + ch * T::kChunkElems, (tv_ / HALVES) * W, hc,
                             bar(C::kBarVFull + vs));
             }
@@ -356,9 +361,11 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
               // S = Q_lo K_lo^T + Q_hi K_hi^T: the Q slots hold the halves, K arrives half by half
               for (int half = 0; ok && half < 2; ++half) {
                 if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
-                issue_rows_x_rows<DT, BF16, W, KT>(elected, tmem_base + C::kColS,
-                                            smem_base + C::kOffQ + half * T::kTileBytes,
-                                            smem_base + C::kOffK + ks * C::kKvBytes, half);
+                const uint32_t qa = smem_base + C::kOffQ + half * T::kTileBytes, ka = smem_base + C::kOffK + ks * C::kKvBytes;
+                if (KT1 == KT || half == 0)
+                  issue_rows_x_rows<DT, BF16, W, KT>(elected, tmem_base + C::kColS, qa, ka, half);
+                else
+                  issue_rows_x_rows<DT, BF16, W, KT1>(elected, tmem_base + C::kColS, qa, ka, 1u);
                 release_k();
               }
               if (!ok) break;
@@ -404,9 +411,11 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
               // O_lo += P V_lo, O_hi += P V_hi: the O0 / O1 columns hold the two halves of O
               for (int half = 0; ok && half < 2; ++half) {
                 if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
-                issue_tmem_x_tile<DT, BF16, W, KT>(elected, tmem_base + C::kColO + half * DT,
-                                            tmem_base + C::kColP, W / 4,
-                                            smem_base + C::kOffV + vs * C::kKvBytes, j > 0);
+                const uint32_t o = tmem_base + C::kColO + half * DT, va = smem_base + C::kOffV + vs * C::kKvBytes;
+                if (KT1 == KT || half == 0)
+                  issue_tmem_x_tile<DT, BF16, W, KT>(elected, o, tmem_base + C::kColP, W / 4, va, j > 0);
+                else
+                  issue_tmem_x_tile<DT, BF16, W, KT1>(elected, o, tmem_base + C::kColP, W / 4, va, j > 0);
                 release_v();
               }
               if (!ok) break;
@@ -637,6 +646,9 @@ cudaError_t launch_fwd(const AttnShape& s, int kv_rows, const CUtensorMap& tq, c
   if (s.D == 128 && s.Dg <= kShortDim128)
     return s.dtype ? launch_fwd_t<128, true, kShortDim128>(s, tq, tk, tv, to, o32, lse, ctx, stream)
                    : launch_fwd_t<128, false, kShortDim128>(s, tq, tk, tv, to, o32, lse, ctx, stream);
+  if (s.D == 256 && s.Dg <= kShortDim256)
+    return s.dtype ? launch_fwd_t<256, true, kShortDim256>(s, tq, tk, tv, to, o32, lse, ctx, stream)
+                   : launch_fwd_t<256, false, kShortDim256>(s, tq, tk, tv, to, o32, lse, ctx, stream);
   switch (s.D) {
     FA2_CASE(32)
     FA2_CASE(64)

@@ -21,6 +21,10 @@ namespace fa2 {
 // columns of an accumulator (KD below: the columns the products run over).  Same results, and
 // [32,20,1024,96] fp16: backward 768 -> 740 us, forward 257 -> 247 us.
 constexpr int kShortDim128 = 96;
+// The same for head dims of 136 to 192: three of four 64-column chunks, the fourth is neither loaded nor multiplied.
+// Same bits.  Forward and backward, us: [4,16,2000,192] bf16 579 -> 513, [2,8,8192,160] 1 745 -> 1 486; forward
+// [1,16,4096,192] 117.7 -> 105.0.
+constexpr int kShortDim256 = 192;
 
 // 64-bit shared-memory descriptor from its two words.
 __device__ __forceinline__ uint64_t desc_from_words(uint32_t lo, uint32_t hi) {
@@ -102,12 +106,12 @@ __device__ __forceinline__ void issue_tileT_x_tile(uint32_t elected, uint32_t d_
 // 2048 bytes apart along the columns.
 constexpr uint32_t kPiecesT_Lbo = 128;   // stride between core matrices along the reduction (K) index
 constexpr uint32_t kPiecesT_Sbo = 2048;  // stride between core matrices along the M index
-template <int D, bool BF16>
+template <int D, bool BF16, int KD = D>
 __device__ __forceinline__ void issue_piecesT_x_tile(uint32_t elected, uint32_t d_tmem,
                                                      uint32_t a_addr, uint32_t b_addr,
                                                      uint32_t accumulate) {
   using T = Tile<D>;
-  constexpr uint32_t idesc = make_idesc_ab(128, D, kInterBF16<BF16>, BF16, true, true);
+  constexpr uint32_t idesc = make_idesc_ab(128, KD, kInterBF16<BF16>, BF16, true, true);
   constexpr uint32_t a_hi = desc_hi_word(kPiecesT_Sbo, 0u);  // no swizzle
   constexpr uint32_t b_hi = desc_hi_word(T::kAtomBytes, T::kSwizzleMode);
   const uint32_t a_lo = desc_lo_word(a_addr, kPiecesT_Lbo), b_lo = desc_lo_word(b_addr, T::kChunkTileBytes);
@@ -125,12 +129,12 @@ __device__ __forceinline__ void issue_piecesT_x_tile(uint32_t elected, uint32_t 
 // B a staged [128, D] tile (MN-major).
 constexpr uint32_t kPieces_Lbo = 2048;  // stride between core matrices along the reduction (K) index
 constexpr uint32_t kPieces_Sbo = 128;   // stride between core matrices along the M index
-template <int D, bool BF16>
+template <int D, bool BF16, int KD = D>
 __device__ __forceinline__ void issue_pieces_x_tile(uint32_t elected, uint32_t d_tmem,
                                                     uint32_t a_addr, uint32_t b_addr,
                                                     uint32_t accumulate) {
   using T = Tile<D>;
-  constexpr uint32_t idesc = make_idesc_ab(128, D, kInterBF16<BF16>, BF16, false, true);
+  constexpr uint32_t idesc = make_idesc_ab(128, KD, kInterBF16<BF16>, BF16, false, true);
   constexpr uint32_t a_hi = desc_hi_word(kPieces_Sbo, 0u);  // no swizzle
   constexpr uint32_t b_hi = desc_hi_word(T::kAtomBytes, T::kSwizzleMode);
   const uint32_t a_lo = desc_lo_word(a_addr, kPieces_Lbo), b_lo = desc_lo_word(b_addr, T::kChunkTileBytes);
@@ -163,11 +167,11 @@ __device__ __forceinline__ void issue_piecesT_half_x_half_tile(uint32_t elected,
 // Half of either product above: the four 16-row reduction steps of half `half` of the piece-major tile,
 // against a staged [64, D] half tile of the operand.  TRANSPOSED selects issue_piecesT_x_tile's use
 // of A.
-template <int D, bool BF16, bool TRANSPOSED>
+template <int D, bool BF16, bool TRANSPOSED, int KD = D>
 __device__ __forceinline__ void issue_pieces_x_half_tile(uint32_t elected, uint32_t d_tmem, uint32_t a_addr,
                                                          int half, uint32_t b_addr, uint32_t accumulate) {
   using T = Tile<D>;
-  constexpr uint32_t idesc = make_idesc_ab(128, D, kInterBF16<BF16>, BF16, TRANSPOSED, true);
+  constexpr uint32_t idesc = make_idesc_ab(128, KD, kInterBF16<BF16>, BF16, TRANSPOSED, true);
   constexpr uint32_t a_hi = desc_hi_word(TRANSPOSED ? kPiecesT_Sbo : kPieces_Sbo, 0u);
   constexpr uint32_t b_hi = desc_hi_word(T::kAtomBytes, T::kSwizzleMode);
   constexpr uint32_t kStep = TRANSPOSED ? 256 : 4096;  // bytes of A per reduction step

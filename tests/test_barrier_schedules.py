@@ -90,3 +90,9 @@ def test_forward_roles_single_tile_items_one_after_the_other(simulator, headdim,
                                             ("consume_pair", 256)])
 def test_spill_roles(simulator, kernel, headdim, rows, keys):
     check(simulator, kernel, headdim, rows, keys)
+
+
+@pytest.mark.parametrize("kernel", ["scores", "consume", "consume_pair", "fwd"])
+def test_roles_of_three_chunk_heads(simulator, kernel):
+    check(simulator, kernel, 192, 449, 300)
+    check(simulator, kernel, 192, 640, 640)
