@@ -26,8 +26,8 @@
 // polynomial on the FMA pipe takes five times the instructions.  With 3 of 8 pairs in the polynomial against
 // none, passes in a loop, microseconds: [2,32,8192,128] bf16 974 -> 921, [1,32,4096,128] 138 -> 129.5,
 // [32,20,1024,96] fp16 223 -> 212, [2,16,8192,256] bf16 974 -> 926, [2,16,8192,64] fp16 373 -> 361.  At
-// head dim 32, where the products are shortest, 2 of 8 pairs measured best: [8,12,4095,32] 258 / 259 / 265
-// with 3, 2 and none.
+// head dim 32, where the products are shortest, 3 of 8 pairs measure best, with 3 / 2 / none: [8,12,4095,32] fp16
+// 258 / 259 / 267, [2,16,8192,32] 321 / 325 / 342, [1,2,32768,32] 343 / 350 / 384, [4,16,2048,32] 53.4 / 53.5 / 54.0.
 //
 // Head dims up to 64, rows up to fwd_kv_rows' line: the MMAs of a tile are short (512 cycles or less per 128 x 128 scores) and the
 // softmax instruction stream is what takes the time; with two softmax warps per scheduler it issues
@@ -52,7 +52,7 @@ struct FwdCfg {
   using T = Tile<D>;
   static constexpr int kW = W;  // rows of a KV tile = columns of a score tile
   static_assert(W == 128 || (W == 64 && D <= 64), "fwd_kv_rows");
-  static constexpr int kPolyShare = kW == 128 && D == 32 ? 2 : 0;  // of every 8 column pairs, this many use ex2_poly2
+  static constexpr int kPolyShare = kW == 128 && D == 32 ? 3 : 0;  // of every 8 column pairs, this many use ex2_poly2
   static constexpr int kCtasPerSm = kW == 64 ? 2 : 1;
   // O is rescaled when the running maximum has moved by more than this (log2 units).  A row's
   // largest P is exactly 1, without rounding error, when its maximum is fresh: 64-row tiles, whose

@@ -1081,3 +1081,22 @@ def test_preprocess_reads_rows_apart_from_each_other(d, rows):
         code, got, used = host.preprocess(a, b, lse)
         assert code == 0 and used.data_ptr() == b.data_ptr() and torch.equal(got, want)
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("d,rows,pairs", [(32, 1152, 3), (32, 1024, 0), (64, 1152, 0), (128, 1152, 0), (256, 1152, 0)])
+def test_forward_columns_of_the_polynomial(d, rows, pairs):
+    """Which of 8 column pairs take the polynomial (3 at head dim 32 with 128-row KV tiles).  Key 0 has score 1, the others 0,
+    the scale is ln 2: every other key's weight is 2^-1, where the polynomial gives 0.99992806 / 2.  lse carries the sum
+    in fp32: exact to 2 ulps of a logarithm below 4 (5e-7) times a sum of at most 9, against a difference of 3.6e-5."""
+    from flash_attention_triton_b200 import api
+
+    q = torch.zeros(1, 1, rows, d, device=DEV, dtype=torch.float16)
+    q[..., 0] = 1
+    k = torch.zeros_like(q)
+    k[:, :, 0, 0] = 1
+    lse = api._flash_attention_forward(q, k, torch.randn_like(q), math.log(2.0))[1][0, 0, :16].double().cpu()
+    sums = torch.exp(lse - math.log(2.0))
+    weights = torch.diff(sums, prepend=torch.zeros(1, dtype=torch.float64))
+    weights[1:] *= 2
+    polynomial = (weights < 1 - 1.8e-5 * torch.tensor([1.0] + [2.0] * 15)).tolist()
+    assert polynomial == [column // 2 < pairs for column in range(16)]
