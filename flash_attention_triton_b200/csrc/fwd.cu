@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
         // K runs one KV tile ahead of V: S(j+1) is issued during KV step j.  Ring entries are
         // staged tiles: entry t holds columns (t % HALVES) * 128 .. of KV tile t / HALVES.
         const int nsub = nkv * HALVES;
+        bool asked = false;  // the next item's number has been drawn
         for (int t = 0; ok && t < nsub + HALVES; ++t) {
           if (t < nsub) {
             if (!(ok = mbar_wait_warp(bar(C::kBarKEmpty + ks), kph ^ 1, w, kSiteLoadK))) break;
@@ -295,7 +296,10 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
           if (t >= HALVES) {
             const int tv_ = t - HALVES;
             // the number of the next item is on its way while the last V tile waits for its stage
-            if (tv_ == nsub - 1 && lane == 0) drawn = atomicAdd(work_counter, 1u);
+            if (tv_ == nsub - 1) {
+              asked = true;
+              if (lane == 0) drawn = atomicAdd(work_counter, 1u);
+            }
             if (!(ok = mbar_wait_warp(bar(C::kBarVEmpty + vs), vph ^ 1, w, kSiteLoadV))) break;
             if (elected) {
               const int chunks = tv_ % HALVES ? kChunks1 : T::kChunks;
@@ -310,9 +314,9 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
             if (tv_ == nsub - 1) break;
           }
         }
-        // A CTA that gives up goes on drawing, so that the counter is left at zero.
+        // A CTA that gives up goes on drawing, once an item, so that the counter is left at zero.
         if (lane == 0) {
-          if (!ok) drawn = atomicAdd(work_counter, 1u);
+          if (!asked) drawn = atomicAdd(work_counter, 1u);
           if (drawn == static_cast<unsigned>(total_items) - 1u) atomicExch(work_counter, 0u);
           *next_slot = static_cast<int>(drawn + gridDim.x);
         }

@@ -4,7 +4,8 @@
 // fails when nothing can go on (deadlock), when a warp arrives twice in one phase of a barrier (it has
 // stood in for another one), when a wait returns on a phase its warp has already seen, or when a warp
 // starts a copy from global memory before it has waited for the kernel before its own.  One CTA runs at a
-// time, one lane of each warp; data does not exist.
+// time, one lane of each warp; data does not exist.  With `giveup` one wait of a launch, drawn at random, runs into
+// its time limit: the CTA must come to its end and leave the forward's work counter at zero.
 #include "cuda_runtime.h"
 #include <ucontext.h>
 #include <unistd.h>
@@ -42,6 +43,9 @@ std::vector<Warp> warps;
 ucontext_t scheduler;
 int current;
 std::mt19937 rng;
+long waits, give_up = -1;  // waits of the launch so far; the one that runs into its limit
+volatile int* abort_flag;  // of the CTA, once a warp has waited
+bool aborted() { return abort_flag && *abort_flag; }
 
 [[noreturn]] void fail(const char* what, uint32_t bar, int warp, int site) {
   printf("%s: block %u, hardware warp %d, barrier +%u, wait site %d\n", what, blockIdx.x, warp, bar, site);
@@ -50,7 +54,7 @@ std::mt19937 rng;
 }
 void arrive(Arrival a) {
   Barrier& b = barriers[a.bar];
-  if (!b.arrived.insert(a.warp).second) fail("second arrival in one phase", a.bar, a.warp, -1);
+  if (!b.arrived.insert(a.warp).second && !aborted()) fail("second arrival in one phase", a.bar, a.warp, -1);
   if (--b.pending == 0) b.pending = b.count, ++b.completed, b.arrived.clear();
 }
 bool passes(uint32_t bar, uint32_t parity) { return (barriers[bar].completed & 1u) != parity; }
@@ -68,15 +72,19 @@ void sim_init(uint32_t bar, uint32_t count) { barriers[bar] = Barrier{count, cou
 void sim_arrive(uint32_t bar) { yield(); arrive({bar, current}); }
 void sim_arrive_later(uint32_t bar) { yield(); copies.push_back({bar, current}); }
 void sim_arrive_after_mma(uint32_t bar) { yield(); pipe_queue.push_back({bar, current}); }
-void sim_wait(uint32_t bar, uint32_t parity, int site) {
+bool sim_wait(uint32_t bar, uint32_t parity, int site, volatile int* flag) {
   Warp& w = warps[current];
+  abort_flag = flag;
+  if (waits++ == give_up) return *flag = 1, false;
   w.bar = bar, w.parity = parity, w.site = site;
-  yield();  // resumed only when the wait passes
+  yield();  // resumed only when the wait passes, or when the CTA gives up
   w.site = -1;
+  if (aborted()) return passes(bar, parity);
   Barrier& b = barriers[bar];
   unsigned& seen = b.seen[current];
   if (seen >= b.completed + 1) fail("wait returned on a phase already seen", bar, current, site);
   seen = b.completed + 1;
+  return true;
 }
 void sim_wait_previous() { warps[current].waited_previous = true; }
 void sim_access() {
@@ -89,6 +97,7 @@ void __syncthreads() {
 void sim_run(unsigned n, void (*body)(void*), void* arg) {
   body_fn = body, body_arg = arg;
   barriers.clear(), copies.clear(), pipe_queue.clear();
+  abort_flag = nullptr;
   warps = std::vector<Warp>(n);
   for (unsigned i = 0; i < n; ++i) {
     Warp& w = warps[i];
@@ -107,7 +116,7 @@ void sim_run(unsigned n, void (*body)(void*), void* arg) {
     unsigned done = 0, synced = 0;
     for (unsigned i = 0; i < n; ++i) {
       done += warps[i].done, synced += warps[i].at_sync;
-      if (!warps[i].done && !warps[i].at_sync && (warps[i].site < 0 || passes(warps[i].bar, warps[i].parity))) offer(i);
+      if (!warps[i].done && !warps[i].at_sync && (warps[i].site < 0 || aborted() || passes(warps[i].bar, warps[i].parity))) offer(i);
     }
     if (done == n) return;
     if (done + synced == n) {
@@ -139,7 +148,7 @@ void sim_run(unsigned n, void (*body)(void*), void* arg) {
 #include "bwd.cu"
 #include "fwd.cu"
 
-// main <kernel> <head dim> <rows> <keys> <schedules> <rows of a step> [<SMs>]
+// main <kernel> <head dim> <rows> <keys> <schedules> <rows of a step> [<SMs> [giveup]]
 int main(int argc, char** argv) {
   using namespace fa2;
   const std::string kernel = argv[1];
@@ -154,9 +163,8 @@ int main(int argc, char** argv) {
   unsigned counter = 0;
   LaunchCtx ctx{&status, &counter, 1};
   const int step = atoi(argv[6]);
-  for (int seed = 0; seed < atoi(argv[5]); ++seed) {
-    rng.seed(seed);
-    ctx.num_sms = argc > 7 ? atoi(argv[7]) : 1 + seed % 2 * 63;  // work items of two Q tiles and of one
+  auto launch = [&] {
+    waits = 0;
     if (kernel == "fwd") launch_fwd(s, step, m, m, m, m, none, lse.data(), ctx, nullptr);
     if (kernel == "dkdv") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, nullptr, 0, step, &status, nullptr);
     if (kernel == "dkdv_atomic") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 1, step, &status, nullptr);
@@ -167,6 +175,16 @@ int main(int argc, char** argv) {
       if (kernel == "consume" && (d > 128 || form == 2)) launch_bwd_consume(s, form, scratch.data(), m, m, none, rs, false, &status, nullptr);
       if (kernel == "consume_pair") launch_bwd_consume(s, form, scratch.data(), m, m, none, rs, true, &status, nullptr);
     }
+    if (counter) fail("work counter not left at zero", 0, -1, -1);
+  };
+  for (int seed = 0; seed < atoi(argv[5]); ++seed) {
+    rng.seed(seed);
+    ctx.num_sms = argc > 7 ? atoi(argv[7]) : 1 + seed % 2 * 63;  // work items of two Q tiles and of one
+    launch();
+    if (argc <= 8) continue;
+    give_up = rng() % waits;
+    launch();
+    give_up = -1;
   }
   return 0;
 }

@@ -96,3 +96,14 @@ def test_spill_roles(simulator, kernel, headdim, rows, keys):
 def test_roles_of_three_chunk_heads(simulator, kernel):
     check(simulator, kernel, 192, 449, 300)
     check(simulator, kernel, 192, 640, 640)
+
+
+@pytest.mark.parametrize("rows,keys", [(128, 64), (449, 300), (1200, 1200)])
+@pytest.mark.parametrize("headdim", [32, 64, 96, 128, 192, 256])
+def test_forward_that_gives_up_a_wait(simulator, headdim, rows, keys):
+    """Whichever wait runs into its limit, every CTA ends and the work counter is at zero for the next launch."""
+    for step in steps_of(headdim):
+        for sms in (1, 2, 3, 64):
+            run = subprocess.run([simulator, "fwd", str(headdim), str(rows), str(keys), "60", str(step), str(sms), "giveup"],
+                                 capture_output=True, text=True, timeout=300)
+            assert run.returncode == 0, (step, sms, run.stdout + run.stderr)
