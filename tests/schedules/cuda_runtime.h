@@ -52,7 +52,7 @@ void sim_arrive(uint32_t bar);
 void sim_arrive_later(uint32_t bar);      // a copy's bytes arrive at some later time
 void sim_arrive_after_mma(uint32_t bar);  // behind everything in the in-order tensor pipe
 void sim_init(uint32_t bar, uint32_t count);
-bool sim_wait(uint32_t bar, uint32_t parity, int site, volatile int* abort_flag);  // false: given up
+bool sim_wait(uint32_t bar, uint32_t parity, int site, volatile int* abort_flag, bool vote);  // false: given up
 void __syncthreads();
 void sim_wait_previous();
 void sim_access();  // of global memory: not before the kernel has waited for its predecessor
@@ -101,8 +101,8 @@ inline void mbar_inval(uint32_t) {}
 inline void mbar_arrive(uint32_t bar) { sim_arrive(bar); }
 inline void mbar_arrive_expect_tx(uint32_t bar, uint32_t) { sim_access(), sim_arrive_later(bar); }
 inline void mma_commit(uint32_t bar) { sim_arrive_after_mma(bar); }
-inline bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx& w, int site) { return sim_wait(bar, parity, site, w.abort_flag); }
-inline bool mbar_wait_warp(uint32_t bar, uint32_t parity, const WaitCtx& w, int site) { return sim_wait(bar, parity, site, w.abort_flag); }
+inline bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx& w, int site) { return sim_wait(bar, parity, site, w.abort_flag, false); }
+inline bool mbar_wait_warp(uint32_t bar, uint32_t parity, const WaitCtx& w, int site) { return sim_wait(bar, parity, site, w.abort_flag, true); }
 template <typename T> T ld_global(const T* p) { return sim_access(), *p; }
 inline void tmem_ld_x32(uint32_t, uint32_t* r) { memset(r, 0, 128); }
 inline void tmem_ld_x16(uint32_t, uint32_t* r) { memset(r, 0, 64); }

@@ -5,7 +5,9 @@
 // stood in for another one), when a wait returns on a phase its warp has already seen, or when a warp
 // starts a copy from global memory before it has waited for the kernel before its own.  One CTA runs at a
 // time, one lane of each warp; data does not exist.  With `giveup` one wait of a launch, drawn at random, runs into
-// its time limit: the CTA must come to its end and leave the forward's work counter at zero.
+// its time limit: the CTA must come to its end and leave the forward's work counter at zero.  The lanes of a warp may
+// part in a wait without a vote that returns while the CTA gives up (some have seen their barrier, others the
+// abort flag), so that warp must not vote again.
 #include "cuda_runtime.h"
 #include <ucontext.h>
 #include <unistd.h>
@@ -35,7 +37,7 @@ std::deque<Arrival> pipe_queue;
 struct Warp {
   ucontext_t ctx;
   std::unique_ptr<char[]> stack;
-  bool done = false, at_sync = false, waited_previous = false;
+  bool done = false, at_sync = false, waited_previous = false, parted = false;
   uint32_t bar = 0, parity = 0;
   int site = -1;  // >= 0: waiting
 };
@@ -72,14 +74,21 @@ void sim_init(uint32_t bar, uint32_t count) { barriers[bar] = Barrier{count, cou
 void sim_arrive(uint32_t bar) { yield(); arrive({bar, current}); }
 void sim_arrive_later(uint32_t bar) { yield(); copies.push_back({bar, current}); }
 void sim_arrive_after_mma(uint32_t bar) { yield(); pipe_queue.push_back({bar, current}); }
-bool sim_wait(uint32_t bar, uint32_t parity, int site, volatile int* flag) {
+bool sim_wait(uint32_t bar, uint32_t parity, int site, volatile int* flag, bool vote) {
   Warp& w = warps[current];
   abort_flag = flag;
-  if (waits++ == give_up) return *flag = 1, false;
+  if (vote && w.parted) fail("vote of a warp whose lanes may have parted", bar, current, site);
+  if (waits++ == give_up) {
+    *flag = 1, w.parted = !vote;
+    return false;
+  }
   w.bar = bar, w.parity = parity, w.site = site;
   yield();  // resumed only when the wait passes, or when the CTA gives up
   w.site = -1;
-  if (aborted()) return passes(bar, parity);
+  if (aborted()) {
+    w.parted |= !vote;
+    return passes(bar, parity);
+  }
   Barrier& b = barriers[bar];
   unsigned& seen = b.seen[current];
   if (seen >= b.completed + 1) fail("wait returned on a phase already seen", bar, current, site);

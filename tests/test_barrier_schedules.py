@@ -107,3 +107,14 @@ def test_forward_that_gives_up_a_wait(simulator, headdim, rows, keys):
             run = subprocess.run([simulator, "fwd", str(headdim), str(rows), str(keys), "60", str(step), str(sms), "giveup"],
                                  capture_output=True, text=True, timeout=300)
             assert run.returncode == 0, (step, sms, run.stdout + run.stderr)
+
+
+@pytest.mark.parametrize("kernel,headdim", [("dkdv", 64), ("dkdv", 128), ("dkdv_atomic", 32), ("dkdv_atomic", 128), ("dkdv_spill", 128),
+                                            ("dq", 64), ("dq", 128), ("scores", 192), ("scores", 256), ("consume", 128),
+                                            ("consume", 256), ("consume_pair", 256)])
+def test_backward_that_gives_up_a_wait(simulator, kernel, headdim):
+    for step in steps_of(headdim):
+        for rows, keys in ((128, 64), (640, 640)):
+            run = subprocess.run([simulator, kernel, str(headdim), str(rows), str(keys), "60", str(step), "1", "giveup"],
+                                 capture_output=True, text=True, timeout=300)
+            assert run.returncode == 0, (step, rows, run.stdout + run.stderr)
