@@ -150,10 +150,10 @@ inline int heads_per_group(const AttnShape& s) {
   return static_cast<int>(g < 1 ? 1 : (g > bh ? bh : g));
 }
 
-// Per-launch context of the forward kernel.  It runs one or two CTAs per SM; a CTA takes work item blockIdx.x
-// and then draws items (pairs of Q tiles) from `work_counter` until none are left, so tensor memory is
+// Per-launch context of the forward kernel.  It runs one or two CTAs per SM.  With more work items (Q tiles or pairs of
+// them) than CTAs, these draw items from `work_counter` until none are left, so tensor memory is
 // allocated once and no SM idles between items.  The counter is zero before the launch; a launch draws
-// total_items numbers in all (one with every item), and whoever draws the last one puts the counter back to zero,
+// total_items + gridDim.x numbers in all, and whoever draws the last one puts the counter back to zero,
 // so no memset sits between launches.
 struct LaunchCtx {
   int* status;                 // device status word (bounded-wait failures)

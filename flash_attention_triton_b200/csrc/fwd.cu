@@ -213,9 +213,13 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
   grid_wait_previous();
   grid_allow_next();
 
-  // One or two CTAs per SM.  A CTA starts with work item blockIdx.x and draws the others from a global counter,
-  // heaviest first within a group of heads (grouped_order).  The roles run through the items without
-  // meeting: the producer draws the next item while the last tiles of the one before are in
+  // One or two CTAs per SM.  A CTA draws its items from a global counter, heaviest first within a group of heads
+  // (grouped_order), unless there is one for each CTA.  The first one is drawn too: with item blockIdx.x to start with,
+  // a CTA that finds no SM at the launch, because another stream or a collective holds some, kept a heavy item
+  // for the end.  Beside a kernel on 4 / 20 SMs, microseconds, item blockIdx.x first against drawn: [1,2,32768,128] 507 -> 391 /
+  // 539 -> 387, [2,16,8192,64] 396 -> 341 / 433 -> 378, [4,16,2048,64] 75.8 -> 61.5 / 79.9 -> 65.5; alone 409 -> 411, 340 -> 343, 54.9 -> 55.4
+  // in a loop (the draw's latency).
+  // The roles run through the items without meeting: the producer draws the next item while the last tiles of the one before are in
   // flight, and loads its first K tile and, once the last score product has read Q, its Q tiles, so that
   // the next item's scores are formed while the softmax groups finish this one.  Every barrier keeps
   // its phase from item to item.  What bounds short rows is this boundary; with all roles meeting there it took
@@ -247,8 +251,24 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
       }
       bool ok = true;
       int ks = 0, kph = 0, vs = 0, vph = 0;  // ring positions
-      unsigned drawn = 0;
-      for (int n = 0, id = blockIdx.x;; ++n) {
+      unsigned drawn = blockIdx.x;  // an item, or beyond total_items
+      const bool draws = total_items > static_cast<int>(gridDim.x);
+      auto draw = [&]() {
+        if (lane == 0) drawn = draws ? atomicAdd(work_counter, 1u) : total_items;
+      };
+      auto drawn_item = [&]() {  // the number drawn, for the whole warp
+        if (lane == 0) {
+          if (draws && drawn == total_items + gridDim.x - 1u) atomicExch(work_counter, 0u);
+          *next_slot = static_cast<int>(drawn);
+        }
+        __syncwarp();
+        const int id = *next_slot;
+        __syncwarp();
+        return id;
+      };
+      if (draws) draw();
+      for (int n = 0;; ++n) {
+        const int id = drawn_item();
         WorkItem item{-1, 0, 0, 0};
         if (id < total_items) {
           const HeadTile ht = grouped_order(id, num_bh, npairs, group);
@@ -300,7 +320,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
             // the number of the next item is on its way while the last V tile waits for its stage
             if (tv_ == nsub - 1) {
               asked = true;
-              if (lane == 0) drawn = atomicAdd(work_counter, 1u);
+              draw();
             }
             if (!(ok = mbar_wait_warp(bar(C::kBarVEmpty + vs), vph ^ 1, w, kSiteLoadV))) break;
             if (elected) {
@@ -316,15 +336,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
             if (tv_ == nsub - 1) break;
           }
         }
-        // A CTA that gives up goes on drawing, once an item, so that the counter is left at zero.
-        if (lane == 0) {
-          if (!asked) drawn = atomicAdd(work_counter, 1u);
-          if (drawn == static_cast<unsigned>(total_items) - 1u) atomicExch(work_counter, 0u);
-          *next_slot = static_cast<int>(drawn + gridDim.x);
-        }
-        __syncwarp();
-        id = *next_slot;
-        __syncwarp();
+        if (!asked) draw();  // a CTA that gives up goes on drawing, once an item, so that the counter is left at zero
       }
     } else if (warp == 8) {
       // ---------------------------------------------------------------- S = Q_i K_j^T issuer

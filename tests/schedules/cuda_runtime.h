@@ -56,6 +56,7 @@ bool sim_wait(uint32_t bar, uint32_t parity, int site, volatile int* abort_flag,
 void __syncthreads();
 void sim_wait_previous();
 void sim_access();  // of global memory: not before the kernel has waited for its predecessor
+void sim_stored(int row);  // of an output
 void sim_run(unsigned warps, void (*body)(void*), void* arg);
 
 template <typename... Params, typename... Args>
@@ -113,11 +114,12 @@ inline float lg2(float) { return 0; }
 inline float max3(float, float, float) { return 0; }
 #define FA2_NOTHING(name) template <typename... A> void name(A&&...) {}
 FA2_NOTHING(fence_mbar_init) FA2_NOTHING(fence_proxy_async_smem) FA2_NOTHING(tma_load_4d) FA2_NOTHING(bulk_load_1d)
-FA2_NOTHING(tma_store_4d) FA2_NOTHING(tma_store_commit) FA2_NOTHING(tma_store_wait_all) FA2_NOTHING(tma_store_wait_read)
+FA2_NOTHING(tma_store_commit) FA2_NOTHING(tma_store_wait_all) FA2_NOTHING(tma_store_wait_read)
 FA2_NOTHING(prefetch_tensormap) FA2_NOTHING(tmem_alloc) FA2_NOTHING(tmem_relinquish) FA2_NOTHING(tmem_dealloc)
 FA2_NOTHING(tc_fence_before) FA2_NOTHING(tc_fence_after) FA2_NOTHING(tmem_wait_ld) FA2_NOTHING(tmem_wait_st)
 FA2_NOTHING(tmem_st_x32) FA2_NOTHING(tmem_st_x16) FA2_NOTHING(mma_ss) FA2_NOTHING(mma_ts) FA2_NOTHING(st_global_8)
 FA2_NOTHING(grid_allow_next)
+inline void tma_store_4d(const CUtensorMap*, int, int row, HeadCoord, uint32_t) { sim_stored(row); }
 inline void grid_wait_previous() { sim_wait_previous(); }
 template <int N> void reg_inc() {}
 template <int N> void reg_dec() {}

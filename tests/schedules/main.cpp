@@ -47,6 +47,7 @@ int current;
 std::mt19937 rng;
 long waits, give_up = -1;  // waits of the launch so far; the one that runs into its limit
 volatile int* abort_flag;  // of the CTA, once a warp has waited
+std::vector<int> stored;  // first rows of the output boxes of the launch, in the order of their stores
 bool aborted() { return abort_flag && *abort_flag; }
 
 [[noreturn]] void fail(const char* what, uint32_t bar, int warp, int site) {
@@ -99,6 +100,7 @@ void sim_wait_previous() { warps[current].waited_previous = true; }
 void sim_access() {
   if (!warps[current].waited_previous) fail("access before the wait for the previous kernel", 0, current, -1);
 }
+void sim_stored(int row) { stored.push_back(row); }
 void __syncthreads() {
   warps[current].at_sync = true;
   yield();
@@ -157,7 +159,7 @@ void sim_run(unsigned n, void (*body)(void*), void* arg) {
 #include "bwd.cu"
 #include "fwd.cu"
 
-// main <kernel> <head dim> <rows> <keys> <schedules> <rows of a step> [<SMs> [giveup]]
+// main <kernel> <head dim> <rows> <keys> <schedules> <rows of a step> [<SMs> [giveup | order]]
 int main(int argc, char** argv) {
   using namespace fa2;
   const std::string kernel = argv[1];
@@ -173,7 +175,7 @@ int main(int argc, char** argv) {
   LaunchCtx ctx{&status, &counter, 1};
   const int step = atoi(argv[6]);
   auto launch = [&] {
-    waits = 0;
+    waits = 0, stored.clear();
     if (kernel == "fwd") launch_fwd(s, step, m, m, m, m, none, lse.data(), ctx, nullptr);
     if (kernel == "dkdv") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, nullptr, 0, step, &status, nullptr);
     if (kernel == "dkdv_atomic") launch_bwd_dkdv(s, m, m, m, m, m, m, none, none, rs, scratch.data(), 1, step, &status, nullptr);
@@ -191,6 +193,11 @@ int main(int argc, char** argv) {
     ctx.num_sms = argc > 7 ? atoi(argv[7]) : 1 + seed % 2 * 63;  // work items of two Q tiles and of one
     launch();
     if (argc <= 8) continue;
+    if (argv[8] == std::string("order")) {
+      for (int row : stored) printf("%d ", row);
+      puts("");
+      continue;
+    }
     give_up = rng() % waits;
     launch();
     give_up = -1;

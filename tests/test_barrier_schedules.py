@@ -118,3 +118,15 @@ def test_backward_that_gives_up_a_wait(simulator, kernel, headdim):
             run = subprocess.run([simulator, kernel, str(headdim), str(rows), str(keys), "60", str(step), "1", "giveup"],
                                  capture_output=True, text=True, timeout=300)
             assert run.returncode == 0, (step, rows, run.stdout + run.stderr)
+
+
+@pytest.mark.parametrize("headdim,step", [(64, 64), (64, 128), (128, 128), (256, 128)])
+@pytest.mark.parametrize("sms", [2, 5, 64])
+def test_forward_items_go_heaviest_first_to_whichever_cta_runs(simulator, headdim, step, sms):
+    """The simulator runs CTAs one after the other, like CTAs of a launch that find an SM late: none of them may have
+    kept an item heavier than those that others have done by then."""
+    run = subprocess.run([simulator, "fwd", str(headdim), "2900", "2900", "20", str(step), str(sms), "order"],
+                         capture_output=True, text=True, timeout=300, check=True)
+    for line in run.stdout.splitlines():
+        items = list(dict.fromkeys(int(row) // 256 for row in line.split()))  # pairs of Q tiles, at their first store
+        assert items == sorted(items, reverse=True) and len(items) == 12
