@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
   // (grouped_order), unless there is one for each CTA.  The first one is drawn too: with item blockIdx.x to start with,
   // a CTA that finds no SM at the launch, because another stream or a collective holds some, kept a heavy item
   // for the end.  Beside a kernel on 4 / 20 SMs, microseconds, item blockIdx.x first against drawn: [1,2,32768,128] 507 -> 391 /
-  // 539 -> 387, [2,16,8192,64] 396 -> 341 / 433 -> 378, [4,16,2048,64] 75.8 -> 61.5 / 79.9 -> 65.5; alone 409 -> 411, 340 -> 343, 54.9 -> 55.4
+  // 539 -> 387, [2,16,8192,64] 396 -> 341 / 433 -> 378, [4,16,2048,64] 75.8 -> 61.5 / 79.9 -> 65.5; alone 409 -> 411, 340 -> 343, 54.0 -> 54.5
   // in a loop (the draw's latency).
   // The roles run through the items without meeting: the producer draws the next item while the last tiles of the one before are in
   // flight, and loads its first K tile and, once the last score product has read Q, its Q tiles, so that
@@ -228,8 +228,9 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
   // 258, [4,16,1000,64] bf16 25.7 -> 23.9, [2,32,8192,128] bf16 973 -> 974, [1,2,32768,128] 463 -> 471.
   //
   // Slot of the n-th item of this CTA, for every role but the producer; false: there is none, or the CTA gives up.
-  // It votes, and so does every other wait here: lanes that left a wait apart, some for the abort flag, would wait for
-  // each other in the next vote.
+  // It votes.  The MMA warps' other waits do not (a vote in each: [8,16,1000,64] 35.4 -> 36.1 us, [4,16,2048,64] 54.5 -> 55.4), so
+  // their lanes may leave one apart when the CTA gives up, some for the abort flag; they meet in a vote at the
+  // end of the item, which every lane reaches.
   auto take_item = [&](int n, WorkItem& item) {
     if (!mbar_wait_warp(bar(C::kBarItemFull + (n & 1)), (n >> 1) & 1, w, kSiteItem)) return false;
     item = reinterpret_cast<const WorkItem*>(smem + C::kOffItems)[n & 1];
@@ -362,23 +363,23 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
       WorkItem item;
       for (int n = 0; ok && take_item(n, item); ++n) {
         const int n0 = kv_tiles(item, 0), n1 = kv_tiles(item, 1), nkv = max(n0, n1);
-        if (!(ok = mbar_wait_warp(bar(C::kBarQFull), n & 1, w, kSiteMmaQ))) break;
+        ok = mbar_wait(bar(C::kBarQFull), n & 1, w, kSiteMmaQ);
         for (int j = 0; ok && j < nkv; ++j) {
           if constexpr (!WIDE) {
-            if (!(ok = mbar_wait_warp(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
+            if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
           }
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             if (j >= (i == 0 ? n0 : n1)) continue;
             if (prev_i >= 0) {
-              if (!(ok = mbar_wait_warp(bar(C::kBarSFree + prev_i), prev_ph, w, kSiteMmaSFree))) break;
+              if (!(ok = mbar_wait(bar(C::kBarSFree + prev_i), prev_ph, w, kSiteMmaSFree))) break;
               tc_fence_after();
             }
             const bool last_of_tile = i == 1 || n1 == 0;
             if constexpr (WIDE) {
               // S = Q_lo K_lo^T + Q_hi K_hi^T: the Q slots hold the halves, K arrives half by half
               for (int half = 0; ok && half < 2; ++half) {
-                if (!(ok = mbar_wait_warp(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
+                if (!(ok = mbar_wait(bar(C::kBarKFull + ks), kph, w, kSiteMmaK))) break;
                 const uint32_t qa = smem_base + C::kOffQ + half * T::kTileBytes, ka = smem_base + C::kOffK + ks * C::kKvBytes;
                 if (KT1 == KT || half == 0)
                   issue_rows_x_rows<DT, BF16, W, KT>(elected, tmem_base + C::kColS, qa, ka, half);
@@ -399,6 +400,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
             prev_ph = count[i]++ & 1;
           }
         }
+        ok = __all_sync(0xffffffffu, ok);  // see take_item
       }
     } else if (warp == 10) {
       // ---------------------------------------------------------------- O_i += P_i V_j issuer
@@ -418,17 +420,17 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
         const int n0 = kv_tiles(item, 0), n1 = kv_tiles(item, 1), nkv = max(n0, n1);
         for (int j = 0; ok && j < nkv; ++j) {
           if constexpr (!WIDE) {
-            if (!(ok = mbar_wait_warp(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
+            if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
           }
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             if (j >= (i == 0 ? n0 : n1)) continue;
-            if (!(ok = mbar_wait_warp(bar(C::kBarPFull + i), count[i]++ & 1, w, kSiteMmaP))) break;
+            if (!(ok = mbar_wait(bar(C::kBarPFull + i), count[i]++ & 1, w, kSiteMmaP))) break;
             tc_fence_after();
             if constexpr (WIDE) {
               // O_lo += P V_lo, O_hi += P V_hi: the O0 / O1 columns hold the two halves of O
               for (int half = 0; ok && half < 2; ++half) {
-                if (!(ok = mbar_wait_warp(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
+                if (!(ok = mbar_wait(bar(C::kBarVFull + vs), vph, w, kSiteMmaV))) break;
                 const uint32_t o = tmem_base + C::kColO + half * DT, va = smem_base + C::kOffV + vs * C::kKvBytes;
                 if (KT1 == KT || half == 0)
                   issue_tmem_x_tile<DT, BF16, W, KT>(elected, o, tmem_base + C::kColP, W / 4, va, j > 0);
@@ -446,6 +448,7 @@ __global__ void __launch_bounds__(kFwdThreads, FwdCfg<D == 256 ? 128 : D, W>::kC
             commit(C::kBarPvDone + i);
           }
         }
+        ok = __all_sync(0xffffffffu, ok);
       }
     }
     __syncwarp();

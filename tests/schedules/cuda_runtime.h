@@ -71,6 +71,8 @@ cudaError_t cudaLaunchKernelEx(const cudaLaunchConfig_t* cfg, void (*kernel)(Par
 }
 
 inline void __syncwarp() {}
+bool sim_meet(bool x);  // false, too, when a lane may have left with false
+inline bool __all_sync(unsigned, bool x) { return sim_meet(x); }
 inline bool __any_sync(unsigned, bool x) { return x; }
 inline unsigned __reduce_max_sync(unsigned, unsigned x) { return x; }
 template <typename T> T atomicAdd(T* p, T v) { T old = *p; *p += v; return old; }

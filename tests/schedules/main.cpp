@@ -7,7 +7,7 @@
 // time, one lane of each warp; data does not exist.  With `giveup` one wait of a launch, drawn at random, runs into
 // its time limit: the CTA must come to its end and leave the forward's work counter at zero.  The lanes of a warp may
 // part in a wait without a vote that returns while the CTA gives up (some have seen their barrier, others the
-// abort flag), so that warp must not vote again.
+// abort flag), so that warp must not wait with a vote before all of its lanes have met.
 #include "cuda_runtime.h"
 #include <ucontext.h>
 #include <unistd.h>
@@ -99,6 +99,11 @@ bool sim_wait(uint32_t bar, uint32_t parity, int site, volatile int* flag, bool 
 void sim_wait_previous() { warps[current].waited_previous = true; }
 void sim_access() {
   if (!warps[current].waited_previous) fail("access before the wait for the previous kernel", 0, current, -1);
+}
+bool sim_meet(bool x) {
+  const bool parted = warps[current].parted;
+  warps[current].parted = false;
+  return x && !parted;
 }
 void sim_stored(int row) { stored.push_back(row); }
 void __syncthreads() {
