@@ -206,7 +206,7 @@ PyObject* backward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 constexpr const char* kApiModule = "flash_attention_triton_b200.api";
 constexpr const char* kLibModule = "flash_attention_triton_b200._lib";
 
-// Environment switches that api.py serves.
+// Environment switches that api.py serves.  Called with the interpreter lock, under which os.environ changes them.
 bool python_path_asked() {
   const char* check = std::getenv("FA2_B200_CHECK_STATUS");
   const char* mode = std::getenv("FA2_B200_BWD_MODE");
@@ -265,6 +265,23 @@ at::Tensor allocate_workspace(const at::Tensor& q, int& mode) {
   }
 }
 
+// Saved-tensor hooks must give back what was saved.  False for what _flash_attention_backward of api.py asserts.
+bool as_saved(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& output, const at::Tensor& lse,
+              const at::Tensor& d_output) {
+  TORCH_CHECK(q.dim() == 4 && k.dim() == 4, "the saved q, k and v must be [B, H, N, D] tensors");
+  if (lse.sizes() != q.sizes().slice(0, 3) || !output.is_contiguous() ||
+      (q.scalar_type() != at::kHalf && q.scalar_type() != at::kBFloat16))
+    return false;
+  TORCH_CHECK(k.size(0) == q.size(0) && k.size(1) == q.size(1) && k.size(3) == q.size(3) && k.size(2) <= q.size(2) &&
+                  v.sizes() == k.sizes() && output.sizes() == q.sizes() && d_output.sizes() == q.sizes(),
+              "the saved tensors have changed their shapes");
+  for (const at::Tensor* t : {&k, &v, &output, &lse, &d_output})
+    TORCH_CHECK(t->device() == q.device() && t->scalar_type() == (t == &lse ? at::kFloat : q.scalar_type()),
+                "the saved tensors have changed their type or device");
+  TORCH_CHECK(q.is_cuda() && lse.is_contiguous(), "the saved tensors have changed their device or strides");
+  return true;
+}
+
 struct Attention : torch::autograd::Function<Attention> {
   // `r` holds the outputs of the forward kernel, already launched on saved_q, saved_k and saved_v.
   static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor&, const at::Tensor&,
@@ -284,10 +301,15 @@ struct Attention : torch::autograd::Function<Attention> {
     const at::Tensor &q = saved[0], &k = saved[1], &v = saved[2], &output = saved[3], &lse = saved[4];
     const double scale = ctx->saved_data["scale"].toDouble();
     const bool deterministic = ctx->saved_data["deterministic"].toBool(), f32 = ctx->saved_data["f32"].toBool();
-    at::Tensor dq = empty_gradient(q, f32), dk = empty_gradient(k, f32), dv = empty_gradient(v, f32);
     at::Tensor d_output = grads[0];
     if (d_output.scalar_type() != q.scalar_type()) d_output = d_output.to(q.scalar_type());
-    if (python_path_asked()) {
+    bool python = !as_saved(q, k, v, output, lse, d_output);
+    if (!python) {
+      pybind11::gil_scoped_acquire gil;
+      python = python_path_asked();
+    }
+    at::Tensor dq = empty_gradient(q, f32), dk = empty_gradient(k, f32), dv = empty_gradient(v, f32);
+    if (python) {
       pybind11::gil_scoped_acquire gil;
       try {
         pybind11::module_::import(kApiModule)

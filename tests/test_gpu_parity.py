@@ -1100,3 +1100,26 @@ def test_forward_columns_of_the_polynomial(d, rows, pairs):
     weights[1:] *= 2
     polynomial = (weights < 1 - 1.8e-5 * torch.tensor([1.0] + [2.0] * 15)).tolist()
     assert polynomial == [column // 2 < pairs for column in range(16)]
+
+
+@pytest.mark.parametrize("index,change,error", [
+    (4, lambda t: t[..., :-1].contiguous(), AssertionError), (4, lambda t: t.half(), RuntimeError),
+    (4, lambda t: t.mT.contiguous().mT, RuntimeError), (3, lambda t: t.mT.contiguous().mT, AssertionError),
+    (3, lambda t: t[:, :, :-1].contiguous(), RuntimeError), (0, lambda t: t.float(), AssertionError),
+    (1, lambda t: t.bfloat16(), RuntimeError), (2, lambda t: t[..., :32].contiguous(), RuntimeError), (1, lambda t: t.cpu(), RuntimeError),
+    (1, lambda t: t[0], RuntimeError)])
+def test_native_backward_refuses_saved_tensors_that_changed(index, change, error):
+    """Saved-tensor hooks that give back another shape, type, device or order than what was saved."""
+    q, k, v, do = (torch.randn(1, 2, 200, 64, device=DEV, dtype=torch.float16) for _ in range(4))
+    q.requires_grad_(True)
+    unpacked = []
+
+    def unpack(t):
+        unpacked.append(t)
+        return change(t) if len(unpacked) == index + 1 else t
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), unpack):
+        out = flash_attention_v2(q, k, v)
+    with pytest.raises(error):
+        torch.autograd.grad(out, q, do)
+    assert len(unpacked) == 5
