@@ -79,7 +79,22 @@ def lib() -> ctypes.CDLL:
 
 
 def host():
-    """Load (once) and return the native host path (``csrc/host.cpp``)."""
+    """The native host path (``csrc/host.cpp``)."""
+    return _load_host()
+
+
+def backward_mode(deterministic: bool, headdim: int, seqlen_q: int) -> int:
+    """The dQ strategy of a call: the rule that calls through the native autograd function follow."""
+    return _load_host().backward_mode(deterministic, headdim, seqlen_q)
+
+
+def allocate_workspace(allocate, batch: int, nheads: int, seqlen_q: int, headdim: int, mode: int):
+    """``(workspace or None, bytes, mode)`` by the steps of the native autograd function; mode -1: no memory.
+    ``allocate(bytes)`` gives a tensor, or None when it has no memory."""
+    return _load_host().allocate_workspace(allocate, batch, nheads, seqlen_q, headdim, mode)
+
+
+def _load_host():
     global _host
     if _host is None:
         lib()

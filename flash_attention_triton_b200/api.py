@@ -91,14 +91,6 @@ def _flash_attention_forward(
 #: dQ strategies of the C library (the ``deterministic`` argument of ``fa2_bwd``)
 _MODE_ATOMIC, _MODE_RECOMPUTE, _MODE_SPILL = 0, 1, 2
 _MODE_NAMES = {"atomic": _MODE_ATOMIC, "recompute": _MODE_RECOMPUTE, "spill": _MODE_SPILL}
-#: the spill mode keeps 32 KiB per tile pair of a head in scratch; when one head's tiles exceed
-#: this much (N above ~45 k) the recompute mode, which needs no scratch, takes over
-_SCRATCH_MAX_BYTES_PER_HEAD = 2 << 30
-
-
-def _scratch_bytes_per_head(seqlen_q: int, headdim: int) -> int:
-    tiles = (seqlen_q + 127) // 128
-    return tiles * (tiles + 1) // 2 * 32768 * (2 if headdim > 128 else 1)
 
 
 def _backward_mode(deterministic: bool, headdim: int, seqlen_q: int) -> int:
@@ -106,24 +98,20 @@ def _backward_mode(deterministic: bool, headdim: int, seqlen_q: int) -> int:
 
     ``True`` must give the same bits whatever the batch / head partitioning, so the choice
     depends on the head dim and the sequence length only.  Head dims above 64: the spill mode
-    (fastest there, 10-25 % ahead of the recompute mode) unless one head's scratch is too
-    large, then the recompute mode.  Head dims up to 64: the recompute mode, which is
-    4-14 % ahead of the spill mode there (the 32 KiB dS tile does not shrink with the head dim, the
-    tensor work does) and needs no scratch, like the reference's O(N) backward.
+    (fastest there, 10-25 % ahead of the recompute mode) unless one head's scratch (32 KiB per tile
+    pair) exceeds 2 GiB (N above ~45 k), then the recompute mode, which needs none.  Head dims up to
+    64: the recompute mode, which is 4-14 % ahead of the spill mode there (the 32 KiB dS tile does not
+    shrink with the head dim, the tensor work does) and needs no scratch, like the reference's O(N) backward.
     ``False`` (the reference's default, atomics there) means "fastest": the atomic kernel at
     head dims up to 64 (14-21 % ahead of the recompute mode from 4096 rows, the same at 2048), the
     deterministic choice above.  ``FA2_B200_BWD_MODE`` =
-    ``atomic`` / ``recompute`` / ``spill`` overrides both (for experiments).
+    ``atomic`` / ``recompute`` / ``spill`` overrides both (for experiments).  The rule itself is
+    ``backward_mode`` of ``csrc/host.cpp``, which calls that do not come here follow as well.
     """
-    if headdim > 128:  # one (deterministic) backward exists there: scores with dV + two consumers
-        return _MODE_SPILL
     forced = os.environ.get("FA2_B200_BWD_MODE")
-    if forced:
+    if forced and headdim <= 128:  # above, one (deterministic) backward exists: scores with dV + two consumers
         return _MODE_NAMES[forced]
-    if headdim <= 64:
-        return _MODE_RECOMPUTE if deterministic else _MODE_ATOMIC
-    scratch_ok = _scratch_bytes_per_head(seqlen_q, headdim) <= _SCRATCH_MAX_BYTES_PER_HEAD
-    return _MODE_SPILL if scratch_ok else _MODE_RECOMPUTE
+    return _lib.backward_mode(bool(deterministic), headdim, seqlen_q)
 
 
 def _allocate_workspace(lib, device, batch, nheads, seqlen_q, headdim, mode):
@@ -134,24 +122,21 @@ def _allocate_workspace(lib, device, batch, nheads, seqlen_q, headdim, mode):
     an eighth of it is tried (more chunks, a few per cent slower), then one head's worth, and
     when even that fails the recompute backward, which needs no scratch and gives the same dK,
     dV and a dQ that differs in the last bit at most, runs instead.  Head dims above 128 have no
-    scratch-free backward: there the out-of-memory error propagates.
+    scratch-free backward: there the out-of-memory error propagates.  The steps themselves are
+    ``allocate_workspace`` of ``csrc/host.cpp``, which calls that do not come here take as well; ``lib``
+    is not asked.
     """
-    want = lib.fa2_bwd_workspace_bytes(batch, nheads, seqlen_q, headdim, mode)
-    if not want:
-        return None, 0, mode
-    sizes = [want]
-    if mode == _MODE_SPILL:
-        one_head = _scratch_bytes_per_head(seqlen_q, headdim)
-        sizes += [n for n in (want // 8 // one_head * one_head, one_head) if one_head <= n < sizes[-1]]
-    for nbytes in sizes:
+
+    def allocate(nbytes):
         try:
-            return torch.empty(nbytes, device=device, dtype=torch.uint8), nbytes, mode
+            return torch.empty(nbytes, device=device, dtype=torch.uint8)
         except torch.cuda.OutOfMemoryError:
-            continue
-    if mode == _MODE_SPILL and headdim <= 128:
-        return None, 0, _MODE_RECOMPUTE
-    raise torch.cuda.OutOfMemoryError(
-        f"no memory for the backward workspace ({sizes[-1]} bytes at least)")
+            return None
+
+    workspace, nbytes, served = _lib.allocate_workspace(allocate, batch, nheads, seqlen_q, headdim, mode)
+    if served < 0:
+        raise torch.cuda.OutOfMemoryError(f"no memory for the backward workspace ({nbytes} bytes at least)")
+    return workspace, nbytes, served
 
 
 def _flash_attention_backward(

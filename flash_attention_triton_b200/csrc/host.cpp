@@ -24,6 +24,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 
 #include "../../include/fa2_b200.h"
 
@@ -235,34 +236,68 @@ long long scratch_bytes_per_head(long long n, int d) {
   return tiles * (tiles + 1) / 2 * 32768 * (d > 128 ? 2 : 1);
 }
 
-// _backward_mode of api.py, without its environment variable
+// Which dQ strategy serves a call (the rule, with its reasons: _backward_mode of api.py).
 int backward_mode(bool deterministic, int d, long long n) {
   if (d > 128) return kModeSpill;
   if (d <= 64) return deterministic ? kModeRecompute : kModeAtomic;
   return scratch_bytes_per_head(n, d) <= kScratchMaxBytesPerHead ? kModeSpill : kModeRecompute;
 }
 
-// _allocate_workspace of api.py: less scratch, or the mode that needs none, when memory is short
-at::Tensor allocate_workspace(const at::Tensor& q, int& mode) {
-  const int b = q.size(0), h = q.size(1), n = q.size(2), d = q.size(3);
+// The workspace of a backward mode, and the mode that will run: less scratch, or the mode that needs none, when memory is
+// short (_allocate_workspace of api.py).  `allocate` gives back an undefined tensor when it has no memory.  False: no
+// memory for the least the mode needs, `bytes`.
+template <typename Allocate>
+bool allocate_workspace(int b, int h, int n, int d, int& mode, long long& bytes, at::Tensor& workspace, Allocate&& allocate) {
   const long long want = static_cast<long long>(fa2_bwd_workspace_bytes(b, h, n, d, mode));
-  if (want == 0) return at::Tensor();
+  workspace = at::Tensor();
+  bytes = want;
+  if (want == 0) return true;
   const long long one_head = scratch_bytes_per_head(n, d);
   long long sizes[3] = {want, 0, 0};
   int count = 1;
   if (mode == kModeSpill)
-    for (const long long bytes : {want / 8 / one_head * one_head, one_head})
-      if (bytes >= one_head && bytes < sizes[count - 1]) sizes[count++] = bytes;
-  for (int i = 0;; ++i) {
-    try {
-      return at::empty({sizes[i]}, q.options().dtype(at::kByte).memory_format(at::MemoryFormat::Contiguous));
-    } catch (const c10::OutOfMemoryError&) {
-      if (i + 1 < count) continue;
-      if (mode != kModeSpill || d > 128) throw;
-      mode = kModeRecompute;
-      return at::Tensor();
-    }
+    for (const long long less : {want / 8 / one_head * one_head, one_head})
+      if (less >= one_head && less < sizes[count - 1]) sizes[count++] = less;
+  for (int i = 0; i < count; ++i) {
+    workspace = allocate(bytes = sizes[i]);
+    if (workspace.defined()) return true;
   }
+  if (mode != kModeSpill || d > 128) return false;
+  mode = kModeRecompute, bytes = 0;
+  return true;
+}
+
+// backward_mode(deterministic, head dim, rows) -> mode
+PyObject* py_backward_mode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 3) return PyErr_Format(PyExc_TypeError, "backward_mode takes 3 arguments");
+  const int deterministic = PyObject_IsTrue(args[0]);
+  const long d = PyLong_AsLong(args[1]);
+  const long long n = PyLong_AsLongLong(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  return PyLong_FromLong(backward_mode(deterministic != 0, static_cast<int>(d), n));
+  END_HANDLE_TH_ERRORS
+}
+
+// allocate_workspace(allocate, batch, heads, rows, head dim, mode) -> (workspace or None, bytes, mode), mode -1: no memory.
+// allocate(bytes) gives a tensor, or None when it has no memory.
+PyObject* py_allocate_workspace(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 6) return PyErr_Format(PyExc_TypeError, "allocate_workspace takes 6 arguments");
+  long v[5];
+  for (int i = 0; i < 5; ++i) v[i] = PyLong_AsLong(args[i + 1]);
+  if (PyErr_Occurred()) return nullptr;
+  int mode = static_cast<int>(v[4]);
+  long long bytes = 0;
+  at::Tensor workspace;
+  const bool ok = allocate_workspace(v[0], v[1], v[2], v[3], mode, bytes, workspace, [&](long long size) {
+    const auto given = pybind11::reinterpret_steal<pybind11::object>(PyObject_CallFunction(args[0], "L", size));
+    if (!given) throw python_error();
+    TORCH_CHECK_TYPE(given.is_none() || THPVariable_Check(given.ptr()), "allocate must give a tensor or None");
+    return given.is_none() ? at::Tensor() : THPVariable_Unpack(given.ptr());
+  });
+  return Py_BuildValue("NLi", THPVariable_Wrap(workspace), bytes, ok ? mode : -1);
+  END_HANDLE_TH_ERRORS
 }
 
 // Saved-tensor hooks must give back what was saved.  False for what _flash_attention_backward of api.py asserts.
@@ -324,7 +359,19 @@ struct Attention : torch::autograd::Function<Attention> {
       at::Tensor rowstats;
       check_code("fa2_bwd_preprocess_strided", run_preprocess(output, d_output, lse, rowstats));
       int mode = backward_mode(deterministic, q.size(3), q.size(2));
-      const at::Tensor workspace = allocate_workspace(q, mode);
+      at::Tensor workspace;
+      long long bytes = 0;
+      std::exception_ptr no_memory;
+      const auto allocate = [&](long long size) {
+        try {
+          return at::empty({size}, q.options().dtype(at::kByte).memory_format(at::MemoryFormat::Contiguous));
+        } catch (const c10::OutOfMemoryError&) {
+          no_memory = std::current_exception();
+          return at::Tensor();
+        }
+      };
+      if (!allocate_workspace(q.size(0), q.size(1), q.size(2), q.size(3), mode, bytes, workspace, allocate))
+        std::rethrow_exception(no_memory);
       at::Tensor t[7] = {q, k, v, d_output, dq, dk, dv};
       check_code("fa2_bwd_strided", run_backward(t, rowstats, workspace, scale, mode));
     }
@@ -401,6 +448,8 @@ PyMethodDef kMethods[] = {
     {"preprocess", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(preprocess)), METH_FASTCALL, nullptr},
     {"gradients", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(gradients)), METH_FASTCALL, nullptr},
     {"backward", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(backward)), METH_FASTCALL, nullptr},
+    {"backward_mode", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_backward_mode)), METH_FASTCALL, nullptr},
+    {"allocate_workspace", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_allocate_workspace)), METH_FASTCALL, nullptr},
     {"readable_in_place", is_readable_in_place, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

@@ -1123,3 +1123,42 @@ def test_native_backward_refuses_saved_tensors_that_changed(index, change, error
     with pytest.raises(error):
         torch.autograd.grad(out, q, do)
     assert len(unpacked) == 5
+
+
+def test_native_backward_when_memory_is_short():
+    """The process may take less and less: an eighth of the recommended scratch, one head's, none (the recompute mode); head
+    dims above 128, which need one head's, raise.  The same dK and dV bits in all of them."""
+    total = torch.cuda.get_device_properties(0).total_memory
+    g = torch.Generator(device=DEV).manual_seed(5)
+
+    def passes(d, heads, limits):
+        q, k, v, do = (torch.randn(1, heads, 8192, d, device=DEV, generator=g, dtype=torch.float16) for _ in range(4))
+        for t in (q, k, v):
+            t.requires_grad_(True)
+        results = []
+        for limit in limits:
+            torch.cuda.empty_cache()  # before and after, so that nothing free is left inside what is held
+            out = flash_attention_v2(q, k, v, None, True)
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+            torch.cuda.reset_peak_memory_stats()
+            held = torch.cuda.memory_reserved()
+            if limit is not None:
+                torch.cuda.set_per_process_memory_fraction((held + limit) / total)
+            try:
+                grads = torch.autograd.grad(out, (q, k, v), do)
+            finally:
+                torch.cuda.set_per_process_memory_fraction(1.0)
+            results.append((grads, torch.cuda.max_memory_reserved() - held))
+        return results
+
+    head, grads = 2080 * 32768, 3 * 8 * 8192 * 128 * 2
+    (want, most), *others = passes(128, 8, [None, 2 * head + grads + (64 << 20), grads + (32 << 20)])
+    assert most >= 8 * head
+    for ((dq, dk, dv), used), heads_of_scratch in zip(others, (1, 0)):
+        assert heads_of_scratch * head <= used - grads < (heads_of_scratch + 1) * head
+        assert torch.equal(dk, want[1]) and torch.equal(dv, want[2])
+        assert (dq.float() - want[0].float()).abs().max() <= 2 ** -7  # an ulp below 16
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        passes(256, 2, [64 << 20])
+    assert _lib.device_status() == 0

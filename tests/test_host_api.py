@@ -224,3 +224,35 @@ def test_native_call_leaves_what_it_does_not_serve_to_the_general_path():
         assert attention(*args) is None
     with pytest.raises(TypeError):
         attention(t, t, t)
+
+
+def test_one_rule_and_one_ladder_for_native_and_python_calls(monkeypatch):
+    """api.py asks the native module, so the tests of its functions test what plain calls do; sizes where the rule changes."""
+    from flash_attention_triton_b200 import _lib, api
+
+    monkeypatch.delenv("FA2_B200_BWD_MODE", raising=False)
+    host = _lib.host()
+    for n in (1, 128, 8192, 46208, 46209, 65536):  # 361 tiles: 65 341 pairs of 32 KiB, below 2 GiB; 362: above
+        for d in (8, 64, 72, 128, 136, 256):
+            for det in (False, True):
+                spill = d > 128 or (d > 64 and n <= 46208)
+                want = api._MODE_SPILL if spill else api._MODE_RECOMPUTE if det or d > 64 else api._MODE_ATOMIC
+                assert host.backward_mode(det, d, n) == want == api._backward_mode(det, d, n)
+    head = 2080 * 32768
+
+    def ladder(limit, d, mode):
+        asked = []
+        take = lambda size: asked.append(size) or (torch.zeros(1) if size <= limit else None)
+        return *host.allocate_workspace(take, 2, 32, 8192, d, mode)[1:], asked
+
+    assert ladder(1 << 62, 128, 2) == (32 * head, 2, [32 * head])
+    assert ladder(4 * head, 128, 2) == (4 * head, 2, [32 * head, 4 * head])
+    assert ladder(head, 128, 2) == (head, 2, [32 * head, 4 * head, head])
+    assert ladder(0, 128, 2) == (0, 1, [32 * head, 4 * head, head])
+    assert ladder(0, 128, 1) == (0, 1, [])
+    assert ladder(0, 64, 0)[1] == -1 and len(ladder(0, 64, 0)[2]) == 1  # the accumulator of the atomic mode is a need
+    assert ladder(0, 256, 2)[1] == -1
+    with pytest.raises(ZeroDivisionError):
+        host.allocate_workspace(lambda size: 1 / 0, 2, 32, 8192, 128, 2)
+    with pytest.raises(TypeError):
+        host.allocate_workspace(lambda size: 3, 2, 32, 8192, 128, 2)
