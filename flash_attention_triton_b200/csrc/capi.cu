@@ -172,11 +172,8 @@ int check_shape(int B, int H, int N, int D, int dtype) {
   return FA2_OK;
 }
 
-// Scratch of the spilling backward modes: one 32 KiB dS tile per (KV tile, Q tile) pair of a head.  Callers are
-// asked for twice that for head dims above 128, which kept a P tile too once; it goes into larger chunks there.
-long long spill_bytes_per_head(int N, int Nk, int D) {
-  return dstile_pairs(N, Nk) * 32768 * (D > 128 ? 2 : 1);
-}
+// Scratch of the spilling backward modes: one 32 KiB dS tile per (KV tile, Q tile) pair of a head.
+long long spill_bytes_per_head(int N, int Nk) { return dstile_pairs(N, Nk) * 32768; }
 // What fa2_bwd_workspace_bytes recommends at most (fa2_set_spill_budget); a workspace of any size
 // that holds one head is accepted by fa2_bwd.
 std::atomic<long long> g_spill_budget{8ll << 30};
@@ -330,9 +327,12 @@ size_t fa2_bwd_workspace_bytes(int B, int H, int N, int D, int deterministic) {
     // 16-bit [128 x 128] tiles of whole heads: as many heads as make a chunk of
     // kSpillChunkTiles tiles, within the budget, never less than one head; then what the chunk
     // plan uses of that
-    const long long per_head = spill_bytes_per_head(N, N, D);
+    const long long per_head = spill_bytes_per_head(N, N);
     const long long ntiles = (static_cast<long long>(N) + 127) / 128;
-    const long long want = (kSpillChunkTiles + ntiles - 1) / ntiles * per_head;
+    // Head dims above 128 gain from chunks twice as large, bf16 backward, us with 4096 / 2048 / 1024 tiles:
+    // [16,32,2048,256] 3 536 / 3 690 / 3 846, [1,32,16384,256] 10 440 / 10 830 / 10 810, [4,16,8192,192] 4 500 / 4 580 / 4 730.
+    const long long chunk_tiles = D > 128 ? 2 * kSpillChunkTiles : kSpillChunkTiles;
+    const long long want = (chunk_tiles + ntiles - 1) / ntiles * per_head;
     const SpillPlan plan =
         spill_plan(B, H, per_head, std::max(per_head, std::min(want, g_spill_budget.load())));
     return static_cast<size_t>(plan.nb) * plan.nh * static_cast<size_t>(per_head);
@@ -369,7 +369,7 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
   // The workspace must hold what the mode needs at least; what lies beyond is used when it
   // helps (more scratch slots, larger chunks) and never written otherwise.
   const long long BH = static_cast<long long>(B) * H;
-  const long long per_head = spill_bytes_per_head(N, Nk, D);
+  const long long per_head = spill_bytes_per_head(N, Nk);
   const long long ws = static_cast<long long>(std::min<size_t>(workspace_bytes, size_t(1) << 62));
   if (deterministic == 0 && workspace_bytes < fa2_bwd_workspace_bytes(B, H, N, D, 0))
     return FA2_ERR_WORKSPACE;
@@ -386,7 +386,7 @@ static int bwd_strided(const void* q, const void* k, const void* v, const void* 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
   if (deterministic == 2) {
-    const SpillPlan plan = spill_plan(B, H, dstile_pairs(N, Nk) * 32768, ws);
+    const SpillPlan plan = spill_plan(B, H, per_head, ws);
     if (plan.nb < B || plan.nh < H) {
       // more than one chunk: the same call on sub-ranges, one after the other on the stream
       // (they share the scratch), with the caller's strides spelled out

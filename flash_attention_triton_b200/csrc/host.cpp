@@ -231,16 +231,16 @@ void check_code(const char* fn, int code) {
 constexpr int kModeAtomic = 0, kModeRecompute = 1, kModeSpill = 2;
 constexpr long long kScratchMaxBytesPerHead = 2ll << 30;
 
-long long scratch_bytes_per_head(long long n, int d) {
+long long scratch_bytes_per_head(long long n) {
   const long long tiles = (n + 127) / 128;
-  return tiles * (tiles + 1) / 2 * 32768 * (d > 128 ? 2 : 1);
+  return tiles * (tiles + 1) / 2 * 32768;
 }
 
 // Which dQ strategy serves a call (the rule, with its reasons: _backward_mode of api.py).
 int backward_mode(bool deterministic, int d, long long n) {
   if (d > 128) return kModeSpill;
   if (d <= 64) return deterministic ? kModeRecompute : kModeAtomic;
-  return scratch_bytes_per_head(n, d) <= kScratchMaxBytesPerHead ? kModeSpill : kModeRecompute;
+  return scratch_bytes_per_head(n) <= kScratchMaxBytesPerHead ? kModeSpill : kModeRecompute;
 }
 
 // The workspace of a backward mode, and the mode that will run: less scratch, or the mode that needs none, when memory is
@@ -252,7 +252,7 @@ bool allocate_workspace(int b, int h, int n, int d, int& mode, long long& bytes,
   workspace = at::Tensor();
   bytes = want;
   if (want == 0) return true;
-  const long long one_head = scratch_bytes_per_head(n, d);
+  const long long one_head = scratch_bytes_per_head(n);
   long long sizes[3] = {want, 0, 0};
   int count = 1;
   if (mode == kModeSpill)

@@ -112,8 +112,8 @@ size_t fa2_rowstats_bytes(int B, int H, int N);
  *     single chunk (1024 tiles: 3 % slower, 512: 11 %, one head of 64 tiles: 3.9x), the minimum
  *     is one head's tiles, and the split never changes a bit of the results.  dQ differs from mode 1 in the last bit at
  *     most (other polynomial / MUFU assignment of the exponentials).  It is the only backward
- *     for head dims above 128, where it is a scores kernel plus dV, dK and dQ kernels over two
- *     scratch tensors (64 KiB per tile pair) and serves every value of `deterministic`.  No
+ *     for head dims above 128, where it is a scores kernel that keeps dV plus dK and dQ kernels over
+ *     the same scratch (32 KiB per tile pair) and serves every value of `deterministic`.  No
  *     counterpart in the reference.
  *   deterministic == 0 ("atomic"): one fused kernel per KV tile adds its dQ contributions into
  *     the fp32 workspace with atomic adds (the reference's SEQUENCE_PARALLEL mode,
@@ -132,7 +132,7 @@ int fa2_bwd(const void* q, const void* k, const void* v, const void* dout,
  * Bytes of workspace fa2_bwd should be given for a value of `deterministic` (see there): the
  * exact size for modes 0 and 1 (0 bytes), the recommended size for mode 2: the tiles of as
  * many heads as make a chunk of 2048 128-row tiles (32 heads at N = 8192: 2.2 GB; about 256 KiB
- * per row of a head, so linear in N and independent of B * H), capped by fa2_set_spill_budget,
+ * per row of a head, so linear in N and independent of B * H), 4096 above head dim 128, capped by fa2_set_spill_budget,
  * never less than one head.
  */
 size_t fa2_bwd_workspace_bytes(int B, int H, int N, int D, int deterministic);

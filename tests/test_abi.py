@@ -163,7 +163,7 @@ def test_spill_scratch_size_follows_the_budget():
         assert lib.fa2_bwd_workspace_bytes(2, 32, 32768, 128, 2) == 8 * pairs4 * 32768
         lib.fa2_set_spill_budget(20 * pairs * 32768)      # 20 heads fit: two chunks of 16
         assert lib.fa2_bwd_workspace_bytes(2, 32, 8192, 128, 2) == 16 * pairs * 32768
-        assert lib.fa2_bwd_workspace_bytes(2, 16, 8192, 256, 0) == 8 * 2 * pairs * 32768  # 64 KiB per pair: 10 heads fit, two chunks of 8
+        assert lib.fa2_bwd_workspace_bytes(2, 16, 8192, 256, 0) == 8 * 2 * pairs * 32768  # 20 heads fit: one batch entry of 16
         lib.fa2_set_spill_budget(1)                       # never below one head
         assert lib.fa2_bwd_workspace_bytes(2, 32, 8192, 128, 2) == pairs * 32768
         assert lib.fa2_set_spill_budget(previous) == 1
@@ -237,3 +237,21 @@ def test_static_scratch_refuses_bad_arguments_before_launching():
     assert lib.fa2_bwd_static_scratch(*p, 1, 2, 256, 64, 1, float("nan"), None) == -9
     assert lib.fa2_bwd_static_scratch(*([0x1000] * 6 + [0x1008] + [0x1000] * 2), 1, 2, 256, 64, 1, 0.1, None) == -4
     assert lib.fa2_bwd_static_scratch(*p, 1, 65, 8192, 128, 1, 0.1, None) == -11
+
+
+def test_head_dims_above_128_ask_for_one_tile_per_pair():
+    """dS alone is kept: 32 KiB a pair for the minimum, the recommendation (chunks of 4096 tiles) and the ladder of the API."""
+    lib = _lib.lib()
+    pairs = 64 * 65 // 2
+    previous = lib.fa2_set_spill_budget(1 << 40)
+    try:
+        assert lib.fa2_bwd_workspace_bytes(2, 16, 8192, 256, 0) == 32 * pairs * 32768  # all there is
+        assert lib.fa2_bwd_workspace_bytes(8, 16, 8192, 136, 2) == 64 * pairs * 32768
+        lib.fa2_set_spill_budget(1)
+        assert lib.fa2_bwd_workspace_bytes(2, 16, 8192, 256, 2) == pairs * 32768
+    finally:
+        lib.fa2_set_spill_budget(previous)
+    asked = []
+    _lib.allocate_workspace(asked.append, 2, 16, 8192, 256, 2)
+    assert asked == [32 * pairs * 32768, 4 * pairs * 32768, pairs * 32768]
+    assert lib.fa2_bwd(*([0x1000] * 8), 0x10000, pairs * 32768 - 1, 1, 1, 8192, 256, 1, 0.1, 2, None) == -10

@@ -347,8 +347,8 @@ def test_spill_mode_chunks_change_no_bit(monkeypatch):
 @pytest.mark.parametrize("d", [64, 256])
 def test_spill_chunks_with_strided_tensors(d, monkeypatch):
     """The chunks of the spill mode are sub-ranges of the caller's tensors addressed through the
-    caller's strides: [B, N, H, D] storage, fewer keys than queries, head dim 64 (one scratch) and
-    256 (two scratches), chunked by a small budget; same bits as in one piece, parity with the oracle."""
+    caller's strides: [B, N, H, D] storage, fewer keys than queries, head dims 64 and
+    256, chunked by a small budget; same bits as in one piece, parity with the oracle."""
     monkeypatch.setenv("FA2_B200_BWD_MODE", "spill")
     g = torch.Generator().manual_seed(11)
     q, do = (torch.randn(3, 500, 4, d, generator=g).to(torch.bfloat16).transpose(1, 2) for _ in range(2))
@@ -359,7 +359,7 @@ def test_spill_chunks_with_strided_tensors(d, monkeypatch):
     try:
         whole = run_api(q, k, v, do, None, True)
         check_against(ref, whole, torch.bfloat16)
-        per_head = 10 * 32768 * (2 if d > 128 else 1)  # T = 4 Q tiles: 10 pairs
+        per_head = 10 * 32768  # T = 4 Q tiles: 10 pairs
         for budget in (3 * per_head, 9 * per_head):     # 2 + 2 heads per batch entry; 2 + 1 batch entries
             lib.fa2_set_spill_budget(budget)
             chunked = run_api(q, k, v, do, None, True)
@@ -1161,4 +1161,29 @@ def test_native_backward_when_memory_is_short():
         assert (dq.float() - want[0].float()).abs().max() <= 2 ** -7  # an ulp below 16
     with pytest.raises(torch.cuda.OutOfMemoryError):
         passes(256, 2, [64 << 20])
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("d", [136, 256])
+@pytest.mark.parametrize("nq,nk", [(300, 300), (1100, 640)])
+def test_wide_heads_in_a_workspace_of_one_head(d, nq, nk):
+    """32 KiB for every pair of tiles of one head, and not a byte more written; the bits of one chunk."""
+    host = _lib.host()
+    q, do = (torch.randn(2, 3, nq, d, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(2, 3, nk, d, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    code, output, lse, _ = host.forward(q, k, v, 0.07, False)
+    assert code == 0
+    rowstats = host.preprocess(output, do, lse)[1]
+    tiles, key_tiles = (nq + 127) // 128, (nk + 127) // 128
+    head = (key_tiles * tiles - key_tiles * (key_tiles - 1) // 2) * 32768
+    results = []
+    for heads in (1, 2, 6):
+        grads = host.gradients(q, k, v, False)
+        room = torch.full((heads * head + 4096,), 0x5A, device=DEV, dtype=torch.uint8)
+        assert host.backward(q, k, v, do, *grads, rowstats, room[: heads * head], 0.07, 2) == 0
+        assert (room[heads * head:] == 0x5A).all()
+        results.append(grads)
+    assert host.backward(q, k, v, do, *grads, rowstats, room[: head - 1], 0.07, 2) == -10
+    for grads in results[1:]:
+        assert all(torch.equal(x, y) for x, y in zip(grads, results[0]))
     assert _lib.device_status() == 0
