@@ -100,7 +100,6 @@ constexpr uint32_t make_idesc(int, int, bool, bool, bool) { return 0; }
 inline uint32_t smem_u32(const void* p) { return uint32_t(static_cast<const uint8_t*>(p) - sim_smem); }
 inline uint32_t elect_one() { return 1; }
 inline void mbar_init(uint32_t bar, uint32_t count) { sim_init(bar, count); }
-inline void mbar_inval(uint32_t) {}
 inline void mbar_arrive(uint32_t bar) { sim_arrive(bar); }
 inline void mbar_arrive_expect_tx(uint32_t bar, uint32_t) { sim_access(), sim_arrive_later(bar); }
 inline void mma_commit(uint32_t bar) { sim_arrive_after_mma(bar); }

@@ -1187,3 +1187,37 @@ def test_wide_heads_in_a_workspace_of_one_head(d, nq, nk):
     for grads in results[1:]:
         assert all(torch.equal(x, y) for x, y in zip(grads, results[0]))
     assert _lib.device_status() == 0
+
+
+def _subclass(t):
+    class Tagged(torch.Tensor):
+        pass
+
+    return t.as_subclass(Tagged)
+
+
+@pytest.mark.parametrize("change", [
+    dict(q=lambda t: t[0]), dict(k=lambda t: t.cpu()), dict(v=lambda t: t.bfloat16()), dict(q=lambda t: t.double()),
+    dict(all=lambda t: t.double()), dict(all=lambda t: t.to(torch.int32)), dict(k=lambda t: t[:, :, :-1]), dict(v=lambda t: t[:, :, :-1]),
+    dict(q=lambda t: t[:, :, :-1]), dict(q=lambda t: t[:1]), dict(q=lambda t: t[:, :1]), dict(all=lambda t: t[..., :20]),
+    dict(all=lambda t: torch.cat([t] * 9, -1)[..., :264]), dict(q=lambda t: t[..., :16]), dict(all=lambda t: t[:0]),
+    dict(all=_subclass), dict(k=_subclass), dict(v=lambda t: torch._neg_view(t)), dict(all=lambda t: t.to_sparse()),
+    dict(k=lambda t: torch.autograd.forward_ad.make_dual(t, t)), dict(scale="x"), dict(scale=1), dict(scale=torch.tensor(0.1)),
+    dict(env=("FA2_B200_CHECK_STATUS", "1")), dict(env=("FA2_B200_BWD_MODE", "spill")),
+    dict(mode=lambda: torch.device("cpu")), dict(mode=lambda: torch.utils._python_dispatch.TorchDispatchMode())])
+def test_native_call_serves_plain_tensors_only(change, monkeypatch):
+    """One property of a served call at a time: the native function leaves the call to the general path (None)."""
+    import contextlib
+
+    attention = _lib.host().attention
+    t = torch.randn(2, 3, 40, 32, device=DEV, dtype=torch.float16)
+    for served in (t, torch.nn.Parameter(t), t.transpose(1, 2).contiguous().transpose(1, 2), t.bfloat16(), t.float()):
+        assert attention(served, served, served, None, False) is not None
+    assert attention(t, t[:, :, :7], t[:, :, :7], 0.1, 1) is not None
+    if "env" in change:
+        monkeypatch.setenv(*change["env"])
+    with torch.autograd.forward_ad.dual_level():
+        args = [change.get(name, change.get("all", lambda x: x))(t) for name in "qkv"]
+        with change.get("mode", contextlib.nullcontext)():
+            assert attention(*args, change.get("scale"), False) is None
+    assert _lib.device_status() == 0

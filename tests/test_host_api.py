@@ -214,14 +214,14 @@ def test_host_module_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
         assert len(runs) == expected
 
 
-def test_native_call_leaves_what_it_does_not_serve_to_the_general_path():
+def test_native_call_leaves_cpu_tensors_to_the_general_path():
+    """What it refuses of CUDA tensors: test_native_call_serves_plain_tensors_only in test_gpu_parity.py."""
     from flash_attention_triton_b200 import _lib
 
     attention = _lib.host().attention
     t = torch.zeros(1, 2, 8, 16, dtype=torch.float16)
-    assert attention(t, t, t, None, False) is None  # not on a GPU
-    for args in ((t[0], t, t, None, False), (t, t, 3, None, False), (t, t, t, "x", False), (t, t.double(), t, None, False)):
-        assert attention(*args) is None
+    assert attention(t, t, t, None, False) is None
+    assert attention(t, t, 3, None, False) is None
     with pytest.raises(TypeError):
         attention(t, t, t)
 
