@@ -38,9 +38,6 @@ struct WaitCtx {
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_inval(uint32_t bar) {
-  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -181,25 +178,6 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, int x, int 
       "r"(x), "r"(y), "r"(hc.h), "r"(hc.b), "r"(src_smem)
       : "memory");
 }
-// 3-D variants for the library's own dense scratch tensors: {x, y, tile index}.
-__device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap* map, int x,
-                                            int y, int z, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst_smem),
-      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int y, int z,
-                                             uint32_t src_smem) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
-          map),
-      "r"(x), "r"(y), "r"(z), "r"(src_smem)
-      : "memory");
-}
-// All bulk stores of this thread have finished READING shared memory (the data may still be
-// in flight to global memory): the source buffer can be rewritten.
 // Untiled bulk copy global -> shared: both addresses 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst_smem, const void* src, uint32_t bytes,
                                              uint32_t bar) {
@@ -209,6 +187,8 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst_smem, const void* src,
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
+// All bulk stores of this thread have finished READING shared memory (the data may still be
+// in flight to global memory): the source buffer can be rewritten.
 __device__ __forceinline__ void tma_store_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
