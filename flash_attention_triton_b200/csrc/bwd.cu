@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(DqCfg<D, W>::kThreads, DqCfg<D, W>::kCtasPerSm
 }
 
 // =========================================================================================
-// One output tile per CTA from spilled 16-bit tiles (head dim 256: dV, dK and dQ; see
+// One output tile per CTA from spilled 16-bit tiles (head dim 256: dK and dQ; see
 // consume_roles).  warps 0-3 epilogue, warp 4 producer, warp 5 MMA issue.
 // =========================================================================================
 // Up to head dim 128 two CTAs run on an SM (rings of three 32 KiB stages at head dim 128).  With one,
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(ConsumeCfg<D>::kThreads, ConsumeCfg<D>::kCtasP
 // half operand tiles (64 reduction rows, 32 KiB each).  Every output tile adds the same products in the
 // same order as above, so the two kernels give the same bits.
 // warps 0-3 and 4-7 epilogue of the first and the second tile, warp 8 producer, warp 9 MMA issue.
-// Measured on the whole backward of [2,16,8192,256] bf16: 3517 -> 3015 us.
+// Measured on the whole backward, bf16, one tile a CTA -> two: [1,32,8192,256] 2690 -> 2542 us, [1,32,8192,192] 2394 -> 2179.
 // =========================================================================================
 struct ConsumePairCfg {
   using T = Tile<256>;
@@ -691,8 +691,9 @@ __global__ void __launch_bounds__(ConsumePairCfg::kThreads, 1)
 //   warp  8    MMA issue, per step:  [Pt(i) ready]  dV += Pt(i) dO(i),  St(i+1) = K Q^T (over Pt(i)),
 //              [dPt(i) copied]  dPt(i+1) = V dO^T.  dPt(i+1) runs under the exponentials of St(i+1).
 //   warp  9    TMA producer
-// Bound by the power limit at long sequences (1.25 GHz under load, 4 500 cycles a pair against 3 072 of tensor and
-// 3 584 of shared-memory time; without the ring's loads 6 % less, without the dS stores 12 %).  The version before
+// Bound by the chain of a step: ncu ([1,16,8192,256] bf16) has the tensor pipe at 66 % of the active cycles (4 660 a pair, 3 072 of
+// them tensor, 3 584 shared-memory time), L1 at 55 %, DRAM at 24 %; without the ring's loads 6 % less, without the dS stores
+// 12 %.  In a loop of long sequences the power limit takes the clock from 1.5 to 1.25 GHz besides.  The version before
 // wrote P^T to a second scratch tensor too, from which a third consumer formed dV: 4.4 of 10.9 GB on
 // [2,16,8192,256] bf16, forward and backward 4 148 -> 3 690 us in a loop.  Same bits.  Walking the Q tiles
 // from the last one, as bwd_dkdv_kernel does, measured the same.

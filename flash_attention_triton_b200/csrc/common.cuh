@@ -224,10 +224,10 @@ cudaError_t launch_bwd_consume(const AttnShape& s, int form, const void* scratch
                                const RowStats& rowstats, bool two_tiles, int* status, cudaStream_t stream);
 
 // Whether the consumers of head dim 256 take two output tiles per CTA: when that still gives every SM a CTA.
-// Below, fewer and longer CTAs leave SMs idle.  Whole bf16 backward, microseconds, one tile against two:
-//     1024 rows: 128 pairs of tiles 111 / 111, 160: 153 / 139, 192: 164 / 158, 256: 200 / 184, 512: 367 / 342
-//     2048 rows: 128 pairs 148 / 160, 160: 227 / 207, 208: 242 / 225, 256: 276 / 252, 320: 352 / 348
-//     8192 rows: 128 pairs 406 / 481, 160: 680 / 616, 192: 680 / 629, 256: 827 / 749, 320: 1133 / 1137
+// Below, fewer and longer CTAs leave SMs idle.  Whole bf16 backward, microseconds, one tile against two, head dim 256 and 192:
+//     1024 rows: 128 pairs of tiles 85 / 88 and 87 / 90, 160: 118 / 109 and 123 / 113, 256: 160 / 151 and 170 / 157, 512: 292 / 275 and 288 / 274
+//     2048 rows: 128 pairs 116 / 127 and 108 / 125, 160: 185 / 172 and 167 / 162, 256: 233 / 214 and 197 / 183, 320: 304 / 309 and 252 / 249
+//     8192 rows: 128 pairs 350 / 414 and 298 / 337, 160: 595 / 578 and 527 / 479, 256: 661 / 620 and 553 / 518, 512: 1352 / 1253 and 1190 / 1072
 inline bool consume_two_tiles(const AttnShape& s, int num_sms) {
   const long long tiles = (s.Nk + 127) / 128;
   return s.D == 256 && (tiles + 1) / 2 * s.B * s.H > num_sms;
